@@ -1,5 +1,6 @@
 // extern "C" entry points declared in include/systemds_cla.h.
 #include "cla_common.cuh"
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -145,6 +146,12 @@ int64_t cla_stats_get(cla_handle h, cla_stats* out) {
   if (!out) return fail(CLA_ERR_BAD_ARG, "null stats pointer");
   if (m->device >= 0) cudaSetDevice(m->device);
   prof_collect(m);
+  if (m->elapsedPending) {  // device time of the last host-buffer call
+    float ms = 0;
+    if (cudaEventSynchronize(m->ev1) == cudaSuccess && cudaEventElapsedTime(&ms, m->ev0, m->ev1) == cudaSuccess)
+      m->stats.last_kernel_ms = ms;
+    m->elapsedPending = false;
+  }
   if (m->finalized) {  // device-buffer calls do not synchronise: this is where their kernels' self-checks surface
     int64_t rc = check_errword(m);
     if (rc < 0) return rc;
@@ -439,10 +446,24 @@ static int64_t rmm_by_vectors(Matrix* m, const double* dV, int32_t vCols, double
   return CLA_OK;
 }
 
-static int64_t rmm_dev(Matrix* m, const double* dV, int32_t vRows, int32_t vCols, double* dOut, cudaStream_t s) {
+// A host-buffer call whose operands and result are small: the product's last kernel may finish the call itself (write
+// the result to the mailbox and raise its flag); otherwise host_call does that with one more kernel.
+struct HostCall {
+  Finish fin;
+  const double* in1 = nullptr;  // the first operand in host memory, where the product may read it there
+  bool used = false;
+};
+
+static int64_t rmm_dev(Matrix* m, const double* dV, int32_t vRows, int32_t vCols, double* dOut, cudaStream_t s,
+                       HostCall* hc = nullptr) {
   if (vRows != m->nCols) return fail(CLA_ERR_SHAPE, "rmm: V must have nCols rows");
   if (vCols < 0) return fail(CLA_ERR_SHAPE, "rmm: negative column count");
   m->stats.calls_rmm++;
+  if (small_block(m)) {
+    const int64_t rc = small_rmm(m, dV, vCols, dOut, nullptr, s, hc ? hc->fin : Finish(), hc ? hc->in1 : nullptr);
+    if (hc) hc->used = rc == 1;
+    if (rc != 0) return rc < 0 ? rc : CLA_OK;
+  }
   if (vCols == 1) {
     int64_t rc = fast_rmm_vec(m, dV, dOut, s);
     if (rc < 0) return rc;
@@ -459,9 +480,14 @@ static int64_t rmm_dev(Matrix* m, const double* dV, int32_t vRows, int32_t vCols
   return launch_rmm_dmma(m, dV, vCols, dOut, s);  // FP64 tensor cores
 }
 
-static int64_t lmm_dev(Matrix* m, const double* dYt, int32_t yRows, double* dOut, cudaStream_t s) {
+static int64_t lmm_dev(Matrix* m, const double* dYt, int32_t yRows, double* dOut, cudaStream_t s, HostCall* hc = nullptr) {
   if (yRows < 0) return fail(CLA_ERR_SHAPE, "lmm: negative row count");
   m->stats.calls_lmm++;
+  if (small_block(m)) {
+    const int64_t rc = small_lmm(m, dYt, yRows, dOut, s, hc ? hc->fin : Finish());
+    if (hc) hc->used = rc == 1;
+    if (rc != 0) return rc < 0 ? rc : CLA_OK;
+  }
   if (yRows == 1) {
     int64_t rc = fast_lmm_vec(m, dYt, dOut, s);
     if (rc < 0) return rc;
@@ -499,7 +525,7 @@ static int64_t lmm_dev(Matrix* m, const double* dYt, int32_t yRows, double* dOut
 }
 
 static int64_t mmchain_dev(Matrix* m, const double* dV, const double* dW, int32_t ctype, double* dOut, double* dU,
-                           cudaStream_t s) {
+                           cudaStream_t s, HostCall* hc = nullptr) {
   if (ctype != CLA_CHAIN_XtXv && ctype != CLA_CHAIN_XtwXv) return fail(CLA_ERR_UNSUPPORTED, "mmchain: unsupported chain type");
   if (ctype == CLA_CHAIN_XtwXv && !dW) return fail(CLA_ERR_BAD_ARG, "mmchain: XtwXv needs w");
   m->stats.calls_mmchain++;
@@ -508,11 +534,18 @@ static int64_t mmchain_dev(Matrix* m, const double* dV, const double* dW, int32_
     if (rc < 0) return rc;
     dU = (double*)m->scratch2;
   }
-  int64_t rc = rmm_dev(m, dV, m->nCols, 1, dU, s);
-  if (rc < 0) return rc;
-  if (ctype == CLA_CHAIN_XtwXv)
-    if ((rc = launch_scale_rows(m, dU, dW, m->nRows, s)) < 0) return rc;
-  return lmm_dev(m, dU, 1, dOut, s);
+  int64_t rc = 0;
+  if (small_block(m)) {  // the weights are applied where the row sums are written
+    rc = small_rmm(m, dV, 1, dU, ctype == CLA_CHAIN_XtwXv ? dW : nullptr, s, Finish());
+    if (rc < 0) return rc;
+  }
+  if (rc == 0) {
+    if ((rc = rmm_dev(m, dV, m->nCols, 1, dU, s)) < 0) return rc;
+    if (ctype == CLA_CHAIN_XtwXv)
+      if ((rc = launch_scale_rows(m, dU, dW, m->nRows, s)) < 0) return rc;
+  } else
+    m->stats.calls_rmm++;
+  return lmm_dev(m, dU, 1, dOut, s, hc);
 }
 
 // Device-buffer calls return once their work is enqueued. All calls on a handle share its scratch buffers, so
@@ -578,13 +611,94 @@ int64_t cla_mmchain_dev(cla_handle h, const double* dV, const double* dW, int32_
 }  // extern "C"
 
 // ---- host-buffer products -------------------------------------------------------------------------
+static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+// Waits for the mailbox flag of call `seq`: polled for as long as a small product takes, then the stream is waited for.
+static int64_t mail_wait(Matrix* m, uint32_t seq) {
+  Mailbox* box = (Mailbox*)m->mail;
+  for (int i = 0; i < 200000; i++) {
+    if (box->flag == seq) {
+      std::atomic_thread_fence(std::memory_order_acquire);
+      return CLA_OK;
+    }
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#endif
+    if ((i & 4095) == 4095 && cudaStreamQuery(m->stream) != cudaErrorNotReady) break;
+  }
+  CLA_CUDA(cudaStreamSynchronize(m->stream));
+  std::atomic_thread_fence(std::memory_order_acquire);
+  if (box->flag != seq) return fail(CLA_ERR_CUDA, "host call: the product ended without its result");
+  return CLA_OK;
+}
+
+// What a product on this handle may take from and put into host memory itself (HostDirect); vCells: size of the right
+// operand, SIZE_MAX for the left products and the chain.
+static int small_direct(Matrix* m, size_t vCells);
+
+enum HostDirect {
+  HD_NONE = 0,
+  HD_OUT = 1,  // the product's kernel for short blocks may store the result in host memory
+  HD_IN = 2,   // ... and reads its first operand once per CTA, so that may stay in host memory too
+};
+
+static int small_direct(Matrix* m, size_t vCells) {
+  if (!small_block(m)) return HD_NONE;
+  if (cudaSetDevice(m->device) != cudaSuccess || ensure_col_plan(m) < 0 || ensure_row_lists(m, m->stream) < 0 || !m->rows.ok) return HD_NONE;
+  // every CTA of the right product reads V once over the bus: worth it while that is less than a copy's latency
+  const bool in = vCells != SIZE_MAX && vCells * 8 * ((m->nRows + 31) / 32) <= 128 * 1024;
+  return in ? HD_OUT | HD_IN : HD_OUT;
+}
+
+// Small operands and results go through the handle's mailbox (pinned): the inputs are one asynchronous copy, or are
+// read by the kernel where they are; the last kernel writes the result, the non-zero count and the self-check word
+// straight into pinned memory and raises a flag the host polls. No synchronisation, no pageable copy, and the device
+// time of the call (events) is read only when asked for (cla_stats_get).
+template <class F>
+static int64_t mail_call(Matrix* m, const double* in1, size_t n1, const double* in2, size_t n2, double* out, size_t nOut,
+                         F&& run, int direct) {
+  const size_t i1 = al256(n1 * 8), i2 = al256(n2 * 8);
+  int64_t rc = ensure_io(m, i1 + i2 + al256(nOut * 8) + 256);
+  if (rc < 0) return rc;
+  char* hin = m->mail + MAIL_HEAD;
+  double* hout = (double*)(m->mail + MAIL_HEAD + MAIL_IN);
+  cudaStream_t s = m->stream;
+  if ((rc = order_begin(m, s)) < 0) return rc;
+  if (n1) memcpy(hin, in1, n1 * 8);
+  if (n2) memcpy(hin + i1, in2, n2 * 8);
+  const bool inHost = (direct & HD_IN) && !n2, outHost = direct & HD_OUT;
+  char* base = (char*)m->io;
+  if ((n1 || n2) && !inHost) CLA_CUDA(cudaMemcpyAsync(base, hin, n2 ? i1 + n2 * 8 : n1 * 8, cudaMemcpyHostToDevice, s));
+  double* d1 = inHost ? (double*)hin : (double*)base;
+  double* dOut = outHost ? hout : (double*)(base + i1 + i2);
+  HostCall hc;
+  hc.in1 = inHost ? in1 : nullptr;
+  hc.fin.box = (Mailbox*)m->mail;
+  hc.fin.nnz = m->dFin;
+  hc.fin.ticket = (unsigned int*)(m->dFin + 1);
+  hc.fin.err = m->dErr;
+  hc.fin.seq = ++m->mailSeq ? m->mailSeq : ++m->mailSeq;
+  CLA_CUDA(cudaEventRecord(m->ev0, s));
+  if ((rc = run(d1, n2 ? (double*)(base + i1) : nullptr, dOut, s, outHost ? &hc : nullptr)) < 0) return rc;
+  CLA_CUDA(cudaEventRecord(m->ev1, s));
+  m->elapsedPending = true;
+  if (!hc.used && (rc = launch_finish(m, dOut, (int)nOut, hout, s, hc.fin)) < 0) return rc;
+  if ((rc = mail_wait(m, hc.fin.seq)) < 0) return rc;
+  m->lastValid = false;  // nothing of this handle is in flight any more
+  const Mailbox* box = (const Mailbox*)m->mail;
+  if (box->err) return fail(CLA_ERR_DEVICE_CHECK, "a kernel self-check tripped (code " + std::to_string(box->err) + ")");
+  if (nOut) memcpy(out, hout, nOut * 8);
+  return (int64_t)box->nnz;
+}
+
 // Staging layout in m->io: [inputs ... | output | nnz counter]
 template <class F>
 static int64_t host_call(Matrix* m, const double* in1, size_t n1, const double* in2, size_t n2, double* out, size_t nOut,
-                         F&& run, bool deferIn1 = false) {
+                         F&& run, bool deferIn1 = false, int direct = HD_NONE) {
   CLA_CUDA(cudaSetDevice(m->device));
-  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t o1 = 0, o2 = al(n1 * 8), oOut = o2 + al(n2 * 8), oCnt = oOut + al(nOut * 8);
+  const size_t o1 = 0, o2 = al256(n1 * 8), oOut = o2 + al256(n2 * 8), oCnt = oOut + al256(nOut * 8);
+  if (!deferIn1 && oOut <= MAIL_IN && nOut > 0 && nOut * 8 <= MAIL_OUT && (m->mail || (m->mail = mailbox_take())))
+    return mail_call(m, in1, n1, in2, n2, out, nOut, run, direct);
   int64_t rc = ensure_io(m, oCnt + 256);
   if (rc < 0) return rc;
   char* base = (char*)m->io;
@@ -603,8 +717,9 @@ static int64_t host_call(Matrix* m, const double* in1, size_t n1, const double* 
   if (n1 && !deferIn1 && (rc = upload(d1, in1, n1)) < 0) return rc;  // deferred: run() uploads it
   if (n2 && (rc = upload(d2, in2, n2)) < 0) return rc;
   CLA_CUDA(cudaEventRecord(m->ev0, s));
-  if ((rc = run(d1, n2 ? d2 : nullptr, dOut, s)) < 0) return rc;
+  if ((rc = run(d1, n2 ? d2 : nullptr, dOut, s, nullptr)) < 0) return rc;
   CLA_CUDA(cudaEventRecord(m->ev1, s));
+  m->elapsedPending = true;
   if ((rc = launch_count_nnz(m, dOut, (int64_t)nOut, dCnt, s)) < 0) return rc;
   if (nOut) {
     if (host_copy_staged(m, out, nOut * 8)) {
@@ -616,8 +731,6 @@ static int64_t host_call(Matrix* m, const double* in1, size_t n1, const double* 
   CLA_CUDA(cudaMemcpyAsync(&nnz, dCnt, sizeof(nnz), cudaMemcpyDeviceToHost, s));
   CLA_CUDA(cudaStreamSynchronize(s));
   m->lastValid = false;  // nothing of this handle is in flight any more
-  float ms = 0;
-  if (cudaEventElapsedTime(&ms, m->ev0, m->ev1) == cudaSuccess) m->stats.last_kernel_ms = ms;
   if ((rc = check_errword(m)) < 0) return rc;
   return (int64_t)nnz;
 }
@@ -664,7 +777,7 @@ int64_t cla_tmm(cla_handle left, cla_handle right, double* out) {
     if ((rc = order_begin(r, l->stream)) < 0) return rc;
   }
   rc = host_call(l, nullptr, 0, nullptr, 0, out, (size_t)l->nCols * r->nCols,
-                 [&](double*, double*, double* dOut, cudaStream_t s) { return tmm_dev(l, r, dOut, s); });
+                 [&](double*, double*, double* dOut, cudaStream_t s, HostCall*) { return tmm_dev(l, r, dOut, s); });
   if (r != l && rc >= 0) r->lastValid = false;  // host_call synchronised the stream both blocks' kernels ran on
   return rc;
 }
@@ -729,7 +842,8 @@ int64_t cla_rmm(cla_handle h, const double* V, int32_t vRows, int32_t vCols, dou
   if (vRows != m->nCols || vCols < 0) return fail(CLA_ERR_SHAPE, "rmm: V must be [nCols x vCols]");
   if ((!V && (size_t)vRows * vCols) || (!out && (size_t)m->nRows * vCols)) return fail(CLA_ERR_BAD_ARG, "rmm: null buffer");
   return host_call(m, V, (size_t)vRows * vCols, nullptr, 0, out, (size_t)m->nRows * vCols,
-                   [&](double* dV, double*, double* dOut, cudaStream_t s) { return rmm_dev(m, dV, vRows, vCols, dOut, s); });
+                   [&](double* dV, double*, double* dOut, cudaStream_t s, HostCall* hc) { return rmm_dev(m, dV, vRows, vCols, dOut, s, hc); },
+                   false, small_direct(m, (size_t)vRows * vCols));
 }
 
 int64_t cla_lmm(cla_handle h, const double* Yt, int32_t yRows, double* out) {
@@ -737,20 +851,24 @@ int64_t cla_lmm(cla_handle h, const double* Yt, int32_t yRows, double* out) {
   REQUIRE_FINAL();
   if (yRows < 0) return fail(CLA_ERR_SHAPE, "lmm: negative row count");
   if ((!Yt && (size_t)yRows * m->nRows) || (!out && (size_t)yRows * m->nCols)) return fail(CLA_ERR_BAD_ARG, "lmm: null buffer");
-  if (yRows == 1)  // one left row: upload it in slices that overlap with the product where the kernel allows
+  if (yRows == 1 && m->nRows >= (1 << 20))  // one long left row: upload it in slices that overlap with the product where the kernel allows
     return host_call(
         m, Yt, (size_t)m->nRows, nullptr, 0, out, (size_t)m->nCols,
-        [&](double* dY, double*, double* dOut, cudaStream_t s) -> int64_t {
+        [&](double* dY, double*, double* dOut, cudaStream_t s, HostCall*) -> int64_t {
           m->stats.calls_lmm++;
           int64_t rc = fast_lmm_vec_host(m, Yt, dY, dOut, s);
           if (rc != 0) return rc < 0 ? rc : CLA_OK;
           m->stats.calls_lmm--;
-          if (m->nRows) CLA_CUDA(cudaMemcpyAsync(dY, Yt, (size_t)m->nRows * 8, cudaMemcpyHostToDevice, s));
+          if (host_copy_staged(m, Yt, (size_t)m->nRows * 8)) {
+            if ((rc = host_to_device_staged(m, dY, Yt, (size_t)m->nRows * 8, s, nullptr)) < 0) return rc;
+          } else
+            CLA_CUDA(cudaMemcpyAsync(dY, Yt, (size_t)m->nRows * 8, cudaMemcpyHostToDevice, s));
           return lmm_dev(m, dY, 1, dOut, s);
         },
         true);
   return host_call(m, Yt, (size_t)yRows * m->nRows, nullptr, 0, out, (size_t)yRows * m->nCols,
-                   [&](double* dY, double*, double* dOut, cudaStream_t s) { return lmm_dev(m, dY, yRows, dOut, s); });
+                   [&](double* dY, double*, double* dOut, cudaStream_t s, HostCall* hc) { return lmm_dev(m, dY, yRows, dOut, s, hc); },
+                   false, small_direct(m, SIZE_MAX));
 }
 
 int64_t cla_tsmm(cla_handle h, double* out) {
@@ -759,7 +877,7 @@ int64_t cla_tsmm(cla_handle h, double* out) {
   if (!out && m->nCols) return fail(CLA_ERR_BAD_ARG, "tsmm: null buffer");
   m->stats.calls_tsmm++;
   return host_call(m, nullptr, 0, nullptr, 0, out, (size_t)m->nCols * m->nCols,
-                   [&](double*, double*, double* dOut, cudaStream_t s) { return launch_tsmm(m, dOut, s); });
+                   [&](double*, double*, double* dOut, cudaStream_t s, HostCall*) { return launch_tsmm(m, dOut, s); });
 }
 
 int64_t cla_mmchain(cla_handle h, const double* v, const double* w, int32_t ctype, double* out) {
@@ -769,9 +887,10 @@ int64_t cla_mmchain(cla_handle h, const double* v, const double* w, int32_t ctyp
   if (ctype == CLA_CHAIN_XtwXv && !w && m->nRows) return fail(CLA_ERR_BAD_ARG, "mmchain: XtwXv needs w");
   const size_t nW = ctype == CLA_CHAIN_XtwXv ? (size_t)m->nRows : 0;
   return host_call(m, v, (size_t)m->nCols, w, nW, out, (size_t)m->nCols,
-                   [&](double* dV, double* dW, double* dOut, cudaStream_t s) {
-                     return mmchain_dev(m, dV, dW, ctype, dOut, nullptr, s);
-                   });
+                   [&](double* dV, double* dW, double* dOut, cudaStream_t s, HostCall* hc) {
+                     return mmchain_dev(m, dV, dW, ctype, dOut, nullptr, s, hc);
+                   },
+                   false, small_direct(m, SIZE_MAX));
 }
 
 // Column sums are t(1) %*% X and row sums X %*% 1, so both run on the product kernels.
@@ -781,7 +900,7 @@ int64_t cla_unary_agg(cla_handle h, int32_t op, double* out) {
   if (op < CLA_AGG_COL_SUMS || op > CLA_AGG_MAX) return fail(CLA_ERR_BAD_ARG, "unary aggregate: unknown operation");
   if (!out) return fail(CLA_ERR_BAD_ARG, "unary aggregate: null buffer");
   if (op == CLA_AGG_ROW_MINS || op == CLA_AGG_ROW_MAXS)
-    return host_call(m, nullptr, 0, nullptr, 0, out, (size_t)m->nRows, [&](double*, double*, double* dOut, cudaStream_t s) {
+    return host_call(m, nullptr, 0, nullptr, 0, out, (size_t)m->nRows, [&](double*, double*, double* dOut, cudaStream_t s, HostCall*) {
       return row_minmax(m, op == CLA_AGG_ROW_MAXS, dOut, s);
     });
   if (op >= CLA_AGG_COL_MINS) {
@@ -810,11 +929,13 @@ int64_t cla_unary_agg(cla_handle h, int32_t op, double* out) {
   if (op == CLA_AGG_ROW_SUMS) {
     std::vector<double> ones((size_t)m->nCols, 1.0);
     return host_call(m, ones.data(), ones.size(), nullptr, 0, out, (size_t)m->nRows,
-                     [&](double* dV, double*, double* dOut, cudaStream_t s) { return rmm_dev(m, dV, m->nCols, 1, dOut, s); });
+                     [&](double* dV, double*, double* dOut, cudaStream_t s, HostCall* hc) { return rmm_dev(m, dV, m->nCols, 1, dOut, s, hc); },
+                     false, small_direct(m, ones.size()));
   }
   std::vector<double> ones((size_t)m->nRows, 1.0), cs((size_t)m->nCols, 0.0);
   int64_t rc = host_call(m, ones.data(), ones.size(), nullptr, 0, op == CLA_AGG_SUM ? cs.data() : out, (size_t)m->nCols,
-                         [&](double* dY, double*, double* dOut, cudaStream_t s) { return lmm_dev(m, dY, 1, dOut, s); });
+                         [&](double* dY, double*, double* dOut, cudaStream_t s, HostCall* hc) { return lmm_dev(m, dY, 1, dOut, s, hc); },
+                         false, small_direct(m, SIZE_MAX));
   if (rc < 0 || op == CLA_AGG_COL_SUMS) return rc;
   double total = 0;
   for (double x : cs) total += x;
@@ -828,7 +949,7 @@ int64_t cla_decompress(cla_handle h, double* out) {
   if (!out && (size_t)m->nRows * m->nCols) return fail(CLA_ERR_BAD_ARG, "decompress: null buffer");
   m->stats.calls_decompress++;
   return host_call(m, nullptr, 0, nullptr, 0, out, (size_t)m->nRows * m->nCols,
-                   [&](double*, double*, double* dOut, cudaStream_t s) { return launch_decompress(m, dOut, s); });
+                   [&](double*, double*, double* dOut, cudaStream_t s, HostCall*) { return launch_decompress(m, dOut, s); });
 }
 
 // ---- decoded index structures -----------------------------------------------------------------------

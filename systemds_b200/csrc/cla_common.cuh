@@ -152,6 +152,62 @@ struct SpItem {
 };
 
 struct FastPlan;  // plans of the specialised DDC kernels (cla_fast.cu)
+
+// One column of one product group, flat (built once per handle, cla_rows.cu).
+struct ColRef {
+  const void* map;
+  const void* mapHi;
+  const double* src;  // dictionary (or dense block) + position of the column inside the group
+  int32_t kind;       // GT_DDC, GT_UNC, GT_SDC or GT_RLE
+  int32_t mapType;
+  int32_t stride;     // columns of the group
+  int32_t col;        // matrix column
+  int32_t group;      // device group index
+  int32_t pad;
+};
+// The tuples of the SDC / RLE groups are numbered through ("sparse table rows", list order, svOff[group] first).
+struct SparseVal {
+  double val;     // the dictionary value, single-column groups
+  int32_t col;    // their matrix column; -1: a group of several columns
+  int32_t group;  // device group index
+};
+// Row-oriented forms of the SDC and RLE groups (cla_rows.cu).
+constexpr int WIN_ROWS = 64;
+struct RowLists {
+  bool tried = false, ok = false;
+  int nSdc = 0, nRle = 0;           // groups with listed rows / with runs
+  int64_t nSv = 0;                  // sparse table rows
+  int32_t* svOff = nullptr;         // [nDev]
+  SparseVal* sv = nullptr;          // [nSv]
+  uint32_t* rowPtr = nullptr;       // [nBlocks * 1024 + 1]: first item of a row; items = table rows of its listed SDC tuples
+  uint32_t* rowItems = nullptr;
+  uint32_t* fullPtr = nullptr;      // [nBlocks * 16 + 1]: runs that cover a whole 64-row window: their table rows
+  uint32_t* fullItems = nullptr;
+  uint32_t* partPtr = nullptr;      // runs that cover part of a window: table row, first row | end row << 8 in the window
+  uint2* partItems = nullptr;
+};
+struct ColPlan {
+  bool built = false;
+  int nDense = 0, nRefs = 0;
+  ColRef* dense = nullptr;     // dense-map and uncompressed columns, list order
+  ColRef* refs = nullptr;      // every column of every group, sorted by matrix column (list order within a column)
+  int32_t* refPtr = nullptr;   // [nCols + 1]
+};
+// Where a host-buffer call's result goes when it is small: pinned memory the kernels write straight into.
+struct alignas(16) Mailbox {  // one 16-byte store: the flag never arrives before what it stands for
+  volatile uint32_t flag;
+  int32_t err;
+  unsigned long long nnz;
+};
+constexpr size_t MAIL_HEAD = 256, MAIL_IN = 64 * 1024, MAIL_OUT = 128 * 1024;
+// Given to the last kernel of a small host-buffer call: it counts the non-zeros and raises the flag.
+struct Finish {
+  Mailbox* box = nullptr;             // null: not wanted
+  unsigned long long* nnz = nullptr;  // device counters, zero between calls
+  unsigned int* ticket = nullptr;
+  int32_t* err = nullptr;             // the handle's self-check word
+  uint32_t seq = 0;
+};
 struct HostStage; // pinned ring for operands in pageable host memory (cla_hostcopy.cu)
 
 struct Matrix;
@@ -225,7 +281,13 @@ struct Matrix {
   cudaStream_t lastStream = nullptr;
   bool lastValid = false;
   FastPlan* fast = nullptr;
+  RowLists rows;
+  ColPlan cols;
   HostStage* hostStage = nullptr;
+  char* mail = nullptr;          // pinned: Mailbox, inputs, outputs (small host-buffer calls)
+  unsigned long long* dFin = nullptr;  // device counters of Finish
+  uint32_t mailSeq = 0;
+  bool elapsedPending = false;   // ev0 / ev1 bracket the last host-buffer call
   bool profile = false;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> profEvents;  // ring of event pairs
   size_t profUsed = 0;
@@ -263,6 +325,18 @@ int64_t device_to_host_staged(Matrix* m, void* host, const void* dSrc, size_t by
 void host_stage_free(Matrix* m);
 int64_t ensure_sparse_list(Matrix* m);
 int64_t ensure_sparse_lists(Matrix* m, cudaStream_t s);  // the row-major work lists; m->spListsOk tells whether they exist  // Matrix::dSparseIdx (cla_generic.cu)
+
+int64_t ensure_col_plan(Matrix* m);                        // Matrix::cols
+int64_t ensure_row_lists(Matrix* m, cudaStream_t s);       // Matrix::rows; rows.ok tells whether they exist
+// Short blocks (cla_small.cu): one kernel per product, every group type. 1 = done, 0 = not covered
+bool small_block(const Matrix* m);
+int64_t small_rmm(Matrix* m, const double* dV, int vCols, double* dOut, const double* dW, cudaStream_t s, const Finish& fin,
+                  const double* hostV = nullptr);
+int64_t small_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s, const Finish& fin);
+int64_t launch_finish(Matrix* m, const double* d, int n, double* out, cudaStream_t s, const Finish& fin);
+// Pinned mailboxes for small host-buffer calls, shared by all handles (cla_hostcopy.cu); null when none can be had
+char* mailbox_take();
+void mailbox_give(char* p);
 
 // launchers implemented in the kernel translation units; all enqueue on `s` and return CLA_OK or an error.
 int64_t launch_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStream_t s, bool afterFast = false);

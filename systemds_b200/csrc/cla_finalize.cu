@@ -41,11 +41,16 @@ static int64_t grow(void** p, size_t* cur, size_t bytes) {
   return CLA_OK;
 }
 int64_t order_begin(Matrix* m, cudaStream_t s) {
-  if (m->lastValid && m->lastStream != s) CLA_CUDA(cudaStreamWaitEvent(s, m->lastDone, 0));
+  if (m->lastValid && m->lastStream != s) {
+    if (m->lastStream == nullptr) CLA_CUDA(cudaEventRecord(m->lastDone, nullptr));  // not recorded by order_end, see there
+    CLA_CUDA(cudaStreamWaitEvent(s, m->lastDone, 0));
+  }
   return CLA_OK;
 }
 int64_t order_end(Matrix* m, cudaStream_t s) {
-  CLA_CUDA(cudaEventRecord(m->lastDone, s));
+  // The legacy default stream always exists, so the event behind a call on it is recorded only when a call on another
+  // stream needs it (everything enqueued there by then is waited for); other streams may be destroyed by their owner.
+  if (s != nullptr) CLA_CUDA(cudaEventRecord(m->lastDone, s));
   m->lastStream = s;
   m->lastValid = true;
   return CLA_OK;
@@ -375,7 +380,7 @@ static size_t map_bytes(int mapType, int64_t size, size_t* hiBytes) {
 static int64_t build_sdc_skip(const HostGroup& hg, int nRows, std::vector<SdcSkip>& skip) {
   const int nb = (nRows + SKIP_ROWS - 1) / SKIP_ROWS;
   skip.assign(std::max(nb, 1), SdcSkip{(int32_t)hg.nOff, nRows, hg.offLen});
-  if (hg.offType != CLA_OFF_BYTE && hg.offType != CLA_OFF_CHAR) return CLA_OK;
+  if (hg.offType != CLA_OFF_BYTE && hg.offType != CLA_OFF_CHAR) return CLA_OK;  // one or two rows: held by the record
   const int maxV = hg.offType == CLA_OFF_BYTE ? 255 : 65535;
   const uint8_t* b = hg.offData.data();
   const uint16_t* c = (const uint16_t*)hg.offData.data();
@@ -415,6 +420,7 @@ int64_t init_device_state(Matrix* m) {
   CLA_CUDA(cudaMalloc(&errp, 64));
   CLA_CUDA(cudaMemset(errp, 0, 64));
   m->dErr = (int32_t*)errp;
+  m->dFin = (unsigned long long*)((char*)errp + 16);
   return CLA_OK;
 }
 
@@ -653,6 +659,7 @@ int64_t finalize_device(Matrix* m) {
     std::vector<double>().swap(hg.dense);
   }
   if ((rc = fast_plan_build(m)) < 0) return rc;
+  if (small_block(m) && (rc = ensure_col_plan(m)) < 0) return rc;
   m->stats.n_rows = m->nRows;
   m->stats.n_cols = m->nCols;
   m->stats.n_groups = (int64_t)m->hg.size();
@@ -691,6 +698,8 @@ void release(Matrix* m) {
   if (m->copyStream) cudaStreamDestroy(m->copyStream);
   m->copyStream = nullptr;
   host_stage_free(m);
+  mailbox_give(m->mail);
+  m->mail = nullptr;
   if (m->stream) cudaStreamDestroy(m->stream);
   m->scratch = m->scratch2 = m->io = nullptr;
   m->dErr = nullptr;

@@ -81,6 +81,42 @@ void host_stage_free(Matrix* m) {
   m->hostStage = nullptr;
 }
 
+// Mailboxes: one pinned, portable buffer per handle that has seen a small host-buffer call. Handles come and go (one per
+// block of a blocked matrix) and pinning costs far more than such a call, so released mailboxes are kept for the next
+// handle, up to MAIL_KEEP of them.
+constexpr size_t MAIL_KEEP = 32;
+static std::mutex g_mailMu;
+static std::vector<char*> g_mailFree;
+char* mailbox_take() {
+  {
+    std::lock_guard<std::mutex> lk(g_mailMu);
+    if (!g_mailFree.empty()) {
+      char* p = g_mailFree.back();
+      g_mailFree.pop_back();
+      return p;
+    }
+  }
+  void* p = nullptr;
+  if (cudaHostAlloc(&p, MAIL_HEAD + MAIL_IN + MAIL_OUT, cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  memset(p, 0, MAIL_HEAD);
+  return (char*)p;
+}
+void mailbox_give(char* p) {
+  if (!p) return;
+  {
+    std::lock_guard<std::mutex> lk(g_mailMu);
+    if (g_mailFree.size() < MAIL_KEEP) {
+      memset(p, 0, MAIL_HEAD);
+      g_mailFree.push_back(p);
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+
 bool host_copy_staged(Matrix* m, const void* host, size_t bytes) {
   return bytes >= STAGE_MIN && stage_threads() > 0 && host_is_pageable(host) && stage_of(m) != nullptr;
 }

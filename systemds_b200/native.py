@@ -107,8 +107,6 @@ def check(rc: int) -> int:
     return int(rc)
 
 
-def ptr(a) -> C.c_void_p:
-    """Address of a numpy array (or None)."""
-    if a is None:
-        return C.c_void_p(0)
-    return C.c_void_p(a.ctypes.data)
+def ptr(a):
+    """Address of a numpy array (or None), as an argument for a ``void*`` parameter."""
+    return None if a is None else a.ctypes.data
