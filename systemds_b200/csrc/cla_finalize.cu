@@ -333,17 +333,71 @@ __global__ void k_check_ids(int mapType, const void* __restrict__ map, int64_t n
 // ------------------------------------------------------------------------------------------------
 // upload
 // ------------------------------------------------------------------------------------------------
+// A block has thousands of small arrays (column lists, dictionaries, skip lists) and a map per group; one allocation and
+// one blocking copy each cost more than the data. They are carved out of two slabs per handle: the small ones are
+// collected in a host image that is copied in one go (flush), the large ones copied from where they are.
+constexpr size_t SLAB_SMALL = 64 * 1024;
+struct Slab {
+  char* base = nullptr;
+  size_t cap = 0, at = 0, flushed = 0;
+  std::vector<char> image;  // host image (small slab only)
+};
+struct Uploads {
+  Slab small_, big;
+  static size_t al(size_t b) { return (b + 255) & ~(size_t)255; }
+};
+static thread_local Uploads* g_up = nullptr;  // the uploads of the finalize call running on this thread
+
+static int64_t slab_open(Matrix* m, Slab& s, size_t cap) {
+  s.cap = cap;
+  if (cap == 0) return CLA_OK;
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, cap);
+  if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  m->allocs.push_back(p);
+  s.base = (char*)p;
+  return CLA_OK;
+}
+static int64_t flush_uploads(Matrix* m) {  // device work on m->stream that follows sees the small arrays registered so far
+  Slab& s = g_up->small_;
+  if (s.at > s.flushed) CLA_CUDA(cudaMemcpyAsync(s.base + s.flushed, s.image.data() + s.flushed, s.at - s.flushed, cudaMemcpyHostToDevice, m->stream));
+  s.flushed = s.at;
+  return CLA_OK;
+}
+static int64_t carve(Matrix* m, size_t bytes, void** dst, Slab** from) {
+  *from = nullptr;
+  if (g_up) {
+    Slab& s = bytes < SLAB_SMALL ? g_up->small_ : g_up->big;
+    const size_t b = Uploads::al(bytes);
+    if (s.at + b <= s.cap) {
+      *dst = s.base + s.at;
+      *from = &s;
+      s.at += b;
+      return CLA_OK;
+    }
+  }
+  cudaError_t e = cudaMalloc(dst, bytes);
+  if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  m->allocs.push_back(*dst);
+  return CLA_OK;
+}
+
 template <typename T>
 static int64_t upload(Matrix* m, const T* src, size_t n, const T** dst, bool index) {
   *dst = nullptr;
   if (n == 0) return CLA_OK;
   void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-  if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  m->allocs.push_back(p);
-  m->deviceBytes += n * sizeof(T);
-  if (index) m->indexBytes += n * sizeof(T);
-  CLA_CUDA(cudaMemcpy(p, src, n * sizeof(T), cudaMemcpyHostToDevice));
+  Slab* from;
+  const size_t bytes = n * sizeof(T);
+  int64_t rc = carve(m, bytes, &p, &from);
+  if (rc < 0) return rc;
+  m->deviceBytes += bytes;
+  if (index) m->indexBytes += bytes;
+  if (from && from == &g_up->small_) {
+    if (from->image.size() < from->at) from->image.resize(from->at);
+    memcpy(from->image.data() + ((char*)p - from->base), src, bytes);
+  } else
+    CLA_CUDA(cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, m->stream));
   *dst = (const T*)p;
   return CLA_OK;
 }
@@ -353,9 +407,16 @@ static int64_t dev_alloc(Matrix* m, size_t n, T** dst) {
   *dst = nullptr;
   if (n == 0) return CLA_OK;
   void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-  if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  m->allocs.push_back(p);
+  // (device-written arrays never come from the small slab, whose host image would overwrite them)
+  const size_t b = Uploads::al(n * sizeof(T));
+  if (g_up && g_up->big.at + b <= g_up->big.cap) {
+    p = g_up->big.base + g_up->big.at;
+    g_up->big.at += b;
+  } else {
+    cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+    if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    m->allocs.push_back(p);
+  }
   m->deviceBytes += n * sizeof(T);
   *dst = (T*)p;
   return CLA_OK;
@@ -443,6 +504,60 @@ int64_t finalize_device(Matrix* m) {
         seen[c] = 1;
       }
   }
+  // sizes of everything below, for the slabs and for the scratch of the run decoder
+  Uploads up;
+  struct UpGuard {
+    UpGuard(Uploads* u) { g_up = u; }
+    ~UpGuard() { g_up = nullptr; }
+  } upGuard(&up);
+  size_t smallB = 0, bigB = 0;
+  int64_t mostPairs = 0;
+  const size_t nb0 = (size_t)std::max(1, (m->nRows + SKIP_ROWS - 1) / SKIP_ROWS);
+  {
+    auto host = [&](size_t b) {
+      if (b) (b < SLAB_SMALL ? smallB : bigB) += Uploads::al(b);
+    };
+    for (auto& hg : m->hg) {
+      if (hg.type == GT_EMPTY || hg.type == GT_CONST) continue;
+      const size_t gc = hg.cols.size();
+      host(gc * 4);
+      if (hg.type != GT_UNC) host((hg.dict.size() + (hg.type == GT_OLE ? gc : 0)) * 8);
+      if (hg.type == GT_SDC && !hg.def.empty()) host(hg.dict.size() * 8);
+      size_t hiB;
+      if (hg.devMap) bigB += Uploads::al(map_bytes(hg.mapType, hg.mapSize, &hiB));
+      host(hg.map.size());
+      host(hg.mapHi.size());
+      host(hg.offData.size());
+      if (hg.type == GT_SDC) host(nb0 * sizeof(SdcSkip));
+      host(hg.ptr.size() * 4);
+      host(hg.data.size() * 2);
+      if (hg.type == GT_RLE) {
+        const int64_t pairs = (int64_t)hg.data.size() / 2;
+        bigB += Uploads::al(nb0 * 4) + Uploads::al((size_t)pairs * sizeof(RleRun));
+        mostPairs = std::max(mostPairs, pairs);
+      }
+      if (hg.type == GT_OLE) bigB += Uploads::al((size_t)m->nRows * (hg.nVals + 1 <= 256 ? 1 : (hg.nVals + 1 <= 65536 ? 2 : 4)));
+      if (hg.type == GT_UNC) bigB += Uploads::al((size_t)m->nRows * gc * 8);
+    }
+    // group records, constants, column table
+    host(m->hg.size() * sizeof(DevGroup));
+    host((size_t)m->nCols * 8);
+    host((size_t)m->nCols * 8);
+  }
+  int64_t rcs;
+  if ((rcs = slab_open(m, up.small_, smallB)) < 0 || (rcs = slab_open(m, up.big, bigB)) < 0) return rcs;
+  struct Scratch {  // of the run decoder, for all groups (stream order keeps them apart)
+    void* p = nullptr;
+    ~Scratch() {
+      if (p) cudaFree(p);
+    }
+  } rleTmp;
+  size_t rleSort = 0;
+  if (mostPairs > 0) {
+    cub::DeviceRadixSort::SortPairs(nullptr, rleSort, (uint32_t*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr,
+                                    (int)mostPairs, 0, 32, m->stream);
+    CLA_CUDA(cudaMalloc(&rleTmp.p, (size_t)mostPairs * (sizeof(RleRun) + 4 * sizeof(uint32_t)) + rleSort + 16));
+  }
   for (size_t gi = 0; gi < m->hg.size(); gi++) {
     HostGroup& hg = m->hg[gi];
     const int gc = (int)hg.cols.size();
@@ -529,22 +644,18 @@ int64_t finalize_device(Matrix* m) {
       if (nPairs > 0) {
         RleRun* tmpRuns = nullptr;
         uint32_t *k0 = nullptr, *k1 = nullptr, *v0 = nullptr, *v1 = nullptr;
-        void* tmp = nullptr;
-        CLA_CUDA(cudaMalloc(&tmp, nPairs * (sizeof(RleRun) + 4 * sizeof(uint32_t))));
+        void* tmp = (char*)rleTmp.p + ((rleSort + 15) & ~(size_t)15);
         tmpRuns = (RleRun*)tmp;
         k0 = (uint32_t*)(tmpRuns + nPairs);
         k1 = k0 + nPairs;
         v0 = k1 + nPairs;
         v1 = v0 + nPairs;
-        if ((rc = dev_alloc(m, (size_t)nPairs, &dRuns)) < 0) return rc;
+        if ((rc = dev_alloc(m, (size_t)nPairs, &dRuns)) < 0 || (rc = flush_uploads(m)) < 0) return rc;
         k_rle_decode<<<(hg.nVals * 32 + 255) / 256, 256, 0, m->stream>>>(g.ptr, g.data, hg.nVals, tmpRuns, k0, m->nRows,
                                                                         m->dErr);
         k_iota<<<(unsigned)((nPairs + 255) / 256), 256, 0, m->stream>>>(v0, nPairs);
-        size_t tb = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, tb, k0, k1, v0, v1, (int)nPairs, 0, 32, m->stream);
-        void* dTmp = nullptr;
-        CLA_CUDA(cudaMalloc(&dTmp, tb + 16));
-        cub::DeviceRadixSort::SortPairs(dTmp, tb, k0, k1, v0, v1, (int)nPairs, 0, 32, m->stream);
+        size_t tb = rleSort;
+        cub::DeviceRadixSort::SortPairs(rleTmp.p, tb, k0, k1, v0, v1, (int)nPairs, 0, 32, m->stream);
         k_rle_gather<<<(unsigned)((nPairs + 255) / 256), 256, 0, m->stream>>>(tmpRuns, v1, dRuns, nPairs);
         // runs of length zero (the (65535, 0) fillers) sorted to the end: count the real ones on the host
         int64_t real = 0;
@@ -552,15 +663,13 @@ int64_t finalize_device(Matrix* m) {
         g.nRuns = real;
         g.runs = dRuns;
         k_rle_skip<<<(nb + 255) / 256, 256, 0, m->stream>>>(dRuns, real, dSkip, nb);
-        CLA_CUDA(cudaStreamSynchronize(m->stream));
-        CLA_CUDA(cudaFree(dTmp));
-        CLA_CUDA(cudaFree(tmp));
       } else {
         CLA_CUDA(cudaMemsetAsync(dSkip, 0, sizeof(int32_t) * std::max(nb, 1), m->stream));
       }
       g.runSkip = dSkip;
     }
     if (hg.type == GT_OLE) {  // transcode to a per-row map; products treat the group as DDC
+      if ((rc = flush_uploads(m)) < 0) return rc;
       const int nv1 = hg.nVals + 1;
       const int64_t n = m->nRows;
       void* dm = nullptr;
@@ -616,6 +725,7 @@ int64_t finalize_device(Matrix* m) {
   m->nDev = (int)m->groups.size();
   m->hasConst = false;
   for (double x : m->constV) m->hasConst |= (x != 0.0);
+  if ((rcs = flush_uploads(m)) < 0) return rcs;
   CLA_CUDA(cudaStreamSynchronize(m->stream));
   int32_t herr = 0;
   CLA_CUDA(cudaMemcpy(&herr, m->dErr, sizeof(herr), cudaMemcpyDeviceToHost));
@@ -650,6 +760,8 @@ int64_t finalize_device(Matrix* m) {
     if ((rc = upload(m, colSrc.data(), colSrc.size(), &dcs, false)) < 0) return rc;
     m->dColSrc = const_cast<int32_t*>(dcs);
   }
+  if ((rc = flush_uploads(m)) < 0) return rc;
+  CLA_CUDA(cudaStreamSynchronize(m->stream));
   // the registered host arrays are no longer needed
   for (auto& hg : m->hg) {
     std::vector<uint8_t>().swap(hg.map);
@@ -687,6 +799,7 @@ void release(Matrix* m) {
   m->profEvents.clear();
   if (m->ev0) cudaEventDestroy(m->ev0);
   if (m->ev1) cudaEventDestroy(m->ev1);
+  m->ev0 = m->ev1 = nullptr;
   if (m->lastDone) cudaEventDestroy(m->lastDone);
   m->lastDone = nullptr;
   m->lastValid = false;
