@@ -434,7 +434,7 @@ static int64_t rmm_by_vectors(Matrix* m, const double* dV, int32_t vCols, double
   k_small_transpose<<<(cells + 255) / 256, 256, 0, s>>>(dV, m->nCols, vCols, Vt);
   for (int j = 0; j < vCols; j++) {
     double* uj = U + rowsPad * j;
-    rc = fast_rmm_vec(m, Vt + (size_t)j * m->nCols, uj, s);
+    rc = fast_rmm_vec(m, Vt + (size_t)j * m->nCols, uj, nullptr, s);
     if (rc < 0) return rc;
     if (rc == 2) rc = launch_rmm(m, Vt + (size_t)j * m->nCols, 1, uj, s, true);
     else if (rc == 0) rc = launch_rmm(m, Vt + (size_t)j * m->nCols, 1, uj, s);
@@ -465,7 +465,7 @@ static int64_t rmm_dev(Matrix* m, const double* dV, int32_t vRows, int32_t vCols
     if (rc != 0) return rc < 0 ? rc : CLA_OK;
   }
   if (vCols == 1) {
-    int64_t rc = fast_rmm_vec(m, dV, dOut, s);
+    int64_t rc = fast_rmm_vec(m, dV, dOut, nullptr, s);
     if (rc < 0) return rc;
     if (rc == 1) return CLA_OK;
     return launch_rmm(m, dV, 1, dOut, s, rc == 2);
@@ -529,6 +529,15 @@ static int64_t mmchain_dev(Matrix* m, const double* dV, const double* dW, int32_
   if (ctype != CLA_CHAIN_XtXv && ctype != CLA_CHAIN_XtwXv) return fail(CLA_ERR_UNSUPPORTED, "mmchain: unsupported chain type");
   if (ctype == CLA_CHAIN_XtwXv && !dW) return fail(CLA_ERR_BAD_ARG, "mmchain: XtwXv needs w");
   m->stats.calls_mmchain++;
+  {
+    const int64_t rc = fast_chain(m, dV, ctype == CLA_CHAIN_XtwXv ? dW : nullptr, dOut, dU, s);
+    if (rc < 0) return rc;
+    if (rc == 1) {
+      m->stats.calls_rmm++;
+      m->stats.calls_lmm++;
+      return CLA_OK;
+    }
+  }
   if (!dU) {
     int64_t rc = ensure_scratch2(m, sizeof(double) * (size_t)std::max(m->nRows, 1));
     if (rc < 0) return rc;
@@ -537,6 +546,9 @@ static int64_t mmchain_dev(Matrix* m, const double* dV, const double* dW, int32_
   int64_t rc = 0;
   if (small_block(m)) {  // the weights are applied where the row sums are written
     rc = small_rmm(m, dV, 1, dU, ctype == CLA_CHAIN_XtwXv ? dW : nullptr, s, Finish());
+    if (rc < 0) return rc;
+  } else if (fast_plan_ok(m) && !fast_plan_partial(m)) {
+    rc = fast_rmm_vec(m, dV, dU, ctype == CLA_CHAIN_XtwXv ? dW : nullptr, s);
     if (rc < 0) return rc;
   }
   if (rc == 0) {

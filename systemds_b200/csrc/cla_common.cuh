@@ -368,7 +368,9 @@ int64_t fast_plan_build(Matrix* m);
 void fast_plan_free(Matrix* m);
 bool fast_plan_ok(const Matrix* m);       // some or all groups are covered by the specialised kernels
 bool fast_plan_partial(const Matrix* m);  // ... some but not all
-int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, cudaStream_t s);
+// dW: null, or factors applied to the rows (0 is returned where the plan does not cover every group)
+int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s);
+int64_t fast_chain(Matrix* m, const double* dV, const double* dW, double* dOut, double* dU, cudaStream_t s);
 int64_t fast_lmm_vec(Matrix* m, const double* dY, double* dOut, cudaStream_t s);
 int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* dOut, cudaStream_t s);  // q = 2 or 4 left rows at once
 int64_t fast_decompress(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s);  // 1 = done, 0 = not covered

@@ -1,26 +1,27 @@
-// Specialised vector products for matrices whose product groups are all dense-map (DDC) groups with
+// Specialised vector products for matrices whose product groups are (all or in part) dense-map (DDC) groups with
 // at most 256 dictionary tuples and one byte per map cell -- the shape of the headline workloads
 // (X %*% v, t(y) %*% X and the two passes of t(X) %*% (X %*% v)).
 //
-// Both kernels are bound by shared-memory lookups (one 8-byte dictionary read per map cell), so the
-// layouts are chosen to make those reads bank-conflict free:
+// The kernels are bound by shared-memory lookups (one 8-byte read per lookup, 16 per clock and SM), so the layout makes
+// those reads bank-conflict free: a lane owns a *column slot*, not rows. Tables are interleaved 16 slots wide, one such
+// "unit" after the other (entry k of slot s of a unit at byte k*128 + s*8), so lane s only ever touches bank pair s
+// whatever the ids are. The two half-warps work on different 16-row blocks of the same slots. The maps are kept in a
+// second, interleaved form (16 slots x 16 rows of ids: one 128-bit load per lane and block), and the address of an
+// entry is one dp4a of the id word (byte * 128 + table base).
 //
-//  * k_rmm_vec_u8: a thread owns 16 consecutive rows (one 128-bit map load per group) and keeps their
-//    16 partial sums in registers; the tables P_g = D_g * v[cols_g] (built per call by k_fast_ptable)
-//    sit in shared memory back to back. A table of <= 16 entries spans each 8-byte bank once, so random
-//    ids never conflict; larger tables conflict in proportion to their size.
+//  * k_lmm_vec: t(y) X, slot = matrix column, table = its dictionary column.
+//  * k_rmm_vec<false>: X v, the same slots and tables; the lane multiplies by its column's v on the fly.
+//  * k_chain_vec: t(X) (w * (X v)) in one pass over the maps, for matrices of up to 112 columns.
+//  * k_rmm_vec<true>: X v on joint slots, when dictionaries are small: several groups share a slot whose one-byte map
+//    holds their joint id (mixed radix, at most 256 joint tuples; combined once at plan time) and whose table, built by
+//    each CTA from v, holds the sum of their terms: one byte of map and one lookup for two to eight cells.
 //
-//  * k_lmm_vec_u8: a lane owns *columns*, not rows. Tables are interleaved 16 columns wide, one such
-//    "unit" after the other (entry k of slot s of a unit at byte k*128 + s*8), so lane s only ever touches
-//    bank pair s whatever the ids are: conflict free for any cardinality, without replicating tables. The
-//    two half-warps of a warp work on different rows of the same 16 column slots per unit; a CTA holds up
-//    to seven units (7 x 32 KB at 256 tuples). The left vector is read with warp-uniform 128-bit loads and
-//    kept in registers for all columns of the CTA.
-//
-// Tables are staged into shared memory with TMA bulk copies (cp.async.bulk + mbarrier, no multicast).
+// Dictionary tables are staged into shared memory with TMA bulk copies (cp.async.bulk + mbarrier, no multicast).
 #include "cla_common.cuh"
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <numeric>
 
 namespace cla {
@@ -31,27 +32,15 @@ int64_t launch_lmm_const_with(Matrix* m, const double* dYt, int q, double* dOut,
 constexpr int FAST_MIN_ROWS = 4096;
 constexpr int SMEM_MAX = 227 * 1024;
 
-// ---- RMM plan ----
-constexpr int RMM_T = 128;            // threads (128 / 256 / 512 measured on 10M x 100, 16 values: 0.313 / 0.320 / 0.496 ms)
-constexpr int RMM_ROWS_PT = 16;       // rows per thread
-constexpr int RMM_TILE = RMM_T * RMM_ROWS_PT;
-
-// ---- LMM plan ----
-// Warps per CTA (one CTA per SM). Measured on the benchmark workloads for 10 / 12 / 14 / 16 warps: t(y) X 10M x 200
-// 0.718 / 0.675 / 0.682 / 0.654 ms (sixteen warps fit 128 registers with 20 bytes of spills), the fused X v 1M x 100
-// 0.0699 / 0.0686 / 0.0688 / 0.0665 ms per step; k_rmm_vec_b is the exception (lmCG step 9.32 / 8.52 / 8.51 / 8.56 ms).
+// ---- plan ----
+// Warps per CTA (one CTA per SM).
 constexpr int LMM_W = 16;
 constexpr int LMM_T = LMM_W * 32;
-constexpr int RB_W = 12;              // k_rmm_vec_b
+constexpr int RB_W = 16;              // k_rmm_vec
 constexpr int LMM_MAX_UNITS = 7;      // 16-column table units per CTA (7 x 32 KB at 256 tuples)
 constexpr int LMM_PART = LMM_MAX_UNITS * 16;  // partial sums a CTA writes
 constexpr int LMM_STEP = 64;          // rows per warp step (32 per half-warp)
 
-struct RmmChunk {
-  int g0, g1;          // range in plan order
-  int tblDoubles;      // table doubles of the chunk (even)
-  int64_t tblOff;      // offset of the chunk's tables in the P image (doubles, even)
-};
 struct LmmChunk {
   int unit0, nUnits;     // units of 16 column slots
   int nk[LMM_MAX_UNITS]; // table depth (max tuples) of each unit
@@ -60,45 +49,49 @@ struct LmmChunk {
   int cta0, nCta;        // CTA range of the launch that works on this chunk
 };
 
+// A joint slot: groups g0..gm-1 of a row with ids a0..am-1 address entry a0 + n0 * (a1 + n1 * (...)).
+constexpr int JS_MAX = 8;
+struct JointSlot {
+  int32_t n;              // groups (0: unused slot)
+  int32_t total;          // joint tuples
+  int32_t group[JS_MAX];  // device group indices
+  int32_t nv[JS_MAX];
+};
+struct JointGroup {  // the i-th group of a slot, what its table is built from
+  const double* dict;
+  const int32_t* cols;
+  int32_t nv, gCols, col, pad;
+};
+constexpr int JS_TERMS = 132;   // terms of a slot with two or more groups: at most 2 + 128
+constexpr int JOINT_UNITS = 6;  // units per chunk: their tables and two units' terms fit shared memory
 struct FastPlan {
   bool ok = false;
-  bool partial = false;  // only some groups are covered; the general kernels add the rest
-  int nG = 0;
-  // RMM
-  std::vector<RmmChunk> rchunks;
-  const uint8_t** dMaps = nullptr;  // [nG] plan order
-  int* dTblOff = nullptr;           // [nG] offset of each group's table inside its chunk (doubles)
-  int* dGroupOf = nullptr;          // [nG] plan order -> device group index
-  int64_t* dImgOff = nullptr;       // [nG] offset of each group's table in the P image (doubles)
-  int64_t pImgDoubles = 0;
-  // LMM
-  int nUnits = 0, nSlots = 0;
-  std::vector<LmmChunk> lchunks;
+  bool partial = false;      // only some groups are covered; the general kernels add the rest
+  bool uniqueCols = true;    // no column in two slots
+  int nUnits = 0, nSlots = 0;  // column slots in use; padded to whole units
+  int nU16 = 0;                // units of 16 slots
+  std::vector<LmmChunk> lchunks;       // decompress: units per CTA fixed at plan time
   LmmChunk* dLChunks = nullptr;
-  const uint8_t** dSlotMap = nullptr;  // [nSlots] column-major byte maps (plan order)
-  uint8_t* dLmmMaps = nullptr;         // the same maps interleaved for the column-per-lane kernel (see k_lmm_interleave)
-  int64_t nRB = 0;                     // 16-row blocks per column in that layout (padded to whole 64-row steps)
-  int* dSlotCol = nullptr;             // [nSlots] output column or -1
-  double* dLmmTables = nullptr;        // image of all chunk tables
   int lmmGrid = 0;
-  int maxNVals = 0;                    // deepest table: <= 16 keeps the row-per-thread kernel conflict free
+  std::vector<int> unitNk;             // table depth of each unit
+  std::vector<int64_t> unitOff;        // its table in the image (doubles)
+  int2* dUnits = nullptr;              // {offset / 16, depth} of each unit
+  const uint8_t** dSlotMap = nullptr;  // [nSlots] column-major byte maps (plan order)
+  uint8_t* dLmmMaps = nullptr;         // the same maps interleaved (see k_lmm_interleave)
+  int64_t nRB = 0;                     // 16-row blocks per slot in that layout (padded to whole 64-row steps)
+  int* dSlotCol = nullptr;             // [nSlots] output column or -1
+  int* dBareCols = nullptr;            // columns without a slot
+  int nBare = 0;
+  double* dLmmTables = nullptr;        // image of all tables
   size_t imageDoubles = 0;
-  // RMM with two groups per lookup (small dictionaries): see k_rmm_vec_f
-  bool fusedOk = false;
-  int nFused = 0;
-  std::vector<LmmChunk> fchunks;
-  LmmChunk* dFChunks = nullptr;
-  struct FusedUnit* dFUnits = nullptr;  // [slots]
-  uint8_t* dFMaps = nullptr;            // [slab16][16-row block][a | b][slot][16 ids]
-  size_t fImageDoubles = 0;
+  // X v on joint slots
+  int nJU16 = 0;                       // 0: not worth it, the column slots serve X v too
+  JointSlot* dJSlots = nullptr;        // [nJU16 * 16]
+  JointGroup* dJGroups = nullptr;      // [nJU16 * 16][JS_MAX]
+  std::vector<int> jNk;
+  int2* dJUnits = nullptr;
+  uint8_t* dJMaps = nullptr;
   std::vector<void*> allocs;
-};
-
-// One column slot of the fused RMM: ids a (group ga) and b (group gb, or none) of a row address entry (a << sh) | b.
-struct FusedUnit {
-  int32_t ga, gb;   // device group indices, gb = -1: no second group
-  int32_t sh;       // bits reserved for b
-  int32_t nva, nvb;
 };
 
 // --------------------------------------------------------------------------------------------------
@@ -174,246 +167,205 @@ __device__ __forceinline__ bool tma_reload(void* dst, const void* src, uint32_t 
   return __syncthreads_and(done != 0) != 0;
 }
 
-// --------------------------------------------------------------------------------------------------
-// RMM: P image (padded per-group tables), then the row kernel
-// --------------------------------------------------------------------------------------------------
-__global__ void k_fast_ptable(const DevGroup* __restrict__ groups, const int* __restrict__ groupOf,
-                              const int64_t* __restrict__ imgOff, int nG, const double* __restrict__ v,
-                              double* __restrict__ P) {
-  const int gi = blockIdx.x;
-  if (gi >= nG) return;
-  const DevGroup& g = groups[groupOf[gi]];
-  for (int k = threadIdx.x; k < g.nVals; k += blockDim.x) {
-    double s = 0;
-    for (int h = 0; h < g.gCols; h++) s += g.dict[(size_t)k * g.gCols + h] * v[g.cols[h]];
-    P[imgOff[gi] + k] = s;
-  }
+__device__ __forceinline__ double lds_f64(uint32_t addr) {
+  double v;
+  asm("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(addr));
+  return v;
+}
+// Address of the table entry of byte i of an id word: base + id * 128, one instruction. (Shift, mask and add took three;
+// with 16 lookups per clock and SM the issue slots were the next limit.)
+// (As asm: the intrinsic with a constant operand is turned back into byte extractions, hoisted and spilled.)
+__device__ __forceinline__ uint32_t entry_at(uint32_t w, int i, uint32_t base) {
+  uint32_t a;
+  asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(a) : "r"(w), "r"(0x80u << (8 * i)), "r"(base));
+  return a;
 }
 
-__device__ __forceinline__ uint32_t byte_x8(uint32_t w, int i) {  // (byte i of w) * 8
-  return i == 0 ? (w << 3) & 0x7F8u : (w >> (8 * i - 3)) & 0x7F8u;
-}
-
-template <int R>
-struct MapWord;
-template <> struct MapWord<16> { typedef uint4 T; };
-template <> struct MapWord<8> { typedef uint2 T; };
-template <> struct MapWord<4> { typedef uint32_t T; };
-
-// R = rows per thread (16, 8 or 4): fewer rows per thread means more threads for short matrices.
-template <int R>
-__global__ void __launch_bounds__(RMM_T)
-k_rmm_vec_u8(const uint8_t* const* __restrict__ maps, const int* __restrict__ tblOff, int g0, int g1,
-             const double* __restrict__ Pchunk, int tblDoubles, int nRows, const double* __restrict__ constRow,
-             double* __restrict__ out, int accumulate, int32_t* err) {
-  extern __shared__ __align__(128) unsigned char smraw[];
-  double* tables = (double*)smraw;
-  const int nG = g1 - g0;
-  const uint8_t** sMaps = (const uint8_t**)(smraw + (size_t)tblDoubles * 8);
-  int* sOff = (int*)(sMaps + nG);
-  __shared__ __align__(8) uint64_t mbar;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < nG; i += RMM_T) {
-    sMaps[i] = maps[g0 + i];
-    sOff[i] = tblOff[g0 + i] * 8;  // byte offset
-  }
-  if (!tma_load_to_smem(tables, Pchunk, (uint32_t)tblDoubles * 8u, &mbar)) {
-    if (tid == 0) atomicExch(err, 100);
-    return;
-  }
-  const double c0 = (constRow != nullptr && !accumulate) ? constRow[0] : 0.0;
-  constexpr int TILE = RMM_T * R;
-  const int nTiles = (nRows + TILE - 1) / TILE;
-  const unsigned char* tb = (const unsigned char*)tables;
-  typedef typename MapWord<R>::T W;
-  for (int tile = blockIdx.x; tile < nTiles; tile += gridDim.x) {
-    const int row = tile * TILE + tid * R;
-    if (row >= nRows) continue;
-    if (row + R <= nRows) {
-      double acc[R];
-#pragma unroll
-      for (int i = 0; i < R; i++) acc[i] = c0;
-#pragma unroll(R == 16 ? 8 : 16)
-      for (int g = 0; g < nG; g++) {
-        const W w = __ldg((const W*)(sMaps[g] + row));
-        const unsigned char* T = tb + sOff[g];
-        uint32_t ww[4];
-        if constexpr (R == 16) { ww[0] = w.x; ww[1] = w.y; ww[2] = w.z; ww[3] = w.w; }
-        else if constexpr (R == 8) { ww[0] = w.x; ww[1] = w.y; }
-        else { ww[0] = w; }
-#pragma unroll
-        for (int i = 0; i < R; i++) acc[i] += *(const double*)(T + byte_x8(ww[i >> 2], i & 3));
-      }
-      if (accumulate) {
-#pragma unroll
-        for (int i = 0; i < R; i++) atomicAdd(out + row + i, acc[i]);
-      } else {
-        double2* o = (double2*)(out + row);
-#pragma unroll
-        for (int i = 0; i < R / 2; i++) o[i] = make_double2(acc[2 * i], acc[2 * i + 1]);
-      }
-    } else {  // ragged last rows
-      for (int r = row; r < nRows; r++) {
-        double a = c0;
-        for (int g = 0; g < nG; g++) a += *(const double*)(tb + sOff[g] + 8 * (int)sMaps[g][r]);
-        if (accumulate) atomicAdd(out + r, a);
-        else out[r] = a;
-      }
-    }
-  }
-}
-
-// --------------------------------------------------------------------------------------------------
-// LMM: column-per-lane kernel
-// --------------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t byte_x128(uint32_t w, int i) {  // (byte i of w) << 7
   return i == 0 ? (w << 7) & 0x7F80u : (i == 3 ? (w >> 17) & 0x7F80u : (w >> (8 * i - 7)) & 0x7F80u);
 }
 
-template <int NU>
-__device__ __forceinline__ void lmm_cells(const uint4 (&m)[NU][2], int sub, const double (&yv)[16],
-                                          const unsigned char* const (&tbase)[NU], double (&acc)[NU]) {
-#pragma unroll
-  for (int u = 0; u < NU; u++) {
-    const uint4 w = m[u][sub];
-    const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-    const unsigned char* T = tbase[u];
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-      const double t = *(const double*)(T + byte_x128(ww[i >> 2], i & 3));
-      acc[u] = fma(yv[i], t, acc[u]);
+constexpr int VSTEP = 32;  // rows of a warp step: one 16-row block per half-warp
+
+// --------------------------------------------------------------------------------------------------
+// LMM: t(y) X. The grid is cut into chunks of U units; a chunk's CTAs split the rows. y is loaded with 128-bit loads
+// that are uniform per half-warp and multiplied into NU accumulators per lane. The CTA's partial sums go to `partial`.
+// k_lmm_final adds them up in a fixed order, a CTA per 16 columns, resident before the last CTA ends (programmatic
+// dependent launch), and stores the result: nothing to clear beforehand. (Left to the last CTA of a chunk, without a second
+// launch: 18.2 instead of 14.3 us for the chain on 50,000 x 100, 17.6 instead of 14.2 for t(y) X on 250,000 x 40 -- one
+// CTA reads 148 partial rows too slowly.)
+// Measured (10M x 200, 256 values): 644 us, 3.2 TB/s; the one-row-step form before, with three instructions per address,
+// a clear, a separately launched sum, 670 us. 100,000 x 500: 36.9 -> 30.5 us, 5000 x 500: 15.4 -> 10.4.
+// --------------------------------------------------------------------------------------------------
+struct LmmArgs {
+  const int2* units;           // {table offset / 16, depth}
+  const uint8_t* imaps;
+  int64_t nRB;
+  const double* tables;
+  const int* slotCol;
+  const double* y;
+  int nRows, nU16, U, nChunks;
+  int ctaFull, ctaLast;        // CTAs of a chunk of U units, of the last chunk
+  int64_t stepBegin, stepEnd;  // warp steps of this launch
+  double* partial;             // [parts][gridDim.x][LMM_PART + 1] (the last: sum of y)
+  int part, parts;             // this launch's part; parts > 0: it is the last one, k_lmm_final follows
+  const double* constV;        // null: none
+  const int* bareCols;
+  int nBare;
+  int addTo;                   // columns may repeat: add with atomics to a cleared result
+  double* out;
+  int32_t* err;
+};
+
+// Adds up the partial sums of unit `u` of a chunk, by one CTA of LMM_T threads: 32 groups of 16 lanes (a lane per
+// column) take every 32nd partial sum, then a tree over the groups: a fixed order.
+constexpr int LMM_FIN = (LMM_T / 16) * 17 + LMM_T / 32;  // doubles of shared memory it needs
+__device__ __forceinline__ void lmm_finish(const LmmArgs& A, int chunk, int cta0, int nCta, int grid, int u, bool withBare,
+                                           double* sm) {
+  double(*red)[17] = (double(*)[17])sm;
+  double* yred = sm + (LMM_T / 16) * 17;
+  const int tid = threadIdx.x, col = tid & 15, sub = tid >> 4;
+  const int n = A.parts * nCta;
+  double s = 0.0, ys = 0.0;
+  for (int i = sub; i < n; i += LMM_T / 16) {
+    const int p = i / nCta, b = i - p * nCta;
+    s += __ldcg(A.partial + ((size_t)p * grid + cta0 + b) * (LMM_PART + 1) + u * 16 + col);
+  }
+  red[sub][col] = s;
+  if (A.constV) {
+    for (int i = tid; i < n; i += LMM_T) {
+      const int p = i / nCta, b = i - p * nCta;
+      ys += __ldcg(A.partial + ((size_t)p * grid + cta0 + b) * (LMM_PART + 1) + LMM_PART);
+    }
+    for (int d = 16; d; d >>= 1) ys += __shfl_xor_sync(0xffffffffu, ys, d);
+    if ((tid & 31) == 0) yred[tid >> 5] = ys;
+  }
+  __syncthreads();
+  for (int h = LMM_T / 32; h; h >>= 1) {
+    if (sub < h) red[sub][col] += red[sub + h][col];
+    __syncthreads();
+  }
+  if (A.constV) {
+    ys = 0.0;
+    for (int w = 0; w < LMM_T / 32; w++) ys += yred[w];
+  }
+  if (tid < 16) {
+    const int c = A.slotCol[(chunk * A.U + u) * 16 + tid];
+    if (c >= 0) {
+      if (A.addTo) atomicAdd(&A.out[c], red[0][tid]);
+      else A.out[c] = A.constV ? fma(ys, A.constV[c], red[0][tid]) : red[0][tid];
     }
   }
+  if (withBare && chunk == 0 && !A.addTo)  // columns of constant groups, and those the general kernels will add to
+    for (int i = tid; i < A.nBare; i += LMM_T) {
+      const int c = A.bareCols[i];
+      A.out[c] = A.constV ? ys * A.constV[c] : 0.0;
+    }
 }
 
-// partial: [gridDim.x][LMM_PART]
+// grid: units
+__global__ void __launch_bounds__(LMM_T) k_lmm_final(const __grid_constant__ LmmArgs A, int grid) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int chunk = blockIdx.x / A.U, u = blockIdx.x - chunk * A.U;
+  __shared__ double sm[LMM_FIN];
+  lmm_finish(A, chunk, chunk * A.ctaFull, chunk == A.nChunks - 1 ? A.ctaLast : A.ctaFull, grid, u, u == 0, sm);
+}
+
 template <int NU>
-__device__ __forceinline__ void lmm_vec_body(const LmmChunk& ch, const uint8_t* __restrict__ imaps, int64_t nRB,
-                                             const double* __restrict__ tablesImg, const double* __restrict__ y,
-                                             int nRows, int64_t stepBegin, int64_t stepEnd,
-                                             double* __restrict__ partial, unsigned char* smraw, uint64_t* mbar,
-                                             int32_t* err) {
+__device__ __forceinline__ void lmm_vec_body(const LmmArgs& A, int chunk, int cta0, int nCta, unsigned char* smraw, uint64_t* mbar) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int slot = lane & 15, half = lane >> 4;
-  if (!tma_load_to_smem(smraw, tablesImg + ch.tblOff, (uint32_t)ch.tblDoubles * 8u, mbar)) {
-    // the tables never arrived: flag it, and make the failure visible in the result as well (the final kernel sums
-    // this row whatever happens, and a device-buffer caller only sees the error word at its next cla_stats_get)
-    if (tid == 0) atomicExch(err, 101);
-    for (int u = tid; u < NU * 16; u += LMM_T) partial[(size_t)blockIdx.x * LMM_PART + u] = __longlong_as_double(0x7ff8000000000000ll);
-    return;
-  }
-  // table base of each unit for this lane (slot offset folded in), and this lane's map pointers
-  const unsigned char* tbase[NU];
-  const uint8_t* mp[NU];
-  {
-    size_t off = 0;
+  const int unit0 = chunk * A.U;
+  double* mine = A.partial + ((size_t)A.part * gridDim.x + blockIdx.x) * (LMM_PART + 1);
+  const int2 first = A.units[unit0], last = A.units[unit0 + NU - 1];
+  const uint32_t bytes = (uint32_t)(last.x + last.y - first.x) * 128u;
+  bool ok = tma_load_to_smem(smraw, A.tables + (size_t)first.x * 16, bytes, mbar);
+  if (!ok) {
+    // the tables never arrived: flag it, and make the failure visible in the result as well (a device-buffer caller
+    // only sees the error word at its next cla_stats_get)
+    if (tid == 0) atomicExch(A.err, 101);
+    for (int u = tid; u <= LMM_PART; u += LMM_T) mine[u] = __longlong_as_double(0x7ff8000000000000ll);
+  } else {
+    uint32_t tb[NU];
 #pragma unroll
-    for (int u = 0; u < NU; u++) {
-      tbase[u] = smraw + off + slot * 8;
-      off += (size_t)ch.nk[u] * 128;
-      mp[u] = imaps + (size_t)(ch.unit0 + u) * nRB * 256 + slot * 16;
+    for (int u = 0; u < NU; u++) tb[u] = smem_u32(smraw) + (uint32_t)(A.units[unit0 + u].x - first.x) * 128u + slot * 8;
+    const uint8_t* mp = A.imaps + (size_t)unit0 * A.nRB * 256 + half * 256 + slot * 16;
+    const size_t ustr = (size_t)A.nRB * 256;
+    double acc[NU], ysum = 0.0;
+#pragma unroll
+    for (int u = 0; u < NU; u++) acc[u] = 0.0;
+    const int64_t nSteps = A.stepEnd - A.stepBegin;
+    const int c = blockIdx.x - cta0;
+    const int64_t s0 = A.stepBegin + nSteps * c / nCta, s1 = A.stepBegin + nSteps * (c + 1) / nCta;
+    uint4 m[NU];
+    int64_t st = s0 + warp;
+    if (st < s1) {
+#pragma unroll
+      for (int u = 0; u < NU; u++) m[u] = __ldg((const uint4*)(mp + u * ustr + st * 512));
     }
-  }
-  double acc[NU];
-#pragma unroll
-  for (int u = 0; u < NU; u++) acc[u] = 0.0;
-
-  // rows of this CTA: contiguous range of 64-row steps
-  const int ctaInChunk = blockIdx.x - ch.cta0;
-  const int64_t nSteps = stepEnd - stepBegin;  // this launch covers the 64-row steps [stepBegin, stepEnd)
-  const int64_t s0 = stepBegin + nSteps * ctaInChunk / ch.nCta, s1 = stepBegin + nSteps * (ctaInChunk + 1) / ch.nCta;
-  for (int64_t st = s0 + warp; st < s1; st += LMM_W) {
-    const int64_t r0 = st * LMM_STEP + half * 32;
-    if (st * LMM_STEP + LMM_STEP <= nRows) {
-      uint4 m[NU][2];
-#pragma unroll
-      for (int u = 0; u < NU; u++) {
-        const uint8_t* src = mp[u] + (r0 >> 4) * 256;
-        m[u][0] = __ldg((const uint4*)src);
-        m[u][1] = __ldg((const uint4*)(src + 256));
-      }
-#pragma unroll
-      for (int sub = 0; sub < 2; sub++) {
+    for (; st < s1; st += LMM_W) {
+      const int64_t r0 = st * VSTEP + half * 16, nxt = st + LMM_W;
+      if (st * VSTEP + VSTEP <= A.nRows) {
         double yv[16];
-        const double2* ys = (const double2*)(y + r0 + sub * 16);
+        const double2* ys = (const double2*)(A.y + r0);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
           const double2 t = __ldg(ys + i);
           yv[2 * i] = t.x;
           yv[2 * i + 1] = t.y;
         }
-        lmm_cells<NU>(m, sub, yv, tbase, acc);
-      }
-    } else {  // ragged last step
-      for (int64_t r = r0; r < min((int64_t)nRows, r0 + 32); r++) {
-        const double yy = y[r];
+        if (A.constV)
 #pragma unroll
-        for (int u = 0; u < NU; u++)
-          acc[u] = fma(yy, *(const double*)(tbase[u] + 128 * (int)mp[u][(r >> 4) * 256 + (r & 15)]), acc[u]);
+          for (int i = 0; i < 16; i++) ysum += yv[i];
+#pragma unroll
+        for (int u = 0; u < NU; u++) {
+          const uint4 w = m[u];
+          if (nxt < s1) m[u] = __ldg((const uint4*)(mp + u * ustr + nxt * 512));  // in flight until the next step
+          const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int i = 0; i < 16; i++) acc[u] = fma(yv[i], lds_f64(entry_at(ww[i >> 2], i & 3, tb[u])), acc[u]);
+        }
+      } else {  // ragged last step
+        for (int i = 0; i < 16 && r0 + i < A.nRows; i++) {
+          const double yy = A.y[r0 + i];
+          ysum += yy;
+#pragma unroll
+          for (int u = 0; u < NU; u++) acc[u] = fma(yy, lds_f64(tb[u] + 128u * mp[u * ustr + st * 512 + i]), acc[u]);
+        }
       }
     }
-  }
-  // combine the two half-warps (same column slots, different rows), then the warps through shared memory
-  __syncthreads();  // tables no longer needed
-  double* red = (double*)smraw;  // [LMM_W][NU*16]
+    // combine the two half-warps (same slots, different rows), then the warps through shared memory
+    __syncthreads();  // tables no longer needed
+    double* red = (double*)smraw;  // [LMM_W][NU * 16 + 1]
 #pragma unroll
-  for (int u = 0; u < NU; u++) {
-    double a = acc[u];
-    a += __shfl_xor_sync(0xffffffffu, a, 16);
-    if (half == 0) red[warp * (NU * 16) + u * 16 + slot] = a;
-  }
-  __syncthreads();
-  for (int u = tid; u < NU * 16; u += LMM_T) {
-    double s = 0;
-    for (int w = 0; w < LMM_W; w++) s += red[w * (NU * 16) + u];
-    partial[(size_t)blockIdx.x * LMM_PART + u] = s;
+    for (int u = 0; u < NU; u++) {
+      double a = acc[u];
+      a += __shfl_xor_sync(0xffffffffu, a, 16);
+      if (half == 0) red[warp * (NU * 16 + 1) + u * 16 + slot] = a;
+    }
+    ysum += __shfl_xor_sync(0xffffffffu, ysum, 16);
+    if (lane == 0) red[warp * (NU * 16 + 1) + NU * 16] = ysum;
+    __syncthreads();
+    for (int u = tid; u <= NU * 16; u += LMM_T) {
+      double s = 0;
+      for (int w = 0; w < LMM_W; w++) s += red[w * (NU * 16 + 1) + u];
+      mine[u < NU * 16 ? u : LMM_PART] = s;
+    }
   }
 }
 
-__global__ void __launch_bounds__(LMM_T, 1)
-k_lmm_vec_u8(const LmmChunk* __restrict__ chunks, int nChunks, const uint8_t* __restrict__ imaps, int64_t nRB,
-             const double* __restrict__ tablesImg, const double* __restrict__ y, int nRows, int64_t stepBegin,
-             int64_t stepEnd, double* __restrict__ partial, int32_t* err) {
+__global__ void __launch_bounds__(LMM_T, 1) k_lmm_vec(const __grid_constant__ LmmArgs A) {
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ __align__(8) uint64_t mbar;
-  __shared__ LmmChunk ch;
-  if (threadIdx.x == 0) {
-    int c = 0;
-    while (c + 1 < nChunks && (int)blockIdx.x >= chunks[c].cta0 + chunks[c].nCta) c++;
-    ch = chunks[c];
-  }
-  __syncthreads();
-#define LMM_CASE(N) case N: lmm_vec_body<N>(ch, imaps, nRB, tablesImg, y, nRows, stepBegin, stepEnd, partial, smraw, &mbar, err); break;
-  switch (ch.nUnits) {
+  const int chunk = min((int)blockIdx.x / A.ctaFull, A.nChunks - 1), cta0 = chunk * A.ctaFull;
+  const int nCta = chunk == A.nChunks - 1 ? A.ctaLast : A.ctaFull;
+  if (A.parts) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#define LMM_CASE(N) case N: lmm_vec_body<N>(A, chunk, cta0, nCta, smraw, &mbar); break;
+  switch (min(A.U, A.nU16 - chunk * A.U)) {
     LMM_CASE(1) LMM_CASE(2) LMM_CASE(3) LMM_CASE(4) LMM_CASE(5) LMM_CASE(6)
-    default: lmm_vec_body<7>(ch, imaps, nRB, tablesImg, y, nRows, stepBegin, stepEnd, partial, smraw, &mbar, err); break;
+    default: lmm_vec_body<7>(A, chunk, cta0, nCta, smraw, &mbar); break;
   }
 #undef LMM_CASE
-}
-
-// out[col] += sum over the chunk's CTAs of partial[cta][slot]. A warp per column slot: lane l adds the partial sums of
-// CTAs l, l + 32, ... (row ranges that were launched separately one after the other), then a shuffle tree adds the
-// 32 lanes -- a fixed order for a given launch geometry, so the result is reproducible, and the 80 or so partial
-// sums of a column are no longer one chain of dependent loads.
-__global__ void k_lmm_vec_final(const LmmChunk* __restrict__ chunks, int nChunks, const int* __restrict__ slotCol,
-                                const double* __restrict__ partial, double* __restrict__ out, int nParts, int gridPerPart) {
-  const int c = blockIdx.x;
-  if (c >= nChunks) return;
-  const LmmChunk ch = chunks[c];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nWarps = (blockDim.x >> 5) * gridDim.y;
-  const int n = nParts * ch.nCta;
-  for (int u = blockIdx.y * (blockDim.x >> 5) + warp; u < ch.nUnits * 16; u += nWarps) {  // gridDim.y CTAs per chunk
-    const int col = slotCol[ch.unit0 * 16 + u];
-    if (col < 0) continue;
-    double s = 0;
-    for (int i = lane; i < n; i += 32) {
-      const int part = i / ch.nCta, b = i - part * ch.nCta;
-      s += partial[((size_t)part * gridPerPart + ch.cta0 + b) * LMM_PART + u];
-    }
-#pragma unroll
-    for (int d = 16; d; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    if (lane == 0) atomicAdd(&out[col], s);
-  }
 }
 
 // --------------------------------------------------------------------------------------------------
@@ -672,194 +624,102 @@ k_decomp_fast(const LmmChunk* __restrict__ chunks, int nChunks, const uint8_t* _
 }
 
 // --------------------------------------------------------------------------------------------------
-// RMM, column-per-lane variant (tables of any depth up to 256 without bank conflicts).
-// Same slabs, interleaved maps and table layout as k_lmm_vec_u8; the table of slot s holds
-// D[:, j] * v[col] (k_rmm_b_tables), so summing a row's lookups over all slots gives the row of X v.
-// A CTA owns a contiguous range of rows and walks the column chunks one after the other, reloading the tables;
-// the first chunk stores its partial sums, later chunks add to them (the CTA owns the rows: no atomics, and the
-// summation order is fixed). Within a chunk each lane accumulates 16 rows x its column slots, then a
-// reduce-scatter over the 16 lanes of the half-warp (15 shuffles) leaves lane s with the sum of row s.
+// RMM: X v. A CTA owns a contiguous range of rows and walks chunks of up to seven units one after the other, reloading
+// the tables; the first chunk stores its partial sums, later chunks add to them (the CTA owns the rows: no atomics,
+// one summation order). Within a chunk a lane accumulates 16 rows over its slots; the sums over the 16 lanes of the
+// half-warps are then formed by the FP64 tensor core, which is idle otherwise: ten m8n8k4 products with 0 / 1 matrices
+// per eight rows of both half-warps. (As shuffles the reduction was 30 of 280 wavefronts of the data pipe that bounds this kernel and a
+// third of its instructions.) A product with 0 would carry an Inf or NaN of one row into its neighbours, so a warp that
+// sees a non-finite result forms its sums again with shuffles.
 // --------------------------------------------------------------------------------------------------
-__global__ void k_rmm_b_tables(const LmmChunk* __restrict__ chunks, const int* __restrict__ slotCol,
-                               const double* __restrict__ T, const double* __restrict__ v, double* __restrict__ P) {
-  const LmmChunk ch = chunks[blockIdx.x];
-  int base = 0;
-  for (int u = 0; u < ch.nUnits; u++) {
-    const int n = ch.nk[u] * 16;
-    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < n; e += gridDim.y * blockDim.x) {  // gridDim.y CTAs per chunk
-      const int col = slotCol[(ch.unit0 + u) * 16 + (e & 15)];
-      P[ch.tblOff + base + e] = col >= 0 ? T[ch.tblOff + base + e] * v[col] : 0.0;
-    }
-    base += n;
-  }
+__device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
 }
 
-template <int NU>
-__device__ __forceinline__ void rmm_b_chunk(const LmmChunk& ch, const uint8_t* __restrict__ imaps, int64_t nRB,
-                                            int64_t s0, int64_t s1, int nRows, double init, bool first,
-                                            double* __restrict__ out, const unsigned char* smraw) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int slot = lane & 15, half = lane >> 4;
-  const unsigned char* tbase[NU];
-  const uint8_t* mp[NU];
-  {
-    size_t off = 0;
+// 1.0 where a == b, else 0.0; volatile: formed where it is used (kept in registers across the main loop, the nine
+// coefficients below pushed the kernel into spilling).
+__device__ __forceinline__ double one_if(int a, int b) {
+  double r;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, %2;\n\tselp.f64 %0, 0d3FF0000000000000, 0d0000000000000000, p;\n\t}" : "=d"(r) : "r"(a), "r"(b));
+  return r;
+}
+// Sums acc[i] over the 16 lanes of each half-warp: lane 4 g returns the sums of row g of the lower half-warp (s0) and of
+// the upper one (s1); the other lanes return nothing of use.
+__device__ __forceinline__ void half_warp_sums(const double (&acc)[8], double& s0, double& s1) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  // C[m][n] = sum over the four lanes of quad n of acc[m]: B = acc[i], A_i = 1 in row i (two chains of four products)
+  double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll
-    for (int u = 0; u < NU; u++) {
-      tbase[u] = smraw + off + slot * 8;
-      off += (size_t)ch.nk[u] * 128;
-      mp[u] = imaps + (size_t)(ch.unit0 + u) * nRB * 256 + slot * 16;
-    }
+  for (int i = 0; i < 4; i++) {
+    dmma884(c[0][0], c[0][1], one_if(g, i), acc[i]);
+    dmma884(c[1][0], c[1][1], one_if(g, i + 4), acc[i + 4]);
   }
-  for (int64_t st = s0 + warp; st < s1; st += RB_W) {
-    const int64_t r0 = st * LMM_STEP + half * 32;
-    uint4 m[NU][2];
-#pragma unroll
-    for (int u = 0; u < NU; u++) {
-      const uint8_t* src = mp[u] + (r0 >> 4) * 256;
-      m[u][0] = __ldg((const uint4*)src);
-      m[u][1] = __ldg((const uint4*)(src + 256));
-    }
-#pragma unroll
-    for (int sub = 0; sub < 2; sub++) {
-      double acc[16];
-#pragma unroll
-      for (int i = 0; i < 16; i++) acc[i] = 0.0;
-#pragma unroll
-      for (int u = 0; u < NU; u++) {
-        const uint4 w = m[u][sub];
-        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-        const unsigned char* T = tbase[u];
-#pragma unroll
-        for (int i = 0; i < 16; i++) acc[i] += *(const double*)(T + byte_x128(ww[i >> 2], i & 3));
-      }
-      // reduce-scatter over the half-warp: after the stage with distance d, a lane keeps the rows whose bit d
-      // equals its own slot bit
-#pragma unroll
-      for (int d = 8; d >= 1; d >>= 1) {
-        const bool up = (slot & d) != 0;
-#pragma unroll
-        for (int i = 0; i < d; i++) {
-          const double lo = acc[i], hi = acc[i + d];
-          const double recv = __shfl_xor_sync(0xffffffffu, up ? lo : hi, d);
-          acc[i] = (up ? hi : lo) + recv;
-        }
-      }
-      const int64_t row = r0 + sub * 16 + slot;
-      if (row < nRows) out[row] = first ? acc[0] + init : out[row] + acc[0];
-    }
-  }
+  // quads 0..3 are the lower half-warp: sum C over n into column 0 for them and into column 1 for the others
+  const double sel = one_if(g, t >> 1);
+  s0 = s1 = 0.0;
+  dmma884(s0, s1, c[0][0] + c[1][0], sel);
+  dmma884(s0, s1, c[0][1] + c[1][1], sel);
 }
 
-__global__ void __launch_bounds__(RB_W * 32, 1)
-k_rmm_vec_b(const LmmChunk* __restrict__ chunks, int nChunks, const uint8_t* __restrict__ imaps, int64_t nRB,
-            const double* __restrict__ P, int nRows, const double* __restrict__ constRow, double* __restrict__ out,
-            int32_t* err) {
-  extern __shared__ __align__(128) unsigned char smraw[];
-  __shared__ __align__(8) uint64_t mbar;
-  __shared__ LmmChunk ch;
-  const int64_t nSteps = ((int64_t)nRows + LMM_STEP - 1) / LMM_STEP;
-  const int64_t s0 = nSteps * blockIdx.x / gridDim.x, s1 = nSteps * (blockIdx.x + 1) / gridDim.x;
-  const double init = constRow ? constRow[0] : 0.0;
-  tma_barrier_init(&mbar);
-  for (int c = 0; c < nChunks; c++) {
-    __syncthreads();  // everyone is done with the previous chunk's tables and with `ch`
-    if (threadIdx.x == 0) ch = chunks[c];
-    __syncthreads();
-    if (!tma_reload(smraw, P + ch.tblOff, (uint32_t)ch.tblDoubles * 8u, &mbar, (uint32_t)(c & 1))) {
-      if (threadIdx.x == 0) atomicExch(err, 102);
-      return;
+struct RmmArgs {
+  const int2* units;       // {table offset / 16, depth}
+  const uint8_t* imaps;
+  int64_t nRB;
+  const double* tables;    // column slots
+  const int* slotCol;
+  const JointSlot* joint;  // joint slots
+  const JointGroup* jointGroups;
+  const double* v;
+  const double* constV;    // null: none
+  int nCols;
+  int nRows, nU16;
+  const double* rowScale;  // null, or a factor per row applied at the end
+  double* out;
+  int32_t* err;
+};
+
+// The sums of step `st` again, for a warp that saw an Inf or NaN: every row by itself, with shuffles. Lane 4 g + t, t < 2,
+// returns rows 8 t + g of the two blocks.
+__device__ __noinline__ double2 rmm_step_by_rows(const uint8_t* mp, size_t ustr, const int2* units, const int* slotCol,
+                                                 const double* v, int nu, uint32_t table0) {
+  const int lane = threadIdx.x & 31, slot = lane & 15, g = lane >> 2, t = lane & 3;
+  double2 r = make_double2(0.0, 0.0);
+  for (int i = 0; i < 16; i++) {
+    double a = 0.0;
+    for (int u = 0; u < nu; u++) {
+      const int col = slotCol[u * 16 + slot];
+      if (col >= 0)
+        a = fma(lds_f64(table0 + (uint32_t)(units[u].x - units[0].x) * 128u + slot * 8 + 128u * mp[u * ustr + i]), v[col], a);
     }
-#define RB_CASE(N) case N: rmm_b_chunk<N>(ch, imaps, nRB, s0, s1, nRows, init, c == 0, out, smraw); break;
-    switch (ch.nUnits) {
-      RB_CASE(1) RB_CASE(2) RB_CASE(3) RB_CASE(4) RB_CASE(5) RB_CASE(6)
-      default: rmm_b_chunk<7>(ch, imaps, nRB, s0, s1, nRows, init, c == 0, out, smraw); break;
-    }
-#undef RB_CASE
+    for (int d = 1; d < 16; d <<= 1) a += __shfl_xor_sync(0xffffffffu, a, d);
+    const double other = __shfl_xor_sync(0xffffffffu, a, 16);
+    if (i == (t & 1) * 8 + g) r = lane < 16 ? make_double2(a, other) : make_double2(other, a);
   }
+  return r;
 }
 
-// --------------------------------------------------------------------------------------------------
-// RMM with two groups per dictionary read. When dictionaries are small, two groups g and h share one column
-// slot: the slot's table holds P_g[a] + P_h[b] at entry (a << sh) | b (at most 256 entries), so one 8-byte read
-// serves two cells -- the lookup bound of 16 reads per clock per SM then allows 32 cells per clock. The maps stay
-// as registered; the kernel reads both groups' ids ([slab16][16-row block][a | b][slot][16 ids], one 128-bit load
-// each) and combines them with one multiply-add per four rows. Otherwise identical to k_rmm_vec_b.
-// --------------------------------------------------------------------------------------------------
-__global__ void k_rmm_f_tables(const DevGroup* __restrict__ groups, const LmmChunk* __restrict__ chunks,
-                               const FusedUnit* __restrict__ units, const double* __restrict__ v,
-                               double* __restrict__ P) {
-  const LmmChunk ch = chunks[blockIdx.x];
-  int base = 0;
-  for (int q = 0; q < ch.nUnits; q++) {
-    const int n = ch.nk[q] * 16;
-    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < n; e += gridDim.y * blockDim.x) {  // gridDim.y CTAs per chunk
-      const FusedUnit u = units[(ch.unit0 + q) * 16 + (e & 15)];
-      const int k = e >> 4;
-      double val = 0.0;
-      if (u.ga >= 0) {
-        const int a = k >> u.sh, b = k & ((1 << u.sh) - 1);
-        if (a < u.nva && (u.gb < 0 ? b == 0 : b < u.nvb)) {
-          const DevGroup& ga = groups[u.ga];
-          for (int h = 0; h < ga.gCols; h++) val += ga.dict[(size_t)a * ga.gCols + h] * v[ga.cols[h]];
-          if (u.gb >= 0) {
-            const DevGroup& gb = groups[u.gb];
-            double vb = 0.0;
-            for (int h = 0; h < gb.gCols; h++) vb += gb.dict[(size_t)b * gb.gCols + h] * v[gb.cols[h]];
-            val += vb;
-          }
-        }
-      }
-      P[ch.tblOff + base + e] = val;
-    }
-    base += n;
-  }
-}
-
-template <int NU>
-__device__ __forceinline__ void rmm_f_chunk(const LmmChunk& ch, const FusedUnit* __restrict__ units,
-                                            const uint8_t* __restrict__ fmaps, int64_t nRB, int64_t s0, int64_t s1,
-                                            int nRows, double init, bool first, double* __restrict__ out,
-                                            const unsigned char* smraw) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int slot = lane & 15, half = lane >> 4;
-  const unsigned char* tbase[NU];
-  const uint8_t* mp[NU];
-  uint32_t mul[NU];  // 1 << sh of this lane's slot
-  {
-    size_t off = 0;
-#pragma unroll
-    for (int u = 0; u < NU; u++) {
-      tbase[u] = smraw + off + slot * 8;
-      off += (size_t)ch.nk[u] * 128;
-      mp[u] = fmaps + (size_t)(ch.unit0 + u) * nRB * 512 + slot * 16;
-      mul[u] = 1u << units[(ch.unit0 + u) * 16 + slot].sh;
-    }
-  }
-  // The ids of the next 16 rows are loaded before the current 16 are looked up (two register buffers): with a few
-  // steps per warp on a short matrix, waiting for each load before issuing the next was most of the run time.
-  auto load_ids = [&](int64_t st, int sub, uint4 (&ma)[NU], uint4 (&mb)[NU]) {
-    const int64_t rb = ((st * LMM_STEP + half * 32) >> 4) + sub;
-#pragma unroll
-    for (int u = 0; u < NU; u++) {
-      const uint8_t* src = mp[u] + rb * 512;
-      ma[u] = __ldg((const uint4*)src);          // 16 lanes x 16 bytes: two full 128-byte lines per half-warp
-      mb[u] = __ldg((const uint4*)(src + 256));
-    }
-  };
-  auto lookup_rows = [&](int64_t st, int sub, const uint4 (&ma)[NU], const uint4 (&mb)[NU]) {
+// Row sums of one step from its id words: lane 4 g + t, t < 2, returns those of rows 8 t + g of the two half-warps' blocks.
+// JOINT: the terms are the table entries themselves, and the reduction is one of shuffles -- with four units or so per
+// step the products with 0 / 1 matrices would keep the FP64 pipe as long as the lookups take (1M x 100, 16 values:
+// 43.6 us with products).
+template <int NU, bool JOINT, int UNROLL_ROWS>
+__device__ __forceinline__ void step_sums(const uint4 (&m)[NU], const uint32_t (&tb)[NU], const double (&v)[NU], double& r0, double& r1) {
+  const int lane = threadIdx.x & 31;
+  if constexpr (JOINT) {
+    const int slot = lane & 15;
     double acc[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) acc[i] = 0.0;
 #pragma unroll
     for (int u = 0; u < NU; u++) {
-      // ids stay below 256 after the shift, so the four bytes of a word never carry into each other
-      const uint32_t ww[4] = {ma[u].x * mul[u] + mb[u].x, ma[u].y * mul[u] + mb[u].y, ma[u].z * mul[u] + mb[u].z,
-                              ma[u].w * mul[u] + mb[u].w};
-      const unsigned char* T = tbase[u];
+      const uint32_t ww[4] = {m[u].x, m[u].y, m[u].z, m[u].w};
 #pragma unroll
-      for (int i = 0; i < 16; i++) acc[i] += *(const double*)(T + byte_x128(ww[i >> 2], i & 3));
+      for (int i = 0; i < 16; i++) acc[i] += lds_f64(entry_at(ww[i >> 2], i & 3, tb[u]));
     }
+    // reduce-scatter over the half-warp: after the stage with distance d, a lane keeps the rows whose bit d equals its
+    // own slot bit
 #pragma unroll
     for (int d = 8; d >= 1; d >>= 1) {
       const bool up = (slot & d) != 0;
@@ -870,74 +730,337 @@ __device__ __forceinline__ void rmm_f_chunk(const LmmChunk& ch, const FusedUnit*
         acc[i] = (up ? hi : lo) + recv;
       }
     }
-    const int64_t row = st * LMM_STEP + half * 32 + sub * 16 + slot;
-    if (row < nRows) out[row] = first ? acc[0] + init : out[row] + acc[0];
-  };
-  uint4 a0[NU], b0[NU], a1[NU], b1[NU];
-  int64_t st = s0 + warp;
-  if (st < s1) load_ids(st, 0, a0, b0);
-  for (; st < s1; st += LMM_W) {
-    load_ids(st, 1, a1, b1);
-    lookup_rows(st, 0, a0, b0);
-    if (st + LMM_W < s1) load_ids(st + LMM_W, 0, a0, b0);
-    lookup_rows(st, 1, a1, b1);
-  }
-}
-
-__global__ void __launch_bounds__(LMM_T, 1)
-k_rmm_vec_f(const LmmChunk* __restrict__ chunks, int nChunks, const FusedUnit* __restrict__ units,
-            const uint8_t* __restrict__ fmaps, int64_t nRB, const double* __restrict__ P, int nRows,
-            const double* __restrict__ constRow, double* __restrict__ out, int32_t* err) {
-  extern __shared__ __align__(128) unsigned char smraw[];
-  __shared__ __align__(8) uint64_t mbar;
-  __shared__ LmmChunk ch;
-  const int64_t nSteps = ((int64_t)nRows + LMM_STEP - 1) / LMM_STEP;
-  const int64_t s0 = nSteps * blockIdx.x / gridDim.x, s1 = nSteps * (blockIdx.x + 1) / gridDim.x;
-  const double init = constRow ? constRow[0] : 0.0;
-  tma_barrier_init(&mbar);
-  for (int c = 0; c < nChunks; c++) {
-    __syncthreads();
-    if (threadIdx.x == 0) ch = chunks[c];
-    __syncthreads();
-    if (!tma_reload(smraw, P + ch.tblOff, (uint32_t)ch.tblDoubles * 8u, &mbar, (uint32_t)(c & 1))) {
-      if (threadIdx.x == 0) atomicExch(err, 103);
-      return;
-    }
-    switch (ch.nUnits) {
-      case 1: rmm_f_chunk<1>(ch, units, fmaps, nRB, s0, s1, nRows, init, c == 0, out, smraw); break;
-      case 2: rmm_f_chunk<2>(ch, units, fmaps, nRB, s0, s1, nRows, init, c == 0, out, smraw); break;
-      case 3: rmm_f_chunk<3>(ch, units, fmaps, nRB, s0, s1, nRows, init, c == 0, out, smraw); break;
-      default: rmm_f_chunk<4>(ch, units, fmaps, nRB, s0, s1, nRows, init, c == 0, out, smraw); break;
-    }
-  }
-}
-
-// [slab16][16-row block][a | b][slot][16 ids]: a half-warp's load of the a ids (and of the b ids) is 256 contiguous bytes
-__global__ void k_rmm_f_interleave(const uint8_t* const* __restrict__ mapA, const uint8_t* const* __restrict__ mapB,
-                                   int nSlots, int nRows, int64_t nRB, uint8_t* __restrict__ out) {
-  const int64_t total = (int64_t)nSlots * nRB * 2;
-  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
-    const int slot = (int)(g & 15);
-    const int which = (int)((g >> 4) & 1);
-    const int64_t rb = (g >> 5) % nRB;
-    const int64_t slab = (g >> 5) / nRB;
-    const int unit = (int)slab * 16 + slot;
-    const uint8_t* map = unit < nSlots ? (which ? mapB[unit] : mapA[unit]) : nullptr;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    const int64_t r = rb * 16;
-    if (map && r < nRows) {
-      if (r + 16 <= nRows) v = *(const uint4*)(map + r);
-      else {
-        __align__(16) uint8_t tmp[16];
-        for (int i = 0; i < 16; i++) tmp[i] = (r + i < nRows) ? map[r + i] : 0;
-        v = *(const uint4*)tmp;
+    r0 = acc[0];  // lane s of a half-warp holds row s of its block
+    r1 = 0.0;
+  } else {
+    const int t = lane & 3;
+#pragma unroll UNROLL_ROWS
+    for (int h = 0; h < 2; h++) {  // rows 0..7 and 8..15 of each half-warp's block
+      double acc[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) acc[i] = 0.0;
+#pragma unroll
+      for (int u = 0; u < NU; u++) {
+        const uint32_t w0 = h ? m[u].z : m[u].x, w1 = h ? m[u].w : m[u].y;
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc[i] = fma(lds_f64(entry_at(i < 4 ? w0 : w1, i & 3, tb[u])), v[u], acc[i]);
+      }
+      double d0, d1;
+      half_warp_sums(acc, d0, d1);
+      if (h == 0) r0 = d0, r1 = d1;
+      else {  // rows 8..15 go to the lanes t = 1
+        d0 = __shfl_up_sync(0xffffffffu, d0, 1);
+        d1 = __shfl_up_sync(0xffffffffu, d1, 1);
+        if (t == 1) r0 = d0, r1 = d1;
       }
     }
-    ((uint4*)out)[g] = v;
   }
 }
 
-// Device layout of the maps for k_lmm_vec_u8: [slab of 16 column slots][16-row block][slot][16 ids].
+template <int NU, bool JOINT>
+__device__ __forceinline__ void rmm_rows(const RmmArgs& A, int unit0, int64_t s0, int64_t s1, double init, bool first, bool last,
+                                         uint32_t table0) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int slot = lane & 15, half = lane >> 4, g = lane >> 2, t = lane & 3;
+  uint32_t tb[NU];
+  double v[NU];
+#pragma unroll
+  for (int u = 0; u < NU; u++) {
+    tb[u] = table0 + (uint32_t)(A.units[unit0 + u].x - A.units[unit0].x) * 128u + slot * 8;
+    v[u] = 0.0;
+    if (!JOINT) {
+      const int col = A.slotCol[(unit0 + u) * 16 + slot];
+      v[u] = col >= 0 ? A.v[col] : 0.0;
+    }
+  }
+  const uint8_t* mp = A.imaps + (size_t)unit0 * A.nRB * 256 + half * 256 + slot * 16;
+  const size_t ustr = (size_t)A.nRB * 256;
+  for (int64_t st = s0 + warp; st < s1; st += RB_W) {
+    // (loading the ids a step ahead costs the registers of a second set, i.e. spills or fewer warps: slower either way)
+    uint4 m[NU];
+#pragma unroll
+    for (int u = 0; u < NU; u++) m[u] = __ldg((const uint4*)(mp + u * ustr + st * 512));
+    const int64_t row = st * VSTEP + (JOINT ? lane : (t & 1) * 8 + g);
+    const bool mine0 = (JOINT || t < 2) && row < A.nRows, mine1 = !JOINT && t < 2 && row + 16 < A.nRows;
+    double o0 = init, o1 = init;  // what these rows hold from the chunks before
+    if (!first) {
+      o0 = mine0 ? A.out[row] : 0.0;
+      o1 = mine1 ? A.out[row + 16] : 0.0;
+    }
+    double r0, r1;
+    step_sums<NU, JOINT, 2>(m, tb, v, r0, r1);
+    if (!JOINT && __any_sync(0xffffffffu, t < 2 && !(isfinite(r0) && isfinite(r1)))) {
+      const double2 r = rmm_step_by_rows(mp + st * 512, ustr, A.units + unit0, A.slotCol + unit0 * 16, A.v, NU, table0);
+      r0 = r.x, r1 = r.y;
+    }
+    r0 += o0;
+    r1 += o1;
+    if (last && A.rowScale) {
+      if (mine0) r0 *= A.rowScale[row];
+      if (mine1) r1 *= A.rowScale[row + 16];
+    }
+    if (mine0) A.out[row] = r0;
+    if (mine1) A.out[row + 16] = r1;
+  }
+}
+
+// Tables of the joint slots of `nu` units, two units at a time: first the terms P_g = D_g v of their groups, then the
+// tables by adding one group after the other (T[k + n a] = T[k] + P[a] for the n joint tuples so far). A lane works for
+// one slot, its entries are spread over the warps. (With every entry taking its id apart by divisions and reading the
+// dictionaries through the group records, this was 40 of the 70 us of a 1M x 100 product.)
+constexpr int RB_T = RB_W * 32;
+__device__ __forceinline__ void joint_tables(const RmmArgs& A, int unit0, int nu, double* tbl, double* terms) {
+  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
+  double* P = terms + lane * JS_TERMS;
+  for (int u0 = 0; u0 < nu; u0 += 2) {
+    const int u = unit0 + min(u0 + (lane >> 4), nu - 1), slot = u * 16 + (lane & 15);
+    const bool on = u0 + (lane >> 4) < nu;
+    const JointSlot& js = A.joint[slot];
+    const int depth = A.units[u].y, n = on ? js.n : 0;
+    double* T = tbl + (size_t)(A.units[u].x - A.units[unit0].x) * 16 + (lane & 15);
+    int off = 0, nvs[JS_MAX];
+#pragma unroll
+    for (int i = 0; i < JS_MAX; i++) {
+      nvs[i] = 0;
+      if (i < n) {
+        const JointGroup G = A.jointGroups[slot * JS_MAX + i];
+        nvs[i] = G.nv;
+        for (int a = r; a < G.nv; a += RB_W) {
+          double x = 0.0;
+          if (G.gCols == 1) x = G.dict[a] * A.v[G.col];
+          else
+            for (int h = 0; h < G.gCols; h++) x += G.dict[(size_t)a * G.gCols + h] * A.v[G.cols[h]];
+          if (i == 0) T[(size_t)a * 16] = x;
+          else P[off + a] = x;
+        }
+        if (i > 0) off += G.nv;
+      }
+    }
+    int cur = n > 0 ? nvs[0] : 0;
+    off = 0;
+#pragma unroll
+    for (int i = 1; i < JS_MAX; i++) {
+      if (!__syncthreads_or(i < n)) break;
+      if (i < n) {
+        // the tuples so far are split over the warps; few tuples: the values of the new group as well
+        const int parts = max(1, RB_W / cur), k0 = cur >= RB_W ? r : r % cur, a0 = cur >= RB_W ? 1 : 1 + r / cur;
+        if (a0 <= parts)
+          for (int k = k0; k < cur; k += RB_W) {
+            const double x = T[(size_t)k * 16];
+            for (int a = a0; a < nvs[i]; a += parts) T[(size_t)(k + cur * a) * 16] = x + P[off + a];
+          }
+      }
+      __syncthreads();
+      if (i < n) {
+        const double p0 = P[off];
+        for (int k = r; k < cur; k += RB_W) T[(size_t)k * 16] += p0;
+        off += nvs[i];
+        cur *= nvs[i];
+      }
+    }
+    if (on)
+      for (int k = cur + r; k < depth; k += RB_W) T[(size_t)k * 16] = 0.0;
+    __syncthreads();
+  }
+}
+
+template <bool JOINT>
+__global__ void __launch_bounds__(RB_T, 1) k_rmm_vec(const __grid_constant__ RmmArgs A) {
+  extern __shared__ __align__(128) unsigned char smraw[];
+  __shared__ __align__(8) uint64_t mbar;
+  __shared__ double cred[RB_W];
+  const int64_t nSteps = ((int64_t)A.nRows + VSTEP - 1) / VSTEP;
+  const int64_t s0 = nSteps * blockIdx.x / gridDim.x, s1 = nSteps * (blockIdx.x + 1) / gridDim.x;
+  double init = 0.0;
+  if (A.constV) {
+    for (int c = threadIdx.x; c < A.nCols; c += RB_T) init = fma(A.constV[c], A.v[c], init);
+    for (int d = 16; d; d >>= 1) init += __shfl_xor_sync(0xffffffffu, init, d);
+    if ((threadIdx.x & 31) == 0) cred[threadIdx.x >> 5] = init;
+    __syncthreads();
+    init = 0.0;
+    for (int w = 0; w < RB_W; w++) init += cred[w];
+  }
+  tma_barrier_init(&mbar);
+  const int most = JOINT ? JOINT_UNITS : LMM_MAX_UNITS, nChunks = (A.nU16 + most - 1) / most, U = (A.nU16 + nChunks - 1) / nChunks;
+  for (int unit0 = 0, c = 0; unit0 < A.nU16; unit0 += U, c++) {
+    const int nu = min(U, A.nU16 - unit0);
+    __syncthreads();  // everyone is done with the previous chunk's tables
+    if (JOINT) {
+      const int rows = A.units[unit0 + nu - 1].x + A.units[unit0 + nu - 1].y - A.units[unit0].x;
+      joint_tables(A, unit0, nu, (double*)smraw, (double*)smraw + (size_t)rows * 16);
+    } else {
+      const int2 f = A.units[unit0], l = A.units[unit0 + nu - 1];
+      if (!tma_reload(smraw, A.tables + (size_t)f.x * 16, (uint32_t)(l.x + l.y - f.x) * 128u, &mbar, (uint32_t)(c & 1))) {
+        if (threadIdx.x == 0) atomicExch(A.err, 102);
+        return;
+      }
+    }
+    const bool last = unit0 + nu == A.nU16;
+    const uint32_t t0 = smem_u32(smraw);
+#define RB_CASE(N) case N: rmm_rows<N, JOINT>(A, unit0, s0, s1, init, c == 0, last, t0); break;
+    switch (nu) {
+      RB_CASE(1) RB_CASE(2) RB_CASE(3) RB_CASE(4) RB_CASE(5) RB_CASE(6)
+      default: rmm_rows<7, JOINT>(A, unit0, s0, s1, init, c == 0, last, t0); break;
+    }
+#undef RB_CASE
+  }
+}
+
+// --------------------------------------------------------------------------------------------------
+// t(X) (w * (X v)) in one kernel, for up to seven units of column slots (112 columns), whose tables fit one SM: a step's
+// row sums are formed as in k_rmm_vec, scaled, put in shared memory, and multiplied into the column sums as in
+// k_lmm_vec with the id words still in registers (row loops not unrolled: the compiler would hoist a step's worth of
+// lookups and spill). The maps are read once instead of twice, the tables are staged once,
+// and u = X v never leaves the SM (it is stored only if the caller gave a buffer for it).
+// --------------------------------------------------------------------------------------------------
+constexpr int CH_W = 11;         // what fits next to seven units of 256 tuples
+constexpr int CH_T = CH_W * 32;
+constexpr int CH_STATIC = 3072;  // static shared memory of the kernel, at most
+struct ChainArgs {
+  LmmArgs L;            // y unused
+  const double* v;
+  const double* w;      // null: no weights
+  double* u;            // null: not wanted
+  int nCols;
+};
+
+template <int NU>
+__device__ __forceinline__ void chain_body(const ChainArgs& C, unsigned char* smraw, uint64_t* mbar, double* ubuf, double init) {
+  const LmmArgs& A = C.L;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slot = lane & 15, half = lane >> 4, g = lane >> 2, t = lane & 3;
+  double* mine = A.partial + (size_t)blockIdx.x * (LMM_PART + 1);
+  const int2 first = A.units[0], last = A.units[NU - 1];
+  if (!tma_load_to_smem(smraw, A.tables, (uint32_t)(last.x + last.y - first.x) * 128u, mbar)) {
+    if (tid == 0) atomicExch(A.err, 103);
+    for (int u = tid; u <= LMM_PART; u += CH_T) mine[u] = __longlong_as_double(0x7ff8000000000000ll);
+    return;
+  }
+  const uint32_t table0 = smem_u32(smraw);
+  uint32_t tb[NU];
+  double v[NU], acc[NU], ysum = 0.0;
+#pragma unroll
+  for (int u = 0; u < NU; u++) {
+    tb[u] = table0 + (uint32_t)(A.units[u].x - first.x) * 128u + slot * 8;
+    const int col = A.slotCol[u * 16 + slot];
+    v[u] = col >= 0 ? C.v[col] : 0.0;
+    acc[u] = 0.0;
+  }
+  const uint8_t* mp = A.imaps + half * 256 + slot * 16;
+  const size_t ustr = (size_t)A.nRB * 256;
+  double* ub = ubuf + warp * 32;
+  const int64_t s0 = A.stepEnd * blockIdx.x / gridDim.x, s1 = A.stepEnd * (blockIdx.x + 1) / gridDim.x;
+  for (int64_t st = s0 + warp; st < s1; st += CH_W) {
+    uint4 m[NU];
+#pragma unroll
+    for (int u = 0; u < NU; u++) m[u] = __ldg((const uint4*)(mp + u * ustr + st * 512));
+    const int64_t row = st * VSTEP + (t & 1) * 8 + g;
+    const bool mine0 = t < 2 && row < A.nRows, mine1 = t < 2 && row + 16 < A.nRows;
+    double w0 = 1.0, w1 = 1.0;
+    if (C.w) {
+      w0 = mine0 ? C.w[row] : 0.0;
+      w1 = mine1 ? C.w[row + 16] : 0.0;
+    }
+    double r0, r1;
+    step_sums<NU, false, 1>(m, tb, v, r0, r1);
+    if (__any_sync(0xffffffffu, t < 2 && !(isfinite(r0) && isfinite(r1)))) {
+      const double2 r = rmm_step_by_rows(mp + st * 512, ustr, A.units, A.slotCol, C.v, NU, table0);
+      r0 = r.x, r1 = r.y;
+    }
+    r0 = (r0 + init) * w0;
+    r1 = (r1 + init) * w1;
+    if (C.u) {
+      if (mine0) C.u[row] = r0;
+      if (mine1) C.u[row + 16] = r1;
+    }
+    if (t < 2) {
+      ub[t * 8 + g] = r0;
+      ub[16 + t * 8 + g] = r1;
+    }
+    __syncwarp();
+    if (st * VSTEP + VSTEP <= A.nRows) {
+#pragma unroll 1
+      for (int b = 0; b < 4; b++) {
+        double y[4];
+        const double2 ya = *(const double2*)&ub[half * 16 + b * 4], yb = *(const double2*)&ub[half * 16 + b * 4 + 2];
+        y[0] = ya.x, y[1] = ya.y, y[2] = yb.x, y[3] = yb.y;
+        if (A.constV) ysum += (y[0] + y[1]) + (y[2] + y[3]);
+#pragma unroll
+        for (int u = 0; u < NU; u++) {
+          const uint32_t w = b == 0 ? m[u].x : (b == 1 ? m[u].y : (b == 2 ? m[u].z : m[u].w));
+#pragma unroll
+          for (int i = 0; i < 4; i++) acc[u] = fma(y[i], lds_f64(entry_at(w, i, tb[u])), acc[u]);
+        }
+      }
+    } else {  // ragged last step
+      for (int i = 0; i < 16 && st * VSTEP + half * 16 + i < A.nRows; i++) {
+        const double yy = ub[half * 16 + i];
+        ysum += yy;
+#pragma unroll
+        for (int u = 0; u < NU; u++) acc[u] = fma(yy, lds_f64(tb[u] + 128u * mp[u * ustr + st * 512 + i]), acc[u]);
+      }
+    }
+    __syncwarp();
+  }
+  __syncthreads();  // tables no longer needed
+  double* red = (double*)smraw;  // [CH_W][NU * 16 + 1]
+#pragma unroll
+  for (int u = 0; u < NU; u++) {
+    double a = acc[u];
+    a += __shfl_xor_sync(0xffffffffu, a, 16);
+    if (half == 0) red[warp * (NU * 16 + 1) + u * 16 + slot] = a;
+  }
+  ysum += __shfl_xor_sync(0xffffffffu, ysum, 16);
+  if (lane == 0) red[warp * (NU * 16 + 1) + NU * 16] = ysum;
+  __syncthreads();
+  for (int u = tid; u <= NU * 16; u += CH_T) {
+    double s = 0;
+    for (int w = 0; w < CH_W; w++) s += red[w * (NU * 16 + 1) + u];
+    mine[u < NU * 16 ? u : LMM_PART] = s;
+  }
+}
+
+__global__ void __launch_bounds__(CH_T, 1) k_chain_vec(const __grid_constant__ ChainArgs C) {
+  extern __shared__ __align__(128) unsigned char smraw[];
+  __shared__ __align__(8) uint64_t mbar;
+  __shared__ __align__(16) double ubuf[CH_W * 32];
+  __shared__ double cred[CH_W];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  double init = 0.0;
+  if (C.L.constV) {
+    for (int c = threadIdx.x; c < C.nCols; c += CH_T) init = fma(C.L.constV[c], C.v[c], init);
+    for (int d = 16; d; d >>= 1) init += __shfl_xor_sync(0xffffffffu, init, d);
+    if ((threadIdx.x & 31) == 0) cred[threadIdx.x >> 5] = init;
+    __syncthreads();
+    init = 0.0;
+    for (int w = 0; w < CH_W; w++) init += cred[w];
+  }
+#define CH_CASE(N) case N: chain_body<N>(C, smraw, &mbar, ubuf, init); break;
+  switch (C.L.nU16) {
+    CH_CASE(1) CH_CASE(2) CH_CASE(3) CH_CASE(4) CH_CASE(5) CH_CASE(6)
+    default: chain_body<7>(C, smraw, &mbar, ubuf, init); break;
+  }
+#undef CH_CASE
+}
+
+// Maps are handed to the interleave kernels as tagged addresses: bit 0 set = MapToBit words, else one byte per row.
+__device__ __forceinline__ uint4 ids16(const uint8_t* tagged, int64_t r, int nRows) {
+  const uintptr_t p = (uintptr_t)tagged & ~(uintptr_t)1;
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (r >= nRows) return v;
+  if ((uintptr_t)tagged & 1) {  // r is a multiple of 16: the 16 bits lie in one word
+    uint32_t bits = (uint32_t)(((const unsigned long long*)p)[r >> 6] >> (r & 63)) & 0xFFFFu;
+    if (r + 16 > nRows) bits &= (1u << (nRows - r)) - 1u;
+    auto four = [](uint32_t x) { return (x & 1u) | ((x & 2u) << 7) | ((x & 4u) << 14) | ((x & 8u) << 21); };
+    return make_uint4(four(bits), four(bits >> 4), four(bits >> 8), four(bits >> 12));
+  }
+  if (r + 16 <= nRows) return *(const uint4*)(p + r);
+  __align__(16) uint8_t tmp[16];
+  for (int i = 0; i < 16; i++) tmp[i] = (r + i < nRows) ? ((const uint8_t*)p)[r + i] : 0;
+  return *(const uint4*)tmp;
+}
+
+// Device layout of the maps for the column-per-lane kernels: [unit of 16 slots][16-row block][slot][16 ids].
 // A half-warp (one lane per slot) then reads 256 contiguous bytes per 128-bit load instead of 16 scattered
 // lines. Built once at plan time; unused slots and rows past the end hold id 0.
 __global__ void k_lmm_interleave(const uint8_t* const* __restrict__ slotMap, int nSlots, int nUnits, int nRows,
@@ -945,46 +1068,35 @@ __global__ void k_lmm_interleave(const uint8_t* const* __restrict__ slotMap, int
   const int64_t total = (int64_t)nSlots * nRB;
   for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
     const int slot = (int)(g & 15);
-    const int64_t rb = (g >> 4) % nRB;
-    const int64_t slab = (g >> 4) / nRB;
+    const int64_t rb = (g >> 4) % nRB, slab = (g >> 4) / nRB;
     const int unit = (int)slab * 16 + slot;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    const int64_t r = rb * 16;
-    if (unit < nUnits && r < nRows) {
-      const uint8_t* src = slotMap[unit] + r;
-      if (r + 16 <= nRows) v = *(const uint4*)src;
-      else {
-        __align__(16) uint8_t tmp[16];
-        for (int i = 0; i < 16; i++) tmp[i] = (r + i < nRows) ? src[i] : 0;
-        v = *(const uint4*)tmp;
-      }
-    }
-    ((uint4*)out)[g] = v;
+    ((uint4*)out)[g] = unit < nUnits ? ids16(slotMap[unit], rb * 16, nRows) : make_uint4(0, 0, 0, 0);
   }
 }
 
-// bit map -> byte map (one id per byte), used once at plan time
-__global__ void k_bits_to_bytes(const unsigned long long* __restrict__ bits, uint8_t* __restrict__ out, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = (uint8_t)((bits[i >> 6] >> (i & 63)) & 1ULL);
+// Joint ids of the slots in the same layout.
+__global__ void k_joint_interleave(const JointSlot* __restrict__ slots, const uint8_t* const* __restrict__ groupMap, int nSlots,
+                                   int nRows, int64_t nRB, uint8_t* __restrict__ out) {
+  const int64_t total = (int64_t)nSlots * nRB;
+  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
+    const int slot = (int)(g & 15);
+    const int64_t rb = (g >> 4) % nRB, slab = (g >> 4) / nRB;
+    const JointSlot& js = slots[slab * 16 + slot];
+    // joint ids stay below 256, so the bytes of a word never carry into each other
+    uint4 id = make_uint4(0, 0, 0, 0);
+    uint32_t stride = 1;
+    for (int k = 0; k < js.n; k++) {
+      const uint4 w = ids16(groupMap[js.group[k]], rb * 16, nRows);
+      id.x += stride * w.x, id.y += stride * w.y, id.z += stride * w.z, id.w += stride * w.w;
+      stride *= js.nv[k];
+    }
+    ((uint4*)out)[g] = id;
+  }
 }
 
 // --------------------------------------------------------------------------------------------------
 // plan
 // --------------------------------------------------------------------------------------------------
-template <typename T>
-static int64_t plan_upload(FastPlan* fp, const std::vector<T>& h, T** d) {
-  *d = nullptr;
-  if (h.empty()) return CLA_OK;
-  void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, h.size() * sizeof(T));
-  if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc plan: ") + cudaGetErrorString(e));
-  fp->allocs.push_back(p);
-  CLA_CUDA(cudaMemcpy(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-  *d = (T*)p;
-  return CLA_OK;
-}
-
 void fast_plan_free(Matrix* m) {
   if (!m->fast) return;
   for (void* p : m->fast->allocs) cudaFree(p);
@@ -992,284 +1104,217 @@ void fast_plan_free(Matrix* m) {
   m->fast = nullptr;
 }
 
+static int64_t plan_malloc(FastPlan* fp, void** p, size_t bytes) {
+  *p = nullptr;
+  cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+  if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc plan: ") + cudaGetErrorString(e));
+  fp->allocs.push_back(*p);
+  return CLA_OK;
+}
+
+// Host arrays of the plan, uploaded with one allocation and one copy.
+struct PlanBlob {
+  std::vector<char> host;
+  template <typename T>
+  size_t add(const std::vector<T>& v) {
+    const size_t at = (host.size() + 255) & ~(size_t)255;
+    host.resize(at + std::max<size_t>(v.size() * sizeof(T), 1));
+    if (!v.empty()) memcpy(host.data() + at, v.data(), v.size() * sizeof(T));
+    return at;
+  }
+};
+
 int64_t fast_plan_build(Matrix* m) {
   FastPlan* fp = new FastPlan();
   m->fast = fp;
   if (m->nRows < FAST_MIN_ROWS || m->nDev == 0) return CLA_OK;
   // the groups these kernels cover: dense maps, at most 256 tuples, one byte (or bit) per cell
-  std::vector<DevGroup> G;
-  std::vector<int> selIdx;
-  for (int gi = 0; gi < m->nDev; gi++) {
+  struct Sel { int dev, reg; };
+  std::vector<Sel> sel;
+  int nUnitsSel = 0;
+  for (size_t hi = 0; hi < m->hg.size(); hi++) {
+    const int gi = m->regToDev[hi];
+    if (gi < 0) continue;
     const DevGroup& g = m->groups[gi];
     if (g.type != GT_DDC || g.nVals > 256 || g.nVals < 1) continue;
     if (g.mapType != CLA_MAP_UBYTE && g.mapType != CLA_MAP_BYTE && g.mapType != CLA_MAP_BIT) continue;
-    G.push_back(g);
-    selIdx.push_back(gi);
+    sel.push_back({gi, (int)hi});
+    nUnitsSel += g.gCols;
   }
-  const bool all = (int)G.size() == m->nDev;
-  int nUnitsSel = 0;
-  for (auto& g : G) nUnitsSel += g.gCols;
-  if (G.empty() || (!all && nUnitsSel < 16)) return CLA_OK;  // too few columns to be worth a separate pass
+  const bool all = (int)sel.size() == m->nDev;
+  if (sel.empty() || (!all && nUnitsSel < 16)) return CLA_OK;  // too few columns to be worth a separate pass
   fp->partial = !all;
-  const int nG = (int)G.size();
-  fp->nG = nG;
+  const int nG = (int)sel.size();
   int64_t rc;
-  // byte maps for every group (bit maps are expanded once)
-  std::vector<const uint8_t*> gmap(nG);
-  for (int gi = 0; gi < nG; gi++) {
-    const DevGroup& g = G[gi];
-    if (g.mapType == CLA_MAP_BIT) {
-      void* p = nullptr;
-      CLA_CUDA(cudaMalloc(&p, (size_t)m->nRows + 64));
-      fp->allocs.push_back(p);
-      m->deviceBytes += m->nRows;
-      k_bits_to_bytes<<<std::min(4096, (m->nRows + 255) / 256), 256, 0, m->stream>>>((const unsigned long long*)g.map,
-                                                                                   (uint8_t*)p, m->nRows);
-      gmap[gi] = (const uint8_t*)p;
-    } else
-      gmap[gi] = (const uint8_t*)g.map;
-  }
-  CLA_CUDA(cudaStreamSynchronize(m->stream));
+  auto G = [&](int i) -> const DevGroup& { return m->groups[sel[i].dev]; };
+  auto tagged = [&](int i) { return (const uint8_t*)((uintptr_t)G(i).map | (G(i).mapType == CLA_MAP_BIT ? 1u : 0u)); };
+  fp->nRB = (((int64_t)m->nRows + LMM_STEP - 1) / LMM_STEP) * (LMM_STEP / 16);
 
-  // ---- RMM: groups ordered by table size so the small (conflict-free) tables pack together ----
-  std::vector<int> order(nG);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return G[a].nVals < G[b].nVals; });
-  int64_t total = 0;
-  for (int gi : order) total += (G[gi].nVals + 1) & ~1;
-  const int budget = total * 8 <= 40 * 1024 ? 40 * 1024 : 96 * 1024;  // small: many CTAs per SM; else two per SM
-  std::vector<const uint8_t*> maps(nG);
-  std::vector<int> tblOff(nG), groupOf(nG);
-  std::vector<int64_t> imgOff(nG);
-  int64_t img = 0;
-  RmmChunk cur{0, 0, 0, 0};
-  for (int i = 0; i < nG; i++) {
-    const int gi = order[i];
-    const int pad = (G[gi].nVals + 1) & ~1;
-    const int perGroup = 8 + 4;  // map pointer + offset kept in shared memory
-    if (cur.g1 > cur.g0 && (cur.tblDoubles + pad) * 8 + (cur.g1 - cur.g0 + 1) * perGroup > budget) {
-      fp->rchunks.push_back(cur);
-      cur = RmmChunk{i, i, 0, img};
-    }
-    maps[i] = gmap[gi];
-    groupOf[i] = selIdx[gi];
-    tblOff[i] = cur.tblDoubles;
-    imgOff[i] = img;
-    cur.tblDoubles += pad;
-    cur.g1 = i + 1;
-    img += pad;
-  }
-  fp->rchunks.push_back(cur);
-  fp->pImgDoubles = img;
-  if ((rc = plan_upload(fp, maps, &fp->dMaps)) < 0) return rc;
-  if ((rc = plan_upload(fp, tblOff, &fp->dTblOff)) < 0) return rc;
-  if ((rc = plan_upload(fp, groupOf, &fp->dGroupOf)) < 0) return rc;
-  if ((rc = plan_upload(fp, imgOff, &fp->dImgOff)) < 0) return rc;
-
-  // ---- LMM: one column slot per (group, column), in output-column order; 16 slots per unit ----
-  // (A chunk holds at most LMM_MAX_UNITS units and their tables fit at any depth, so nothing is gained by packing
-  // shallow tables together; in column order the 16 slots of a unit are neighbours in a decompressed row.)
+  // ---- column slots: one per (group, column), in output-column order; 16 slots per unit ----
+  // (in column order the 16 slots of a unit are neighbours in a decompressed row)
   struct Unit { int g, j, nv, col; };
   std::vector<Unit> units;
-  for (int gi = 0; gi < nG; gi++) {
-    std::vector<int32_t> cols(G[gi].gCols);
-    CLA_CUDA(cudaMemcpy(cols.data(), G[gi].cols, cols.size() * 4, cudaMemcpyDeviceToHost));
-    for (int j = 0; j < G[gi].gCols; j++) units.push_back({gi, j, G[gi].nVals, cols[j]});
-  }
+  for (int i = 0; i < nG; i++)
+    for (int j = 0; j < G(i).gCols; j++) units.push_back({i, j, G(i).nVals, m->hg[sel[i].reg].cols[j]});
   std::stable_sort(units.begin(), units.end(), [](const Unit& a, const Unit& b) { return a.col < b.col; });
   fp->nUnits = (int)units.size();
-  const int nU16 = (fp->nUnits + 15) / 16;
+  const int nU16 = fp->nU16 = (fp->nUnits + 15) / 16;
   fp->nSlots = nU16 * 16;
-  // unused slots of the last unit read the map of the last column (its ids stay inside the unit's table depth)
-  std::vector<const uint8_t*> slotMap(fp->nSlots, gmap[units.back().g]);
+  std::vector<const uint8_t*> slotMap(fp->nSlots, nullptr);
   std::vector<int> slotCol(fp->nSlots, -1);
-  std::vector<int> unitNk(nU16, 1);
-  // host copies of the dictionaries
-  std::vector<std::vector<double>> dicts(nG);
-  for (int gi = 0; gi < nG; gi++) {
-    dicts[gi].resize((size_t)G[gi].nVals * G[gi].gCols);
-    CLA_CUDA(cudaMemcpy(dicts[gi].data(), G[gi].dict, dicts[gi].size() * 8, cudaMemcpyDeviceToHost));
+  fp->unitNk.assign(nU16, 1);
+  fp->unitOff.assign(nU16, 0);
+  std::vector<uint8_t> held(m->nCols, 0);
+  for (int u = 0; u < fp->nUnits; u++) {
+    slotMap[u] = tagged(units[u].g);
+    slotCol[u] = units[u].col;
+    if (held[units[u].col]) fp->uniqueCols = false;
+    held[units[u].col] = 1;
+    fp->unitNk[u / 16] = std::max(fp->unitNk[u / 16], units[u].nv);
   }
-  for (int u = 0; u < fp->nUnits; u++) unitNk[u / 16] = std::max(unitNk[u / 16], units[u].nv);
-  // chunks: greedily pack units up to the shared-memory budget and LMM_MAX_UNITS
-  const size_t redBytes = (size_t)LMM_W * LMM_PART * 8;
-  const size_t lmmBudget = SMEM_MAX - 2048;
-  std::vector<double> image;
-  LmmChunk lc{};
-  lc.unit0 = 0;
-  auto flush = [&]() {
-    lc.tblDoubles = 0;
-    for (int q = 0; q < lc.nUnits; q++) lc.tblDoubles += lc.nk[q] * 16;
-    lc.tblOff = (int64_t)image.size();
-    image.resize(image.size() + lc.tblDoubles, 0.0);
-    size_t off = lc.tblOff;
-    for (int q = 0; q < lc.nUnits; q++) {
-      for (int s = 0; s < 16; s++) {
-        const int u = (lc.unit0 + q) * 16 + s;
-        if (u >= fp->nUnits) continue;
-        const Unit& un = units[u];
-        const int gc = G[un.g].gCols;
-        for (int k = 0; k < un.nv; k++) image[off + (size_t)k * 16 + s] = dicts[un.g][(size_t)k * gc + un.j];
+  std::vector<int> bare;
+  for (int c = 0; c < m->nCols; c++)
+    if (!held[c]) bare.push_back(c);
+  fp->nBare = (int)bare.size();
+  // table image, unit after unit
+  std::vector<int2> unitRec(nU16);
+  int64_t imgD = 0;
+  for (int q = 0; q < nU16; q++) {
+    fp->unitOff[q] = imgD;
+    unitRec[q] = make_int2((int)(imgD / 16), fp->unitNk[q]);
+    imgD += (int64_t)fp->unitNk[q] * 16;
+  }
+  std::vector<double> image(imgD, 0.0);
+  for (int u = 0; u < fp->nUnits; u++) {
+    const HostGroup& hg = m->hg[sel[units[u].g].reg];
+    const int gc = (int)hg.cols.size(), nv = hg.nVals;  // (an OLE group's extra "no tuple" entry stays zero)
+    double* T = image.data() + fp->unitOff[u / 16] + (u & 15);
+    for (int k = 0; k < nv; k++) T[(size_t)k * 16] = hg.dict[(size_t)k * gc + units[u].j];
+  }
+  fp->imageDoubles = image.size();
+  // chunks of up to LMM_MAX_UNITS units for the kernels that fix them at plan time (several left rows, decompress):
+  // CTAs per chunk in proportion to its cost in L1 data-pipe wavefronts per 64-row step: 64 per unit for the dictionary
+  // reads, 8 for the map loads and 64 for the left vector
+  {
+    LmmChunk lc{};
+    for (int q = 0; q < nU16; q++) {
+      if (lc.nUnits == LMM_MAX_UNITS) {
+        fp->lchunks.push_back(lc);
+        lc = LmmChunk{};
       }
-      off += (size_t)lc.nk[q] * 16;
+      if (lc.nUnits == 0) {
+        lc.unit0 = q;
+        lc.tblOff = fp->unitOff[q];
+      }
+      lc.nk[lc.nUnits++] = fp->unitNk[q];
+      lc.tblDoubles += fp->unitNk[q] * 16;
     }
     fp->lchunks.push_back(lc);
-  };
-  size_t curBytes = 0;
-  lc.nUnits = 0;
-  for (int q = 0; q < nU16; q++) {
-    const size_t b = (size_t)unitNk[q] * 128;
-    if (lc.nUnits == LMM_MAX_UNITS || (lc.nUnits > 0 && std::max(curBytes + b, redBytes) > lmmBudget)) {
-      flush();
-      lc = LmmChunk{};
-      lc.unit0 = q;
-      lc.nUnits = 0;
-      curBytes = 0;
+    const int totalCta = std::max(m->smCount, (int)fp->lchunks.size());
+    double totalCost = 0;
+    auto chunkCost = [](const LmmChunk& c) { return 72.0 * c.nUnits + 64.0; };
+    for (auto& c : fp->lchunks) totalCost += chunkCost(c);
+    const int64_t nSteps = ((int64_t)m->nRows + LMM_STEP - 1) / LMM_STEP;
+    std::vector<int> share(fp->lchunks.size());
+    int used = 0, cta = 0;
+    for (size_t i = 0; i < fp->lchunks.size(); i++) {
+      share[i] = std::max(1, (int)(totalCta * chunkCost(fp->lchunks[i]) / totalCost));
+      used += share[i];
     }
-    lc.nk[lc.nUnits++] = unitNk[q];
-    curBytes += b;
+    for (size_t i = 0; used < totalCta; i = (i + 1) % fp->lchunks.size(), used++) share[i]++;  // hand out the remainder
+    for (size_t i = 0; i < fp->lchunks.size(); i++) {
+      auto& c = fp->lchunks[i];
+      const int n = (int)std::min<int64_t>(share[i], nSteps);
+      c.cta0 = cta;
+      c.nCta = n;
+      cta += n;
+    }
+    fp->lmmGrid = cta;
   }
-  flush();
-  for (int u = 0; u < fp->nUnits; u++) {
-    slotMap[u] = gmap[units[u].g];
-    slotCol[u] = units[u].col;
-  }
-  // CTAs per chunk in proportion to its cost, one CTA per SM in total. Cost per 64-row warp step in
-  // L1 data-pipe wavefronts: 64 per unit for the dictionary reads, 8 per unit for the map loads and
-  // 64 for the left vector (which does not depend on the number of units).
-  const int totalCta = std::max(m->smCount, (int)fp->lchunks.size());
-  double totalCost = 0;
-  auto chunkCost = [](const LmmChunk& c) { return 72.0 * c.nUnits + 64.0; };
-  for (auto& c : fp->lchunks) totalCost += chunkCost(c);
-  int cta = 0;
-  const int64_t nSteps = ((int64_t)m->nRows + LMM_STEP - 1) / LMM_STEP;
-  std::vector<int> share(fp->lchunks.size());
-  int used = 0;
-  for (size_t i = 0; i < fp->lchunks.size(); i++) {
-    share[i] = std::max(1, (int)(totalCta * chunkCost(fp->lchunks[i]) / totalCost));
-    used += share[i];
-  }
-  for (size_t i = 0; used < totalCta; i = (i + 1) % fp->lchunks.size(), used++) share[i]++;  // hand out the remainder
-  for (size_t i = 0; i < fp->lchunks.size(); i++) {
-    auto& c = fp->lchunks[i];
-    const int n = (int)std::min<int64_t>(share[i], nSteps);
-    c.cta0 = cta;
-    c.nCta = n;
-    cta += n;
-  }
-  fp->lmmGrid = cta;
-  if ((rc = plan_upload(fp, fp->lchunks, &fp->dLChunks)) < 0) return rc;
-  if ((rc = plan_upload(fp, slotMap, &fp->dSlotMap)) < 0) return rc;
-  if ((rc = plan_upload(fp, slotCol, &fp->dSlotCol)) < 0) return rc;
-  {
-    fp->nRB = (((int64_t)m->nRows + LMM_STEP - 1) / LMM_STEP) * (LMM_STEP / 16);
-    const size_t bytes = (size_t)fp->nSlots * fp->nRB * 16;
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc interleaved maps: ") + cudaGetErrorString(e));
-    fp->allocs.push_back(p);
-    fp->dLmmMaps = (uint8_t*)p;
-    m->deviceBytes += (int64_t)bytes;
-    k_lmm_interleave<<<m->smCount * 8, 256, 0, m->stream>>>(fp->dSlotMap, fp->nSlots, fp->nUnits, m->nRows, fp->nRB,
-                                                           fp->dLmmMaps);
-    CLA_CUDA(cudaStreamSynchronize(m->stream));
-  }
-  if ((rc = plan_upload(fp, image, &fp->dLmmTables)) < 0) return rc;
-  fp->imageDoubles = image.size();
-  for (auto& g : G) fp->maxNVals = std::max(fp->maxNVals, g.nVals);
-  m->deviceBytes += (int64_t)image.size() * 8;
-  CLA_CUDA(cudaFuncSetAttribute(k_lmm_vec_u8, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
-  CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec_b, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
-  CLA_CUDA(cudaFuncSetAttribute(k_decomp_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 2048));
-  CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec_u8<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-  CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec_u8<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-  CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec_u8<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-  // ---- RMM with two groups per lookup, when at least half of the groups find a partner ----
+
+  // ---- joint slots for X v: the smallest dictionaries first, as many groups per slot as 256 joint tuples allow ----
+  std::vector<JointSlot> js;
+  std::vector<const uint8_t*> groupMap(m->nDev, nullptr);
   {
     std::vector<int> byNv(nG);
     std::iota(byNv.begin(), byNv.end(), 0);
-    std::stable_sort(byNv.begin(), byNv.end(), [&](int a, int b) { return G[a].nVals < G[b].nVals; });
-    auto bitsFor = [](int nv) { int sh = 0; while ((1 << sh) < nv) sh++; return sh; };
-    std::vector<FusedUnit> fu;
-    int lo = 0, hi = nG - 1, paired = 0;
-    while (lo <= hi) {  // the largest remaining dictionary takes the smallest remaining partner that still fits
-      const int a = byNv[hi];
-      if (lo < hi) {
-        const int b = byNv[lo];
-        const int sh = bitsFor(G[b].nVals);
-        if ((G[a].nVals << sh) <= 256) {
-          fu.push_back(FusedUnit{a, b, sh, G[a].nVals, G[b].nVals});
-          paired += 2;
-          lo++;
-          hi--;
-          continue;
-        }
+    std::stable_sort(byNv.begin(), byNv.end(), [&](int a, int b) { return G(a).nVals < G(b).nVals; });
+    for (int i : byNv) {
+      const int nv = G(i).nVals;
+      int terms = nv;
+      if (!js.empty())
+        for (int k = 0; k < js.back().n; k++) terms += js.back().nv[k];
+      if (js.empty() || js.back().n == JS_MAX || js.back().total * nv > 256 || terms > JS_TERMS) {
+        JointSlot s{};
+        s.total = 1;
+        js.push_back(s);
       }
-      fu.push_back(FusedUnit{a, -1, 0, G[a].nVals, 1});
-      hi--;
+      JointSlot& s = js.back();
+      s.group[s.n] = sel[i].dev;
+      s.nv[s.n++] = nv;
+      s.total *= nv;
+      groupMap[sel[i].dev] = tagged(i);
     }
-    // (fast_rmm_vec takes this kernel below 4M rows only: no second copy of the maps for taller matrices)
-    if (paired * 2 >= nG && !fp->partial && m->nRows < (4 << 20)) {
-      std::stable_sort(fu.begin(), fu.end(), [](const FusedUnit& x, const FusedUnit& y) { return (x.nva << x.sh) > (y.nva << y.sh); });
-      fp->nFused = (int)fu.size();
-      const int nU16F = (fp->nFused + 15) / 16;
-      const int nSlotsF = nU16F * 16;
-      std::vector<const uint8_t*> mapA(nSlotsF, nullptr), mapB(nSlotsF, nullptr);
-      std::vector<FusedUnit> units(nSlotsF, FusedUnit{-1, -1, 0, 1, 1});
-      std::vector<int> nk(nU16F, 1);
-      for (int u = 0; u < fp->nFused; u++) {
-        mapA[u] = gmap[fu[u].ga];
-        mapB[u] = fu[u].gb >= 0 ? gmap[fu[u].gb] : nullptr;
-        units[u] = FusedUnit{selIdx[fu[u].ga], fu[u].gb >= 0 ? selIdx[fu[u].gb] : -1, fu[u].sh, fu[u].nva, fu[u].nvb};
-        nk[u / 16] = std::max(nk[u / 16], fu[u].nva << fu[u].sh);
-      }
-      LmmChunk fc{};
-      int64_t img = 0;
-      size_t cur = 0;
-      auto flushF = [&]() {
-        fc.tblDoubles = 0;
-        for (int q = 0; q < fc.nUnits; q++) fc.tblDoubles += fc.nk[q] * 16;
-        fc.tblOff = img;
-        img += fc.tblDoubles;
-        fp->fchunks.push_back(fc);
-      };
-      fc.unit0 = 0;
-      fc.nUnits = 0;
-      for (int q = 0; q < nU16F; q++) {
-        const size_t b = (size_t)nk[q] * 128;
-        if (fc.nUnits == 4 || (fc.nUnits > 0 && cur + b > (size_t)SMEM_MAX - 2048)) {
-          flushF();
-          fc = LmmChunk{};
-          fc.unit0 = q;
-          fc.nUnits = 0;
-          cur = 0;
-        }
-        fc.nk[fc.nUnits++] = nk[q];
-        cur += b;
-      }
-      flushF();
-      fp->fImageDoubles = (size_t)img;
-      const uint8_t** dA = nullptr;
-      const uint8_t** dB = nullptr;
-      if ((rc = plan_upload(fp, mapA, &dA)) < 0) return rc;
-      if ((rc = plan_upload(fp, mapB, &dB)) < 0) return rc;
-      if ((rc = plan_upload(fp, units, &fp->dFUnits)) < 0) return rc;
-      if ((rc = plan_upload(fp, fp->fchunks, &fp->dFChunks)) < 0) return rc;
-      const size_t bytes = (size_t)nSlotsF * fp->nRB * 32;
-      void* pm = nullptr;
-      cudaError_t e = cudaMalloc(&pm, bytes);
-      if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc fused maps: ") + cudaGetErrorString(e));
-      fp->allocs.push_back(pm);
-      fp->dFMaps = (uint8_t*)pm;
-      m->deviceBytes += (int64_t)bytes;
-      k_rmm_f_interleave<<<m->smCount * 8, 256, 0, m->stream>>>(dA, dB, nSlotsF, m->nRows, fp->nRB, fp->dFMaps);
-      CLA_CUDA(cudaStreamSynchronize(m->stream));
-      CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec_f, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
-      fp->fusedOk = true;
+    // a second copy of the maps pays from a quarter fewer lookups on
+    if (js.size() * 4 > (size_t)fp->nUnits * 3) js.clear();
+    std::stable_sort(js.begin(), js.end(), [](const JointSlot& a, const JointSlot& b) { return a.total > b.total; });
+    fp->nJU16 = (int)(js.size() + 15) / 16;
+    js.resize((size_t)fp->nJU16 * 16, JointSlot{});
+  }
+  std::vector<JointGroup> jg(js.size() * JS_MAX, JointGroup{});
+  for (size_t i = 0; i < js.size(); i++)
+    for (int k = 0; k < js[i].n; k++) {
+      const DevGroup& g = m->groups[js[i].group[k]];
+      int col = 0;
+      for (auto& x : sel)
+        if (x.dev == js[i].group[k]) col = m->hg[x.reg].cols[0];
+      jg[i * JS_MAX + k] = JointGroup{g.dict, g.cols, js[i].nv[k], g.gCols, col, 0};
     }
+  std::vector<int2> jRec(fp->nJU16);
+  fp->jNk.assign(fp->nJU16, 1);
+  int jAt = 0;
+  for (int q = 0; q < fp->nJU16; q++) {
+    for (int s = 0; s < 16; s++) fp->jNk[q] = std::max(fp->jNk[q], js[q * 16 + s].total);
+    jRec[q] = make_int2(jAt, fp->jNk[q]);
+    jAt += fp->jNk[q];
+  }
+
+  PlanBlob blob;
+  const size_t oChunks = blob.add(fp->lchunks), oMap = blob.add(slotMap), oCol = blob.add(slotCol), oBare = blob.add(bare);
+  const size_t oUnits = blob.add(unitRec), oImage = blob.add(image);
+  const size_t oJs = blob.add(js), oJg = blob.add(jg), oJRec = blob.add(jRec), oGMap = blob.add(groupMap);
+  const size_t mapBytes = (size_t)fp->nSlots * fp->nRB * 16, jMapBytes = (size_t)fp->nJU16 * 16 * fp->nRB * 16;
+  void *d = nullptr, *maps = nullptr;
+  if ((rc = plan_malloc(fp, &d, blob.host.size())) < 0 || (rc = plan_malloc(fp, &maps, mapBytes + jMapBytes)) < 0) return rc;
+  CLA_CUDA(cudaMemcpyAsync(d, blob.host.data(), blob.host.size(), cudaMemcpyHostToDevice, m->stream));
+  char* base = (char*)d;
+  fp->dLChunks = (LmmChunk*)(base + oChunks);
+  fp->dSlotMap = (const uint8_t**)(base + oMap);
+  fp->dSlotCol = (int*)(base + oCol);
+  fp->dBareCols = (int*)(base + oBare);
+  fp->dUnits = (int2*)(base + oUnits);
+  fp->dLmmTables = (double*)(base + oImage);
+  fp->dJSlots = (JointSlot*)(base + oJs);
+  fp->dJGroups = (JointGroup*)(base + oJg);
+  fp->dJUnits = (int2*)(base + oJRec);
+  fp->dLmmMaps = (uint8_t*)maps;
+  fp->dJMaps = (uint8_t*)maps + mapBytes;
+  m->deviceBytes += (int64_t)(mapBytes + jMapBytes + blob.host.size());
+  k_lmm_interleave<<<m->smCount * 8, 256, 0, m->stream>>>(fp->dSlotMap, fp->nSlots, fp->nUnits, m->nRows, fp->nRB, fp->dLmmMaps);
+  if (fp->nJU16)
+    k_joint_interleave<<<m->smCount * 8, 256, 0, m->stream>>>(fp->dJSlots, (const uint8_t* const*)(base + oGMap), fp->nJU16 * 16,
+                                                             m->nRows, fp->nRB, fp->dJMaps);
+  CLA_CUDA(cudaStreamSynchronize(m->stream));
+  static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
+  if (!attrSet[m->device & 63]) {
+    CLA_CUDA(cudaFuncSetAttribute(k_lmm_vec, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
+    CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
+    CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
+    CLA_CUDA(cudaFuncSetAttribute(k_decomp_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 2048));
+    attrSet[m->device & 63] = true;
   }
   if (fp->partial) {  // tell the general kernels which groups are taken care of
-    for (int gi : selIdx) m->groups[gi].inFast = 1;
+    for (auto& x : sel) m->groups[x.dev].inFast = 1;
     CLA_CUDA(cudaMemcpy(m->dGroups, m->groups.data(), sizeof(DevGroup) * m->groups.size(), cudaMemcpyHostToDevice));
   }
   fp->ok = true;
@@ -1279,71 +1324,6 @@ int64_t fast_plan_build(Matrix* m) {
 // --------------------------------------------------------------------------------------------------
 // launchers
 // --------------------------------------------------------------------------------------------------
-__global__ void k_const_dot(const double* __restrict__ constV, const double* __restrict__ v, int n, double* out) {
-  double s = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += constV[i] * v[i];
-  __shared__ double sh[256];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int d = 128; d; d >>= 1) {
-    if ((int)threadIdx.x < d) sh[threadIdx.x] += sh[threadIdx.x + d];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[0] = sh[0];
-}
-
-static int64_t fast_rmm_vec_b(Matrix* m, FastPlan* fp, const double* dV, double* dOut, cudaStream_t s) {
-  int64_t rc;
-  const size_t pBytes = ((size_t)fp->imageDoubles * 8 + 255) & ~(size_t)255;
-  if ((rc = ensure_scratch(m, pBytes + 256)) < 0) return rc;
-  double* P = (double*)m->scratch;
-  double* constRow = nullptr;
-  k_rmm_b_tables<<<dim3((unsigned)fp->lchunks.size(), 16), 256, 0, s>>>(fp->dLChunks, fp->dSlotCol, fp->dLmmTables, dV, P);
-  m->stats.kernel_launches++;
-  if (m->hasConst) {
-    constRow = (double*)((char*)m->scratch + pBytes);
-    k_const_dot<<<1, 256, 0, s>>>(m->dConstV, dV, m->nCols, constRow);
-    m->stats.kernel_launches++;
-  }
-  size_t smem = 1024;
-  for (auto& c : fp->lchunks) smem = std::max(smem, (size_t)c.tblDoubles * 8);
-  const int64_t nSteps = ((int64_t)m->nRows + LMM_STEP - 1) / LMM_STEP;
-  const int grid = (int)std::min<int64_t>(m->smCount, nSteps);
-  prof_begin(m, s);
-  k_rmm_vec_b<<<grid, RB_W * 32, smem, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dLmmMaps, fp->nRB, P, m->nRows, constRow,
-                                        dOut, m->dErr);
-  prof_end(m, s);
-  m->stats.kernel_launches++;
-  CLA_CUDA(cudaGetLastError());
-  return fp->partial ? 2 : 1;
-}
-
-static int64_t fast_rmm_vec_f(Matrix* m, FastPlan* fp, const double* dV, double* dOut, cudaStream_t s) {
-  int64_t rc;
-  const size_t pBytes = ((size_t)fp->fImageDoubles * 8 + 255) & ~(size_t)255;
-  if ((rc = ensure_scratch(m, pBytes + 256)) < 0) return rc;
-  double* P = (double*)m->scratch;
-  double* constRow = nullptr;
-  k_rmm_f_tables<<<dim3((unsigned)fp->fchunks.size(), 16), 256, 0, s>>>(m->dGroups, fp->dFChunks, fp->dFUnits, dV, P);
-  m->stats.kernel_launches++;
-  if (m->hasConst) {
-    constRow = (double*)((char*)m->scratch + pBytes);
-    k_const_dot<<<1, 256, 0, s>>>(m->dConstV, dV, m->nCols, constRow);
-    m->stats.kernel_launches++;
-  }
-  size_t smem = 1024;
-  for (auto& c : fp->fchunks) smem = std::max(smem, (size_t)c.tblDoubles * 8);
-  const int64_t nSteps = ((int64_t)m->nRows + LMM_STEP - 1) / LMM_STEP;
-  const int grid = (int)std::min<int64_t>(m->smCount, nSteps);
-  prof_begin(m, s);
-  k_rmm_vec_f<<<grid, LMM_T, smem, s>>>(fp->dFChunks, (int)fp->fchunks.size(), fp->dFUnits, fp->dFMaps, fp->nRB, P, m->nRows,
-                                        constRow, dOut, m->dErr);
-  prof_end(m, s);
-  m->stats.kernel_launches++;
-  CLA_CUDA(cudaGetLastError());
-  return 1;
-}
-
 bool fast_plan_ok(const Matrix* m) { return m->fast && m->fast->ok; }
 bool fast_plan_partial(const Matrix* m) { return m->fast && m->fast->ok && m->fast->partial; }
 
@@ -1364,81 +1344,182 @@ int64_t fast_decompress(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s)
   return 1;
 }
 
-int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, cudaStream_t s) {
+int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s) {
   FastPlan* fp = m->fast;
-  if (!fp || !fp->ok || ((uintptr_t)dOut & 15)) return 0;  // 128-bit stores need an aligned output
-  // Two groups per lookup pays off on short matrices, where the row-per-thread kernel cannot keep enough loads
-  // in flight (measured: 1M rows 46.6 vs 52.5 us); on tall ones the second map load and the shuffles cost more
-  // than the saved reads (10M rows: 344 vs 326 us).
-  if (fp->fusedOk && m->nRows < (4 << 20) && !getenv("CLA_NO_FUSED_RMM")) return fast_rmm_vec_f(m, fp, dV, dOut, s);
-  if (fp->maxNVals > 16) return fast_rmm_vec_b(m, fp, dV, dOut, s);  // deep tables: the conflict-free layout
-  int64_t rc;
-  const size_t pBytes = ((size_t)fp->pImgDoubles * 8 + 255) & ~(size_t)255;
-  if ((rc = ensure_scratch(m, pBytes + 256)) < 0) return rc;
-  double* P = (double*)m->scratch;
-  double* constRow = nullptr;
-  k_fast_ptable<<<fp->nG, 128, 0, s>>>(m->dGroups, fp->dGroupOf, fp->dImgOff, fp->nG, dV, P);
+  if (!fp || !fp->ok || (dW && fp->partial)) return 0;
+  // (short matrices: building the joint tables takes longer than the lookups they save)
+  const bool joint = fp->nJU16 > 0 && m->nRows >= 300000;
+  RmmArgs A{};
+  A.units = joint ? fp->dJUnits : fp->dUnits;
+  A.imaps = joint ? fp->dJMaps : fp->dLmmMaps;
+  A.nRB = fp->nRB;
+  A.tables = fp->dLmmTables;
+  A.slotCol = fp->dSlotCol;
+  A.joint = fp->dJSlots;
+  A.jointGroups = fp->dJGroups;
+  A.v = dV;
+  A.constV = m->hasConst ? m->dConstV : nullptr;
+  A.nCols = m->nCols;
+  A.nRows = m->nRows;
+  A.nU16 = joint ? fp->nJU16 : fp->nU16;
+  A.rowScale = dW;
+  A.out = dOut;
+  A.err = m->dErr;
+  const std::vector<int>& nk = joint ? fp->jNk : fp->unitNk;
+  const int most = joint ? JOINT_UNITS : LMM_MAX_UNITS, nChunks = (A.nU16 + most - 1) / most, U = (A.nU16 + nChunks - 1) / nChunks;
+  size_t smem = 1024;
+  for (int q = 0; q < A.nU16; q += U) {
+    size_t b = 0;
+    for (int i = q; i < std::min(A.nU16, q + U); i++) b += (size_t)nk[i] * 128;
+    smem = std::max(smem, b);
+  }
+  if (joint) smem += 32 * JS_TERMS * sizeof(double);
+  const int64_t nSteps = ((int64_t)m->nRows + VSTEP - 1) / VSTEP;
+  const int grid = (int)std::min<int64_t>(m->smCount, nSteps);
+  prof_begin(m, s);
+  if (joint) k_rmm_vec<true><<<grid, RB_T, smem, s>>>(A);
+  else k_rmm_vec<false><<<grid, RB_T, smem, s>>>(A);
+  prof_end(m, s);
   m->stats.kernel_launches++;
-  if (m->hasConst) {
-    constRow = (double*)((char*)m->scratch + pBytes);
-    k_const_dot<<<1, 256, 0, s>>>(m->dConstV, dV, m->nCols, constRow);
-    m->stats.kernel_launches++;
-  }
-  // rows per thread: 128-bit map loads from about two million rows on, 32-bit ones below (measured on 100 groups of
-  // 16 values, ms per product for 4 / 8 / 16 rows per thread: 1M rows 0.052 / 0.071 / 0.057, 3M rows 0.127 / 0.142 /
-  // 0.127, 10M rows 0.358 / 0.449 / 0.322; eight rows per thread lose at every size)
-  int R = m->nRows >= (2 << 20) - 200000 ? 16 : 4;
-  if (const char* e = getenv("CLA_RMM_ROWS_PER_THREAD")) {  // tuning aid
-    const int v = atoi(e);
-    if (v == 4 || v == 8 || v == 16) R = v;
-  }
-  const int nTiles = (m->nRows + RMM_T * R - 1) / (RMM_T * R);
-  for (size_t c = 0; c < fp->rchunks.size(); c++) {
-    const RmmChunk& ch = fp->rchunks[c];
-    const size_t smem = (size_t)ch.tblDoubles * 8 + (size_t)(ch.g1 - ch.g0) * 12 + 16;
-    auto kern = R == 16 ? k_rmm_vec_u8<16> : (R == 8 ? k_rmm_vec_u8<8> : k_rmm_vec_u8<4>);
-    // as many CTAs as are resident at once (registers and shared memory decide): the tile loop does the rest, and
-    // no partial second wave is left over
-    int perSm = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kern, RMM_T, smem) != cudaSuccess || perSm < 1) {
-      cudaGetLastError();
-      perSm = 1;
-    }
-    const int grid = std::min(nTiles, m->smCount * perSm);
-    if (c == 0) prof_begin(m, s);
-    kern<<<grid, RMM_T, smem, s>>>(fp->dMaps, fp->dTblOff, ch.g0, ch.g1, P + ch.tblOff, ch.tblDoubles, m->nRows, constRow,
-                                   dOut, c > 0 ? 1 : 0, m->dErr);
-    if (c + 1 == fp->rchunks.size()) prof_end(m, s);
-    m->stats.kernel_launches++;
-  }
   CLA_CUDA(cudaGetLastError());
   return fp->partial ? 2 : 1;
+}
+
+// Units per chunk of k_lmm_vec: with few rows per CTA, staging the tables (32 KB per unit) costs more than the rows, so
+// the columns are spread over more CTAs; with many, wide chunks read y less often. Clocks, from the pipe's
+// wavefronts: 512 per unit staged, 1.13 per unit and 1 for y per row, and at least one round of steps.
+static int lmm_chunk_units(const FastPlan* fp, int nRows, int sm) {
+  int best = 1;
+  double bestCost = 1e300;
+  for (int U = 1; U <= LMM_MAX_UNITS; U++) {
+    const int nChunks = (fp->nU16 + U - 1) / U, u = (fp->nU16 + nChunks - 1) / nChunks;
+    if (nChunks > sm && U < LMM_MAX_UNITS) continue;
+    const double ctas = std::max(1.0, (double)sm / nChunks), rows = nRows / ctas, waves = std::ceil((double)nChunks / sm);
+    const double rounds = std::ceil(rows / (VSTEP * LMM_W));
+    const double cost = waves * (512.0 * u + std::max(rows * (1.13 * u + 1.0), rounds * (600.0 + 40.0 * u)));
+    if (cost < bestCost) bestCost = cost, best = u;
+  }
+  return best;
+}
+
+static size_t lmm_args(Matrix* m, FastPlan* fp, LmmArgs& A, int* grid) {
+  A.units = fp->dUnits;
+  A.imaps = fp->dLmmMaps;
+  A.nRB = fp->nRB;
+  A.tables = fp->dLmmTables;
+  A.slotCol = fp->dSlotCol;
+  A.nRows = m->nRows;
+  A.nU16 = fp->nU16;
+  A.U = lmm_chunk_units(fp, m->nRows, m->smCount);
+  A.nChunks = (fp->nU16 + A.U - 1) / A.U;
+  A.addTo = fp->uniqueCols ? 0 : 1;
+  A.constV = (m->hasConst && fp->uniqueCols) ? m->dConstV : nullptr;
+  A.bareCols = fp->dBareCols;
+  A.nBare = fp->nBare;
+  A.err = m->dErr;
+  A.part = 0;
+  A.parts = 1;
+  A.stepBegin = 0;
+  A.stepEnd = ((int64_t)m->nRows + VSTEP - 1) / VSTEP;
+  const int uLast = fp->nU16 - (A.nChunks - 1) * A.U;
+  const double w = 1.13 * A.U + 1.0, wl = 1.13 * uLast + 1.0, all = (A.nChunks - 1) * w + wl;
+  const int steps = (int)std::min<int64_t>(A.stepEnd, 1 << 20);
+  A.ctaFull = std::max(1, std::min(steps, (int)(m->smCount * w / all + 0.5)));
+  if (A.nChunks > 1 && A.ctaFull * (A.nChunks - 1) >= m->smCount) A.ctaFull = std::max(1, (m->smCount - 1) / (A.nChunks - 1));
+  A.ctaLast = std::max(1, std::min(steps, m->smCount - A.ctaFull * (A.nChunks - 1)));
+  *grid = A.ctaFull * (A.nChunks - 1) + A.ctaLast;
+  size_t smem = (size_t)LMM_W * (LMM_PART + 1) * 8;
+  for (int q = 0; q < fp->nU16; q += A.U) {
+    size_t b = 0;
+    for (int i = q; i < std::min(fp->nU16, q + A.U); i++) b += (size_t)fp->unitNk[i] * 128;
+    smem = std::max(smem, b);
+  }
+  return smem;
+}
+
+// k_lmm_final behind a kernel that lets it start early
+static int64_t launch_lmm_final(Matrix* m, const LmmArgs& A, int grid, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)A.nU16);
+  cfg.blockDim = dim3(LMM_T);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  CLA_CUDA(cudaLaunchKernelEx(&cfg, k_lmm_final, A, grid));
+  m->stats.kernel_launches++;
+  return CLA_OK;
+}
+// The product's last (or only) launch of k_lmm_vec and what finishes it
+static int64_t launch_lmm_vec(Matrix* m, const LmmArgs& A, int grid, size_t smem, cudaStream_t s) {
+  k_lmm_vec<<<grid, LMM_T, smem, s>>>(A);
+  m->stats.kernel_launches++;
+  if (A.parts) return launch_lmm_final(m, A, grid, s);
+  return CLA_OK;
+}
+
+// t(X) (w * (X v)) where one kernel can do it (see k_chain_vec); 0: not covered
+int64_t fast_chain(Matrix* m, const double* dV, const double* dW, double* dOut, double* dU, cudaStream_t s) {
+  FastPlan* fp = m->fast;
+  if (!fp || !fp->ok || fp->partial || !fp->uniqueCols || fp->nU16 > LMM_MAX_UNITS) return 0;
+  // many rows of small dictionaries: X v by joint slots and t(X) u by themselves take fewer lookups
+  if (fp->nJU16 > 0 && fp->nJU16 * 2 <= fp->nU16 && m->nRows >= (1 << 20)) return 0;
+  ChainArgs C{};
+  int grid;
+  lmm_args(m, fp, C.L, &grid);
+  C.L.U = fp->nU16;
+  C.L.nChunks = 1;
+  grid = (int)std::min<int64_t>(m->smCount, C.L.stepEnd);
+  C.L.ctaFull = C.L.ctaLast = grid;
+  size_t smem = (size_t)CH_W * (LMM_PART + 1) * 8, b = 0;
+  for (int nk : fp->unitNk) b += (size_t)nk * 128;
+  smem = std::max(smem, b);
+  if (smem > SMEM_MAX - CH_STATIC) return 0;
+  int64_t rc;
+  if ((rc = ensure_scratch(m, (size_t)grid * (LMM_PART + 1) * 8 + 256)) < 0) return rc;
+  C.L.partial = (double*)m->scratch;
+  C.L.out = dOut;
+  C.v = dV;
+  C.w = dW;
+  C.u = dU;
+  C.nCols = m->nCols;
+  static bool attrSet[64] = {};  // per device
+  if (!attrSet[m->device & 63]) {
+    CLA_CUDA(cudaFuncSetAttribute(k_chain_vec, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  SMEM_MAX - CH_STATIC));
+    attrSet[m->device & 63] = true;
+  }
+  prof_begin(m, s);
+  k_chain_vec<<<grid, CH_T, smem, s>>>(C);
+  m->stats.kernel_launches++;
+  if ((rc = launch_lmm_final(m, C.L, grid, s)) < 0) return rc;
+  prof_end(m, s);
+  CLA_CUDA(cudaGetLastError());
+  return 1;
 }
 
 int64_t fast_lmm_vec(Matrix* m, const double* dY, double* dOut, cudaStream_t s) {
   FastPlan* fp = m->fast;
   if (!fp || !fp->ok || ((uintptr_t)dY & 15)) return 0;  // 128-bit loads of the left vector need alignment
+  LmmArgs A{};
+  int grid;
+  const size_t smem = lmm_args(m, fp, A, &grid);
   int64_t rc;
-  const size_t partBytes = (size_t)fp->lmmGrid * LMM_PART * 8;
-  if ((rc = ensure_scratch(m, partBytes + 256)) < 0) return rc;
-  double* partial = (double*)m->scratch;
-  CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)m->nCols, s));
-  size_t smem = (size_t)LMM_W * LMM_PART * 8;
-  for (auto& c : fp->lchunks) smem = std::max(smem, (size_t)c.tblDoubles * 8);
+  if ((rc = ensure_scratch(m, (size_t)grid * (LMM_PART + 1) * 8 + 256)) < 0) return rc;
+  A.partial = (double*)m->scratch;
+  A.y = dY;
+  A.out = dOut;
+  if (A.addTo) CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)m->nCols, s));
   prof_begin(m, s);
-  const int64_t nSteps = ((int64_t)m->nRows + LMM_STEP - 1) / LMM_STEP;
-  k_lmm_vec_u8<<<fp->lmmGrid, LMM_T, smem, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dLmmMaps, fp->nRB, fp->dLmmTables, dY,
-                                               m->nRows, 0, nSteps, partial, m->dErr);
+  if ((rc = launch_lmm_vec(m, A, grid, smem, s)) < 0) return rc;
   prof_end(m, s);
-  k_lmm_vec_final<<<dim3((unsigned)fp->lchunks.size(), LMM_MAX_UNITS), 512, 0, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dSlotCol,
-                                                              partial, dOut, 1, fp->lmmGrid);
-  m->stats.kernel_launches += 2;
-  if (m->hasConst)
+  if (m->hasConst && !A.constV)
     if ((rc = launch_lmm_const(m, dY, 1, dOut, s)) < 0) return rc;
   CLA_CUDA(cudaGetLastError());
   return fp->partial ? 2 : 1;
 }
-
 
 // Q = 2 or 4 left rows (rows q of y at y + q * pitch, 16-byte aligned) in one pass; same return values as fast_lmm_vec.
 template <int Q>
@@ -1450,7 +1531,7 @@ static int64_t fast_lmm_rows_t(Matrix* m, FastPlan* fp, const double* dY, size_t
   CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)Q * m->nCols, s));
   size_t smem = (size_t)LQ_W * Q * LMM_PART * 8;
   for (auto& c : fp->lchunks) smem = std::max(smem, (size_t)c.tblDoubles * 8);
-  static bool attr[64] = {};
+  static bool attr[64] = {};  // per device
   if (!attr[m->device & 63]) {
     CLA_CUDA(cudaFuncSetAttribute(k_lmm_vecq_u8<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
     attr[m->device & 63] = true;
@@ -1491,19 +1572,21 @@ static int lmm_pipe_depth() {
 int64_t fast_lmm_vec_host(Matrix* m, const double* hostY, double* dY, double* dOut, cudaStream_t s) {
   FastPlan* fp = m->fast;
   if (!fp || !fp->ok || fp->partial || ((uintptr_t)dY & 15) || m->nRows < (1 << 20)) return 0;
+  LmmArgs A{};
+  int grid;
+  const size_t smem = lmm_args(m, fp, A, &grid);
   int64_t rc;
   const int LMM_PIPE = lmm_pipe_depth();
-  const size_t partBytes = (size_t)LMM_PIPE * fp->lmmGrid * LMM_PART * 8;
-  if ((rc = ensure_scratch(m, partBytes + 256)) < 0) return rc;
+  if ((rc = ensure_scratch(m, (size_t)LMM_PIPE * grid * (LMM_PART + 1) * 8 + 256)) < 0) return rc;
   if (!m->copyStream) {
     CLA_CUDA(cudaStreamCreateWithFlags(&m->copyStream, cudaStreamNonBlocking));
     for (int i = 0; i < LMM_PIPE_MAX; i++) CLA_CUDA(cudaEventCreateWithFlags(&m->copyDone[i], cudaEventDisableTiming));
   }
-  double* partial = (double*)m->scratch;
-  CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)m->nCols, s));
-  size_t smem = (size_t)LMM_W * LMM_PART * 8;
-  for (auto& c : fp->lchunks) smem = std::max(smem, (size_t)c.tblDoubles * 8);
-  const int64_t nSteps = ((int64_t)m->nRows + LMM_STEP - 1) / LMM_STEP;
+  A.partial = (double*)m->scratch;
+  A.y = dY;
+  A.out = dOut;
+  if (A.addTo) CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)m->nCols, s));
+  const int64_t nSteps = A.stepEnd;
   // the copy stream must not run ahead of work already queued on s that still reads dY
   CLA_CUDA(cudaEventRecord(m->ev1, s));
   CLA_CUDA(cudaStreamWaitEvent(m->copyStream, m->ev1, 0));
@@ -1514,7 +1597,7 @@ int64_t fast_lmm_vec_host(Matrix* m, const double* hostY, double* dY, double* dO
   auto range_start = [&](int i) { return nSteps * ((int64_t)i * (2 * LMM_PIPE - i + 1) / 2) / wSum; };  // i ranges: n + ... + (n - i + 1)
   auto range_rows = [&](int i, int64_t& sb, int64_t& se, int64_t& rb, int64_t& re) {
     sb = range_start(i), se = i + 1 == LMM_PIPE ? nSteps : range_start(i + 1);
-    rb = sb * LMM_STEP, re = std::min<int64_t>(m->nRows, se * LMM_STEP);
+    rb = sb * VSTEP, re = std::min<int64_t>(m->nRows, se * VSTEP);
   };
   // the kernel of row range i, once that range of y is on the copy stream
   auto launch_range = [&](int i) -> int64_t {
@@ -1523,11 +1606,13 @@ int64_t fast_lmm_vec_host(Matrix* m, const double* hostY, double* dY, double* dO
     CLA_CUDA(cudaEventRecord(m->copyDone[i], m->copyStream));
     CLA_CUDA(cudaStreamWaitEvent(s, m->copyDone[i], 0));
     if (i == 0) prof_begin(m, s);
-    k_lmm_vec_u8<<<fp->lmmGrid, LMM_T, smem, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dLmmMaps, fp->nRB, fp->dLmmTables,
-                                                 dY, m->nRows, sb, se, partial + (size_t)i * fp->lmmGrid * LMM_PART,
-                                                 m->dErr);
+    A.stepBegin = sb;
+    A.stepEnd = se;
+    A.part = i;
+    A.parts = i == LMM_PIPE - 1 ? LMM_PIPE : 0;  // the last range's launch adds up all ranges' partial sums
+    const int64_t r = launch_lmm_vec(m, A, grid, smem, s);
+    if (r < 0) return r;
     if (i == LMM_PIPE - 1) prof_end(m, s);
-    m->stats.kernel_launches++;
     return CLA_OK;
   };
   if (host_copy_staged(m, hostY, (size_t)m->nRows * 8)) {
@@ -1555,10 +1640,7 @@ int64_t fast_lmm_vec_host(Matrix* m, const double* hostY, double* dY, double* dO
       if ((rc = launch_range(i)) < 0) return rc;
     }
   }
-  k_lmm_vec_final<<<dim3((unsigned)fp->lchunks.size(), LMM_MAX_UNITS), 512, 0, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dSlotCol, partial,
-                                                              dOut, LMM_PIPE, fp->lmmGrid);
-  m->stats.kernel_launches++;
-  if (m->hasConst)
+  if (m->hasConst && !A.constV)
     if ((rc = launch_lmm_const(m, dY, 1, dOut, s)) < 0) return rc;
   CLA_CUDA(cudaGetLastError());
   return 1;
@@ -1574,7 +1656,7 @@ int64_t fast_lmm_vec_host(Matrix* m, const double* hostY, double* dY, double* dO
 // whose context loads the library holds the array (about 450 KB) until the process exits.
 // --------------------------------------------------------------------------------------------------
 constexpr int NOALLOC_MAX_CTAS = 512;  // partial-sum rows available; one CTA per SM is launched, more only with > 148 column chunks
-constexpr size_t NOALLOC_PARTIAL_DOUBLES = (size_t)NOALLOC_MAX_CTAS * LMM_PART;
+constexpr size_t NOALLOC_PARTIAL_DOUBLES = (size_t)NOALLOC_MAX_CTAS * (LMM_PART + 1);
 static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_PARTIAL_DOUBLES + 32];
 
 static std::mutex g_noallocMu;
@@ -1601,25 +1683,23 @@ int64_t fast_lmm_vec_noalloc(Matrix* m, const double* dY, double* dOut, cudaStre
   if (!fp || !fp->ok || fp->partial)
     return fail(CLA_ERR_UNSUPPORTED, "no-allocation product: needs dense-map groups with at most 256 tuples and byte maps");
   if ((uintptr_t)dY & 15) return fail(CLA_ERR_BAD_ARG, "no-allocation product: the left vector must be 16-byte aligned");
-  if (fp->lmmGrid > NOALLOC_MAX_CTAS)
-    return fail(CLA_ERR_UNSUPPORTED, "no-allocation product: the matrix needs " + std::to_string(fp->lmmGrid) +
+  LmmArgs A{};
+  int grid;
+  const size_t smem = lmm_args(m, fp, A, &grid);
+  if (grid > NOALLOC_MAX_CTAS)
+    return fail(CLA_ERR_UNSUPPORTED, "no-allocation product: the matrix needs " + std::to_string(grid) +
                                          " partial-sum rows, the fixed scratch holds " + std::to_string(NOALLOC_MAX_CTAS));
   double* scratch = nullptr;
   int64_t rc = noalloc_address(m->device, &scratch);
   if (rc < 0) return rc;
   m->stats.calls_lmm++;
-  double* partial = scratch;                           // fully rewritten by every launch
+  A.partial = scratch;                                 // fully rewritten by every launch
   double* rowSum = scratch + NOALLOC_PARTIAL_DOUBLES;  // accumulated with atomics: cleared below before use
-  CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)m->nCols, s));
-  size_t smem = (size_t)LMM_W * LMM_PART * 8;
-  for (auto& c : fp->lchunks) smem = std::max(smem, (size_t)c.tblDoubles * 8);
-  const int64_t nSteps = ((int64_t)m->nRows + LMM_STEP - 1) / LMM_STEP;
-  k_lmm_vec_u8<<<fp->lmmGrid, LMM_T, smem, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dLmmMaps, fp->nRB, fp->dLmmTables,
-                                               dY, m->nRows, 0, nSteps, partial, m->dErr);
-  k_lmm_vec_final<<<dim3((unsigned)fp->lchunks.size(), LMM_MAX_UNITS), 512, 0, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dSlotCol,
-                                                              partial, dOut, 1, fp->lmmGrid);
-  m->stats.kernel_launches += 2;
-  if (m->hasConst)
+  A.y = dY;
+  A.out = dOut;
+  if (A.addTo) CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)m->nCols, s));
+  if ((rc = launch_lmm_vec(m, A, grid, smem, s)) < 0) return rc;
+  if (m->hasConst && !A.constV)
     if ((rc = launch_lmm_const_with(m, dY, 1, dOut, rowSum, s)) < 0) return rc;
   CLA_CUDA(cudaGetLastError());
   return CLA_OK;

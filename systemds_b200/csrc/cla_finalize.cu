@@ -479,7 +479,9 @@ int64_t init_device_state(Matrix* m) {
   CLA_CUDA(cudaEventCreateWithFlags(&m->lastDone, cudaEventDisableTiming));
   void* errp = nullptr;
   CLA_CUDA(cudaMalloc(&errp, 64));
-  CLA_CUDA(cudaMemset(errp, 0, 64));
+  // (on the handle's own stream: a clear on the default stream could run after the first checks have reported)
+  CLA_CUDA(cudaMemsetAsync(errp, 0, 64, m->stream));
+  CLA_CUDA(cudaStreamSynchronize(m->stream));
   m->dErr = (int32_t*)errp;
   m->dFin = (unsigned long long*)((char*)errp + 16);
   return CLA_OK;
@@ -489,6 +491,9 @@ int64_t finalize_device(Matrix* m) {
   int64_t rc0 = init_device_state(m);
   if (rc0 < 0) return rc0;
 
+  // maps and dense blocks registered from device memory may still be being written by work on the default stream
+  CLA_CUDA(cudaEventRecord(m->lastDone, nullptr));
+  CLA_CUDA(cudaStreamWaitEvent(m->stream, m->lastDone, 0));
   m->constV.assign(m->nCols, 0.0);
   m->regToDev.assign(m->hg.size(), -1);
   m->groups.clear();

@@ -1,0 +1,111 @@
+"""Products at the sizes where the specialised kernels change over: edges of tiles, remainders, smallest and largest of
+their ranges. Checked against the dense product of the decompressed block, relative to the summed magnitudes."""
+import numpy as np
+import pytest
+
+from systemds_b200 import CompressedMatrixBlock, datagen
+from systemds_b200 import colgroup as cg
+from systemds_b200.cmb import CHAIN_XtwXv, CLALibDecompress, CLALibLeftMultBy, CLALibMMChain, CLALibRightMultBy, CLALibTSMM
+from systemds_b200.mapping import MapToFactory
+from tests.util import TOL, dense_of, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _ddc(nRows, cards, seed, const=False, width=1):
+    rng = np.random.default_rng(seed)
+    groups, c = [], 0
+    for k in cards:
+        groups.append(cg.ColGroupDDC(list(range(c, c + width)), rng.standard_normal((k, width)),
+                                     MapToFactory.create_from(rng.integers(0, k, nRows), k)))
+        c += width
+    if const:
+        groups.append(cg.ColGroupConst([c], [[0.75]]))
+        c += 1
+    return CompressedMatrixBlock(nRows, c, groups)
+
+
+def _check(cmb, ks=(1,), qs=(1,), chain=True, seed=0):
+    X = dense_of(cmb)
+    aX = np.abs(X)
+    n, m = X.shape
+    rng = np.random.default_rng(seed)
+    for k in ks:
+        V = rng.standard_normal((m, k))
+        got = CLALibRightMultBy.rightMultByMatrix(cmb, V)
+        assert rel_err(got, X @ V, aX @ np.abs(V) + 1e-300) < TOL, ("rmm", k)
+        assert got.nnz == np.count_nonzero(got)
+    for q in qs:
+        Y = rng.standard_normal((q, n))
+        got = CLALibLeftMultBy.leftMultByMatrix(cmb, Y)
+        assert rel_err(got, Y @ X, np.abs(Y) @ aX + 1e-300) < TOL, ("lmm", q)
+        assert got.nnz == np.count_nonzero(got)
+    if chain:
+        v, w = rng.standard_normal(m), rng.standard_normal(n)
+        s = aX.T @ (np.abs(w) * (aX @ np.abs(v))) + 1e-300
+        assert rel_err(CLALibMMChain.mmChain(cmb, v, w, CHAIN_XtwXv).ravel(), X.T @ (w * (X @ v)), s) < 10 * TOL
+        s = aX.T @ (aX @ np.abs(v)) + 1e-300
+        assert rel_err(CLALibMMChain.mmChain(cmb, v).ravel(), X.T @ (X @ v), s) < 10 * TOL
+
+
+@pytest.mark.parametrize("nRows", [1, 31, 33, 1025, 4095, 4096])
+def test_short_blocks_every_group_type(nRows):
+    """The one-kernel products on blocks below 4096 rows, and the first row count above them."""
+    kinds = datagen.KINDS + ("ddcfor", "ddc2", "ole", "rle", "sdc")
+    cmb = datagen.random_cmb(31 * nRows + 7, nRows, kinds).to_device()
+    _check(cmb, ks=(1, 3, 5, 8, 9), qs=(1, 2, 4, 5))
+    cmb.free()
+
+
+@pytest.mark.parametrize("nCols", [450, 900])
+def test_short_blocks_wide_right_operand(nCols):
+    """V beyond what travels with the launch (448 values) and beyond what fits shared memory (6144)."""
+    cmb = _ddc(77, [5] * nCols, nCols, const=True).to_device()
+    _check(cmb, ks=(1, 8), chain=False)
+    cmb.free()
+
+
+@pytest.mark.parametrize("nRows,nCols", [(4097, 16), (4127, 17), (5000, 112), (5000, 113), (9000, 240), (300007, 20)])
+@pytest.mark.parametrize("card", [2, 7, 16, 256])
+def test_byte_map_units(nRows, nCols, card):
+    """Column-per-lane kernels: last unit partly filled, one unit more than the fused chain takes, several chunks, joint
+    slots (tall blocks of small dictionaries), bit maps; a constant column."""
+    cmb = _ddc(nRows, [card] * nCols, nRows + nCols + card, const=nCols % 2 == 1).to_device()
+    _check(cmb)
+    cmb.free()
+
+
+def test_joint_slots_of_uneven_dictionaries():
+    """Mixed-radix joint ids: one to eight groups per slot, single tuples, co-coded columns."""
+    cards = [1, 1, 2, 2, 2, 3, 3, 5, 7, 11, 13, 16, 17, 40, 128, 255, 256] + [2] * 20 + [3] * 15
+    for width in (1, 2):
+        cmb = _ddc(300001, cards, 5 + width, width=width).to_device()
+        _check(cmb)
+        cmb.free()
+
+
+@pytest.mark.parametrize("nRows", [5000, 300007])
+def test_non_finite_values_stay_in_their_rows(nRows):
+    """Inf and NaN dictionary entries reach the rows that hold them and no other (the row sums of neighbouring rows are
+    formed by one matrix product)."""
+    rng = np.random.default_rng(1)
+    groups = []
+    for c in range(40):
+        d = rng.standard_normal((100, 1))
+        if c % 13 == 0:
+            d[5], d[6] = np.inf, np.nan
+        ids = rng.integers(7, 100, nRows)
+        hit = rng.random(nRows) < 0.01
+        ids[hit] = rng.integers(5, 7, int(hit.sum()))
+        groups.append(cg.ColGroupDDC([c], d, MapToFactory.create_from(ids, 100)))
+    cmb = CompressedMatrixBlock(nRows, 40, groups).to_device()
+    X = dense_of(cmb)
+    v = rng.standard_normal(40)
+    with np.errstate(invalid="ignore"):
+        want = X @ v
+    got = np.asarray(CLALibRightMultBy.rightMultByMatrix(cmb, v)).ravel()
+    fine = np.isfinite(X).all(axis=1)
+    assert 0 < fine.sum() < nRows
+    assert np.array_equal(np.isfinite(got), fine)
+    assert rel_err(got[fine], want[fine], np.abs(X[fine]) @ np.abs(v)) < TOL
+    cmb.free()
