@@ -423,6 +423,14 @@ __global__ void k_vectors_to_rows(const double* __restrict__ U, int64_t nRows, i
     for (int j = 0; j < vCols; j++) out[r * vCols + j] = U[(int64_t)j * stride + r];
 }
 
+// One right-hand column; dW: factors applied to the rows (null: none)
+static int64_t rmm_vec(Matrix* m, const double* dV, const double* dW, double* dOut, cudaStream_t s) {
+  const int64_t rc = fast_rmm_vec(m, dV, dOut, fast_plan_partial(m) ? nullptr : dW, s);
+  if (rc < 0) return rc;
+  if (rc == 1) return CLA_OK;
+  return launch_rmm(m, dV, dW, dOut, s, rc == 2);
+}
+
 static int64_t rmm_by_vectors(Matrix* m, const double* dV, int32_t vCols, double* dOut, cudaStream_t s) {
   const size_t vtBytes = (((size_t)vCols * m->nCols * sizeof(double)) + 255) & ~(size_t)255;
   const size_t rowsPad = ((size_t)m->nRows + 31) & ~(size_t)31;
@@ -434,11 +442,7 @@ static int64_t rmm_by_vectors(Matrix* m, const double* dV, int32_t vCols, double
   k_small_transpose<<<(cells + 255) / 256, 256, 0, s>>>(dV, m->nCols, vCols, Vt);
   for (int j = 0; j < vCols; j++) {
     double* uj = U + rowsPad * j;
-    rc = fast_rmm_vec(m, Vt + (size_t)j * m->nCols, uj, nullptr, s);
-    if (rc < 0) return rc;
-    if (rc == 2) rc = launch_rmm(m, Vt + (size_t)j * m->nCols, 1, uj, s, true);
-    else if (rc == 0) rc = launch_rmm(m, Vt + (size_t)j * m->nCols, 1, uj, s);
-    if (rc < 0) return rc;
+    if ((rc = rmm_vec(m, Vt + (size_t)j * m->nCols, nullptr, uj, s)) < 0) return rc;
   }
   k_vectors_to_rows<<<m->smCount * 8, 256, 0, s>>>(U, m->nRows, (int64_t)rowsPad, vCols, dOut);
   m->stats.kernel_launches += 2;
@@ -464,12 +468,7 @@ static int64_t rmm_dev(Matrix* m, const double* dV, int32_t vRows, int32_t vCols
     if (hc) hc->used = rc == 1;
     if (rc != 0) return rc < 0 ? rc : CLA_OK;
   }
-  if (vCols == 1) {
-    int64_t rc = fast_rmm_vec(m, dV, dOut, nullptr, s);
-    if (rc < 0) return rc;
-    if (rc == 1) return CLA_OK;
-    return launch_rmm(m, dV, 1, dOut, s, rc == 2);
-  }
+  if (vCols == 1) return rmm_vec(m, dV, nullptr, dOut, s);
   // A pass of the one-column kernels per column beats the tensor-core kernel (whose time hardly depends on
   // the width up to 64 columns) for a few columns; measured crossover: about 16 columns when every group is
   // a byte-map DDC group (2M x 200: 0.26 ms per column against 4.3 ms), about 7 when SDC / RLE groups take
@@ -488,21 +487,14 @@ static int64_t lmm_dev(Matrix* m, const double* dYt, int32_t yRows, double* dOut
     if (hc) hc->used = rc == 1;
     if (rc != 0) return rc < 0 ? rc : CLA_OK;
   }
-  if (yRows == 1) {
-    int64_t rc = fast_lmm_vec(m, dYt, dOut, s);
-    if (rc < 0) return rc;
-    if (rc == 1) return CLA_OK;
-    if (rc == 2) return launch_lmm(m, dYt, yRows, dOut, s, true);
-  }
-  // Several left rows: passes of the column-per-lane kernels over four, two or one row at a time for the groups they
-  // cover (measured 0.17 ms per row on 2M x 200 for the one-row kernel against 1.5 ms per row in the general
-  // pre-aggregation kernel), the general kernels for the rest. Rows of an odd-length Yt are not 16-byte aligned, so they are copied to a padded pitch first.
-  static const int lmmLoopMax = loop_limit("CLA_LMM_LOOP_MAX", 1 << 30);  // tuning aid
-  if (yRows >= 2 && yRows <= lmmLoopMax && fast_plan_ok(m) && m->nRows > 0) {
+  // Passes of the column-per-lane kernels over four, two or one left rows at a time for the groups they cover; the
+  // other groups eight at a time. The former read the left rows with 128-bit loads: rows that are not 16-byte aligned
+  // are copied to an even pitch first.
+  if (yRows >= 1 && fast_plan_ok(m) && m->nRows > 0) {
     const double* rows = dYt;
     size_t pitch = (size_t)m->nRows;
-    if (m->nRows & 1) {
-      pitch = (size_t)m->nRows + 1;
+    if (((uintptr_t)dYt & 15) || (yRows > 1 && (m->nRows & 1))) {
+      pitch = ((size_t)m->nRows + 1) & ~(size_t)1;
       int64_t rc = ensure_scratch2(m, pitch * yRows * sizeof(double));
       if (rc < 0) return rc;
       CLA_CUDA(cudaMemcpy2DAsync(m->scratch2, pitch * sizeof(double), dYt, (size_t)m->nRows * sizeof(double),
@@ -510,7 +502,7 @@ static int64_t lmm_dev(Matrix* m, const double* dYt, int32_t yRows, double* dOut
       rows = (const double*)m->scratch2;
     }
     int64_t rc = 0;
-    for (int i = 0; i < yRows;) {  // four rows per pass over the maps, then two, then one
+    for (int i = 0; i < yRows;) {
       const int q = yRows - i >= 4 ? 4 : (yRows - i >= 2 ? 2 : 1);
       rc = q == 1 ? fast_lmm_vec(m, rows + pitch * i, dOut + (size_t)i * m->nCols, s)
                   : fast_lmm_rows(m, rows + pitch * i, pitch, q, dOut + (size_t)i * m->nCols, s);
@@ -544,19 +536,10 @@ static int64_t mmchain_dev(Matrix* m, const double* dV, const double* dW, int32_
     dU = (double*)m->scratch2;
   }
   int64_t rc = 0;
-  if (small_block(m)) {  // the weights are applied where the row sums are written
-    rc = small_rmm(m, dV, 1, dU, ctype == CLA_CHAIN_XtwXv ? dW : nullptr, s, Finish());
-    if (rc < 0) return rc;
-  } else if (fast_plan_ok(m) && !fast_plan_partial(m)) {
-    rc = fast_rmm_vec(m, dV, dU, ctype == CLA_CHAIN_XtwXv ? dW : nullptr, s);
-    if (rc < 0) return rc;
-  }
-  if (rc == 0) {
-    if ((rc = rmm_dev(m, dV, m->nCols, 1, dU, s)) < 0) return rc;
-    if (ctype == CLA_CHAIN_XtwXv)
-      if ((rc = launch_scale_rows(m, dU, dW, m->nRows, s)) < 0) return rc;
-  } else
-    m->stats.calls_rmm++;
+  const double* w = ctype == CLA_CHAIN_XtwXv ? dW : nullptr;  // applied where the row sums are written
+  if (small_block(m) && (rc = small_rmm(m, dV, 1, dU, w, s, Finish())) < 0) return rc;
+  if (rc == 0 && (rc = rmm_vec(m, dV, w, dU, s)) < 0) return rc;
+  m->stats.calls_rmm++;
   return lmm_dev(m, dU, 1, dOut, s, hc);
 }
 

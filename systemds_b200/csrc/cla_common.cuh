@@ -185,6 +185,24 @@ struct RowLists {
   uint32_t* fullItems = nullptr;
   uint32_t* partPtr = nullptr;      // runs that cover part of a window: table row, first row | end row << 8 in the window
   uint2* partItems = nullptr;
+  // the same listed rows group by group, element order: row in its 1024-row block | tuple << 10
+  uint32_t* sdcItems = nullptr;
+  std::vector<int64_t> sdcBase;     // [nDev] first item of a group
+};
+// One column of a group the column-per-lane kernels do not take, as the left product walks it (cla_rest.cu).
+struct RestTask {
+  const double* src;   // dictionary + position of the column
+  const void* a;       // SDC: items; RLE: runs; dense map: map
+  const void* b;       // SDC: skip entries; RLE: first run of every block; dense map: high bytes
+  int64_t n;           // SDC: listed rows; RLE: runs
+  int32_t kind, mapType, stride, col;
+};
+struct RestPlan {
+  bool tried = false, ok = false;
+  int nTasks = 0, nUnc = 0, nDense = 0;
+  RestTask* tasks = nullptr;      // SDC, RLE and remaining dense-map columns
+  ColRef* dense = nullptr;        // the remaining dense-map columns, list order
+  std::vector<int> unc;           // device group indices of the uncompressed groups
 };
 struct ColPlan {
   bool built = false;
@@ -283,6 +301,7 @@ struct Matrix {
   FastPlan* fast = nullptr;
   RowLists rows;
   ColPlan cols;
+  RestPlan rest;
   HostStage* hostStage = nullptr;
   char* mail = nullptr;          // pinned: Mailbox, inputs, outputs (small host-buffer calls)
   unsigned long long* dFin = nullptr;  // device counters of Finish
@@ -328,6 +347,10 @@ int64_t ensure_sparse_lists(Matrix* m, cudaStream_t s);  // the row-major work l
 
 int64_t ensure_col_plan(Matrix* m);                        // Matrix::cols
 int64_t ensure_row_lists(Matrix* m, cudaStream_t s);       // Matrix::rows; rows.ok tells whether they exist
+// The groups the specialised kernels leave (cla_rest.cu): 1 = done, 0 = not covered (the general kernels then run)
+int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s, bool addTo);
+int64_t rest_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s);
+int64_t plan_alloc(Matrix* m, void** p, size_t bytes);
 // Short blocks (cla_small.cu): one kernel per product, every group type. 1 = done, 0 = not covered
 bool small_block(const Matrix* m);
 int64_t small_rmm(Matrix* m, const double* dV, int vCols, double* dOut, const double* dW, cudaStream_t s, const Finish& fin,
@@ -339,7 +362,8 @@ char* mailbox_take();
 void mailbox_give(char* p);
 
 // launchers implemented in the kernel translation units; all enqueue on `s` and return CLA_OK or an error.
-int64_t launch_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStream_t s, bool afterFast = false);
+// X v over the groups the specialised kernels leave (all without them), scaled by dW (null: not)
+int64_t launch_rmm(Matrix* m, const double* dV, const double* dW, double* dOut, cudaStream_t s, bool afterFast = false);
 int64_t launch_rmm_dmma(Matrix* m, const double* dV, int vCols, double* dOut, cudaStream_t s);
 int64_t launch_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s, bool afterFast = false);
 void minmax_of_group(const HostGroup& hg, int nRows, std::vector<double>& colMin, std::vector<double>& colMax);

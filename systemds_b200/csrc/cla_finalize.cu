@@ -441,7 +441,14 @@ static size_t map_bytes(int mapType, int64_t size, size_t* hiBytes) {
 static int64_t build_sdc_skip(const HostGroup& hg, int nRows, std::vector<SdcSkip>& skip) {
   const int nb = (nRows + SKIP_ROWS - 1) / SKIP_ROWS;
   skip.assign(std::max(nb, 1), SdcSkip{(int32_t)hg.nOff, nRows, hg.offLen});
-  if (hg.offType != CLA_OFF_BYTE && hg.offType != CLA_OFF_CHAR) return CLA_OK;  // one or two rows: held by the record
+  if (hg.offType == CLA_OFF_SINGLE || hg.offType == CLA_OFF_TWO) {  // rows held by the record: only the positions matter
+    for (int b = 0; b < nb; b++) {
+      const int64_t r = (int64_t)b * SKIP_ROWS;
+      skip[b].elem = r <= hg.first ? 0 : ((hg.offType == CLA_OFF_TWO && r <= hg.last) ? 1 : (int32_t)hg.nOff);
+    }
+    return CLA_OK;
+  }
+  if (hg.offType != CLA_OFF_BYTE && hg.offType != CLA_OFF_CHAR) return CLA_OK;
   const int maxV = hg.offType == CLA_OFF_BYTE ? 255 : 65535;
   const uint8_t* b = hg.offData.data();
   const uint16_t* c = (const uint16_t*)hg.offData.data();

@@ -69,21 +69,13 @@ __global__ void k_const_times_v(const double* __restrict__ constV, int nCols, co
 constexpr int RV_THREADS = 256;
 constexpr int RV_WARPS = RV_THREADS / 32;
 constexpr size_t RV_SMEM = (size_t)(RV_WARPS + 1) * SKIP_ROWS * sizeof(double);
-// LISTS: the SDC / RLE contributions come from the row-major work lists (8-row steps, 64-row windows) instead of the
-// rounds of step 3: a thread owns one step of the block and applies its items in list order to its own eight sums,
-// a thread per window sums the runs that cover the window. No staging tile, two shared-memory updates per listed
-// row instead of sixteen per row and round.
-constexpr size_t RV_SMEM_LISTS = (size_t)(2 * SKIP_ROWS + 16) * sizeof(double);
-template <bool LISTS>
 __global__ void __launch_bounds__(RV_THREADS)
 k_rmm_vec_general(const DevGroup* __restrict__ groups, const int32_t* __restrict__ ddcIdx, int nDdc,
                   const int32_t* __restrict__ uncIdx, int nUnc, const int32_t* __restrict__ sparseIdx, int nSparse, int nRows, const double* __restrict__ P, const double* __restrict__ v,
-                  const double* __restrict__ constRow, double* __restrict__ out, int afterFast,
-                  const SpItem* __restrict__ stepItems, const uint32_t* __restrict__ stepPtr, int64_t nStepPtr,
-                  const SpItem* __restrict__ winItems, const uint32_t* __restrict__ winPtr, int64_t nWinPtr) {
+                  const double* __restrict__ constRow, double* __restrict__ out, int afterFast) {
   extern __shared__ __align__(16) double rvsm[];
   double* acc = rvsm;                  // [SKIP_ROWS]
-  double* stage = rvsm + SKIP_ROWS;    // [RV_WARPS][SKIP_ROWS]; LISTS: sums of the steps [8][128], then 16 window sums
+  double* stage = rvsm + SKIP_ROWS;    // [RV_WARPS][SKIP_ROWS]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r0 = blockIdx.x * SKIP_ROWS, r1 = min(nRows, r0 + SKIP_ROWS);
   for (int i = tid; i < SKIP_ROWS; i += RV_THREADS) acc[i] = 0.0;
@@ -125,43 +117,6 @@ k_rmm_vec_general(const DevGroup* __restrict__ groups, const int32_t* __restrict
     }
   }
   if (nUnc) __syncthreads();
-  if (LISTS) {
-    constexpr int NSTEP = SKIP_ROWS / G3_STEP, NWIN = SKIP_ROWS / G3_WIN;  // 128 steps, 16 windows per block
-    double* sacc = stage;                 // row i of step t at [i * NSTEP + t]: neighbouring threads, neighbouring words
-    double* wbase = stage + SKIP_ROWS;    // [NWIN]
-    for (int i = tid; i < SKIP_ROWS; i += RV_THREADS) sacc[i] = 0.0;
-    __syncthreads();
-    if (tid < NWIN) {  // runs that cover a whole window
-      const int64_t w = (int64_t)blockIdx.x * NWIN + tid;
-      const uint32_t p0 = winPtr[min(w, nWinPtr - 1)], p1 = winPtr[min(w + 1, nWinPtr - 1)];
-      double sum = 0.0;
-      for (uint32_t i = p0; i < p1; i++) sum += P[winItems[i].prow];
-      wbase[tid] = sum;
-    } else if (tid >= RV_THREADS - NSTEP) {  // listed rows and run pieces of one 8-row step, in list order
-      const int t = tid - (RV_THREADS - NSTEP);
-      const int64_t st = (int64_t)blockIdx.x * NSTEP + t;
-      const uint32_t p0 = stepPtr[min(st, nStepPtr - 1)], p1 = stepPtr[min(st + 1, nStepPtr - 1)];
-      SpItem e = p0 < p1 ? stepItems[p0] : SpItem{0, 0};
-      for (uint32_t i = p0; i < p1; i++) {
-        const SpItem nxt = i + 1 < p1 ? stepItems[i + 1] : SpItem{0, 0};  // next item in flight during this one's table read
-        const double p = P[e.prow];
-        const int ra = e.rows & 0xFF, rb = (e.rows >> 8) & 0xFF;
-        for (int r = ra; r < rb; r++) sacc[r * NSTEP + t] += p;
-        e = nxt;
-      }
-    }
-    __syncthreads();
-    const double c0 = (constRow != nullptr && !afterFast) ? constRow[0] : 0.0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int rr = tid * 4 + i, r = r0 + rr;
-      if (r < r1) {
-        const double val = ((acc[rr] + sacc[(rr & 7) * NSTEP + (rr >> 3)]) + wbase[rr >> 6]) + c0;
-        out[r] = afterFast ? out[r] + val : val;
-      }
-    }
-    return;
-  }
   // SDC / RLE groups, eight per round. From here on thread t owns rows 4 t .. 4 t + 3.
   double a4[4];
   {
@@ -247,9 +202,16 @@ int64_t ensure_sparse_list(Matrix* m) {
   return CLA_OK;
 }
 
-int64_t launch_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStream_t s, bool afterFast) {
-  if (m->nRows == 0 || vCols == 0) return CLA_OK;
-  if (vCols != 1) return fail(CLA_ERR_UNSUPPORTED, "rmm: the general kernel takes one right-hand column");
+int64_t launch_rmm(Matrix* m, const double* dV, const double* dW, double* dOut, cudaStream_t s, bool afterFast) {
+  if (m->nRows == 0) return CLA_OK;
+  {
+    const int64_t rc = rest_rmm(m, dV, dOut, dW, s, afterFast);
+    if (rc != 0) return rc < 0 ? rc : CLA_OK;
+  }
+  if (dW) {  // no row lists: the kernel below does not scale
+    const int64_t rc = launch_rmm(m, dV, nullptr, dOut, s, afterFast);
+    return rc < 0 ? rc : launch_scale_rows(m, dOut, dW, m->nRows, s);
+  }
   if (afterFast) {  // nothing left for this pass if the specialised kernels covered every group
     bool rest = false;
     for (auto& g : m->groups) rest |= !g.inFast;
@@ -277,27 +239,15 @@ int64_t launch_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStr
   static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
   bool& attr = attrSet[m->device & 63];
   if (!attr) {
-    CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec_general<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RV_SMEM));
+    CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec_general, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RV_SMEM));
     attr = true;
-  }
-  // matrices with many listed rows: the row-major work lists (shared with the tensor-core right product), built once
-  bool lists = false;
-  if (m->nSparse > 0 && m->nRows >= 4 * SKIP_ROWS) {
-    if ((rc = ensure_sparse_lists(m, s)) < 0) return rc;
-    lists = m->spListsOk && m->dStepPtr != nullptr;
   }
   const int32_t* ddcIdx = afterFast ? m->dDdcRestIdx : m->dDdcIdx;
   const int nDdc = afterFast ? m->nDdcRest : m->nDdc;
   prof_begin(m, s);
   const unsigned grid = (unsigned)((m->nRows + SKIP_ROWS - 1) / SKIP_ROWS);
-  if (lists)
-    k_rmm_vec_general<true><<<grid, RV_THREADS, RV_SMEM_LISTS, s>>>(
-        m->dGroups, ddcIdx, nDdc, m->dUncIdx, m->nUnc, m->dSparseIdx, m->nSparse, m->nRows, P, dV, constRow, dOut, afterFast ? 1 : 0,
-        (const SpItem*)m->dStepItems, m->dStepPtr, m->nStepPtr, (const SpItem*)m->dWinItems, m->dWinPtr, m->nWinPtr);
-  else
-    k_rmm_vec_general<false><<<grid, RV_THREADS, RV_SMEM, s>>>(m->dGroups, ddcIdx, nDdc, m->dUncIdx, m->nUnc, m->dSparseIdx, m->nSparse, m->nRows, P, dV,
-                                                             constRow, dOut, afterFast ? 1 : 0, nullptr, nullptr, 0, nullptr,
-                                                             nullptr, 0);
+  k_rmm_vec_general<<<grid, RV_THREADS, RV_SMEM, s>>>(m->dGroups, ddcIdx, nDdc, m->dUncIdx, m->nUnc, m->dSparseIdx, m->nSparse, m->nRows, P, dV,
+                                                     constRow, dOut, afterFast ? 1 : 0);
   prof_end(m, s);
   m->stats.kernel_launches++;
   CLA_CUDA(cudaGetLastError());
@@ -623,11 +573,10 @@ constexpr int LMM_HIST_MAX = 6144;        // doubles of shared histogram (48 KB)
 // grid: (row chunks, dictionary groups, q tiles). A: [totalVals x q]
 __global__ void __launch_bounds__(LMM_THREADS)
 k_lmm_preagg(const DevGroup* __restrict__ groups, int nRows, int rowsPerChunk, const double* __restrict__ Yt, int q,
-             double* __restrict__ A, int skipFast, int skipSparse) {
+             double* __restrict__ A, int skipFast) {
   __shared__ double hist[LMM_HIST_MAX];
   const DevGroup& g = groups[blockIdx.y];
   if (g.type == GT_UNC || (skipFast && g.inFast)) return;
-  if (skipSparse && (g.type == GT_SDC || g.type == GT_RLE)) return;  // taken from the row-major work lists (k_lmm_lists)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ra = blockIdx.x * rowsPerChunk, rb = min(nRows, ra + rowsPerChunk);
   if (ra >= rb) return;
@@ -746,64 +695,17 @@ __global__ void k_lmm_const(const double* __restrict__ sums, const double* __res
     out[e] += sums[e / nCols] * constV[e % nCols];
 }
 
-// Pre-aggregation of the SDC / RLE groups for one left row from the row-major work lists: A[table row] += the left
-// values of the rows an item covers. A CTA walks 1024-row blocks (left values staged in shared memory, with their
-// sums per 64-row window); the block's items are read coalesced, a thread per item (an item names its step or window
-// inside the block), and added to a table in shared memory that goes to A once per CTA. (The per-group form walks
-// every offset stream and, for RLE, reads the whole left row once per group.) Like the general left product this
-// combines partial sums with atomics.
-constexpr int LL_THREADS = 256;
-__global__ void __launch_bounds__(LL_THREADS)
-k_lmm_lists(const SpItem* __restrict__ stepItems, const uint32_t* __restrict__ stepPtr, int64_t nStepPtr,
-            const SpItem* __restrict__ winItems, const uint32_t* __restrict__ winPtr, int64_t nWinPtr, int nRows,
-            const double* __restrict__ y, int nVals, double* __restrict__ A) {
-  extern __shared__ __align__(16) double llsm[];
-  constexpr int NSTEP = SKIP_ROWS / G3_STEP, NWIN = SKIP_ROWS / G3_WIN;
-  double* ys = llsm;                        // [SKIP_ROWS]
-  double* ywin = llsm + SKIP_ROWS;          // [NWIN]
-  double* hist = llsm + SKIP_ROWS + NWIN;   // [nVals]
-  const int tid = threadIdx.x;
-  for (int i = tid; i < nVals; i += LL_THREADS) hist[i] = 0.0;
-  const int nBlocks = (nRows + SKIP_ROWS - 1) / SKIP_ROWS;
-  for (int b = blockIdx.x; b < nBlocks; b += gridDim.x) {
-    __syncthreads();  // the previous block's readers of ys are done (and hist is cleared before the first block)
-    const int r0 = b * SKIP_ROWS;
-    for (int i = tid; i < SKIP_ROWS; i += LL_THREADS) ys[i] = r0 + i < nRows ? y[r0 + i] : 0.0;
-    __syncthreads();
-    if (tid < NWIN) {
-      double sum = 0.0;
-      for (int i = 0; i < G3_WIN; i++) sum += ys[tid * G3_WIN + i];
-      ywin[tid] = sum;
-    }
-    __syncthreads();
-    const int64_t w0 = (int64_t)b * NWIN, s0 = (int64_t)b * NSTEP;
-    const uint32_t wa = winPtr[min(w0, nWinPtr - 1)], wb = winPtr[min(w0 + NWIN, nWinPtr - 1)];
-    for (uint32_t i = wa + tid; i < wb; i += LL_THREADS) {
-      const SpItem e = winItems[i];
-      atomicAdd(&hist[e.prow], ywin[(e.rows >> 16) & (NWIN - 1)]);
-    }
-    const uint32_t sa = stepPtr[min(s0, nStepPtr - 1)], sb = stepPtr[min(s0 + NSTEP, nStepPtr - 1)];
-    for (uint32_t i = sa + tid; i < sb; i += LL_THREADS) {
-      const SpItem e = stepItems[i];
-      const int ra = e.rows & 0xFF, rb = (e.rows >> 8) & 0xFF;
-      const double* yr = ys + ((e.rows >> 16) & (NSTEP - 1)) * G3_STEP;
-      double sum = 0.0;
-      for (int r = ra; r < rb; r++) sum += yr[r];
-      atomicAdd(&hist[e.prow], sum);
-    }
-  }
-  __syncthreads();
-  for (int i = tid; i < nVals; i += LL_THREADS) {
-    const double v = hist[i];
-    if (v != 0.0) atomicAdd(&A[i], v);
-  }
-}
+int64_t launch_lmm_const(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s);
 
 int64_t launch_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s, bool afterFast) {
   if (q == 0 || m->nCols == 0) return CLA_OK;
   if (!afterFast) CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)q * m->nCols, s));
   if (m->nRows == 0) return CLA_OK;
   int64_t rc;
+  if (m->nDev > 0 && (afterFast || !fast_plan_partial(m))) {  // (without the specialised kernels' part only where they leave no group)
+    if ((rc = rest_lmm(m, dYt, q, dOut, s)) < 0) return rc;
+    if (rc == 1) return afterFast ? CLA_OK : launch_lmm_const(m, dYt, q, dOut, s);
+  }
   const size_t aBytes = (size_t)std::max<int64_t>(m->totalVals, 1) * q * sizeof(double);
   const size_t sOff = (aBytes + 255) & ~(size_t)255;
   if ((rc = ensure_scratch(m, sOff + (size_t)q * sizeof(double))) < 0) return rc;
@@ -816,30 +718,8 @@ int64_t launch_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream
     rowsPerChunk = std::max(SKIP_ROWS * 4, ((rowsPerChunk + SKIP_ROWS - 1) / SKIP_ROWS) * SKIP_ROWS);
     const int chunks = (m->nRows + rowsPerChunk - 1) / rowsPerChunk;
     dim3 grid(chunks, m->nDev, (q + LMM_QT - 1) / LMM_QT);
-    // one left row on a tall matrix with SDC / RLE groups: those come from the row-major work lists
-    bool lists = false;
-    const size_t llSmem = (size_t)(SKIP_ROWS + SKIP_ROWS / G3_WIN + std::max<int64_t>(m->totalVals, 1)) * sizeof(double);
-    if (q == 1 && m->nRows >= 4 * SKIP_ROWS && llSmem <= 160 * 1024) {
-      if ((rc = ensure_sparse_list(m)) < 0) return rc;
-      if (m->nSparse > 0) {
-        if ((rc = ensure_sparse_lists(m, s)) < 0) return rc;
-        lists = m->spListsOk && m->dStepPtr != nullptr;
-      }
-    }
     prof_begin(m, s);
-    k_lmm_preagg<<<grid, LMM_THREADS, 0, s>>>(m->dGroups, m->nRows, rowsPerChunk, dYt, q, A, afterFast ? 1 : 0, lists ? 1 : 0);
-    if (lists) {
-      static bool llAttr[64] = {};
-      if (!llAttr[m->device & 63]) {
-        CLA_CUDA(cudaFuncSetAttribute(k_lmm_lists, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-        llAttr[m->device & 63] = true;
-      }
-      const int nBlocks = (m->nRows + SKIP_ROWS - 1) / SKIP_ROWS;
-      k_lmm_lists<<<std::min(nBlocks, 2 * m->smCount), LL_THREADS, llSmem, s>>>(
-          (const SpItem*)m->dStepItems, m->dStepPtr, m->nStepPtr, (const SpItem*)m->dWinItems, m->dWinPtr, m->nWinPtr, m->nRows,
-          dYt, (int)m->totalVals, A);
-      m->stats.kernel_launches++;
-    }
+    k_lmm_preagg<<<grid, LMM_THREADS, 0, s>>>(m->dGroups, m->nRows, rowsPerChunk, dYt, q, A, afterFast ? 1 : 0);
     prof_end(m, s);
     k_lmm_post<<<m->nDev, 128, 0, s>>>(m->dGroups, A, q, m->nCols, dOut, afterFast ? 1 : 0);
     m->stats.kernel_launches += 2;

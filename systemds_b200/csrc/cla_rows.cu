@@ -24,7 +24,7 @@ namespace cla {
 constexpr int RL_WIN = SKIP_ROWS / WIN_ROWS;  // windows per block
 constexpr int RL_THREADS = 256;
 
-static int64_t plan_alloc(Matrix* m, void** p, size_t bytes) {
+int64_t plan_alloc(Matrix* m, void** p, size_t bytes) {
   *p = nullptr;
   cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
   if (e != cudaSuccess) {
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(RL_THREADS)
 k_row_lists(const DevGroup* __restrict__ groups, const int32_t* __restrict__ list, int nSdc, int nRle, int nRows,
             const int32_t* __restrict__ svOff, uint32_t* __restrict__ rowPtr, uint32_t* __restrict__ rowItems,
             uint32_t* __restrict__ fullPtr, uint32_t* __restrict__ fullItems, uint32_t* __restrict__ partPtr,
-            uint2* __restrict__ partItems) {
+            uint2* __restrict__ partItems, uint32_t* __restrict__ sdcItems, const int64_t* __restrict__ sdcBase) {
   __shared__ uint32_t cnt[SKIP_ROWS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int blk = blockIdx.x, b0 = blk * SKIP_ROWS, b1 = min(nRows, b0 + SKIP_ROWS);
@@ -115,7 +115,11 @@ k_row_lists(const DevGroup* __restrict__ groups, const int32_t* __restrict__ lis
       const uint32_t o = (uint32_t)svOff[gi];
       sdc_walk_block(g, b0, b1, [&](int row, int e) {
         const uint32_t p = atomicAdd(&cnt[row - b0], 1u);
-        if (FILL) rowItems[p] = o + (uint32_t)(g.single ? 0 : map_get(g.mapType, g.map, g.mapHi, e));
+        if (FILL) {
+          const uint32_t id = (uint32_t)(g.single ? 0 : map_get(g.mapType, g.map, g.mapHi, e));
+          rowItems[p] = o + id;
+          sdcItems[sdcBase[gi] + e] = (uint32_t)(row - b0) | (id << 10);
+        }
       });
       __syncwarp();
     }
@@ -211,10 +215,17 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   }
   const int nBlocks = (m->nRows + SKIP_ROWS - 1) / SKIP_ROWS;
   const int64_t nRowPtr = (int64_t)nBlocks * SKIP_ROWS + 1, nWinPtr = (int64_t)nBlocks * RL_WIN + 1;
-  int64_t rc;
   std::vector<int32_t> list(sdc);
   list.insert(list.end(), rle.begin(), rle.end());
   // pointers, group list, table-row numbering and values in one allocation
+  L.sdcBase.assign(m->nDev, 0);
+  int64_t nListed = 0;
+  for (int gi : sdc) {
+    L.sdcBase[gi] = nListed;
+    nListed += m->groups[gi].nOff;
+    if (m->groups[gi].nVals > (1 << 22)) return CLA_OK;  // an item holds 22 bits of tuple
+  }
+  const size_t bBase = (size_t)m->nDev * 8;
   const size_t bOff = ((size_t)m->nDev * 4 + 15) & ~(size_t)15, bList = (list.size() * 4 + 15) & ~(size_t)15;
   const size_t bSv = (size_t)std::max<int64_t>(nSv, 1) * sizeof(SparseVal);
   const size_t bRow = (L.nSdc ? (size_t)nRowPtr * 4 : 0), bWin = (L.nRle ? (size_t)nWinPtr * 4 : 0);
@@ -223,9 +234,10 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   cub::DeviceScan::ExclusiveSum(nullptr, tb2, (uint32_t*)nullptr, (uint32_t*)nullptr, (int)nWinPtr, s);
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   void* base = nullptr;
-  if ((rc = plan_alloc(m, &base, al(bOff) + al(bList) + al(bSv) + al(bRow) + 2 * al(bWin) + std::max(tb1, tb2))) < 0) return CLA_OK;
+  if (plan_alloc(m, &base, al(bBase) + al(bOff) + al(bList) + al(bSv) + al(bRow) + 2 * al(bWin) + std::max(tb1, tb2)) < 0) return CLA_OK;
   char* p = (char*)base;
   L.svOff = (int32_t*)p; p += al(bOff);
+  int64_t* dBase = (int64_t*)p; p += al(bBase);
   int32_t* dList = (int32_t*)p; p += al(bList);
   L.sv = (SparseVal*)p; p += al(bSv);
   if (L.nSdc) L.rowPtr = (uint32_t*)p;
@@ -236,10 +248,11 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   p += al(bWin);
   void* tmp = p;
   CLA_CUDA(cudaMemcpyAsync(L.svOff, off.data(), (size_t)m->nDev * 4, cudaMemcpyHostToDevice, s));
+  CLA_CUDA(cudaMemcpyAsync(dBase, L.sdcBase.data(), bBase, cudaMemcpyHostToDevice, s));
   CLA_CUDA(cudaMemcpyAsync(dList, list.data(), list.size() * 4, cudaMemcpyHostToDevice, s));
   k_sparse_vals<<<m->nDev, 128, 0, s>>>(m->dGroups, L.svOff, L.sv);
   k_row_lists<false><<<nBlocks, RL_THREADS, 0, s>>>(m->dGroups, dList, L.nSdc, L.nRle, m->nRows, L.svOff, L.rowPtr, nullptr,
-                                                   L.fullPtr, nullptr, L.partPtr, nullptr);
+                                                   L.fullPtr, nullptr, L.partPtr, nullptr, nullptr, nullptr);
   uint32_t tot[3] = {0, 0, 0};
   if (L.nSdc) {
     CLA_CUDA(cudaMemsetAsync(L.rowPtr + nRowPtr - 1, 0, 4, s));
@@ -257,12 +270,13 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   CLA_CUDA(cudaStreamSynchronize(s));
   void* items = nullptr;
   const size_t i0 = al((size_t)tot[0] * 4), i1 = al((size_t)tot[1] * 4), i2 = al((size_t)tot[2] * 8);
-  if ((rc = plan_alloc(m, &items, i0 + i1 + i2)) < 0) return CLA_OK;
+  if (plan_alloc(m, &items, 2 * i0 + i1 + i2) < 0) return CLA_OK;
+  L.sdcItems = (uint32_t*)((char*)items + i0 + i1 + i2);
   L.rowItems = (uint32_t*)items;
   L.fullItems = (uint32_t*)((char*)items + i0);
   L.partItems = (uint2*)((char*)items + i0 + i1);
   k_row_lists<true><<<nBlocks, RL_THREADS, 0, s>>>(m->dGroups, dList, L.nSdc, L.nRle, m->nRows, L.svOff, L.rowPtr, L.rowItems,
-                                                  L.fullPtr, L.fullItems, L.partPtr, L.partItems);
+                                                  L.fullPtr, L.fullItems, L.partPtr, L.partItems, L.sdcItems, dBase);
   CLA_CUDA(cudaGetLastError());
   CLA_CUDA(cudaStreamSynchronize(s));
   L.ok = true;
