@@ -48,15 +48,17 @@ __global__ void k_rest_terms(const SparseVal* __restrict__ sv, int nSv, const De
 struct UncGroup {
   const double* dense;
   const int32_t* cols;
-  int32_t gCols, pad;
+  int32_t gCols, at;  // at: its first column among the launch's
 };
-constexpr int RR_UNC = 8;  // uncompressed groups per launch
+constexpr int RR_UNC = 8;       // uncompressed groups per launch
+constexpr int RR_UCOLS = 1024;  // their columns (their part of v in shared memory); a wider group goes by itself, v unstaged
 struct RestRmmArgs {
   const SparseVal* sv;
   const int32_t* svOff;
   const DevGroup* groups;
   const double* P;          // null: the CTA builds the table in shared memory
   int nSv, nRows, nDense, nUnc, nCols, addTo;
+  int nUncCols;             // 0: v of the uncompressed columns is not staged
   const uint32_t *rowPtr, *rowItems, *fullPtr, *fullItems, *partPtr;
   const uint2* partItems;
   const ColRef* dense;
@@ -82,6 +84,9 @@ __global__ void __launch_bounds__(RR_T, 4) k_rest_rmm(const __grid_constant__ Re
     for (int d = 16; d; d >>= 1) c0 += __shfl_xor_sync(0xffffffffu, c0, d);
     if (lane == 0) cred[warp] = c0;
   }
+  double* uv = ps + (A.P ? 0 : A.nSv);
+  for (int i = 0; i < A.nUnc && A.nUncCols; i++)
+    for (int c = tid; c < A.unc[i].gCols; c += RR_T) uv[A.unc[i].at + c] = A.v[A.unc[i].cols[c]];
   __syncthreads();
   if (A.constV) {
     c0 = 0.0;
@@ -101,6 +106,8 @@ __global__ void __launch_bounds__(RR_T, 4) k_rest_rmm(const __grid_constant__ Re
     for (int i = 0; i < A.nUnc; i++) {
       const UncGroup& U = A.unc[i];
       const int gc = U.gCols;
+      const double* vs = uv + U.at;
+      auto v_at = [&](int c) { return g == 0 ? (A.nUncCols ? vs[c] : A.v[U.cols[c]]) : 0.0; };
 #pragma unroll 1
       for (int j = 0; j < 4; j++) {
         const int row = min(r0 + 8 * j + g, A.nRows - 1);
@@ -112,10 +119,7 @@ __global__ void __launch_bounds__(RR_T, 4) k_rest_rmm(const __grid_constant__ Re
 #pragma unroll
           for (int u = 0; u < 8; u++) xv[u] = __ldcs(x + c + 4 * u);
 #pragma unroll
-          for (int u = 0; u < 8; u++) {
-            const double b = g == 0 ? A.v[U.cols[c + 4 * u + t]] : 0.0;
-            dmma884(s0, s1, xv[u], b);
-          }
+          for (int u = 0; u < 8; u++) dmma884(s0, s1, xv[u], v_at(c + 4 * u + t));
         }
         {
           double xv[8];
@@ -124,8 +128,7 @@ __global__ void __launch_bounds__(RR_T, 4) k_rest_rmm(const __grid_constant__ Re
 #pragma unroll
           for (int u = 0; u < 8; u++)
             if (c + 4 * u < gc) {
-              const double b = (g == 0 && c + 4 * u + t < gc) ? A.v[U.cols[c + 4 * u + t]] : 0.0;
-              dmma884(s0, s1, xv[u], b);
+              dmma884(s0, s1, xv[u], c + 4 * u + t < gc ? v_at(c + 4 * u + t) : 0.0);
             }
         }
         // lane 4 g' holds row g' of the eight: hand it to the lane of that row
@@ -156,17 +159,37 @@ __global__ void __launch_bounds__(RR_T, 4) k_rest_rmm(const __grid_constant__ Re
         if (col[u] >= 0) acc = fma(x[u], A.v[col[u]], acc);
     }
     // listed tuples of this lane's row
-    for (uint32_t p = p0; p < p1; p++) acc += P[A.rowItems[p]];
+    for (; p0 + 4 <= p1; p0 += 4) {
+      uint32_t it[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) it[u] = A.rowItems[p0 + u];
+#pragma unroll
+      for (int u = 0; u < 4; u++) acc += P[it[u]];
+    }
+    {
+      uint32_t it[3];
+#pragma unroll
+      for (int u = 0; u < 3; u++) it[u] = p0 + u < p1 ? A.rowItems[p0 + u] : 0u;
+#pragma unroll
+      for (int u = 0; u < 3; u++)
+        if (p0 + u < p1) acc += P[it[u]];
+    }
     if (A.fullPtr) {
       const int w = r0 / WIN_ROWS, rw = r0 + lane - w * WIN_ROWS;
       double full = 0.0;  // runs over the whole window: lanes share the sum
       for (uint32_t p = A.fullPtr[w] + lane; p < A.fullPtr[w + 1]; p += 32) full += P[A.fullItems[p]];
       for (int d = 16; d; d >>= 1) full += __shfl_xor_sync(0xffffffffu, full, d);
       acc += full;
-      for (uint32_t p = A.partPtr[w]; p < A.partPtr[w + 1]; p++) {
-        const uint2 it = A.partItems[p];
-        const double x = P[it.x];
-        if (rw >= (int)(it.y & 0xFF) && rw < (int)(it.y >> 8)) acc += x;
+      const uint32_t q1 = A.partPtr[w + 1];
+      for (uint32_t p = A.partPtr[w]; p < q1; p += 4) {
+        uint2 it[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) it[u] = p + u < q1 ? A.partItems[p + u] : make_uint2(0, 0);  // no rows
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const double x = P[it[u].x];
+          if (rw >= (int)(it[u].y & 0xFF) && rw < (int)(it[u].y >> 8)) acc += x;
+        }
       }
     }
     if (r0 + lane < A.nRows) {
@@ -187,7 +210,8 @@ constexpr int RL_UC = 64;       // columns per CTA of the second
 constexpr int RL_WIN = SKIP_ROWS / WIN_ROWS;
 struct RestLmmArgs {
   const RestTask* tasks;
-  int nTasks, nChunks;       // chunks of RL_TASKS columns
+  int nTasks, nChunks;       // chunks of RL_TASKS columns; the first nSparse are SDC / RLE columns
+  int nSparse;
   int ctaTasks;              // CTAs per chunk
   const double* dense;       // uncompressed group (null: none), its width, chunks of RL_UC columns, CTAs per chunk
   const int32_t* uncCols;
@@ -206,7 +230,7 @@ __device__ __forceinline__ void rest_lmm_tasks(const RestLmmArgs& A, int chunk, 
   double* sums = ws + QT * RL_WIN;                  // [RL_TASKS][QT]
   RestTask* T = (RestTask*)(sums + RL_TASKS * QT);  // [RL_TASKS]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t0 = chunk * RL_TASKS, nt = min(RL_TASKS, A.nTasks - t0);
+  const int t0 = chunk * RL_TASKS, nt = min(RL_TASKS, A.nTasks - t0), nSparse = max(0, min(nt, A.nSparse - t0));
   for (int i = tid; i < nt; i += RL_T) T[i] = A.tasks[t0 + i];
   for (int i = tid; i < nt * QT; i += RL_T) sums[i] = 0.0;
   const int nBlocks = (A.nRows + SKIP_ROWS - 1) / SKIP_ROWS;
@@ -226,123 +250,108 @@ __device__ __forceinline__ void rest_lmm_tasks(const RestLmmArgs& A, int chunk, 
       if (lane == 0) ws[e] = s;
     }
     __syncthreads();
-    for (int i0 = warp; i0 < nt; i0 += 32 * RL_WARPS) {
-      // this warp's next 32 columns: lane l looks up where column i0 + RL_WARPS l starts in the block
-      const int ti = i0 + lane * RL_WARPS;
-      int64_t e0 = 0, e1 = 0;
-      if (ti < nt) {
-        const RestTask& k = T[ti];
+    // SDC and RLE columns: eight lanes each, four columns of a warp at a time (a column has a few dozen items per block,
+    // and with eight lanes the walks of four columns and one reduction of three steps serve what took four)
+    const int l8 = lane & 7, grp = lane >> 3;
+    const unsigned gmask = 0xFFu << (grp * 8);
+    for (int i0 = warp * 4; i0 < nSparse; i0 += RL_WARPS * 4) {
+      const int task = i0 + grp;
+      double acc[QT];
+#pragma unroll
+      for (int i = 0; i < QT; i++) acc[i] = 0.0;
+      if (task < nSparse) {
+        const RestTask& k = T[task];
         if (k.kind == GT_SDC) {
           const SdcSkip* sk = (const SdcSkip*)k.b;
-          e0 = sk[b].elem;
-          e1 = b + 1 < nBlocks ? (int64_t)sk[b + 1].elem : k.n;
-        } else if (k.kind == GT_RLE) {
-          e0 = ((const int32_t*)k.b)[b];
-          e1 = k.n;
-        }
-      }
-      const int n = min(32, (nt - i0 + RL_WARPS - 1) / RL_WARPS);
-      uint2 next = make_uint2(0, 0);
-      auto fetch = [&](int j) {  // the first 32 items of column j of the 32
-        const int64_t a = __shfl_sync(0xffffffffu, e0, j & 31), z = __shfl_sync(0xffffffffu, e1, j & 31);
-        uint2 v = make_uint2(0xFFFFFFFFu, 0);
-        if (j < n) {
-          const RestTask& k = T[i0 + j * RL_WARPS];
-          if (a + lane < z) {
-            if (k.kind == GT_SDC) v.x = ((const uint32_t*)k.a)[a + lane];
-            else if (k.kind == GT_RLE) v = ((const uint2*)k.a)[a + lane];
+          const int64_t e1 = b + 1 < nBlocks ? (int64_t)sk[b + 1].elem : k.n;
+          const uint32_t* items = (const uint32_t*)k.a;
+          for (int64_t e = (int64_t)sk[b].elem + l8; e < e1; e += 32) {
+            uint32_t it[4];
+            double x[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) it[u] = e + 8 * u < e1 ? items[e + 8 * u] : 0u;
+#pragma unroll
+            for (int u = 0; u < 4; u++) x[u] = k.src[(size_t)(it[u] >> 10) * k.stride];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+              if (e + 8 * u < e1) {
+                const double* y = ys + (it[u] & 1023u);
+#pragma unroll
+                for (int i = 0; i < QT; i++) acc[i] = fma(x[u], y[i * SKIP_ROWS], acc[i]);
+              }
           }
-        }
-        return v;
-      };
-      next = fetch(0);
-      for (int j = 0; j < n; j++) {
-        const uint2 item = next;
-        next = fetch(j + 1);
-        const int task = i0 + j * RL_WARPS;
-        const RestTask& k = T[task];
-        const int64_t a = __shfl_sync(0xffffffffu, e0, j), z = __shfl_sync(0xffffffffu, e1, j);
-        double acc[QT];
-#pragma unroll
-        for (int i = 0; i < QT; i++) acc[i] = 0.0;
-        if (k.kind == GT_SDC) {
-          auto one = [&](uint32_t it) {
-            const double x = k.src[(size_t)(it >> 10) * k.stride];
-            const double* y = ys + (it & 1023u);
-#pragma unroll
-            for (int i = 0; i < QT; i++) acc[i] = fma(x, y[i * SKIP_ROWS], acc[i]);
-          };
-          if (a + lane < z) one(item.x);
-          for (int64_t e = a + 32 + lane; e < z; e += 32) one(((const uint32_t*)k.a)[e]);
-        } else if (k.kind == GT_RLE) {
-          for (int64_t e = a;; e += 32) {
-            uint2 it = item;
-            if (e > a) it = e + lane < z ? ((const uint2*)k.a)[e + lane] : make_uint2(0xFFFFFFFFu, 0);
-            const bool in = e + lane < z && (int)it.x < r0 + nr;  // the runs of a group are sorted by row
-            const unsigned mask = __ballot_sync(0xffffffffu, in);
-            for (unsigned left = mask; left; left &= left - 1) {
-              const int l = __ffs(left) - 1;
-              const int start = (int)__shfl_sync(0xffffffffu, it.x, l) - r0;
-              const uint32_t lk = __shfl_sync(0xffffffffu, it.y, l);
-              const int ra = max(start, 0), rb = min(start + (int)(lk & 0xFFFF), nr);
-              if (ra >= rb) continue;
-              const double x = k.src[(size_t)(lk >> 16) * k.stride];
-              const int wa = (ra + WIN_ROWS - 1) / WIN_ROWS, wb = rb / WIN_ROWS;  // whole windows [wa, wb)
-              double s[QT];
-#pragma unroll
-              for (int i = 0; i < QT; i++) s[i] = 0.0;
-              if (wa < wb) {
-                if (lane >= wa && lane < wb)
-#pragma unroll
-                  for (int i = 0; i < QT; i++) s[i] += ws[i * RL_WIN + lane];
-                for (int r = ra + lane; r < wa * WIN_ROWS; r += 32)
-#pragma unroll
-                  for (int i = 0; i < QT; i++) s[i] += ys[i * SKIP_ROWS + r];
-                for (int r = wb * WIN_ROWS + lane; r < rb; r += 32)
-#pragma unroll
-                  for (int i = 0; i < QT; i++) s[i] += ys[i * SKIP_ROWS + r];
-              } else
-                for (int r = ra + lane; r < rb; r += 32)
-#pragma unroll
-                  for (int i = 0; i < QT; i++) s[i] += ys[i * SKIP_ROWS + r];
-#pragma unroll
-              for (int i = 0; i < QT; i++) acc[i] = fma(x, s[i], acc[i]);
-            }
-            if (mask != 0xffffffffu) break;
-          }
-        } else {  // dense map, lanes along the rows
-          for (int rr = lane; rr < nr; rr += 256) {
-            int64_t at[8];
-            double x[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) at[u] = rr + 32 * u < nr ? (int64_t)map_get(k.mapType, k.a, k.b, r0 + rr + 32 * u) * k.stride : 0;
-#pragma unroll
-            for (int u = 0; u < 8; u++) x[u] = rr + 32 * u < nr ? k.src[at[u]] : 0.0;
-#pragma unroll
-            for (int u = 0; u < 8; u++)
-              if (rr + 32 * u < nr)
-#pragma unroll
-                for (int i = 0; i < QT; i++) acc[i] = fma(x[u], ys[i * SKIP_ROWS + rr + 32 * u], acc[i]);
-          }
-        }
-        // lane i ends with the sum of left row i (reduce-scatter while there are several)
-        if constexpr (QT == 1) {
-          for (int d = 16; d; d >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], d);
-          if (lane == 0) sums[task] += acc[0];
         } else {
+          const RleRun* runs = (const RleRun*)k.a;
+          for (int64_t e = ((const int32_t*)k.b)[b]; e < k.n; e++) {
+            const RleRun run = runs[e];
+            if (run.start >= r0 + nr) break;  // the runs of a group are sorted by row
+            const int ra = max(run.start - r0, 0), rb = min(run.start - r0 + (int)run.len, nr);
+            if (ra >= rb) continue;
+            const double x = k.src[(size_t)run.k * k.stride];
+            const int wa = (ra + WIN_ROWS - 1) / WIN_ROWS, wb = rb / WIN_ROWS;  // whole windows [wa, wb)
+            double s[QT];
 #pragma unroll
-          for (int d = QT / 2; d; d >>= 1) {
-            const bool up = (lane & d) != 0;
+            for (int i = 0; i < QT; i++) s[i] = 0.0;
+            const int h = wa < wb ? wa * WIN_ROWS : rb;  // rows [ra, h) and, behind the windows, [wb * 64, rb)
+            for (int r = ra + l8; r < h; r += 8)
 #pragma unroll
-            for (int i = 0; i < d; i++) {
-              const double recv = __shfl_xor_sync(0xffffffffu, up ? acc[i] : acc[i + d], d);
-              acc[i] = (up ? acc[i + d] : acc[i]) + recv;
+              for (int i = 0; i < QT; i++) s[i] += ys[i * SKIP_ROWS + r];
+            if (wa < wb) {
+              for (int w = wa + l8; w < wb; w += 8)
+#pragma unroll
+                for (int i = 0; i < QT; i++) s[i] += ws[i * RL_WIN + w];
+              for (int r = wb * WIN_ROWS + l8; r < rb; r += 8)
+#pragma unroll
+                for (int i = 0; i < QT; i++) s[i] += ys[i * SKIP_ROWS + r];
             }
+#pragma unroll
+            for (int i = 0; i < QT; i++) acc[i] = fma(x, s[i], acc[i]);
           }
-          for (int d = 16; d >= QT; d >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], d);
-          if (lane < QT) sums[task * QT + lane] += acc[0];
         }
       }
+      __syncwarp();
+      // lane i of the eight ends with the sum of left row i (reduce-scatter while there are several)
+#pragma unroll
+      for (int d = QT / 2; d; d >>= 1) {
+        const bool up = (lane & d) != 0;
+#pragma unroll
+        for (int i = 0; i < d; i++) {
+          const double recv = __shfl_xor_sync(gmask, up ? acc[i] : acc[i + d], d);
+          acc[i] = (up ? acc[i + d] : acc[i]) + recv;
+        }
+      }
+      for (int d = 4; d >= QT; d >>= 1) acc[0] += __shfl_xor_sync(gmask, acc[0], d);
+      if (task < nSparse && l8 < QT) sums[task * QT + l8] += acc[0];
+    }
+    for (int task = nSparse + warp; task < nt; task += RL_WARPS) {  // dense map, lanes along the rows
+      const RestTask& k = T[task];
+      double acc[QT];
+#pragma unroll
+      for (int i = 0; i < QT; i++) acc[i] = 0.0;
+      for (int rr = lane; rr < nr; rr += 256) {
+        int64_t at[8];
+        double x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) at[u] = rr + 32 * u < nr ? (int64_t)map_get(k.mapType, k.a, k.b, r0 + rr + 32 * u) * k.stride : 0;
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = rr + 32 * u < nr ? k.src[at[u]] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+          if (rr + 32 * u < nr)
+#pragma unroll
+            for (int i = 0; i < QT; i++) acc[i] = fma(x[u], ys[i * SKIP_ROWS + rr + 32 * u], acc[i]);
+      }
+#pragma unroll
+      for (int d = QT / 2; d; d >>= 1) {
+        const bool up = (lane & d) != 0;
+#pragma unroll
+        for (int i = 0; i < d; i++) {
+          const double recv = __shfl_xor_sync(0xffffffffu, up ? acc[i] : acc[i + d], d);
+          acc[i] = (up ? acc[i + d] : acc[i]) + recv;
+        }
+      }
+      for (int d = 16; d >= QT; d >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], d);
+      if (lane < QT) sums[task * QT + lane] += acc[0];
     }
   }
   __syncthreads();
@@ -533,30 +542,32 @@ int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cu
   A.partItems = L.partItems;
   A.v = dV;
   A.out = dOut;
-  size_t smem = 0;
   if (A.nSv > RR_PMAX) {
     if ((rc = ensure_scratch(m, (size_t)A.nSv * sizeof(double))) < 0) return rc;
     k_rest_terms<<<std::min(1024, (A.nSv + 255) / 256), 256, 0, s>>>(L.sv, A.nSv, m->dGroups, L.svOff, dV, (double*)m->scratch);
     m->stats.kernel_launches++;
     A.P = (const double*)m->scratch;
-  } else
-    smem = (size_t)A.nSv * sizeof(double);
+  }
   static bool attrSet[64] = {};  // per device
   if (!attrSet[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_rest_rmm, cudaFuncAttributeMaxDynamicSharedMemorySize, RR_PMAX * (int)sizeof(double)));
+    CLA_CUDA(cudaFuncSetAttribute(k_rest_rmm, cudaFuncAttributeMaxDynamicSharedMemorySize, (RR_PMAX + RR_UCOLS) * (int)sizeof(double)));
     attrSet[m->device & 63] = true;
   }
-  const int perSm = smem <= 50 * 1024 ? 4 : 3;
-  const int grid = std::max(1, std::min((m->nRows + RR_T - 1) / RR_T, perSm * m->smCount));
   int u0 = 0;
   prof_begin(m, s);
-  do {  // uncompressed groups RR_UNC at a time; the first launch adds everything else
-    A.nUnc = std::min(RR_UNC, R.nUnc - u0);
-    for (int i = 0; i < A.nUnc; i++) {
-      const DevGroup& g = m->groups[R.unc[u0 + i]];
-      A.unc[i] = UncGroup{g.dense, g.cols, g.gCols, 0};
+  do {  // uncompressed groups up to RR_UNC and RR_UCOLS columns at a time; the first launch adds everything else
+    A.nUnc = A.nUncCols = 0;
+    while (u0 < R.nUnc && A.nUnc < RR_UNC) {
+      const DevGroup& g = m->groups[R.unc[u0]];
+      if (A.nUnc > 0 && A.nUncCols + g.gCols > RR_UCOLS) break;
+      A.unc[A.nUnc++] = UncGroup{g.dense, g.cols, g.gCols, A.nUncCols};
+      A.nUncCols += g.gCols;
+      u0++;
     }
-    u0 += A.nUnc;
+    if (A.nUncCols > RR_UCOLS) A.nUncCols = 0;
+    const size_t smem = ((A.P ? 0 : A.nSv) + (size_t)A.nUncCols) * sizeof(double);
+    const int perSm = smem <= 50 * 1024 ? 4 : 3;
+    const int grid = std::max(1, std::min((m->nRows + RR_T - 1) / RR_T, perSm * m->smCount));
     A.addTo = addTo ? 1 : 0;
     A.constV = (!addTo && m->hasConst) ? m->dConstV : nullptr;
     A.rowScale = u0 >= R.nUnc ? dW : nullptr;
@@ -605,6 +616,7 @@ int64_t rest_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t
       RestLmmArgs A{};
       A.tasks = R.tasks;
       A.nTasks = u == 0 ? R.nTasks : 0;
+      A.nSparse = R.nTasks - R.nDense;
       if (u < R.nUnc) {
         const DevGroup& g = m->groups[R.unc[u]];
         A.dense = g.dense;
