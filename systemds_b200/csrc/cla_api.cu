@@ -404,50 +404,12 @@ static int64_t check_errword(Matrix* m) {
   return CLA_OK;
 }
 
-// Few right-hand columns (or few left-hand rows) are served by the one-vector kernels, once per vector: each
-// pass re-reads the maps, which is cheaper than the general tile kernels up to the limits below.
-static int loop_limit(const char* env, int dflt) {
-  const char* e = getenv(env);
-  return e ? atoi(e) : dflt;
-}
-
-__global__ void k_small_transpose(const double* __restrict__ in, int rows, int cols, double* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < rows * cols) out[(size_t)(i % cols) * rows + i / cols] = in[i];
-}
-
-// U holds vCols result vectors of nRows each; out is row-major nRows x vCols.
-__global__ void k_vectors_to_rows(const double* __restrict__ U, int64_t nRows, int64_t stride, int vCols,
-                                  double* __restrict__ out) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nRows; r += (int64_t)gridDim.x * blockDim.x)
-    for (int j = 0; j < vCols; j++) out[r * vCols + j] = U[(int64_t)j * stride + r];
-}
-
 // One right-hand column; dW: factors applied to the rows (null: none)
 static int64_t rmm_vec(Matrix* m, const double* dV, const double* dW, double* dOut, cudaStream_t s) {
   const int64_t rc = fast_rmm_vec(m, dV, dOut, fast_plan_partial(m) ? nullptr : dW, s);
   if (rc < 0) return rc;
   if (rc == 1) return CLA_OK;
   return launch_rmm(m, dV, dW, dOut, s, rc == 2);
-}
-
-static int64_t rmm_by_vectors(Matrix* m, const double* dV, int32_t vCols, double* dOut, cudaStream_t s) {
-  const size_t vtBytes = (((size_t)vCols * m->nCols * sizeof(double)) + 255) & ~(size_t)255;
-  const size_t rowsPad = ((size_t)m->nRows + 31) & ~(size_t)31;
-  int64_t rc = ensure_scratch2(m, vtBytes + rowsPad * vCols * sizeof(double));
-  if (rc < 0) return rc;
-  double* Vt = (double*)m->scratch2;
-  double* U = (double*)((char*)m->scratch2 + vtBytes);
-  const int cells = m->nCols * vCols;
-  k_small_transpose<<<(cells + 255) / 256, 256, 0, s>>>(dV, m->nCols, vCols, Vt);
-  for (int j = 0; j < vCols; j++) {
-    double* uj = U + rowsPad * j;
-    if ((rc = rmm_vec(m, Vt + (size_t)j * m->nCols, nullptr, uj, s)) < 0) return rc;
-  }
-  k_vectors_to_rows<<<m->smCount * 8, 256, 0, s>>>(U, m->nRows, (int64_t)rowsPad, vCols, dOut);
-  m->stats.kernel_launches += 2;
-  CLA_CUDA(cudaGetLastError());
-  return CLA_OK;
 }
 
 // A host-buffer call whose operands and result are small: the product's last kernel may finish the call itself (write
@@ -469,13 +431,16 @@ static int64_t rmm_dev(Matrix* m, const double* dV, int32_t vRows, int32_t vCols
     if (rc != 0) return rc < 0 ? rc : CLA_OK;
   }
   if (vCols == 1) return rmm_vec(m, dV, nullptr, dOut, s);
-  // A pass of the one-column kernels per column beats the tensor-core kernel (whose time hardly depends on
-  // the width up to 64 columns) for a few columns; measured crossover: about 16 columns when every group is
-  // a byte-map DDC group (2M x 200: 0.26 ms per column against 4.3 ms), about 7 when SDC / RLE groups take
-  // the general pass as well (1M x 500, 451 groups: 0.25 ms per column against 1.9 ms).
-  static const int loopEnv = loop_limit("CLA_RMM_LOOP_MAX", -1);  // tuning aid
-  const int loopMax = loopEnv >= 0 ? loopEnv : (fast_plan_partial(m) ? 7 : 12);
-  if (vCols >= 2 && vCols <= loopMax && fast_plan_ok(m) && m->nRows > 0) return rmm_by_vectors(m, dV, vCols, dOut, s);
+  if (vCols == 2 && fast_plan_ok(m) && !fast_plan_partial(m) && m->nRows > 0) {
+    // two passes of the one-column kernel (1M x 200: 2 x 80 us) beat one of the tensor-core kernel (253 us); three do not
+    for (int j = 0; j < 2; j++) {
+      const int64_t rc = fast_rmm_vec(m, dV + j, dOut + j, nullptr, s, 2);
+      if (rc < 0) return rc;
+    }
+    return CLA_OK;
+  }
+  const int64_t rc = wide_rmm(m, dV, vCols, dOut, s);
+  if (rc != 0) return rc < 0 ? rc : CLA_OK;
   return launch_rmm_dmma(m, dV, vCols, dOut, s);  // FP64 tensor cores
 }
 

@@ -140,17 +140,6 @@ struct HostGroup {
   int devSrcDevice = -1;
 };
 
-// Row-major work lists of the SDC / RLE groups (built by ensure_sparse_lists, cla_rmm_dmma.cu): rows are cut into
-// steps of 8 and windows of 64, a warp work unit of the tensor-core right product is 512 rows.
-constexpr int G3_UNIT = 512;
-constexpr int G3_STEP = 8;
-constexpr int G3_WIN = 64;
-// One piece of work: rows [ra, rb) of an 8-row step (or a whole 64-row window) receive table row prow.
-struct SpItem {
-  uint32_t prow;
-  uint32_t rows;  // ra | rb << 8 | (index of the step or window inside its 1024-row block) << 16
-};
-
 struct FastPlan;  // plans of the specialised DDC kernels (cla_fast.cu)
 
 // One column of one product group, flat (built once per handle, cla_rows.cu).
@@ -226,6 +215,7 @@ struct Finish {
   int32_t* err = nullptr;             // the handle's self-check word
   uint32_t seq = 0;
 };
+struct WidePlan;  // plan of the wide right product (cla_wide.cu)
 struct HostStage; // pinned ring for operands in pageable host memory (cla_hostcopy.cu)
 
 struct Matrix;
@@ -253,10 +243,6 @@ struct Matrix {
   double* dConstV = nullptr;     // [nCols]
   void* dDenseCols = nullptr;    // list of dense-operand columns for the tensor-core RMM (built on first use)
   int nDenseCols = 0;
-  void* dDenseDesc = nullptr;    // the same columns as flat records (map, dictionary column, V row)
-  void* dSdcIdx = nullptr;       // device group indices of the SDC / RLE groups
-  void* dRleIdx = nullptr;
-  int nSdcGroups = 0, nRleGroups = 0;
   bool denseColsBuilt = false;
   int32_t* dSparseIdx = nullptr;  // device group indices of the SDC groups with listed rows and RLE groups with runs, list order
   int nSparse = 0;
@@ -266,13 +252,6 @@ struct Matrix {
   int32_t* dUncIdx = nullptr;
   int nDdc = 0, nDdcRest = 0, nUnc = 0;
   bool sparseListBuilt = false;
-  // row-major work lists of the SDC / RLE groups for the tensor-core right product (cla_rmm_dmma.cu), built on first use
-  void* dStepItems = nullptr;
-  uint32_t* dStepPtr = nullptr;
-  void* dWinItems = nullptr;
-  uint32_t* dWinPtr = nullptr;
-  bool spListsTried = false, spListsOk = false;
-  int64_t nStepPtr = 0, nWinPtr = 0;  // entries of dStepPtr / dWinPtr (the last one = number of items)
   int32_t* dColSrc = nullptr;    // [nCols][2]: dense-map / uncompressed group holding the column and the position in it (-1: none)
   bool colSrcValid = false;      // false when some column is held by more than one such group (overlapping input)
   bool hasConst = false;
@@ -302,6 +281,7 @@ struct Matrix {
   RowLists rows;
   ColPlan cols;
   RestPlan rest;
+  WidePlan* wide = nullptr;
   HostStage* hostStage = nullptr;
   char* mail = nullptr;          // pinned: Mailbox, inputs, outputs (small host-buffer calls)
   unsigned long long* dFin = nullptr;  // device counters of Finish
@@ -342,8 +322,7 @@ int64_t host_to_device_staged(Matrix* m, void* dDst, const void* host, size_t by
                               const std::function<int64_t(size_t)>& enqueued);
 int64_t device_to_host_staged(Matrix* m, void* host, const void* dSrc, size_t bytes, cudaStream_t s);
 void host_stage_free(Matrix* m);
-int64_t ensure_sparse_list(Matrix* m);
-int64_t ensure_sparse_lists(Matrix* m, cudaStream_t s);  // the row-major work lists; m->spListsOk tells whether they exist  // Matrix::dSparseIdx (cla_generic.cu)
+int64_t ensure_sparse_list(Matrix* m);  // Matrix::dSparseIdx (cla_generic.cu)
 
 int64_t ensure_col_plan(Matrix* m);                        // Matrix::cols
 int64_t ensure_row_lists(Matrix* m, cudaStream_t s);       // Matrix::rows; rows.ok tells whether they exist
@@ -351,6 +330,8 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s);       // Matrix::rows; rows
 int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s, bool addTo);
 int64_t rest_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s);
 int64_t plan_alloc(Matrix* m, void** p, size_t bytes);
+int64_t wide_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStream_t s);  // cla_wide.cu: 1 = done, 0 = not covered
+void wide_plan_free(Matrix* m);
 // Short blocks (cla_small.cu): one kernel per product, every group type. 1 = done, 0 = not covered
 bool small_block(const Matrix* m);
 int64_t small_rmm(Matrix* m, const double* dV, int vCols, double* dOut, const double* dW, cudaStream_t s, const Finish& fin,
@@ -393,7 +374,7 @@ void fast_plan_free(Matrix* m);
 bool fast_plan_ok(const Matrix* m);       // some or all groups are covered by the specialised kernels
 bool fast_plan_partial(const Matrix* m);  // ... some but not all
 // dW: null, or factors applied to the rows (0 is returned where the plan does not cover every group)
-int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s);
+int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s, int64_t stride = 1);
 int64_t fast_chain(Matrix* m, const double* dV, const double* dW, double* dOut, double* dU, cudaStream_t s);
 int64_t fast_lmm_vec(Matrix* m, const double* dY, double* dOut, cudaStream_t s);
 int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* dOut, cudaStream_t s);  // q = 2 or 4 left rows at once

@@ -676,6 +676,7 @@ struct RmmArgs {
   int nCols;
   int nRows, nU16;
   const double* rowScale;  // null, or a factor per row applied at the end
+  int64_t stride;          // of v and out (column of a row-major matrix)
   double* out;
   int32_t* err;
 };
@@ -683,7 +684,7 @@ struct RmmArgs {
 // The sums of step `st` again, for a warp that saw an Inf or NaN: every row by itself, with shuffles. Lane 4 g + t, t < 2,
 // returns rows 8 t + g of the two blocks.
 __device__ __noinline__ double2 rmm_step_by_rows(const uint8_t* mp, size_t ustr, const int2* units, const int* slotCol,
-                                                 const double* v, int nu, uint32_t table0) {
+                                                 const double* v, int64_t stride, int nu, uint32_t table0) {
   const int lane = threadIdx.x & 31, slot = lane & 15, g = lane >> 2, t = lane & 3;
   double2 r = make_double2(0.0, 0.0);
   for (int i = 0; i < 16; i++) {
@@ -691,7 +692,7 @@ __device__ __noinline__ double2 rmm_step_by_rows(const uint8_t* mp, size_t ustr,
     for (int u = 0; u < nu; u++) {
       const int col = slotCol[u * 16 + slot];
       if (col >= 0)
-        a = fma(lds_f64(table0 + (uint32_t)(units[u].x - units[0].x) * 128u + slot * 8 + 128u * mp[u * ustr + i]), v[col], a);
+        a = fma(lds_f64(table0 + (uint32_t)(units[u].x - units[0].x) * 128u + slot * 8 + 128u * mp[u * ustr + i]), v[col * stride], a);
     }
     for (int d = 1; d < 16; d <<= 1) a += __shfl_xor_sync(0xffffffffu, a, d);
     const double other = __shfl_xor_sync(0xffffffffu, a, 16);
@@ -770,7 +771,7 @@ __device__ __forceinline__ void rmm_rows(const RmmArgs& A, int unit0, int64_t s0
     v[u] = 0.0;
     if (!JOINT) {
       const int col = A.slotCol[(unit0 + u) * 16 + slot];
-      v[u] = col >= 0 ? A.v[col] : 0.0;
+      v[u] = col >= 0 ? A.v[col * A.stride] : 0.0;
     }
   }
   const uint8_t* mp = A.imaps + (size_t)unit0 * A.nRB * 256 + half * 256 + slot * 16;
@@ -784,13 +785,13 @@ __device__ __forceinline__ void rmm_rows(const RmmArgs& A, int unit0, int64_t s0
     const bool mine0 = (JOINT || t < 2) && row < A.nRows, mine1 = !JOINT && t < 2 && row + 16 < A.nRows;
     double o0 = init, o1 = init;  // what these rows hold from the chunks before
     if (!first) {
-      o0 = mine0 ? A.out[row] : 0.0;
-      o1 = mine1 ? A.out[row + 16] : 0.0;
+      o0 = mine0 ? A.out[row * A.stride] : 0.0;
+      o1 = mine1 ? A.out[(row + 16) * A.stride] : 0.0;
     }
     double r0, r1;
     step_sums<NU, JOINT, 2>(m, tb, v, r0, r1);
     if (!JOINT && __any_sync(0xffffffffu, t < 2 && !(isfinite(r0) && isfinite(r1)))) {
-      const double2 r = rmm_step_by_rows(mp + st * 512, ustr, A.units + unit0, A.slotCol + unit0 * 16, A.v, NU, table0);
+      const double2 r = rmm_step_by_rows(mp + st * 512, ustr, A.units + unit0, A.slotCol + unit0 * 16, A.v, A.stride, NU, table0);
       r0 = r.x, r1 = r.y;
     }
     r0 += o0;
@@ -799,8 +800,8 @@ __device__ __forceinline__ void rmm_rows(const RmmArgs& A, int unit0, int64_t s0
       if (mine0) r0 *= A.rowScale[row];
       if (mine1) r1 *= A.rowScale[row + 16];
     }
-    if (mine0) A.out[row] = r0;
-    if (mine1) A.out[row + 16] = r1;
+    if (mine0) A.out[row * A.stride] = r0;
+    if (mine1) A.out[(row + 16) * A.stride] = r1;
   }
 }
 
@@ -827,9 +828,9 @@ __device__ __forceinline__ void joint_tables(const RmmArgs& A, int unit0, int nu
         nvs[i] = G.nv;
         for (int a = r; a < G.nv; a += RB_W) {
           double x = 0.0;
-          if (G.gCols == 1) x = G.dict[a] * A.v[G.col];
+          if (G.gCols == 1) x = G.dict[a] * A.v[G.col * A.stride];
           else
-            for (int h = 0; h < G.gCols; h++) x += G.dict[(size_t)a * G.gCols + h] * A.v[G.cols[h]];
+            for (int h = 0; h < G.gCols; h++) x += G.dict[(size_t)a * G.gCols + h] * A.v[G.cols[h] * A.stride];
           if (i == 0) T[(size_t)a * 16] = x;
           else P[off + a] = x;
         }
@@ -873,7 +874,7 @@ __global__ void __launch_bounds__(RB_T, 1) k_rmm_vec(const __grid_constant__ Rmm
   const int64_t s0 = nSteps * blockIdx.x / gridDim.x, s1 = nSteps * (blockIdx.x + 1) / gridDim.x;
   double init = 0.0;
   if (A.constV) {
-    for (int c = threadIdx.x; c < A.nCols; c += RB_T) init = fma(A.constV[c], A.v[c], init);
+    for (int c = threadIdx.x; c < A.nCols; c += RB_T) init = fma(A.constV[c], A.v[c * A.stride], init);
     for (int d = 16; d; d >>= 1) init += __shfl_xor_sync(0xffffffffu, init, d);
     if ((threadIdx.x & 31) == 0) cred[threadIdx.x >> 5] = init;
     __syncthreads();
@@ -964,7 +965,7 @@ __device__ __forceinline__ void chain_body(const ChainArgs& C, unsigned char* sm
     double r0, r1;
     step_sums<NU, false, 1>(m, tb, v, r0, r1);
     if (__any_sync(0xffffffffu, t < 2 && !(isfinite(r0) && isfinite(r1)))) {
-      const double2 r = rmm_step_by_rows(mp + st * 512, ustr, A.units, A.slotCol, C.v, NU, table0);
+      const double2 r = rmm_step_by_rows(mp + st * 512, ustr, A.units, A.slotCol, C.v, 1, NU, table0);
       r0 = r.x, r1 = r.y;
     }
     r0 = (r0 + init) * w0;
@@ -1344,7 +1345,7 @@ int64_t fast_decompress(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s)
   return 1;
 }
 
-int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s) {
+int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s, int64_t stride) {
   FastPlan* fp = m->fast;
   if (!fp || !fp->ok || (dW && fp->partial)) return 0;
   // (short matrices: building the joint tables takes longer than the lookups they save)
@@ -1363,6 +1364,7 @@ int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW
   A.nRows = m->nRows;
   A.nU16 = joint ? fp->nJU16 : fp->nU16;
   A.rowScale = dW;
+  A.stride = stride;
   A.out = dOut;
   A.err = m->dErr;
   const std::vector<int>& nk = joint ? fp->jNk : fp->unitNk;

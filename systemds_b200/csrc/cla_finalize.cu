@@ -796,6 +796,7 @@ int64_t finalize_device(Matrix* m) {
 void release(Matrix* m) {
   if (m->device >= 0) cudaSetDevice(m->device);
   fast_plan_free(m);
+  wide_plan_free(m);
   for (void* p : m->allocs) cudaFree(p);
   m->allocs.clear();
   if (m->scratch) cudaFree(m->scratch);
