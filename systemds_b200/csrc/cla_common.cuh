@@ -193,6 +193,12 @@ struct RestPlan {
   ColRef* dense = nullptr;        // the remaining dense-map columns, list order
   std::vector<int> unc;           // device group indices of the uncompressed groups
 };
+struct DecPlan {  // column-per-lane decompress (cla_generic.cu)
+  bool tried = false;
+  void* cols = nullptr;
+  int warps = 0;
+  size_t smem = 0;
+};
 struct ColPlan {
   bool built = false;
   int nDense = 0, nRefs = 0;
@@ -281,6 +287,7 @@ struct Matrix {
   RowLists rows;
   ColPlan cols;
   RestPlan rest;
+  DecPlan dec;
   WidePlan* wide = nullptr;
   HostStage* hostStage = nullptr;
   char* mail = nullptr;          // pinned: Mailbox, inputs, outputs (small host-buffer calls)
@@ -359,7 +366,7 @@ int64_t launch_decompress(Matrix* m, double* dOut, cudaStream_t s);
 // X %*% V kept compressed: fills `child` (fresh Matrix) with groups that alias m's index structures (cla_generic.cu)
 int64_t make_overlapping(Matrix* m, Matrix* child, const double* dV, int vCols, cudaStream_t s);
 int64_t init_device_state(Matrix* m);  // stream, events, error word of a Matrix whose device is set (cla_finalize.cu)
-int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s);
+int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s, size_t ld = 0);  // ld 0: nCols
 int64_t launch_group_decode(Matrix* m, int devGroup, int32_t* dIds, cudaStream_t s);
 int64_t launch_group_counts(Matrix* m, int devGroup, unsigned long long* dCounts, cudaStream_t s);
 int64_t launch_count_nnz(Matrix* m, const double* d, int64_t n, unsigned long long* dCount, cudaStream_t s);
@@ -378,7 +385,7 @@ int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW
 int64_t fast_chain(Matrix* m, const double* dV, const double* dW, double* dOut, double* dU, cudaStream_t s);
 int64_t fast_lmm_vec(Matrix* m, const double* dY, double* dOut, cudaStream_t s);
 int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* dOut, cudaStream_t s);  // q = 2 or 4 left rows at once
-int64_t fast_decompress(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s);  // 1 = done, 0 = not covered
+int64_t fast_decompress(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s, size_t ld);  // 1 = done, 0 = not covered
 int64_t fast_lmm_vec_host(Matrix* m, const double* hostY, double* dY, double* dOut, cudaStream_t s);
 int64_t fast_lmm_vec_noalloc(Matrix* m, const double* dY, double* dOut, cudaStream_t s);
 

@@ -521,7 +521,7 @@ constexpr int DEC_NP = (LMM_MAX_UNITS + 1) / 2;  // unit pairs of a chunk: a war
 __global__ void __launch_bounds__(DEC_T, 1)
 k_decomp_fast(const LmmChunk* __restrict__ chunks, int nChunks, const uint8_t* __restrict__ imaps, int64_t nRB,
               const double* __restrict__ tablesImg, const int* __restrict__ slotCol, const double* __restrict__ constV,
-              double* __restrict__ out, int nCols, int r0, int r1, int32_t* err) {
+              double* __restrict__ out, size_t ld, int r0, int r1, int32_t* err) {
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ __align__(8) uint64_t mbar;
   __shared__ LmmChunk ch;
@@ -551,7 +551,6 @@ k_decomp_fast(const LmmChunk* __restrict__ chunks, int nChunks, const uint8_t* _
   const int64_t stepBegin = r0 / LMM_STEP, stepEnd = ((int64_t)r1 + LMM_STEP - 1) / LMM_STEP;  // r0 is a multiple of LMM_STEP
   const int64_t nSteps = stepEnd - stepBegin;
   const int64_t s0 = stepBegin + nSteps * ctaInChunk / ch.nCta, s1 = stepBegin + nSteps * (ctaInChunk + 1) / ch.nCta;
-  const size_t ld = (size_t)nCols;
   if (!tma_load_to_smem(smraw, tablesImg + ch.tblOff, (uint32_t)ch.tblDoubles * 8u, &mbar)) {
     // the tables never arrived: flag it, and make the failure visible in this CTA's cells as well (a device-buffer
     // caller only sees the error word at its next cla_stats_get)
@@ -1330,7 +1329,7 @@ bool fast_plan_partial(const Matrix* m) { return m->fast && m->fast->ok && m->fa
 
 // Rows [r0, r1) of the decompressed matrix into dOut (row r0 first) when every column is a slot of the plan and no
 // column belongs to two groups; 0 = not covered (the caller takes the tile kernel).
-int64_t fast_decompress(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s) {
+int64_t fast_decompress(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s, size_t ld) {
   FastPlan* fp = m->fast;
   if (!fp || !fp->ok || fp->partial || !fp->dLmmMaps || !m->colSrcValid || fp->nUnits != m->nCols || (r0 % LMM_STEP)) return 0;
   static const bool off = getenv("CLA_DECOMP_TILES") != nullptr;
@@ -1338,7 +1337,7 @@ int64_t fast_decompress(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s)
   size_t smem = 0;
   for (auto& c : fp->lchunks) smem = std::max(smem, (size_t)c.tblDoubles * 8);
   k_decomp_fast<<<fp->lmmGrid, DEC_T, smem, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dLmmMaps, fp->nRB, fp->dLmmTables,
-                                                fp->dSlotCol, m->hasConst ? m->dConstV : nullptr, dOut, m->nCols, r0, r1,
+                                                fp->dSlotCol, m->hasConst ? m->dConstV : nullptr, dOut, ld, r0, r1,
                                                 m->dErr);
   m->stats.kernel_launches++;
   CLA_CUDA(cudaGetLastError());

@@ -371,13 +371,13 @@ int64_t make_overlapping(Matrix* m, Matrix* child, const double* dV, int vCols, 
 // One launch per group keeps the reference's "groups in list order" summation
 // (lib/CLALibDecompress.java:427-434) without atomics.
 // --------------------------------------------------------------------------------------------------
-__global__ void k_decomp_init(double* __restrict__ out, const double* __restrict__ constV, int64_t nRows, int nCols) {
+__global__ void k_decomp_init(double* __restrict__ out, size_t ld, const double* __restrict__ constV, int64_t nRows, int nCols) {
   const int64_t n = nRows * nCols;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = constV ? constV[i % nCols] : 0.0;
+    out[(size_t)(i / nCols) * ld + i % nCols] = constV ? constV[i % nCols] : 0.0;
 }
 // rows [r0, r1); out points at row r0
-__global__ void k_decomp_dense(DevGroup g, double* __restrict__ out, int r0, int r1, int nCols) {
+__global__ void k_decomp_dense(DevGroup g, double* __restrict__ out, int r0, int r1, size_t ld) {
   const int64_t n = (int64_t)(r1 - r0) * g.gCols;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = e / g.gCols;
@@ -385,20 +385,20 @@ __global__ void k_decomp_dense(DevGroup g, double* __restrict__ out, int r0, int
     double v;
     if (g.type == GT_UNC) v = g.dense[(size_t)(r0 + r) * g.gCols + c];
     else v = g.dict[(size_t)map_get(g.mapType, g.map, g.mapHi, r0 + r) * g.gCols + c];
-    out[r * nCols + g.cols[c]] += v;
+    out[r * ld + g.cols[c]] += v;
   }
 }
-__global__ void k_decomp_sdc(DevGroup g, double* __restrict__ out, int r0, int r1, int nCols) {
+__global__ void k_decomp_sdc(DevGroup g, double* __restrict__ out, int r0, int r1, size_t ld) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int rb = r0 + warp * SKIP_ROWS;
   if (rb >= r1) return;
   const int re = min(r1, rb + SKIP_ROWS);
   sdc_walk_block(g, rb, re, [&](int row, int e) {
     const int id = g.single ? 0 : map_get(g.mapType, g.map, g.mapHi, e);
-    for (int c = 0; c < g.gCols; c++) out[(size_t)(row - r0) * nCols + g.cols[c]] += g.dict[(size_t)id * g.gCols + c];
+    for (int c = 0; c < g.gCols; c++) out[(size_t)(row - r0) * ld + g.cols[c]] += g.dict[(size_t)id * g.gCols + c];
   });
 }
-__global__ void k_decomp_rle(DevGroup g, double* __restrict__ out, int r0, int r1, int nCols) {
+__global__ void k_decomp_rle(DevGroup g, double* __restrict__ out, int r0, int r1, size_t ld) {
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nWarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -407,7 +407,7 @@ __global__ void k_decomp_rle(DevGroup g, double* __restrict__ out, int r0, int r
     if (r.start >= r1) break;
     const int a = max(r.start, r0), b = min(r.start + (int)r.len, r1);
     for (int i = a + lane; i < b; i += 32)
-      for (int c = 0; c < g.gCols; c++) out[(size_t)(i - r0) * nCols + g.cols[c]] += g.dict[(size_t)r.k * g.gCols + c];
+      for (int c = 0; c < g.gCols; c++) out[(size_t)(i - r0) * ld + g.cols[c]] += g.dict[(size_t)r.k * g.gCols + c];
   }
 }
 
@@ -430,7 +430,7 @@ __device__ __forceinline__ int db_pos(int r) { return (r & 3) * 32 + (r >> 2); }
 constexpr int DB_WARPS = 16;  // two columns per warp (measured 4 / 8 / 16 / 32 warps on 1M x 500 mixed: 2.54 / 2.11 / 1.87 / 2.07 ms)
 __global__ void __launch_bounds__(DB_WARPS * 32)
 k_decomp_block(const DevGroup* __restrict__ groups, const int32_t* __restrict__ colSrc, const double* __restrict__ constV,
-               double* __restrict__ out, int r0, int r1, int nCols, int exactSdc) {
+               double* __restrict__ out, size_t ld, int r0, int r1, int nCols, int exactSdc) {
   extern __shared__ double dtile[];  // [DB_COLS][DB_LD]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rb = r0 + blockIdx.x * DB_ROWS, re = min(r1, rb + DB_ROWS), nr = re - rb;
@@ -515,19 +515,246 @@ k_decomp_block(const DevGroup* __restrict__ groups, const int32_t* __restrict__ 
     const size_t ustride = us ? (size_t)uncStride[lane] : 0;
     const double ucst = us ? uncCst[lane] : 0.0;
     const double* tcol = dtile + lane * DB_LD;
-    double* o = out + (size_t)(rb - r0) * nCols + c0 + lane;
+    double* o = out + (size_t)(rb - r0) * ld + c0 + lane;
     for (int rr = warp; rr < nr; rr += DB_WARPS)
-      o[(size_t)rr * nCols] = us ? ucst + us[(size_t)(rb + rr) * ustride] : tcol[db_pos(rr)];
+      o[(size_t)rr * ld] = us ? ucst + us[(size_t)(rb + rr) * ustride] : tcol[db_pos(rr)];
   }
 }
 
-// r0 must be a multiple of SKIP_ROWS
-int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s) {
+// Decompress, column per lane: a warp owns 32 neighbouring columns and DC_ROWS rows and walks down the rows, every lane
+// in its own column: 16 ids per load and a table in shared memory (entry k of lane l at k * 32 + l: no bank conflicts) for
+// small dense-map groups, the next listed row and its value for an SDC column, the current run for an RLE column, the dense
+// block itself for an uncompressed one. Each cell is formed in the register it is stored from, and the warps of a CTA
+// write whole stretches of a row at the same time. The tile kernel above builds every cell in shared memory and reads
+// it back, and finds its way into the offset streams by a scan. What is left is the latency of the chains item -> value and
+// run -> value. 250,001 x 500 mixed (1 GB): 482 -> 310 us, 3.2 TB/s written.
+struct DecCol {
+  const double* dict;  // dictionary (or dense block) + position in the group
+  const void* a;       // byte / bit map; SDC items; RLE runs
+  const void* b;       // SDC skip entries; RLE first run of every block
+  int64_t n;           // SDC listed rows; RLE runs
+  double cst;          // column constant
+  int32_t kind;        // DC_*
+  int32_t stride, tbl, nVals;
+  int32_t mapType, pad;
+};
+enum { DC_CONST = 0, DC_BYTES = 1, DC_BITS = 2, DC_MAP = 3, DC_SDC = 4, DC_RLE = 5, DC_UNC = 6 };
+constexpr int DC_ROWS = 64;            // (256 / 128 / 64 rows on 250,001 x 500: 346 / 319 / 310 us)
+constexpr size_t DC_TBL = 100 * 1024;  // table bytes of a CTA
+__global__ void __launch_bounds__(512) k_decomp_cols(const DecCol* __restrict__ cols, double* __restrict__ out, size_t ld, int r0, int r1,
+                                                     int nRows, int nCols, int exactSdc) {
+  extern __shared__ double dct[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nW = blockDim.x >> 5;
+  const int c = (blockIdx.y * nW + warp) * 32 + lane;
+  const int rb = r0 + blockIdx.x * DC_ROWS, re = min(r1, rb + DC_ROWS), blk = rb / SKIP_ROWS, nBlocks = (nRows + SKIP_ROWS - 1) / SKIP_ROWS;
+  DecCol d;
+  d.kind = -1;
+  if (c < nCols) d = cols[c];
+  const double cst = c < nCols ? d.cst : 0.0;
+  double* T = dct;
+  if (d.kind == DC_BYTES || d.kind == DC_BITS) {
+    T = dct + d.tbl + lane;
+    for (int k = 0; k < d.nVals; k++) T[k * 32] = cst + d.dict[(size_t)k * d.stride];
+  }
+  double* o = out + (size_t)(rb - r0) * ld + c;
+  if (d.kind == DC_BYTES || d.kind == DC_BITS) {  // (a lane reads only what it wrote itself)
+    for (int r = rb; r < re; r += 16, o += 16 * ld) {
+      if (r + 16 <= re) {
+        uint32_t w[4];
+        if (d.kind == DC_BYTES) {
+          const uint4 v = __ldg((const uint4*)((const uint8_t*)d.a + r));
+          w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+        } else {
+          const uint32_t bits = (uint32_t)(((const unsigned long long*)d.a)[r >> 6] >> (r & 63));
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const uint32_t x = bits >> (4 * q);
+            w[q] = (x & 1u) | ((x & 2u) << 7) | ((x & 4u) << 14) | ((x & 8u) << 21);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i++) o[i * ld] = T[((w[i >> 2] >> (8 * (i & 3))) & 0xFF) * 32];
+      } else
+        for (int i = 0; r + i < re; i++) o[i * ld] = T[map_get(d.mapType, d.a, nullptr, r + i) * 32];
+    }
+  } else if (d.kind == DC_UNC) {
+    const double* x = d.dict + (size_t)rb * d.stride;
+    const size_t xs = d.stride;
+    for (int r = rb; r < re; r += 16, o += 16 * ld, x += 16 * xs) {
+      if (r + 16 <= re) {
+        double v[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = __ldcs(x + i * xs);
+#pragma unroll
+        for (int i = 0; i < 16; i++) o[i * ld] = cst + v[i];
+      } else
+        for (int i = 0; r + i < re; i++) o[i * ld] = cst + x[i * xs];
+    }
+  } else if (d.kind == DC_SDC) {
+    const uint32_t* items = (const uint32_t*)d.a;
+    const SdcSkip* sk = (const SdcSkip*)d.b;
+    const int64_t end = blk + 1 < nBlocks ? (int64_t)sk[blk + 1].elem : d.n;
+    int64_t p = sk[blk].elem, hi = end;
+    const uint32_t first = (uint32_t)(rb & (SKIP_ROWS - 1));
+    while (p < hi) {  // first item at or behind row rb
+      const int64_t mid = (p + hi) >> 1;
+      if ((items[mid] & 1023u) < first) p = mid + 1;
+      else hi = mid;
+    }
+    const int base = blk * SKIP_ROWS;
+    auto value = [&](uint32_t it) { return exactSdc ? d.dict[(size_t)(it >> 10) * d.stride] : cst + d.dict[(size_t)(it >> 10) * d.stride]; };
+    // the next listed row and its value, and the item behind it
+    uint32_t it = p < end ? items[p] : 0u, ahead = p + 1 < end ? items[p + 1] : 0u;
+    int row = p < end ? base + (int)(it & 1023u) : INT_MAX;
+    double val = p < end ? value(it) : 0.0;
+    for (int r = rb; r < re; r++, o += ld) {
+      double v = cst;
+      if (r == row) {
+        v = val;
+        p++;
+        row = p < end ? base + (int)(ahead & 1023u) : INT_MAX;
+        if (p < end) val = value(ahead);
+        ahead = p + 1 < end ? items[p + 1] : 0u;
+      }
+      *o = v;
+    }
+  } else if (d.kind == DC_RLE) {
+    const RleRun* runs = (const RleRun*)d.a;
+    int64_t ri = ((const int32_t*)d.b)[blk];
+    int start = INT_MAX, end = INT_MAX;  // the current or next run
+    double val = 0.0;
+    auto next = [&]() {
+      if (ri < d.n) {
+        const RleRun run = runs[ri++];
+        start = run.start;
+        end = run.start + (int)run.len;
+        val = cst + d.dict[(size_t)run.k * d.stride];
+      } else
+        start = end = INT_MAX;
+    };
+    next();
+    for (int r = rb; r < re; r++, o += ld) {
+      while (end <= r) next();
+      *o = r >= start ? val : cst;
+    }
+  } else if (d.kind == DC_MAP) {
+    for (int r = rb; r < re; r++, o += ld) *o = cst + d.dict[(size_t)map_get(d.mapType, d.a, d.b, r) * d.stride];
+  } else if (d.kind == DC_CONST) {
+    for (int r = rb; r < re; r++, o += ld) *o = cst;
+  }
+}
+
+// Column records of k_decomp_cols; m->dec.warps tells how many warps a CTA has (0: the tile kernel is the better one).
+static int64_t ensure_dec(Matrix* m, cudaStream_t s) {
+  DecPlan& D = m->dec;
+  if (D.tried) return CLA_OK;
+  D.tried = true;
+  int64_t rc;
+  if ((rc = ensure_row_lists(m, s)) < 0) return rc;
+  if (!m->rows.ok) return CLA_OK;
+  std::vector<DecCol> cols(m->nCols);
+  for (int c = 0; c < m->nCols; c++) {
+    cols[c] = DecCol{};
+    cols[c].kind = DC_CONST;
+    cols[c].cst = m->hasConst ? m->constV[c] : 0.0;
+  }
+  int scattered = 0;
+  for (size_t hi = 0; hi < m->hg.size(); hi++) {
+    const int gi = m->regToDev[hi];
+    if (gi < 0) continue;
+    const DevGroup& g = m->groups[gi];
+    for (int j = 0; j < g.gCols; j++) {
+      DecCol& d = cols[m->hg[hi].cols[j]];
+      d.stride = g.gCols;
+      d.nVals = g.nVals;
+      d.mapType = g.mapType;
+      d.dict = (g.type == GT_UNC ? g.dense : g.dict) + j;
+      if (g.type == GT_DDC) {
+        d.a = g.map;
+        d.b = g.mapHi;
+        d.kind = g.nVals > 256 ? DC_MAP
+                 : (g.mapType == CLA_MAP_UBYTE || g.mapType == CLA_MAP_BYTE ? DC_BYTES : (g.mapType == CLA_MAP_BIT ? DC_BITS : DC_MAP));
+        scattered += d.kind == DC_MAP;
+      } else if (g.type == GT_SDC) {
+        if (g.nOff == 0) continue;
+        d.kind = DC_SDC;
+        d.a = m->rows.sdcItems + m->rows.sdcBase[gi];
+        d.b = g.skip;
+        d.n = g.nOff;
+        if (!m->multiCover) d.dict = g.dictRaw + j;
+      } else if (g.type == GT_RLE) {
+        if (g.nRuns == 0) continue;
+        d.kind = DC_RLE;
+        d.a = g.runs;
+        d.b = g.runSkip;
+        d.n = g.nRuns;
+      } else
+        d.kind = DC_UNC;
+    }
+  }
+  // A lane-private gather from a large dictionary touches 32 lines per row, and a warp whose columns are of several kinds
+  // walks its rows once per kind: matrices with many such columns keep the tile kernel (1M x 60 with four kinds in two
+  // warps: 280 us there, 342 here).
+  int kinds = 0;
+  for (int c0 = 0; c0 < m->nCols; c0 += 32) {
+    unsigned seen = 0;
+    for (int c = c0; c < std::min(m->nCols, c0 + 32); c++) seen |= 1u << (cols[c].kind == DC_BITS ? DC_BYTES : cols[c].kind);
+    kinds += __builtin_popcount(seen);
+  }
+  if (scattered * 16 > m->nCols || kinds * 5 > (m->nCols + 31) / 32 * 7) return CLA_OK;
+  // tables: 256 bytes per tuple of the deepest small dictionary of every 32 columns; fewer columns per CTA if they are deep
+  int warps = std::max(1, std::min(16, (m->nCols + 31) / 32));
+  size_t most = 0;
+  for (; warps >= 1; warps /= 2) {
+    most = 0;
+    for (int c0 = 0; c0 < m->nCols; c0 += warps * 32) {
+      size_t b = 0;
+      for (int g0 = c0; g0 < std::min(m->nCols, c0 + warps * 32); g0 += 32) {
+        int deep = 0;
+        for (int c = g0; c < std::min(m->nCols, g0 + 32); c++)
+          if (cols[c].kind == DC_BYTES || cols[c].kind == DC_BITS) deep = std::max(deep, cols[c].nVals);
+        for (int c = g0; c < std::min(m->nCols, g0 + 32); c++) cols[c].tbl = (int)(b / 8);
+        b += (size_t)deep * 256;
+      }
+      most = std::max(most, b);
+    }
+    if (most <= DC_TBL) break;
+  }
+  if (warps < 1) return CLA_OK;
+  void* p = nullptr;
+  if ((rc = plan_alloc(m, &p, cols.size() * sizeof(DecCol))) < 0) return rc;
+  CLA_CUDA(cudaMemcpyAsync(p, cols.data(), cols.size() * sizeof(DecCol), cudaMemcpyHostToDevice, s));
+  CLA_CUDA(cudaStreamSynchronize(s));
+  D.cols = p;
+  D.warps = warps;
+  D.smem = most;
+  return CLA_OK;
+}
+
+// r0 must be a multiple of SKIP_ROWS; a row of dOut is ld doubles wide
+int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStream_t s, size_t ld) {
+  if (ld == 0) ld = (size_t)m->nCols;
   const int64_t n = (int64_t)(r1 - r0) * m->nCols;
   if (n <= 0) return CLA_OK;
   if (m->colSrcValid) {  // no column held by two groups: one pass, every cell written once
-    const int64_t rf = fast_decompress(m, r0, r1, dOut, s);  // byte-map matrices: straight from the column-per-lane layout
+    const int64_t rf = fast_decompress(m, r0, r1, dOut, s, ld);  // byte-map matrices: straight from the column-per-lane layout
     if (rf != 0) return rf < 0 ? rf : CLA_OK;
+    int64_t rc;
+    const bool byCols = n >= (4 << 20);  // (below, too few of its warps are in flight)
+    if (byCols && (rc = ensure_dec(m, s)) < 0) return rc;
+    if (byCols && m->dec.warps > 0) {
+      static bool decAttr[64] = {};  // per device
+      if (!decAttr[m->device & 63]) {
+        CLA_CUDA(cudaFuncSetAttribute(k_decomp_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DC_TBL));
+        decAttr[m->device & 63] = true;
+      }
+      dim3 grid((r1 - r0 + DC_ROWS - 1) / DC_ROWS, (m->nCols + m->dec.warps * 32 - 1) / (m->dec.warps * 32));
+      k_decomp_cols<<<grid, m->dec.warps * 32, m->dec.smem, s>>>((const DecCol*)m->dec.cols, dOut, ld, r0, r1, m->nRows, m->nCols,
+                                                                m->multiCover ? 0 : 1);
+      m->stats.kernel_launches++;
+      CLA_CUDA(cudaGetLastError());
+      return CLA_OK;
+    }
     const size_t smem = (size_t)DB_COLS * DB_LD * sizeof(double);
     static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
     bool& attr = attrSet[m->device & 63];
@@ -536,23 +763,23 @@ int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStr
       attr = true;
     }
     dim3 grid((r1 - r0 + DB_ROWS - 1) / DB_ROWS, (m->nCols + DB_COLS - 1) / DB_COLS);
-    k_decomp_block<<<grid, DB_WARPS * 32, smem, s>>>(m->dGroups, m->dColSrc, m->hasConst ? m->dConstV : nullptr, dOut, r0, r1, m->nCols,
+    k_decomp_block<<<grid, DB_WARPS * 32, smem, s>>>(m->dGroups, m->dColSrc, m->hasConst ? m->dConstV : nullptr, dOut, ld, r0, r1, m->nCols,
                                            m->multiCover ? 0 : 1);
     m->stats.kernel_launches++;
     CLA_CUDA(cudaGetLastError());
     return CLA_OK;
   }
   // overlapping groups: constants first, then every group adds its values (the reference's list-order summation)
-  k_decomp_init<<<grid_for(n, 256), 256, 0, s>>>(dOut, m->hasConst ? m->dConstV : nullptr, r1 - r0, m->nCols);
+  k_decomp_init<<<grid_for(n, 256), 256, 0, s>>>(dOut, ld, m->hasConst ? m->dConstV : nullptr, r1 - r0, m->nCols);
   m->stats.kernel_launches++;
   for (auto& g : m->groups) {
     if (g.type == GT_DDC || g.type == GT_UNC)
-      k_decomp_dense<<<grid_for((int64_t)(r1 - r0) * g.gCols, 256), 256, 0, s>>>(g, dOut, r0, r1, m->nCols);
+      k_decomp_dense<<<grid_for((int64_t)(r1 - r0) * g.gCols, 256), 256, 0, s>>>(g, dOut, r0, r1, ld);
     else if (g.type == GT_SDC) {
       const int nb = (r1 - r0 + SKIP_ROWS - 1) / SKIP_ROWS;
-      k_decomp_sdc<<<(nb * 32 + 255) / 256, 256, 0, s>>>(g, dOut, r0, r1, m->nCols);
+      k_decomp_sdc<<<(nb * 32 + 255) / 256, 256, 0, s>>>(g, dOut, r0, r1, ld);
     } else if (g.type == GT_RLE && g.nRuns)
-      k_decomp_rle<<<64, 256, 0, s>>>(g, dOut, r0, r1, m->nCols);
+      k_decomp_rle<<<64, 256, 0, s>>>(g, dOut, r0, r1, ld);
     m->stats.kernel_launches++;
   }
   CLA_CUDA(cudaGetLastError());

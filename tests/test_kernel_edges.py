@@ -109,3 +109,28 @@ def test_non_finite_values_stay_in_their_rows(nRows):
     assert np.array_equal(np.isfinite(got), fine)
     assert rel_err(got[fine], want[fine], np.abs(X[fine]) @ np.abs(v)) < TOL
     cmb.free()
+
+
+@pytest.mark.parametrize("nRows", [33, 5000])
+@pytest.mark.parametrize("nCols", [127, 129, 160, 257])
+def test_self_product_blocks(oracle, nRows, nCols):
+    """t(X) X with and without SDC / RLE columns around the edges of the 128 x 128 blocks and their 32 x 32 tiles."""
+    for kinds in (("ddc",) * nCols, ("ddc", "sdc", "rle") * (nCols // 3) + ("ddc",) * (nCols % 3)):
+        cmb = datagen.random_cmb(nCols + nRows, nRows, kinds).to_device()
+        X = dense_of(cmb)
+        got = CLALibTSMM.leftMultByTransposeSelf(cmb)
+        assert rel_err(got, oracle.dense_tsmm_ld(X), np.abs(X).T @ np.abs(X) + 1e-300) < TOL
+        assert np.array_equal(got, got.T)
+        cmb.free()
+
+
+@pytest.mark.parametrize("nRows", [1, 255, 257, 1040, 5001])
+@pytest.mark.parametrize("nCols", [31, 33, 530])
+def test_decompress_columns(nRows, nCols):
+    """Decompress with the columns of a CTA of every kind, row remainders and part blocks: the cells are the registered
+    values."""
+    kinds = ("ddc", "sdcz", "rle", "unc", "ddc_bit", "sdc", "const", "empty", "ole", "sdcs")
+    kinds = kinds * (nCols // 11) + ("ddc",) * (nCols % 11)
+    cmb = datagen.random_cmb(nRows + nCols, nRows, kinds).to_device()
+    assert np.array_equal(np.array(CLALibDecompress.decompress(cmb)), dense_of(cmb))
+    cmb.free()
