@@ -2,20 +2,14 @@
 //
 // The reference multiplies dictionaries when there are few groups and otherwise decompresses the
 // whole matrix and runs a dense self product (:73-77). Here the second strategy is used for all
-// inputs, but blocked so the dense form never exists in full: a chunk of rows small enough to stay
-// resident in L2 is decompressed into scratch, an FP64 tensor-core (DMMA m8n8k4) SYRK adds
-// chunk^T * chunk into the upper 64 x 64 blocks of the result, and the next chunk reuses the scratch.
+// inputs, but blocked so the dense form never exists in full: a chunk of rows is decompressed into scratch, an FP64
+// tensor-core SYRK adds chunk^T * chunk into the upper triangle of the result, and the next chunk reuses the scratch.
 // Constant columns are part of the decompressed chunk, so no correction layer is needed.
 #include "cla_common.cuh"
 #include <algorithm>
 #include <cstdlib>
 
 namespace cla {
-
-constexpr int TS_BLK = 64;      // C block edge
-constexpr int TS_KT = 16;       // rows per shared-memory stage
-constexpr int TS_LD = 68;       // padded row stride (doubles): k * 68 mod 16 = {0,4,8,12} keeps fragment loads conflict free
-constexpr int TS_THREADS = 256;
 
 __device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -51,85 +45,211 @@ __device__ __forceinline__ uint32_t ld_u16_here(const uint16_t* p) {
   return v;
 }
 
-// grid: (blocks of A columns x blocks of B columns, k splits). A: [rows x aCols], B: [rows x bCols], both row-major
-// chunks of the same rows. C [aCols x bCols] += A^T B. A CTA owns one 64 x 64 block of C; warp w its rows 8 w .. 8 w + 8.
-// 16-row stages, double buffered (static shared memory, 35 KB): the loads of the next stage are issued into registers before the DMMAs of the
-// current one and stored to the other buffer after them, so one barrier per stage and no exposed load latency.
-// SYRK: B is A, blockIdx.x enumerates the block pairs bi <= bj of the upper triangle, only cells on or above the
-// diagonal are added (t(X) %*% X with more than 128 columns).
+// C [aCols x bCols] += A^T B for row-major chunks A [rows x lda], B [rows x ldb] of the same rows, on 128 x 128 blocks of C:
+// a CTA owns one block (or, on the diagonal of a self product, its upper triangle of 32 x 32 tiles) over a range of rows,
+// a warp one 32 x 32 tile in registers (eight m16n8k8 per eight rows from 16 fragment loads). 16-row stages arrive row by
+// row by TMA bulk copies in a ring of six, issued four stages ahead; full / empty mbarriers let the warps drift apart, so
+// that one's fragment loads hide behind the others' products. Rows of a stage are 132 doubles apart (4 mod 16:
+// conflict-free fragment loads). The blocks get CTAs in proportion to their tiles.
+// Bound: the FP64 tensor pipe, 128 clocks per warp and eight rows against 32 wavefronts of the L1 data pipe; it is busy 73 %
+// of the time, 90 % being the most that the 3 : 3 : 2 : 2 split of a triangle's ten tiles allows. 98,304 rows x 250
+// columns: 308 us (64 x 64 blocks of m8n8k4 with the stage loaded through registers: 316 at 45 % and atomics four times as
+// often; with cp.async by all threads and a barrier per stage: 318 at 67 %).
 constexpr int GT_KT = 16;
+constexpr int GT_BLK = 128;
+constexpr int GT_LD = GT_BLK + 4;
+constexpr int GT_WARPS = 16;
+constexpr int GT_T = GT_WARPS * 32;
+constexpr int GT_STAGES = 6;
+constexpr int GT_STAGE = 2 * GT_KT * GT_LD;  // doubles
+constexpr size_t GT_SMEM = (size_t)GT_STAGES * GT_STAGE * sizeof(double) + 2 * GT_STAGES * sizeof(uint64_t);
+constexpr int GT_PAIRS = 64;  // blocks per launch
+struct GemmBlocks {
+  int n;
+  int cta0[GT_PAIRS + 1];   // CTAs [cta0[p], cta0[p + 1]) split the rows of block p
+  int16_t bi[GT_PAIRS], bj[GT_PAIRS];
+};
+__device__ __forceinline__ bool gt_wait(uint32_t bar, uint32_t parity) {
+  uint32_t done = 0;
+  for (int it = 0; it < (1 << 20) && !done; it++)
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+  return done != 0;
+}
+// lda, ldb: even, rows 16-byte aligned; the rows up to the next multiple of GT_KT behind `rows` are zero.
 template <bool SYRK>
-__global__ void __launch_bounds__(TS_THREADS)
-k_gemm_tn_dmma(const double* __restrict__ A, int aCols, const double* __restrict__ B, int bCols, int rows, int nBlkB,
-               double* __restrict__ C, int rowsPerSplit) {
-  __shared__ double sI[2][GT_KT * TS_LD];
-  __shared__ double sJ[2][GT_KT * TS_LD];
-  int bi, bj;
-  if (SYRK) {  // decode the linear pair index into (bi <= bj)
-    int p = blockIdx.x;
-    bi = 0;
-    while (p >= nBlkB - bi) {
-      p -= nBlkB - bi;
-      bi++;
+__global__ void __launch_bounds__(GT_T, 1)
+k_gemm_tn(const double* __restrict__ A, int aCols, int lda, const double* __restrict__ B, int bCols, int ldb, int rows,
+          double* __restrict__ C, const __grid_constant__ GemmBlocks G, int32_t* err) {
+  extern __shared__ __align__(128) double gts[];  // [GT_STAGES][A | B][GT_KT][GT_LD], full and empty barriers
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  int p = 0;
+  while (p + 1 < G.n && (int)blockIdx.x >= G.cta0[p + 1]) p++;
+  const int i0 = G.bi[p] * GT_BLK, j0 = G.bj[p] * GT_BLK;
+  const bool diag = SYRK && i0 == j0;
+  const int nCta = G.cta0[p + 1] - G.cta0[p], c = blockIdx.x - G.cta0[p];
+  const int nSt = (rows + GT_KT - 1) / GT_KT;
+  const int s0 = (int)((int64_t)nSt * c / nCta), s1 = (int)((int64_t)nSt * (c + 1) / nCta);
+  // The block's tiles are dealt to the warps in turn, so that they spread over the SM's four schedulers (by position in
+  // the block, the triangle's tiles fell 1 : 2 : 3 : 4 on them and cost as much as a whole block); with eight tiles or
+  // fewer two warps share a tile, one for each eight rows of a stage.
+  const int ti = (min(GT_BLK, aCols - i0) + 31) / 32, tj = (min(GT_BLK, bCols - j0) + 31) / 32;
+  const int nT = diag ? ti * (ti + 1) / 2 : ti * tj, split = nT <= GT_WARPS / 2 ? 2 : 1;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(gts);
+  const uint32_t full = base + (uint32_t)(GT_STAGES * GT_STAGE * 8), empty = full + GT_STAGES * 8;
+  if (tid == 0) {
+    for (int i = 0; i < GT_STAGES; i++) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + 8 * i));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty + 8 * i), "r"(nT * split));
     }
-    bj = bi + p;
-  } else {
-    bi = blockIdx.x / nBlkB;
-    bj = blockIdx.x - bi * nBlkB;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int rBeg = blockIdx.y * rowsPerSplit, rEnd = min(rows, rBeg + rowsPerSplit);
-  if (rBeg >= rEnd) return;
-  double c[8][2];
-#pragma unroll
-  for (int t = 0; t < 8; t++) c[t][0] = c[t][1] = 0.0;
-  const int am = lane >> 2, ak = lane & 3;
-  // this thread's cells of a stage: column cc of rows kk0, kk0 + 4, ... (GT_KT * 64 / 256 = 4 cells per operand)
-  const int cc = tid & 63, kk0 = tid >> 6;
-  const int ci = bi * TS_BLK + cc, cj = bj * TS_BLK + cc;
-  constexpr int GT_CELLS = GT_KT * TS_BLK / TS_THREADS;
-  double va[GT_CELLS], vb[GT_CELLS];
-  auto load = [&](int r) {
-#pragma unroll
-    for (int u = 0; u < GT_CELLS; u++) {
-      const int row = r + kk0 + 4 * u;
-      va[u] = (row < rEnd && ci < aCols) ? ld_f64_here(A + (size_t)row * aCols + ci) : 0.0;
-      vb[u] = (row < rEnd && cj < bCols) ? ld_f64_here(B + (size_t)row * bCols + cj) : 0.0;
-    }
-  };
-  auto store = [&](int buf) {
-#pragma unroll
-    for (int u = 0; u < GT_CELLS; u++) {
-      sI[buf][(kk0 + 4 * u) * TS_LD + cc] = va[u];
-      sJ[buf][(kk0 + 4 * u) * TS_LD + cc] = vb[u];
-    }
-  };
-  load(rBeg);
-  store(0);
   __syncthreads();
-  int cur = 0;
-  for (int r = rBeg; r < rEnd; r += GT_KT) {
-    const bool more = r + GT_KT < rEnd;
-    if (more) load(r + GT_KT);
+  // the copies, by warp 0: lane = row of the stage, lanes 0..15 A, lanes 16..31 B
+  const uint32_t wA = (uint32_t)min(GT_BLK, lda - i0) * 8u, wB = diag ? 0u : (uint32_t)min(GT_BLK, ldb - j0) * 8u;
+  const bool isB = lane >= GT_KT;
+  const uint32_t bytes = isB ? wB : wA;
+  const double* src = isB ? B + (size_t)(lane - GT_KT) * ldb + j0 : A + (size_t)lane * lda + i0;
+  const size_t step = (size_t)GT_KT * (isB ? ldb : lda);
+  auto issue = [&](int st) -> bool {
+    if (st >= s1) return true;
+    const int k = st - s0, b = k % GT_STAGES;
+    if (k >= GT_STAGES && !gt_wait(empty + 8 * b, (uint32_t)(k / GT_STAGES - 1) & 1u)) return false;
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + 8 * b), "r"((wA + wB) * GT_KT) : "memory");
+    __syncwarp();
+    if (bytes)
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       base + (uint32_t)(b * GT_STAGE + lane * GT_LD) * 8u),
+                   "l"(src + (size_t)st * step), "r"(bytes), "r"(full + 8 * b)
+                   : "memory");
+    return true;
+  };
+  if (warp == 0)
+    for (int i = 0; i < GT_STAGES - 2; i++) issue(s0 + i);
+  const int tile = split == 2 ? warp & (GT_WARPS / 2 - 1) : warp;
+  if (tile >= nT) return;
+  const int kBeg = split == 2 ? warp / (GT_WARPS / 2) * 8 : 0, kEnd = split == 2 ? kBeg + 8 : GT_KT;
+  int wi = 0, wj = tile;
+  if (diag) {
+    int rest = tile;
+    while (wi + 1 < ti && rest >= ti - wi) rest -= ti - wi, wi++;
+    wj = wi + rest;
+  } else
+    wi = tile / tj, wj = tile - wi * tj;
+  double acc[2][4][4];
 #pragma unroll
-    for (int k0 = 0; k0 < GT_KT; k0 += 4) {
-      const double a = sI[cur][(k0 + ak) * TS_LD + warp * 8 + am];  // A[m][k] = A[k][bi*64 + warp*8 + m]
+  for (int i = 0; i < 2; i++)
 #pragma unroll
-      for (int t = 0; t < 8; t++) dmma884(c[t][0], c[t][1], a, sJ[cur][(k0 + ak) * TS_LD + t * 8 + am]);
+    for (int j = 0; j < 4; j++)
+#pragma unroll
+      for (int u = 0; u < 4; u++) acc[i][j][u] = 0.0;
+  for (int st = s0; st < s1; st++) {
+    const int n = st - s0, b = n % GT_STAGES;
+    // four stages ahead, into the buffer of the stage before last: the other warps have long left that one
+    if (warp == 0 && !issue(st + GT_STAGES - 2)) {
+      if (lane == 0) atomicExch(err, 111);
+      return;
     }
-    if (more) store(cur ^ 1);
-    __syncthreads();
-    cur ^= 1;
-  }
-  const int gi = bi * TS_BLK + warp * 8 + (lane >> 2);
-#pragma unroll
-  for (int t = 0; t < 8; t++) {
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const int gj = bj * TS_BLK + t * 8 + (lane & 3) * 2 + u;
-      if (gi < aCols && gj < bCols && (!SYRK || gi <= gj) && c[t][u] != 0.0) atomicAdd(&C[(size_t)gi * bCols + gj], c[t][u]);
+    if (!gt_wait(full + 8 * b, (uint32_t)(n / GT_STAGES) & 1u)) {
+      if (lane == 0) atomicExch(err, 112);
+      return;
     }
+    const double* sA = gts + (size_t)b * GT_STAGE + wi * 32 + g;
+    const double* sB = gts + (size_t)b * GT_STAGE + (diag ? 0 : GT_KT * GT_LD) + wj * 32 + g;
+#pragma unroll 1
+    for (int k = kBeg; k < kEnd; k += 8) {
+      double a[2][4], bb[4][2];
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const double* x = sA + (k + t) * GT_LD + i * 16;
+        a[i][0] = x[0];
+        a[i][1] = x[8];
+        a[i][2] = x[4 * GT_LD];
+        a[i][3] = x[4 * GT_LD + 8];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        bb[j][0] = sB[(k + t) * GT_LD + j * 8];
+        bb[j][1] = sB[(k + 4 + t) * GT_LD + j * 8];
+      }
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) dmma1688(acc[i][j], a[i][0], a[i][1], a[i][2], a[i][3], bb[j][0], bb[j][1]);
+    }
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * b) : "memory");
   }
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int gi = i0 + wi * 32 + i * 16 + g + 8 * (u >> 1), gj = j0 + wj * 32 + j * 8 + 2 * t + (u & 1);
+        if (gi < aCols && gj < bCols && (!SYRK || gi <= gj) && acc[i][j][u] != 0.0) atomicAdd(&C[(size_t)gi * bCols + gj], acc[i][j][u]);
+      }
+}
+
+template <bool SYRK>
+static int64_t launch_gemm_tn(Matrix* m, const double* A, int aCols, int lda, const double* B, int bCols, int ldb, int rows, double* C,
+                              cudaStream_t s) {
+  static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
+  if (!attrSet[m->device & 63]) {
+    CLA_CUDA(cudaFuncSetAttribute(k_gemm_tn<SYRK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM));
+    attrSet[m->device & 63] = true;
+  }
+  const int nA = (aCols + GT_BLK - 1) / GT_BLK, nB = (bCols + GT_BLK - 1) / GT_BLK, nSt = (rows + GT_KT - 1) / GT_KT;
+  auto tiles = [](int cols, int b) { return (std::min(GT_BLK, cols - b * GT_BLK) + 31) / 32; };
+  int bi = 0, bj = 0;
+  while (bi < nA) {  // up to GT_PAIRS blocks per launch
+    GemmBlocks G;
+    G.n = 0;
+    double w[GT_PAIRS], sum = 0.0;
+    while (bi < nA && G.n < GT_PAIRS) {
+      G.bi[G.n] = (int16_t)bi;
+      G.bj[G.n] = (int16_t)bj;
+      const int ti = tiles(aCols, bi), tj = tiles(bCols, bj);
+      const int nT = (SYRK && bi == bj) ? ti * (ti + 1) / 2 : ti * tj;
+      sum += w[G.n++] = nT <= 8 ? (nT + 1) / 2 * 2 : (nT + 3) / 4 * 4;  // what the busiest scheduler has to do
+      if (++bj == nB) {
+        bi++;
+        bj = SYRK ? bi : 0;
+      }
+    }
+    int at = 0;
+    double cum = 0.0;
+    for (int p = 0; p < G.n; p++) {
+      G.cta0[p] = at;
+      cum += w[p];
+      const int want = std::max(at + 1, (int)(cum / sum * m->smCount + 0.5));
+      at += std::max(1, std::min(want - at, (nSt + 1) / 2));  // at least two stages each
+    }
+    G.cta0[G.n] = at;
+    k_gemm_tn<SYRK><<<at, GT_T, GT_SMEM, s>>>(A, aCols, lda, B, bCols, ldb, rows, C, G, m->dErr);
+    m->stats.kernel_launches++;
+  }
+  CLA_CUDA(cudaGetLastError());
+  return CLA_OK;
+}
+
+// Rows [r0, r1) decompressed into X as k_gemm_tn wants them: ld even, zeros up to a whole stage.
+static int64_t decompress_chunk(Matrix* m, int r0, int r1, double* X, int ld, cudaStream_t s) {
+  const int rows = r1 - r0, pad = (rows + GT_KT - 1) / GT_KT * GT_KT - rows;
+  if (pad) CLA_CUDA(cudaMemsetAsync(X + (size_t)rows * ld, 0, (size_t)pad * ld * sizeof(double), s));
+  return launch_decompress_range(m, r0, r1, X, s, (size_t)ld);
+}
+
+// Rows of a decompressed chunk: enough that the partial sums every CTA adds to the result at its end do not count, little
+// enough not to matter in 180 GB.
+static int64_t chunk_rows(int64_t nRows, int64_t cols) {
+  int64_t chunk = (192ll << 20) / (cols * 8);
+  chunk = std::max<int64_t>(SKIP_ROWS, (chunk / SKIP_ROWS) * SKIP_ROWS);
+  return std::min<int64_t>(chunk, (nRows + SKIP_ROWS - 1) / SKIP_ROWS * SKIP_ROWS);
 }
 
 // --------------------------------------------------------------------------------------------------
@@ -625,30 +745,21 @@ int64_t launch_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
     prof_end(m, s);
     m->stats.kernel_launches++;
   } else {
-    // chunk of rows whose dense form stays well inside L2 (48 MB)
-    int64_t chunk = (48ll << 20) / ((int64_t)n * 8);
-    chunk = std::max<int64_t>(SKIP_ROWS, (chunk / SKIP_ROWS) * SKIP_ROWS);
-    chunk = std::min<int64_t>(chunk, ((int64_t)m->nRows + SKIP_ROWS - 1) / SKIP_ROWS * SKIP_ROWS);
-    if ((rc = ensure_scratch2(m, (size_t)chunk * n * sizeof(double))) < 0) return rc;
+    const int64_t chunk = chunk_rows(m->nRows, n);
+    const int ld = tri ? n : (n + 1) & ~1;
+    if ((rc = ensure_scratch2(m, (size_t)chunk * ld * sizeof(double))) < 0) return rc;
     double* X = (double*)m->scratch2;
-    const int nBlk = (n + TS_BLK - 1) / TS_BLK;
-    const int nPairs = nBlk * (nBlk + 1) / 2;
     for (int64_t r0 = 0; r0 < m->nRows; r0 += chunk) {
       const int r1 = (int)std::min<int64_t>(m->nRows, r0 + chunk);
-      if ((rc = launch_decompress_range(m, (int)r0, r1, X, s)) < 0) return rc;
       const int rows = r1 - (int)r0;
+      if ((rc = tri ? launch_decompress_range(m, (int)r0, r1, X, s) : decompress_chunk(m, (int)r0, r1, X, ld, s)) < 0) return rc;
       if (tri) {
         const int64_t nStages = ((int64_t)rows + TT_KT - 1) / TT_KT;
         launch_tri16(false, -2, 0, n, (int)std::min<int64_t>(m->smCount, nStages), tri16Smem, s, nullptr, nullptr, nullptr,
                      X, rows, dOut, m->dErr);
-      } else {
-        int splits = std::max(1, std::min((rows + TS_KT * 8 - 1) / (TS_KT * 8), (4 * m->smCount + nPairs - 1) / nPairs));
-        int rowsPerSplit = ((rows + splits - 1) / splits + GT_KT - 1) / GT_KT * GT_KT;
-        splits = (rows + rowsPerSplit - 1) / rowsPerSplit;
-        dim3 grid(nPairs, splits);
-        k_gemm_tn_dmma<true><<<grid, TS_THREADS, 0, s>>>(X, n, X, n, rows, nBlk, dOut, rowsPerSplit);
-      }
-      m->stats.kernel_launches++;
+        m->stats.kernel_launches++;
+      } else if ((rc = launch_gemm_tn<true>(m, X, n, ld, X, n, ld, rows, dOut, s)) < 0)
+        return rc;
     }
   }
   k_mirror<<<std::max(1, std::min(1024, (int)(((int64_t)n * n + 255) / 256))), 256, 0, s>>>(dOut, n);
@@ -668,28 +779,20 @@ int64_t launch_tmm(Matrix* L, Matrix* R, double* dOut, cudaStream_t s) {
   CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)a * b, s));
   if (L->nRows == 0) return CLA_OK;
   int64_t rc;
-  int64_t chunk = (48ll << 20) / ((int64_t)(a + b) * 8);
-  chunk = std::max<int64_t>(SKIP_ROWS, (chunk / SKIP_ROWS) * SKIP_ROWS);
-  chunk = std::min<int64_t>(chunk, ((int64_t)L->nRows + SKIP_ROWS - 1) / SKIP_ROWS * SKIP_ROWS);
-  if ((rc = ensure_scratch2(L, (size_t)chunk * a * sizeof(double))) < 0) return rc;
-  if ((rc = ensure_scratch2(R, (size_t)chunk * b * sizeof(double))) < 0) return rc;
+  const int64_t chunk = chunk_rows(L->nRows, a + b);
+  const int la = (a + 1) & ~1, lb = (b + 1) & ~1;
+  if ((rc = ensure_scratch2(L, (size_t)chunk * la * sizeof(double))) < 0) return rc;
+  if ((rc = ensure_scratch2(R, (size_t)chunk * lb * sizeof(double))) < 0) return rc;
   double* XL = (double*)L->scratch2;
   double* XR = (double*)R->scratch2;
-  const int nBlkA = (a + TS_BLK - 1) / TS_BLK, nBlkB = (b + TS_BLK - 1) / TS_BLK;
-  const int nBlocks = nBlkA * nBlkB;
   for (int64_t r0 = 0; r0 < L->nRows; r0 += chunk) {
     const int r1 = (int)std::min<int64_t>(L->nRows, r0 + chunk);
-    if ((rc = launch_decompress_range(L, (int)r0, r1, XL, s)) < 0) return rc;
-    if ((rc = launch_decompress_range(R, (int)r0, r1, XR, s)) < 0) return rc;
+    if ((rc = decompress_chunk(L, (int)r0, r1, XL, la, s)) < 0) return rc;
+    if ((rc = decompress_chunk(R, (int)r0, r1, XR, lb, s)) < 0) return rc;
     const int rows = r1 - (int)r0;
-    int splits = std::max(1, std::min((rows + TS_KT * 8 - 1) / (TS_KT * 8), (4 * L->smCount + nBlocks - 1) / nBlocks));
-    int rowsPerSplit = ((rows + splits - 1) / splits + GT_KT - 1) / GT_KT * GT_KT;
-    splits = (rows + rowsPerSplit - 1) / rowsPerSplit;
-    dim3 grid(nBlocks, splits);
     if (r0 == 0) prof_begin(L, s);
-    k_gemm_tn_dmma<false><<<grid, TS_THREADS, 0, s>>>(XL, a, XR, b, rows, nBlkB, dOut, rowsPerSplit);
+    if ((rc = launch_gemm_tn<false>(L, XL, a, la, XR, b, lb, rows, dOut, s)) < 0) return rc;
     if (r0 == 0) prof_end(L, s);
-    L->stats.kernel_launches++;
   }
   CLA_CUDA(cudaGetLastError());
   return CLA_OK;
