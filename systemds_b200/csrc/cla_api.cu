@@ -452,8 +452,8 @@ static int64_t lmm_dev(Matrix* m, const double* dYt, int32_t yRows, double* dOut
     if (hc) hc->used = rc == 1;
     if (rc != 0) return rc < 0 ? rc : CLA_OK;
   }
-  // Passes of the column-per-lane kernels over four, two or one left rows at a time for the groups they cover; the
-  // other groups eight at a time. The former read the left rows with 128-bit loads: rows that are not 16-byte aligned
+  // Passes of the column-per-lane kernels over up to eight left rows at a time for the groups they cover; the other
+  // groups likewise. The former read the left rows with 128-bit loads: rows that are not 16-byte aligned
   // are copied to an even pitch first.
   if (yRows >= 1 && fast_plan_ok(m) && m->nRows > 0) {
     const double* rows = dYt;
@@ -468,7 +468,7 @@ static int64_t lmm_dev(Matrix* m, const double* dYt, int32_t yRows, double* dOut
     }
     int64_t rc = 0;
     for (int i = 0; i < yRows;) {
-      const int q = yRows - i >= 4 ? 4 : (yRows - i >= 2 ? 2 : 1);
+      const int q = std::min(8, yRows - i);
       rc = q == 1 ? fast_lmm_vec(m, rows + pitch * i, dOut + (size_t)i * m->nCols, s)
                   : fast_lmm_rows(m, rows + pitch * i, pitch, q, dOut + (size_t)i * m->nCols, s);
       if (rc <= 0) break;

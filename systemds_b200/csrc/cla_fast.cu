@@ -369,137 +369,189 @@ __global__ void __launch_bounds__(LMM_T, 1) k_lmm_vec(const __grid_constant__ Lm
 }
 
 // --------------------------------------------------------------------------------------------------
-// LMM with Q left rows at once (Q = 2 or 4; the reference's left-multiply blocks four rows too,
-// lib/CLALibLeftMultBy.java:731-819). Same layout and lookups as k_lmm_vec_u8, but a dictionary value fetched for a
-// cell multiplies the cell's Q left values: one pass over the maps and one lookup per cell serve Q rows, where Q
-// passes of the one-row kernel would fetch each value Q times. partial: [gridDim.x][Q][LMM_PART].
+// LMM with two to eight left rows at once, on the FP64 tensor core: m8n8k4 with A = left rows x matrix rows, B = matrix
+// rows x eight column slots. Lane (g, t) looks up slot g's values of rows 4 t .. 4 t + 3 of a 16-row block (one word of
+// ids), the four products of the block taking one of them each, so a lookup serves all left rows and nothing is staged.
+// Four lanes share a slot, so its table is kept four times: entry k of slot s for lane t at (k * 16 + (s & 3) * 4 + t) * 8,
+// which gives each of the 16 lanes of a half-warp a bank pair of its own.
+// Bound: the FP64 rate, 16 clocks of the tensor pipe per 16 rows and eight slots (half of it with four left rows or fewer
+// wasted), against 8 for the lookups, 1 for the ids and 8 for the left values of all the CTA's slots. (FMA on scalar
+// accumulators, four left rows per lookup, took 47 us per pass of four rows over 500k x 100 columns of four tuples.)
 // --------------------------------------------------------------------------------------------------
-constexpr int LQ_W = 12;              // warps per CTA (Q x NU accumulators per lane: up to 170 registers)
-constexpr int LQ_T = LQ_W * 32;
+__device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+constexpr int LR_W = 16;
+constexpr int LR_T = LR_W * 32;
+constexpr int LR_MAXT = 8;                    // tiles of eight slots per CTA
+constexpr int LR_PART = LR_MAXT * 64 + 8;     // partial sums of a CTA: [slot][left row], then the sums of the left rows
+constexpr int LR_SMEM = 220 * 1024;
+struct LmmRowsArgs {
+  const int2* units;           // {table offset / 16, depth} of a unit = two tiles
+  const uint8_t* imaps;
+  int64_t nRB;
+  const double* tables;
+  const int* slotCol;
+  const double* y;
+  size_t pitch;
+  int q, nRows, nTiles, U, nChunks, ctaFull, ctaLast;  // chunks of U tiles; CTAs of a chunk, of the last one
+  double* partial;             // [gridDim.x][LR_PART]
+  const double* constV;        // null: none
+  const int* bareCols;
+  int nBare, nCols, addTo;
+  double* out;
+};
 
-template <int NU, int Q>
-__device__ __forceinline__ void lmmq_body(const LmmChunk& ch, const uint8_t* __restrict__ imaps, int64_t nRB,
-                                          const double* __restrict__ tablesImg, const double* __restrict__ y, size_t pitch,
-                                          int nRows, double* __restrict__ partial, unsigned char* smraw, uint64_t* mbar,
-                                          int32_t* err) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int slot = lane & 15, half = lane >> 4;
-  if (!tma_load_to_smem(smraw, tablesImg + ch.tblOff, (uint32_t)ch.tblDoubles * 8u, mbar)) {
-    if (tid == 0) atomicExch(err, 105);
-    for (int u = tid; u < Q * LMM_PART; u += LQ_T) partial[(size_t)blockIdx.x * Q * LMM_PART + u] = __longlong_as_double(0x7ff8000000000000ll);
-    return;
-  }
-  const unsigned char* tbase[NU];
-  const uint8_t* mp[NU];
+template <int NT>
+__device__ __forceinline__ void lmm_rows_body(const LmmRowsArgs& A, int chunk, int cta0, int nCta, double* sm) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int tile0 = chunk * A.U;
+  uint32_t tb[NT];
   {
-    size_t off = 0;
+    uint32_t at = 0;  // entries of 128 bytes
 #pragma unroll
-    for (int u = 0; u < NU; u++) {
-      tbase[u] = smraw + off + slot * 8;
-      off += (size_t)ch.nk[u] * 128;
-      mp[u] = imaps + (size_t)(ch.unit0 + u) * nRB * 256 + slot * 16;
+    for (int u = 0; u < NT; u++) {
+      const int2 un = A.units[(tile0 + u) >> 1];
+      const double* src = A.tables + (size_t)un.x * 16 + ((tile0 + u) & 1) * 8;
+      double* dst = sm + (size_t)at * 16;
+      for (int e = tid; e < un.y * 32; e += LR_T) {  // entry, quad, slot of the quad, copy
+        const int k = e >> 5, quad = (e >> 4) & 1, s = (e >> 2) & 3;
+        dst[((size_t)quad * un.y + k) * 16 + (e & 15)] = src[(size_t)k * 16 + quad * 4 + s];
+      }
+      tb[u] = smem_u32(sm) + (at + (uint32_t)((g >> 2) * un.y)) * 128u + (uint32_t)((g & 3) * 4 + t) * 8u;
+      at += 2u * un.y;
     }
   }
-  double acc[NU][Q];
+  __syncthreads();
+  double c[NT][2], ys = 0.0;
 #pragma unroll
-  for (int u = 0; u < NU; u++)
+  for (int u = 0; u < NT; u++) c[u][0] = c[u][1] = 0.0;
+  const bool live = g < A.q;
+  const double* yr = A.y + (size_t)(live ? g : 0) * A.pitch + 4 * t;
+  const size_t ustr = (size_t)A.nRB * 256;
+  // tile tl: slots (tl & 1) * 8 .. + 8 of unit tl >> 1
+  auto ids_at = [&](int u, int64_t blk) {
+    const int tl = tile0 + u;
+    return __ldg((const uint32_t*)(A.imaps + (size_t)(tl >> 1) * ustr + blk * 256 + ((tl & 1) * 8 + g) * 16 + 4 * t));
+  };
+  const int64_t nBlk = ((int64_t)A.nRows + 15) / 16, whole = A.nRows / 16;
+  const int ci = blockIdx.x - cta0;
+  const int64_t b0 = nBlk * ci / nCta, b1 = nBlk * (ci + 1) / nCta;
+  // NB blocks per turn, their loads issued together: with few tiles a block is little work, and the left values come from
+  // L2 (500k x 200, 256 values, eight left rows, three tiles: 301 us with one block per turn, its loads one turn ahead)
+  constexpr int NB = NT <= 3 ? 4 : (NT <= 5 ? 2 : 1);
+  for (int64_t blk = b0 + warp * NB; blk < b1; blk += LR_W * NB) {
+    uint32_t id[NB][NT];
+    double yv[NB][4];
 #pragma unroll
-    for (int q = 0; q < Q; q++) acc[u][q] = 0.0;
-  const int ctaInChunk = blockIdx.x - ch.cta0;
-  const int64_t nSteps = ((int64_t)nRows + LMM_STEP - 1) / LMM_STEP;
-  const int64_t s0 = nSteps * ctaInChunk / ch.nCta, s1 = nSteps * (ctaInChunk + 1) / ch.nCta;
-  for (int64_t st = s0 + warp; st < s1; st += LQ_W) {
-    const int64_t r0 = st * LMM_STEP + half * 32;
-    if (st * LMM_STEP + LMM_STEP <= nRows) {
-#pragma unroll 1
-      for (int sub = 0; sub < 2; sub++) {
-        uint4 m[NU];
+    for (int n = 0; n < NB; n++) {
+      const int64_t k = blk + n;
+      const bool in = k < b1;
 #pragma unroll
-        for (int u = 0; u < NU; u++) m[u] = __ldg((const uint4*)(mp[u] + ((r0 >> 4) + sub) * 256));
-        const double* yr = y + r0 + sub * 16;
+      for (int u = 0; u < NT; u++) id[n][u] = in ? ids_at(u, k) : 0u;
 #pragma unroll
-        for (int i = 0; i < 16; i += 2) {  // two rows per 128-bit load of every left row
-          double2 yq[Q];
-#pragma unroll
-          for (int q = 0; q < Q; q++) yq[q] = __ldg((const double2*)(yr + q * pitch + i));
-#pragma unroll
-          for (int u = 0; u < NU; u++) {
-            const uint32_t w = (i >> 2) == 0 ? m[u].x : ((i >> 2) == 1 ? m[u].y : ((i >> 2) == 2 ? m[u].z : m[u].w));
-            const double t0 = *(const double*)(tbase[u] + byte_x128(w, i & 3));
-            const double t1 = *(const double*)(tbase[u] + byte_x128(w, (i & 3) + 1));
-#pragma unroll
-            for (int q = 0; q < Q; q++) acc[u][q] = fma(yq[q].y, t1, fma(yq[q].x, t0, acc[u][q]));
-          }
-        }
+      for (int i = 0; i < 4; i++) yv[n][i] = 0.0;
+      if (in && k < whole) {
+        const double2 ya = __ldg((const double2*)(yr + k * 16)), yb = __ldg((const double2*)(yr + k * 16) + 1);
+        yv[n][0] = ya.x, yv[n][1] = ya.y, yv[n][2] = yb.x, yv[n][3] = yb.y;
       }
-    } else {  // ragged last step
-      for (int64_t r = r0; r < min((int64_t)nRows, r0 + 32); r++) {
+    }
 #pragma unroll
-        for (int u = 0; u < NU; u++) {
-          const double t = *(const double*)(tbase[u] + 128 * (int)mp[u][(r >> 4) * 256 + (r & 15)]);
+    for (int n = 0; n < NB; n++) {
+      if (blk + n >= b1) break;
+      if (blk + n < whole) {
 #pragma unroll
-          for (int q = 0; q < Q; q++) acc[u][q] = fma(y[q * pitch + r], t, acc[u][q]);
+        for (int u = 0; u < NT; u++) {
+          double x[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) x[i] = lds_f64(entry_at(id[n][u], i, tb[u]));
+#pragma unroll
+          for (int i = 0; i < 4; i++) dmma884(c[u][0], c[u][1], yv[n][i], x[i]);
         }
+      } else {  // the last rows: nothing of the padding enters the products
+        const int64_t r0 = (blk + n) * 16 + 4 * t;
+#pragma unroll
+        for (int i = 0; i < 4; i++) yv[n][i] = r0 + i < A.nRows ? yr[(blk + n) * 16 + i] : 0.0;
+#pragma unroll
+        for (int u = 0; u < NT; u++)
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+            dmma884(c[u][0], c[u][1], yv[n][i], r0 + i < A.nRows ? lds_f64(entry_at(id[n][u], i, tb[u])) : 0.0);
       }
+      if (A.constV) ys += (yv[n][0] + yv[n][1]) + (yv[n][2] + yv[n][3]);
     }
   }
   __syncthreads();  // tables no longer needed
-  double* red = (double*)smraw;  // [LQ_W][Q][NU*16]
+  // c: left row g, slots 2 t, 2 t + 1; the warps through shared memory
+  double* red = sm;  // [LR_W][NT * 64 + 8]
+  constexpr int N = NT * 64 + 8;
 #pragma unroll
-  for (int u = 0; u < NU; u++)
+  for (int u = 0; u < NT; u++)
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
-      double a = acc[u][q];
-      a += __shfl_xor_sync(0xffffffffu, a, 16);
-      if (half == 0) red[(warp * Q + q) * (NU * 16) + u * 16 + slot] = a;
+    for (int e = 0; e < 2; e++) red[warp * N + (u * 8 + 2 * t + e) * 8 + g] = c[u][e];
+  ys += __shfl_xor_sync(0xffffffffu, ys, 1);
+  ys += __shfl_xor_sync(0xffffffffu, ys, 2);
+  if (t == 0) red[warp * N + NT * 64 + g] = ys;
+  __syncthreads();
+  double* mine = A.partial + (size_t)blockIdx.x * LR_PART;
+  for (int e = tid; e < N; e += LR_T) {
+    double s = 0.0;
+    for (int k = 0; k < LR_W; k++) s += red[k * N + e];
+    mine[e < NT * 64 ? e : LR_MAXT * 64 + e - NT * 64] = s;
+  }
+}
+
+__global__ void __launch_bounds__(LR_T, 1) k_lmm_rows(const __grid_constant__ LmmRowsArgs A) {
+  extern __shared__ __align__(128) double lrsm[];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int chunk = min((int)blockIdx.x / A.ctaFull, A.nChunks - 1), cta0 = chunk * A.ctaFull;
+  const int nCta = chunk == A.nChunks - 1 ? A.ctaLast : A.ctaFull;
+#define LR_CASE(N) case N: lmm_rows_body<N>(A, chunk, cta0, nCta, lrsm); break;
+  switch (min(A.U, A.nTiles - chunk * A.U)) {
+    LR_CASE(1) LR_CASE(2) LR_CASE(3) LR_CASE(4) LR_CASE(5) LR_CASE(6) LR_CASE(7)
+    default: lmm_rows_body<LR_MAXT>(A, chunk, cta0, nCta, lrsm); break;
+  }
+#undef LR_CASE
+}
+
+// Adds up the partial sums of one tile (64 cells by 8 threads each, a fixed order) and stores the results. grid: tiles
+__global__ void __launch_bounds__(512) k_lmm_rows_final(const __grid_constant__ LmmRowsArgs A) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  __shared__ double red[8][64], yred[8][8];
+  const int chunk = blockIdx.x / A.U, u = blockIdx.x - chunk * A.U, cta0 = chunk * A.ctaFull;
+  const int nCta = chunk == A.nChunks - 1 ? A.ctaLast : A.ctaFull;
+  const int cell = threadIdx.x & 63, sub = threadIdx.x >> 6;
+  double s = 0.0, ys = 0.0;
+#pragma unroll 4
+  for (int i = sub; i < nCta; i += 8) {
+    const double* p = A.partial + (size_t)(cta0 + i) * LR_PART;
+    s += __ldcg(p + u * 64 + cell);
+    if (A.constV && cell < 8) ys += __ldcg(p + LR_MAXT * 64 + cell);
+  }
+  red[sub][cell] = s;
+  if (cell < 8) yred[sub][cell] = ys;
+  __syncthreads();
+  auto row_sum = [&](int g) {
+    double x = 0.0;
+    for (int k = 0; k < 8; k++) x += yred[k][g];
+    return x;
+  };
+  if (sub == 0) {
+    for (int k = 1; k < 8; k++) s += red[k][cell];
+    const int g = cell & 7, col = A.slotCol[blockIdx.x * 8 + (cell >> 3)];
+    if (g < A.q && col >= 0) {
+      double* o = A.out + (size_t)g * A.nCols + col;
+      if (A.addTo) atomicAdd(o, s);
+      else *o = A.constV ? fma(row_sum(g), A.constV[col], s) : s;
     }
-  __syncthreads();
-  for (int e = tid; e < Q * NU * 16; e += LQ_T) {
-    const int q = e / (NU * 16), u = e - q * (NU * 16);
-    double s = 0;
-    for (int w = 0; w < LQ_W; w++) s += red[(w * Q + q) * (NU * 16) + u];
-    partial[((size_t)blockIdx.x * Q + q) * LMM_PART + u] = s;
   }
-}
-
-template <int Q>
-__global__ void __launch_bounds__(LQ_T, 1)
-k_lmm_vecq_u8(const LmmChunk* __restrict__ chunks, int nChunks, const uint8_t* __restrict__ imaps, int64_t nRB,
-              const double* __restrict__ tablesImg, const double* __restrict__ y, size_t pitch, int nRows,
-              double* __restrict__ partial, int32_t* err) {
-  extern __shared__ __align__(128) unsigned char smraw[];
-  __shared__ __align__(8) uint64_t mbar;
-  __shared__ LmmChunk ch;
-  if (threadIdx.x == 0) {
-    int c = 0;
-    while (c + 1 < nChunks && (int)blockIdx.x >= chunks[c].cta0 + chunks[c].nCta) c++;
-    ch = chunks[c];
-  }
-  __syncthreads();
-#define LQ_CASE(N) case N: lmmq_body<N, Q>(ch, imaps, nRB, tablesImg, y, pitch, nRows, partial, smraw, &mbar, err); break;
-  switch (ch.nUnits) {
-    LQ_CASE(1) LQ_CASE(2) LQ_CASE(3) LQ_CASE(4) LQ_CASE(5) LQ_CASE(6)
-    default: lmmq_body<7, Q>(ch, imaps, nRB, tablesImg, y, pitch, nRows, partial, smraw, &mbar, err); break;
-  }
-#undef LQ_CASE
-}
-
-// out[q][col] += sum over the chunk's CTAs of partial[cta][q][slot]; blockIdx.z = q
-__global__ void k_lmm_vecq_final(const LmmChunk* __restrict__ chunks, int nChunks, const int* __restrict__ slotCol,
-                                 const double* __restrict__ partial, double* __restrict__ out, int Q, int nCols) {
-  const int c = blockIdx.x, q = blockIdx.z;
-  if (c >= nChunks) return;
-  const LmmChunk ch = chunks[c];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nWarps = (blockDim.x >> 5) * gridDim.y;
-  for (int u = blockIdx.y * (blockDim.x >> 5) + warp; u < ch.nUnits * 16; u += nWarps) {
-    const int col = slotCol[ch.unit0 * 16 + u];
-    if (col < 0) continue;
-    double s = 0;
-    for (int i = lane; i < ch.nCta; i += 32) s += partial[((size_t)(ch.cta0 + i) * Q + q) * LMM_PART + u];
-#pragma unroll
-    for (int d = 16; d; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    if (lane == 0) atomicAdd(&out[(size_t)q * nCols + col], s);
-  }
+  if (blockIdx.x == 0 && !A.addTo)  // columns of constant groups, and those the general kernels will add to
+    for (int e = threadIdx.x; e < A.nBare * A.q; e += 512) {
+      const int g = e / A.nBare, col = A.bareCols[e - g * A.nBare];
+      A.out[(size_t)g * A.nCols + col] = A.constV ? row_sum(g) * A.constV[col] : 0.0;
+    }
 }
 
 // --------------------------------------------------------------------------------------------------
@@ -631,12 +683,6 @@ k_decomp_fast(const LmmChunk* __restrict__ chunks, int nChunks, const uint8_t* _
 // third of its instructions.) A product with 0 would carry an Inf or NaN of one row into its neighbours, so a warp that
 // sees a non-finite result forms its sums again with shuffles.
 // --------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
-
 // 1.0 where a == b, else 0.0; volatile: formed where it is used (kept in registers across the main loop, the nine
 // coefficients below pushed the kernel into spilling).
 __device__ __forceinline__ double one_if(int a, int b) {
@@ -1522,40 +1568,91 @@ int64_t fast_lmm_vec(Matrix* m, const double* dY, double* dOut, cudaStream_t s) 
   return fp->partial ? 2 : 1;
 }
 
-// Q = 2 or 4 left rows (rows q of y at y + q * pitch, 16-byte aligned) in one pass; same return values as fast_lmm_vec.
-template <int Q>
-static int64_t fast_lmm_rows_t(Matrix* m, FastPlan* fp, const double* dY, size_t pitch, double* dOut, cudaStream_t s) {
-  int64_t rc;
-  const size_t partBytes = (size_t)fp->lmmGrid * Q * LMM_PART * 8;
-  if ((rc = ensure_scratch(m, partBytes + 256)) < 0) return rc;
-  double* partial = (double*)m->scratch;
-  CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)Q * m->nCols, s));
-  size_t smem = (size_t)LQ_W * Q * LMM_PART * 8;
-  for (auto& c : fp->lchunks) smem = std::max(smem, (size_t)c.tblDoubles * 8);
-  static bool attr[64] = {};  // per device
-  if (!attr[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_lmm_vecq_u8<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
-    attr[m->device & 63] = true;
-  }
-  prof_begin(m, s);
-  k_lmm_vecq_u8<Q><<<fp->lmmGrid, LQ_T, smem, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dLmmMaps, fp->nRB, fp->dLmmTables, dY,
-                                                  pitch, m->nRows, partial, m->dErr);
-  prof_end(m, s);
-  k_lmm_vecq_final<<<dim3((unsigned)fp->lchunks.size(), LMM_MAX_UNITS, Q), 512, 0, s>>>(fp->dLChunks, (int)fp->lchunks.size(),
-                                                                                       fp->dSlotCol, partial, dOut, Q, m->nCols);
-  m->stats.kernel_launches += 2;
-  if (m->hasConst)
-    for (int q = 0; q < Q; q++)
-      if ((rc = launch_lmm_const(m, dY + q * pitch, 1, dOut + (size_t)q * m->nCols, s)) < 0) return rc;
-  CLA_CUDA(cudaGetLastError());
-  return fp->partial ? 2 : 1;
-}
+// q = 2 .. 8 left rows (row i at y + i * pitch, 16-byte aligned) in one pass; same return values as fast_lmm_vec.
 int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* dOut, cudaStream_t s) {
   FastPlan* fp = m->fast;
   if (!fp || !fp->ok || ((uintptr_t)dY & 15) || (pitch & 1)) return 0;
-  if (q == 4) return fast_lmm_rows_t<4>(m, fp, dY, pitch, dOut, s);
-  if (q == 2) return fast_lmm_rows_t<2>(m, fp, dY, pitch, dOut, s);
-  return fail(CLA_ERR_BAD_ARG, "fast_lmm_rows: 2 or 4 rows");
+  if (q < 1 || q > 8) return fail(CLA_ERR_BAD_ARG, "fast_lmm_rows: up to 8 rows");
+  LmmRowsArgs A{};
+  A.units = fp->dUnits;
+  A.imaps = fp->dLmmMaps;
+  A.nRB = fp->nRB;
+  A.tables = fp->dLmmTables;
+  A.slotCol = fp->dSlotCol;
+  A.y = dY;
+  A.pitch = pitch;
+  A.q = q;
+  A.nRows = m->nRows;
+  A.nTiles = (fp->nUnits + 7) / 8;
+  A.constV = (m->hasConst && fp->uniqueCols) ? m->dConstV : nullptr;
+  A.bareCols = fp->dBareCols;
+  A.nBare = fp->nBare;
+  A.nCols = m->nCols;
+  A.addTo = fp->uniqueCols ? 0 : 1;
+  A.out = dOut;
+  auto bytes_of = [&](int t0, int n) {
+    size_t b = 0;
+    for (int i = t0; i < std::min(A.nTiles, t0 + n); i++) b += (size_t)fp->unitNk[i >> 1] * 256;
+    return b;
+  };
+  // Tiles per chunk: what fits, and by the same balance as lmm_chunk_units -- clocks per 16 rows 16 a tile and 10 for the
+  // left values, 2 per tuple of a staged tile, at least one round of blocks.
+  size_t smem = 0;
+  double bestCost = 1e300;
+  const int64_t nBlk = ((int64_t)m->nRows + 15) / 16;
+  for (int U = 1; U <= LR_MAXT; U++) {
+    size_t most = (size_t)LR_W * (std::min(U, A.nTiles) * 64 + 8) * 8, stage = 0;
+    for (int t0 = 0; t0 < A.nTiles; t0 += U) {
+      const size_t b = bytes_of(t0, U);
+      stage = std::max(stage, b);
+      most = std::max(most, b);
+    }
+    if (most > (size_t)LR_SMEM) break;
+    const int nChunks = (A.nTiles + U - 1) / U;
+    const double ctas = std::max(1.0, (double)m->smCount / nChunks), blocks = nBlk / ctas, waves = std::ceil((double)nChunks / m->smCount);
+    const double cost = waves * (stage / 128.0 + std::max(blocks * (16.0 * U + 10.0), std::ceil(blocks / LR_W) * (700.0 + 60.0 * U)));
+    if (cost < bestCost) {
+      bestCost = cost;
+      A.U = U;
+      smem = most;
+    }
+  }
+  if (A.U == 0) return fail(CLA_ERR_STATE, "left product: a table does not fit shared memory");
+  A.nChunks = (A.nTiles + A.U - 1) / A.U;
+  const int blocks = (int)std::min<int64_t>((nBlk + 3) / 4, 1 << 20);
+  const double full = 16.0 * A.U + 10.0, last = 16.0 * (A.nTiles - (A.nChunks - 1) * A.U) + 10.0, all = (A.nChunks - 1) * full + last;
+  A.ctaFull = std::max(1, std::min(blocks, (int)(m->smCount * full / all + 0.5)));
+  if (A.nChunks > 1 && A.ctaFull * (A.nChunks - 1) >= m->smCount) A.ctaFull = std::max(1, (m->smCount - 1) / (A.nChunks - 1));
+  A.ctaLast = std::max(1, std::min(blocks, m->smCount - A.ctaFull * (A.nChunks - 1)));
+  const int grid = A.ctaFull * (A.nChunks - 1) + A.ctaLast;
+  int64_t rc;
+  if ((rc = ensure_scratch(m, (size_t)grid * LR_PART * 8 + 256)) < 0) return rc;
+  A.partial = (double*)m->scratch;
+  if (A.addTo) CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)q * m->nCols, s));
+  static bool attr[64] = {};  // per device
+  if (!attr[m->device & 63]) {
+    CLA_CUDA(cudaFuncSetAttribute(k_lmm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, LR_SMEM));
+    attr[m->device & 63] = true;
+  }
+  prof_begin(m, s);
+  k_lmm_rows<<<grid, LR_T, smem, s>>>(A);
+  prof_end(m, s);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)A.nTiles);
+  cfg.blockDim = dim3(512);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  CLA_CUDA(cudaLaunchKernelEx(&cfg, k_lmm_rows_final, A));
+  m->stats.kernel_launches += 2;
+  if (m->hasConst && !A.constV)
+    for (int i = 0; i < q; i++)
+      if ((rc = launch_lmm_const(m, dY + i * pitch, 1, dOut + (size_t)i * m->nCols, s)) < 0) return rc;
+  CLA_CUDA(cudaGetLastError());
+  return fp->partial ? 2 : 1;
 }
 
 // Host-buffer t(y) %*% X with the upload of y overlapped with the product: y is copied in up to LMM_PIPE_MAX row ranges

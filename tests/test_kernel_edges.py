@@ -71,7 +71,7 @@ def test_byte_map_units(nRows, nCols, card):
     """Column-per-lane kernels: last unit partly filled, one unit more than the fused chain takes, several chunks, joint
     slots (tall blocks of small dictionaries), bit maps; a constant column."""
     cmb = _ddc(nRows, [card] * nCols, nRows + nCols + card, const=nCols % 2 == 1).to_device()
-    _check(cmb)
+    _check(cmb, qs=(1, 2, 5, 8, 9))
     cmb.free()
 
 
@@ -133,4 +133,22 @@ def test_decompress_columns(nRows, nCols):
     kinds = kinds * (nCols // 11) + ("ddc",) * (nCols % 11)
     cmb = datagen.random_cmb(nRows + nCols, nRows, kinds).to_device()
     assert np.array_equal(np.array(CLALibDecompress.decompress(cmb)), dense_of(cmb))
+    cmb.free()
+
+
+@pytest.mark.parametrize("nRows", [4096, 4127, 4161])
+@pytest.mark.parametrize("kinds", ["bytes", "chars", "mixed", "sparse"])
+def test_wide_right_operand(nRows, kinds):
+    """X %*% V around the tile widths (8, 16, 24, 32 columns, two slices) and row remainders: several chunks of columns,
+    padding columns of every kind, dictionaries too large to stay resident, odd column counts, no dense column at all."""
+    if kinds == "bytes":
+        cmb = _ddc(nRows, [256] * 130 + [2, 2, 3], 3, const=True)
+    elif kinds == "chars":
+        cmb = _ddc(nRows, [300, 1000, 4096, 5000] * 3 + [9], 4)
+    elif kinds == "mixed":
+        cmb = datagen.random_cmb(nRows, nRows, datagen.KINDS + ("unc", "ddc2", "ddc_char", "rle", "sdcz"))
+    else:
+        cmb = datagen.random_cmb(nRows, nRows, ("sdc", "sdcz", "rle", "sdcs", "const", "rle"))
+    cmb.to_device()
+    _check(cmb, ks=(2, 3, 7, 8, 9, 16, 17, 24, 25, 32, 33, 64, 65), qs=(2, 3, 8, 9), chain=False)
     cmb.free()
