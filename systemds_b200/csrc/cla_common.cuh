@@ -318,6 +318,9 @@ void prof_collect(Matrix* m);
 
 int64_t order_begin(Matrix* m, cudaStream_t s);  // see Matrix::lastDone
 int64_t order_end(Matrix* m, cudaStream_t s);
+// device memory of a handle, from the device's pool (cla_finalize.cu); free only what no stream uses any more
+cudaError_t dev_malloc(const Matrix* m, void** p, size_t bytes);
+void dev_free(const Matrix* m, void* p);
 int64_t ensure_scratch(Matrix* m, size_t bytes);
 int64_t ensure_scratch2(Matrix* m, size_t bytes);
 int64_t ensure_io(Matrix* m, size_t bytes);

@@ -396,7 +396,16 @@ struct LmmRowsArgs {
   const int* slotCol;
   const double* y;
   size_t pitch;
-  int q, nRows, nTiles, U, nChunks, ctaFull, ctaLast;  // chunks of U tiles; CTAs of a chunk, of the last one
+  int q, nRows, nTiles, nChunks, grid;
+  // chunk c: tiles [tile0(c), tile0(c + 1)), even to one tile, and CTAs in proportion
+  __host__ __device__ int tile0(int c) const { return (int)((int64_t)nTiles * c / nChunks); }
+  __host__ __device__ int cta0(int c) const { return (int)((int64_t)grid * tile0(c) / nTiles); }
+  __host__ __device__ int chunk_of(int cta) const {
+    int c = (int)((int64_t)cta * nChunks / grid);
+    while (c > 0 && cta0(c) > cta) c--;
+    while (c + 1 < nChunks && cta0(c + 1) <= cta) c++;
+    return c;
+  }
   double* partial;             // [gridDim.x][LR_PART]
   const double* constV;        // null: none
   const int* bareCols;
@@ -407,7 +416,7 @@ struct LmmRowsArgs {
 template <int NT>
 __device__ __forceinline__ void lmm_rows_body(const LmmRowsArgs& A, int chunk, int cta0, int nCta, double* sm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int tile0 = chunk * A.U;
+  const int tile0 = A.tile0(chunk);
   uint32_t tb[NT];
   {
     uint32_t at = 0;  // entries of 128 bytes
@@ -506,10 +515,9 @@ __device__ __forceinline__ void lmm_rows_body(const LmmRowsArgs& A, int chunk, i
 __global__ void __launch_bounds__(LR_T, 1) k_lmm_rows(const __grid_constant__ LmmRowsArgs A) {
   extern __shared__ __align__(128) double lrsm[];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int chunk = min((int)blockIdx.x / A.ctaFull, A.nChunks - 1), cta0 = chunk * A.ctaFull;
-  const int nCta = chunk == A.nChunks - 1 ? A.ctaLast : A.ctaFull;
+  const int chunk = A.chunk_of(blockIdx.x), cta0 = A.cta0(chunk), nCta = A.cta0(chunk + 1) - cta0;
 #define LR_CASE(N) case N: lmm_rows_body<N>(A, chunk, cta0, nCta, lrsm); break;
-  switch (min(A.U, A.nTiles - chunk * A.U)) {
+  switch (A.tile0(chunk + 1) - A.tile0(chunk)) {
     LR_CASE(1) LR_CASE(2) LR_CASE(3) LR_CASE(4) LR_CASE(5) LR_CASE(6) LR_CASE(7)
     default: lmm_rows_body<LR_MAXT>(A, chunk, cta0, nCta, lrsm); break;
   }
@@ -520,8 +528,10 @@ __global__ void __launch_bounds__(LR_T, 1) k_lmm_rows(const __grid_constant__ Lm
 __global__ void __launch_bounds__(512) k_lmm_rows_final(const __grid_constant__ LmmRowsArgs A) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ double red[8][64], yred[8][8];
-  const int chunk = blockIdx.x / A.U, u = blockIdx.x - chunk * A.U, cta0 = chunk * A.ctaFull;
-  const int nCta = chunk == A.nChunks - 1 ? A.ctaLast : A.ctaFull;
+  int chunk = (int)((int64_t)blockIdx.x * A.nChunks / A.nTiles);  // this tile's chunk
+  while (chunk > 0 && A.tile0(chunk) > (int)blockIdx.x) chunk--;
+  while (chunk + 1 < A.nChunks && A.tile0(chunk + 1) <= (int)blockIdx.x) chunk++;
+  const int u = blockIdx.x - A.tile0(chunk), cta0 = A.cta0(chunk), nCta = A.cta0(chunk + 1) - cta0;
   const int cell = threadIdx.x & 63, sub = threadIdx.x >> 6;
   double s = 0.0, ys = 0.0;
 #pragma unroll 4
@@ -1145,14 +1155,14 @@ __global__ void k_joint_interleave(const JointSlot* __restrict__ slots, const ui
 // --------------------------------------------------------------------------------------------------
 void fast_plan_free(Matrix* m) {
   if (!m->fast) return;
-  for (void* p : m->fast->allocs) cudaFree(p);
+  for (void* p : m->fast->allocs) dev_free(m, p);
   delete m->fast;
   m->fast = nullptr;
 }
 
-static int64_t plan_malloc(FastPlan* fp, void** p, size_t bytes) {
+static int64_t plan_malloc(Matrix* m, FastPlan* fp, void** p, size_t bytes) {
   *p = nullptr;
-  cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+  cudaError_t e = dev_malloc(m, p, std::max<size_t>(bytes, 16));
   if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc plan: ") + cudaGetErrorString(e));
   fp->allocs.push_back(*p);
   return CLA_OK;
@@ -1331,7 +1341,7 @@ int64_t fast_plan_build(Matrix* m) {
   const size_t oJs = blob.add(js), oJg = blob.add(jg), oJRec = blob.add(jRec), oGMap = blob.add(groupMap);
   const size_t mapBytes = (size_t)fp->nSlots * fp->nRB * 16, jMapBytes = (size_t)fp->nJU16 * 16 * fp->nRB * 16;
   void *d = nullptr, *maps = nullptr;
-  if ((rc = plan_malloc(fp, &d, blob.host.size())) < 0 || (rc = plan_malloc(fp, &maps, mapBytes + jMapBytes)) < 0) return rc;
+  if ((rc = plan_malloc(m, fp, &d, blob.host.size())) < 0 || (rc = plan_malloc(m, fp, &maps, mapBytes + jMapBytes)) < 0) return rc;
   CLA_CUDA(cudaMemcpyAsync(d, blob.host.data(), blob.host.size(), cudaMemcpyHostToDevice, m->stream));
   char* base = (char*)d;
   fp->dLChunks = (LmmChunk*)(base + oChunks);
@@ -1601,30 +1611,24 @@ int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* 
   double bestCost = 1e300;
   const int64_t nBlk = ((int64_t)m->nRows + 15) / 16;
   for (int U = 1; U <= LR_MAXT; U++) {
+    LmmRowsArgs T = A;
+    T.nChunks = (A.nTiles + U - 1) / U;
     size_t most = (size_t)LR_W * (std::min(U, A.nTiles) * 64 + 8) * 8, stage = 0;
-    for (int t0 = 0; t0 < A.nTiles; t0 += U) {
-      const size_t b = bytes_of(t0, U);
-      stage = std::max(stage, b);
-      most = std::max(most, b);
-    }
-    if (most > (size_t)LR_SMEM) break;
-    const int nChunks = (A.nTiles + U - 1) / U;
-    const double ctas = std::max(1.0, (double)m->smCount / nChunks), blocks = nBlk / ctas, waves = std::ceil((double)nChunks / m->smCount);
+    for (int c = 0; c < T.nChunks; c++) stage = std::max(stage, bytes_of(T.tile0(c), T.tile0(c + 1) - T.tile0(c)));
+    most = std::max(most, stage);
+    if (most > (size_t)LR_SMEM) continue;
+    const double ctas = std::max(1.0, (double)m->smCount / T.nChunks), blocks = nBlk / ctas, waves = std::ceil((double)T.nChunks / m->smCount);
     const double cost = waves * (stage / 128.0 + std::max(blocks * (16.0 * U + 10.0), std::ceil(blocks / LR_W) * (700.0 + 60.0 * U)));
     if (cost < bestCost) {
       bestCost = cost;
-      A.U = U;
+      A.nChunks = T.nChunks;
       smem = most;
     }
   }
-  if (A.U == 0) return fail(CLA_ERR_STATE, "left product: a table does not fit shared memory");
-  A.nChunks = (A.nTiles + A.U - 1) / A.U;
-  const int blocks = (int)std::min<int64_t>((nBlk + 3) / 4, 1 << 20);
-  const double full = 16.0 * A.U + 10.0, last = 16.0 * (A.nTiles - (A.nChunks - 1) * A.U) + 10.0, all = (A.nChunks - 1) * full + last;
-  A.ctaFull = std::max(1, std::min(blocks, (int)(m->smCount * full / all + 0.5)));
-  if (A.nChunks > 1 && A.ctaFull * (A.nChunks - 1) >= m->smCount) A.ctaFull = std::max(1, (m->smCount - 1) / (A.nChunks - 1));
-  A.ctaLast = std::max(1, std::min(blocks, m->smCount - A.ctaFull * (A.nChunks - 1)));
-  const int grid = A.ctaFull * (A.nChunks - 1) + A.ctaLast;
+  if (A.nChunks == 0) return fail(CLA_ERR_STATE, "left product: a table does not fit shared memory");
+  // at least one CTA for every chunk, however the shares round; no more than four blocks of rows justify
+  const int64_t most = std::max<int64_t>((int64_t)2 * A.nChunks, ((nBlk + 3) / 4) * A.nChunks);
+  const int grid = A.grid = (int)std::min<int64_t>(most, 2 * A.nChunks > m->smCount ? 2 * A.nChunks : m->smCount);
   int64_t rc;
   if ((rc = ensure_scratch(m, (size_t)grid * LR_PART * 8 + 256)) < 0) return rc;
   A.partial = (double*)m->scratch;

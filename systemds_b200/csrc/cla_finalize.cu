@@ -29,13 +29,71 @@ std::shared_ptr<Matrix> lookup(cla_handle h) {
   return it == g_table.end() ? nullptr : it->second;
 }
 
-static int64_t grow(void** p, size_t* cur, size_t bytes) {
+// Device memory of all handles comes from one pool per device. A block of a blocked matrix lives for a few products, and
+// mapping and unmapping its memory (cudaMalloc, cudaFree: up to a millisecond each) took longer than those. The pool keeps
+// at most POOL_KEEP of what handles have returned, and nothing once the last handle on the device is gone. Allocations
+// are complete when dev_malloc returns, so they may be used on any stream; who frees has waited for the device first.
+constexpr uint64_t POOL_KEEP = 1ull << 30;
+static std::mutex g_poolMu;
+static cudaMemPool_t g_pool[64] = {};
+static bool g_poolTried[64] = {};
+static int64_t g_poolHandles[64] = {};
+static cudaMemPool_t pool_of(int device) {
+  if (device < 0 || device >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(g_poolMu);
+  if (!g_poolTried[device]) {
+    g_poolTried[device] = true;
+    int ok = 0;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = POOL_KEEP;
+    if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, device) != cudaSuccess || !ok ||
+        cudaMemPoolCreate(&g_pool[device], &props) != cudaSuccess) {
+      cudaGetLastError();
+      g_pool[device] = nullptr;
+    } else
+      cudaMemPoolSetAttribute(g_pool[device], cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  return g_pool[device];
+}
+cudaError_t dev_malloc(const Matrix* m, void** p, size_t bytes) {
+  *p = nullptr;
+  cudaMemPool_t pool = pool_of(m->device);
+  if (!pool) return cudaMalloc(p, bytes);
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, m->stream);
+  if (e == cudaErrorMemoryAllocation) {  // what the pool keeps may be in pieces
+    cudaGetLastError();
+    cudaMemPoolTrimTo(pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, m->stream);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+void dev_free(const Matrix* m, void* p) {
+  if (!p) return;
+  if (pool_of(m->device)) cudaFreeAsync(p, m->stream);
+  else cudaFree(p);
+}
+static void pool_handles(int device, int by) {
+  cudaMemPool_t pool = pool_of(device);
+  if (!pool) return;
+  std::lock_guard<std::mutex> lk(g_poolMu);
+  if ((g_poolHandles[device] += by) == 0) cudaMemPoolTrimTo(pool, 0);
+}
+
+static int64_t grow(Matrix* m, void** p, size_t* cur, size_t bytes) {
   if (bytes <= *cur) return CLA_OK;
-  if (*p) cudaFree(*p);
+  if (*p) {
+    CLA_CUDA(cudaDeviceSynchronize());
+    dev_free(m, *p);
+  }
   *p = nullptr;
   *cur = 0;
   size_t want = bytes + bytes / 4 + 256;
-  cudaError_t e = cudaMalloc(p, want);
+  cudaError_t e = dev_malloc(m, p, want);
   if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc scratch: ") + cudaGetErrorString(e));
   *cur = want;
   return CLA_OK;
@@ -55,10 +113,10 @@ int64_t order_end(Matrix* m, cudaStream_t s) {
   m->lastValid = true;
   return CLA_OK;
 }
-int64_t ensure_scratch(Matrix* m, size_t bytes) { return grow(&m->scratch, &m->scratchBytes, bytes); }
-int64_t ensure_scratch2(Matrix* m, size_t bytes) { return grow(&m->scratch2, &m->scratch2Bytes, bytes); }
-int64_t ensure_io(Matrix* m, size_t bytes) { return grow(&m->io, &m->ioBytes, bytes); }
-int64_t ensure_small(Matrix* m, size_t bytes) { return grow(&m->small_, &m->smallBytes, bytes); }
+int64_t ensure_scratch(Matrix* m, size_t bytes) { return grow(m, &m->scratch, &m->scratchBytes, bytes); }
+int64_t ensure_scratch2(Matrix* m, size_t bytes) { return grow(m, &m->scratch2, &m->scratch2Bytes, bytes); }
+int64_t ensure_io(Matrix* m, size_t bytes) { return grow(m, &m->io, &m->ioBytes, bytes); }
+int64_t ensure_small(Matrix* m, size_t bytes) { return grow(m, &m->small_, &m->smallBytes, bytes); }
 
 constexpr size_t PROF_MAX = 512;
 void prof_begin(Matrix* m, cudaStream_t s) {
@@ -352,7 +410,7 @@ static int64_t slab_open(Matrix* m, Slab& s, size_t cap) {
   s.cap = cap;
   if (cap == 0) return CLA_OK;
   void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, cap);
+  cudaError_t e = dev_malloc(m, &p, cap);
   if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   m->allocs.push_back(p);
   s.base = (char*)p;
@@ -376,7 +434,7 @@ static int64_t carve(Matrix* m, size_t bytes, void** dst, Slab** from) {
       return CLA_OK;
     }
   }
-  cudaError_t e = cudaMalloc(dst, bytes);
+  cudaError_t e = dev_malloc(m, dst, bytes);
   if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   m->allocs.push_back(*dst);
   return CLA_OK;
@@ -413,7 +471,7 @@ static int64_t dev_alloc(Matrix* m, size_t n, T** dst) {
     p = g_up->big.base + g_up->big.at;
     g_up->big.at += b;
   } else {
-    cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+    cudaError_t e = dev_malloc(m, &p, n * sizeof(T));
     if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     m->allocs.push_back(p);
   }
@@ -477,15 +535,14 @@ static int64_t build_sdc_skip(const HostGroup& hg, int nRows, std::vector<SdcSki
 
 int64_t init_device_state(Matrix* m) {
   CLA_CUDA(cudaSetDevice(m->device));
-  cudaDeviceProp prop;
-  CLA_CUDA(cudaGetDeviceProperties(&prop, m->device));
-  m->smCount = prop.multiProcessorCount;
+  CLA_CUDA(cudaDeviceGetAttribute(&m->smCount, cudaDevAttrMultiProcessorCount, m->device));
   CLA_CUDA(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
+  pool_handles(m->device, 1);
   CLA_CUDA(cudaEventCreate(&m->ev0));
   CLA_CUDA(cudaEventCreate(&m->ev1));
   CLA_CUDA(cudaEventCreateWithFlags(&m->lastDone, cudaEventDisableTiming));
   void* errp = nullptr;
-  CLA_CUDA(cudaMalloc(&errp, 64));
+  CLA_CUDA(dev_malloc(m, &errp, 64));
   // (on the handle's own stream: a clear on the default stream could run after the first checks have reported)
   CLA_CUDA(cudaMemsetAsync(errp, 0, 64, m->stream));
   CLA_CUDA(cudaStreamSynchronize(m->stream));
@@ -559,16 +616,15 @@ int64_t finalize_device(Matrix* m) {
   int64_t rcs;
   if ((rcs = slab_open(m, up.small_, smallB)) < 0 || (rcs = slab_open(m, up.big, bigB)) < 0) return rcs;
   struct Scratch {  // of the run decoder, for all groups (stream order keeps them apart)
+    const Matrix* m;
     void* p = nullptr;
-    ~Scratch() {
-      if (p) cudaFree(p);
-    }
-  } rleTmp;
+    ~Scratch() { dev_free(m, p); }
+  } rleTmp{m};
   size_t rleSort = 0;
   if (mostPairs > 0) {
     cub::DeviceRadixSort::SortPairs(nullptr, rleSort, (uint32_t*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                     (int)mostPairs, 0, 32, m->stream);
-    CLA_CUDA(cudaMalloc(&rleTmp.p, (size_t)mostPairs * (sizeof(RleRun) + 4 * sizeof(uint32_t)) + rleSort + 16));
+    CLA_CUDA(dev_malloc(m, &rleTmp.p, (size_t)mostPairs * (sizeof(RleRun) + 4 * sizeof(uint32_t)) + rleSort + 16));
   }
   for (size_t gi = 0; gi < m->hg.size(); gi++) {
     HostGroup& hg = m->hg[gi];
@@ -795,16 +851,13 @@ int64_t finalize_device(Matrix* m) {
 
 void release(Matrix* m) {
   if (m->device >= 0) cudaSetDevice(m->device);
+  if (m->stream) cudaDeviceSynchronize();  // nothing on any stream uses the handle's memory any more
   fast_plan_free(m);
   wide_plan_free(m);
-  for (void* p : m->allocs) cudaFree(p);
+  for (void* p : m->allocs) dev_free(m, p);
   m->allocs.clear();
-  if (m->scratch) cudaFree(m->scratch);
-  if (m->scratch2) cudaFree(m->scratch2);
-  if (m->io) cudaFree(m->io);
-  if (m->small_) cudaFree(m->small_);
+  for (void* p : {m->scratch, m->scratch2, m->io, m->small_, (void*)m->dErr}) dev_free(m, p);
   m->small_ = nullptr;
-  if (m->dErr) cudaFree(m->dErr);
   for (auto& pr : m->profEvents) {
     cudaEventDestroy(pr.first);
     cudaEventDestroy(pr.second);
@@ -826,7 +879,11 @@ void release(Matrix* m) {
   host_stage_free(m);
   mailbox_give(m->mail);
   m->mail = nullptr;
-  if (m->stream) cudaStreamDestroy(m->stream);
+  if (m->stream) {
+    cudaStreamSynchronize(m->stream);
+    cudaStreamDestroy(m->stream);
+    pool_handles(m->device, -1);
+  }
   m->scratch = m->scratch2 = m->io = nullptr;
   m->dErr = nullptr;
   m->stream = nullptr;

@@ -183,7 +183,7 @@ int64_t ensure_sparse_list(Matrix* m) {
   auto up = [&](const std::vector<int32_t>& idx, int32_t** d) -> int64_t {
     if (idx.empty()) return CLA_OK;
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, idx.size() * sizeof(int32_t));
+    cudaError_t e = dev_malloc(m, &p, idx.size() * sizeof(int32_t));
     if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc group list: ") + cudaGetErrorString(e));
     m->allocs.push_back(p);
     CLA_CUDA(cudaMemcpy(p, idx.data(), idx.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -281,7 +281,7 @@ __global__ void k_iota_cols(int32_t* p, int n) {
 int64_t make_overlapping(Matrix* m, Matrix* child, const double* dV, int vCols, cudaStream_t s) {
   auto dalloc = [&](void** p, size_t bytes) -> int64_t {
     *p = nullptr;
-    cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+    cudaError_t e = dev_malloc(child, p, std::max<size_t>(bytes, 16));
     if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc overlapping result: ") + cudaGetErrorString(e));
     child->allocs.push_back(*p);
     child->deviceBytes += (int64_t)bytes;

@@ -26,7 +26,7 @@ constexpr int RL_THREADS = 256;
 
 int64_t plan_alloc(Matrix* m, void** p, size_t bytes) {
   *p = nullptr;
-  cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+  cudaError_t e = dev_malloc(m, p, std::max<size_t>(bytes, 16));
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(CLA_ERR_NOMEM, std::string("cudaMalloc row plan: ") + cudaGetErrorString(e));
