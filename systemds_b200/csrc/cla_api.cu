@@ -457,7 +457,8 @@ static int64_t lmm_dev(Matrix* m, const double* dYt, int32_t yRows, double* dOut
   // are copied to an even pitch first.
   if (yRows >= 1 && fast_plan_ok(m) && m->nRows > 0) {
     const double* rows = dYt;
-    size_t pitch = (size_t)m->nRows;
+    size_t pitch = (size_t)m->nRows;  // (of no meaning for one row)
+    if (yRows == 1) pitch &= ~(size_t)1;
     if (((uintptr_t)dYt & 15) || (yRows > 1 && (m->nRows & 1))) {
       pitch = ((size_t)m->nRows + 1) & ~(size_t)1;
       int64_t rc = ensure_scratch2(m, pitch * yRows * sizeof(double));
@@ -466,14 +467,7 @@ static int64_t lmm_dev(Matrix* m, const double* dYt, int32_t yRows, double* dOut
                                  (size_t)m->nRows * sizeof(double), yRows, cudaMemcpyDeviceToDevice, s));
       rows = (const double*)m->scratch2;
     }
-    int64_t rc = 0;
-    for (int i = 0; i < yRows;) {
-      const int q = std::min(8, yRows - i);
-      rc = q == 1 ? fast_lmm_vec(m, rows + pitch * i, dOut + (size_t)i * m->nCols, s)
-                  : fast_lmm_rows(m, rows + pitch * i, pitch, q, dOut + (size_t)i * m->nCols, s);
-      if (rc <= 0) break;
-      i += q;
-    }
+    const int64_t rc = fast_lmm_rows(m, rows, pitch, yRows, dOut, s);
     if (rc < 0) return rc;
     if (rc == 1) return CLA_OK;
     if (rc == 2) return launch_lmm(m, dYt, yRows, dOut, s, true);

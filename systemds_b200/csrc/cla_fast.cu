@@ -369,6 +369,140 @@ __global__ void __launch_bounds__(LMM_T, 1) k_lmm_vec(const __grid_constant__ Lm
 }
 
 // --------------------------------------------------------------------------------------------------
+// LMM with Q left rows at once (Q = 2 or 4; the reference's left-multiply blocks four rows too,
+// lib/CLALibLeftMultBy.java:731-819). Same layout and lookups as k_lmm_vec_u8, but a dictionary value fetched for a
+// cell multiplies the cell's Q left values: one pass over the maps and one lookup per cell serve Q rows, where Q
+// passes of the one-row kernel would fetch each value Q times. partial: [gridDim.x][Q][LMM_PART].
+// --------------------------------------------------------------------------------------------------
+constexpr int LQ_W = 12;              // warps per CTA (Q x NU accumulators per lane: up to 170 registers)
+constexpr int LQ_T = LQ_W * 32;
+
+template <int NU, int Q>
+__device__ __forceinline__ void lmmq_body(const LmmChunk& ch, const uint8_t* __restrict__ imaps, int64_t nRB,
+                                          const double* __restrict__ tablesImg, const double* __restrict__ y, size_t pitch,
+                                          int nRows, double* __restrict__ partial, unsigned char* smraw, uint64_t* mbar,
+                                          int32_t* err) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slot = lane & 15, half = lane >> 4;
+  if (!tma_load_to_smem(smraw, tablesImg + ch.tblOff, (uint32_t)ch.tblDoubles * 8u, mbar)) {
+    if (tid == 0) atomicExch(err, 105);
+    for (int u = tid; u < Q * LMM_PART; u += LQ_T) partial[(size_t)blockIdx.x * Q * LMM_PART + u] = __longlong_as_double(0x7ff8000000000000ll);
+    return;
+  }
+  const unsigned char* tbase[NU];
+  const uint8_t* mp[NU];
+  {
+    size_t off = 0;
+#pragma unroll
+    for (int u = 0; u < NU; u++) {
+      tbase[u] = smraw + off + slot * 8;
+      off += (size_t)ch.nk[u] * 128;
+      mp[u] = imaps + (size_t)(ch.unit0 + u) * nRB * 256 + slot * 16;
+    }
+  }
+  double acc[NU][Q];
+#pragma unroll
+  for (int u = 0; u < NU; u++)
+#pragma unroll
+    for (int q = 0; q < Q; q++) acc[u][q] = 0.0;
+  const int ctaInChunk = blockIdx.x - ch.cta0;
+  const int64_t nSteps = ((int64_t)nRows + LMM_STEP - 1) / LMM_STEP;
+  const int64_t s0 = nSteps * ctaInChunk / ch.nCta, s1 = nSteps * (ctaInChunk + 1) / ch.nCta;
+  for (int64_t st = s0 + warp; st < s1; st += LQ_W) {
+    const int64_t r0 = st * LMM_STEP + half * 32;
+    if (st * LMM_STEP + LMM_STEP <= nRows) {
+#pragma unroll 1
+      for (int sub = 0; sub < 2; sub++) {
+        uint4 m[NU];
+#pragma unroll
+        for (int u = 0; u < NU; u++) m[u] = __ldg((const uint4*)(mp[u] + ((r0 >> 4) + sub) * 256));
+        const double* yr = y + r0 + sub * 16;
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {  // two rows per 128-bit load of every left row
+          double2 yq[Q];
+#pragma unroll
+          for (int q = 0; q < Q; q++) yq[q] = __ldg((const double2*)(yr + q * pitch + i));
+#pragma unroll
+          for (int u = 0; u < NU; u++) {
+            const uint32_t w = (i >> 2) == 0 ? m[u].x : ((i >> 2) == 1 ? m[u].y : ((i >> 2) == 2 ? m[u].z : m[u].w));
+            const double t0 = *(const double*)(tbase[u] + byte_x128(w, i & 3));
+            const double t1 = *(const double*)(tbase[u] + byte_x128(w, (i & 3) + 1));
+#pragma unroll
+            for (int q = 0; q < Q; q++) acc[u][q] = fma(yq[q].y, t1, fma(yq[q].x, t0, acc[u][q]));
+          }
+        }
+      }
+    } else {  // ragged last step
+      for (int64_t r = r0; r < min((int64_t)nRows, r0 + 32); r++) {
+#pragma unroll
+        for (int u = 0; u < NU; u++) {
+          const double t = *(const double*)(tbase[u] + 128 * (int)mp[u][(r >> 4) * 256 + (r & 15)]);
+#pragma unroll
+          for (int q = 0; q < Q; q++) acc[u][q] = fma(y[q * pitch + r], t, acc[u][q]);
+        }
+      }
+    }
+  }
+  __syncthreads();  // tables no longer needed
+  double* red = (double*)smraw;  // [LQ_W][Q][NU*16]
+#pragma unroll
+  for (int u = 0; u < NU; u++)
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      double a = acc[u][q];
+      a += __shfl_xor_sync(0xffffffffu, a, 16);
+      if (half == 0) red[(warp * Q + q) * (NU * 16) + u * 16 + slot] = a;
+    }
+  __syncthreads();
+  for (int e = tid; e < Q * NU * 16; e += LQ_T) {
+    const int q = e / (NU * 16), u = e - q * (NU * 16);
+    double s = 0;
+    for (int w = 0; w < LQ_W; w++) s += red[(w * Q + q) * (NU * 16) + u];
+    partial[((size_t)blockIdx.x * Q + q) * LMM_PART + u] = s;
+  }
+}
+
+template <int Q>
+__global__ void __launch_bounds__(LQ_T, 1)
+k_lmm_vecq_u8(const LmmChunk* __restrict__ chunks, int nChunks, const uint8_t* __restrict__ imaps, int64_t nRB,
+              const double* __restrict__ tablesImg, const double* __restrict__ y, size_t pitch, int nRows,
+              double* __restrict__ partial, int32_t* err) {
+  extern __shared__ __align__(128) unsigned char smraw[];
+  __shared__ __align__(8) uint64_t mbar;
+  __shared__ LmmChunk ch;
+  if (threadIdx.x == 0) {
+    int c = 0;
+    while (c + 1 < nChunks && (int)blockIdx.x >= chunks[c].cta0 + chunks[c].nCta) c++;
+    ch = chunks[c];
+  }
+  __syncthreads();
+#define LQ_CASE(N) case N: lmmq_body<N, Q>(ch, imaps, nRB, tablesImg, y, pitch, nRows, partial, smraw, &mbar, err); break;
+  switch (ch.nUnits) {
+    LQ_CASE(1) LQ_CASE(2) LQ_CASE(3) LQ_CASE(4) LQ_CASE(5) LQ_CASE(6)
+    default: lmmq_body<7, Q>(ch, imaps, nRB, tablesImg, y, pitch, nRows, partial, smraw, &mbar, err); break;
+  }
+#undef LQ_CASE
+}
+
+// out[q][col] += sum over the chunk's CTAs of partial[cta][q][slot]; blockIdx.z = q
+__global__ void k_lmm_vecq_final(const LmmChunk* __restrict__ chunks, int nChunks, const int* __restrict__ slotCol,
+                                 const double* __restrict__ partial, double* __restrict__ out, int Q, int nCols) {
+  const int c = blockIdx.x, q = blockIdx.z;
+  if (c >= nChunks) return;
+  const LmmChunk ch = chunks[c];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nWarps = (blockDim.x >> 5) * gridDim.y;
+  for (int u = blockIdx.y * (blockDim.x >> 5) + warp; u < ch.nUnits * 16; u += nWarps) {
+    const int col = slotCol[ch.unit0 * 16 + u];
+    if (col < 0) continue;
+    double s = 0;
+    for (int i = lane; i < ch.nCta; i += 32) s += partial[((size_t)(ch.cta0 + i) * Q + q) * LMM_PART + u];
+#pragma unroll
+    for (int d = 16; d; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    if (lane == 0) atomicAdd(&out[(size_t)q * nCols + col], s);
+  }
+}
+
+// --------------------------------------------------------------------------------------------------
 // LMM with two to eight left rows at once, on the FP64 tensor core: m8n8k4 with A = left rows x matrix rows, B = matrix
 // rows x eight column slots. Lane (g, t) looks up slot g's values of rows 4 t .. 4 t + 3 of a 16-row block (one word of
 // ids), the four products of the block taking one of them each, so a lookup serves all left rows and nothing is staged.
@@ -448,25 +582,35 @@ __device__ __forceinline__ void lmm_rows_body(const LmmRowsArgs& A, int chunk, i
   const int64_t nBlk = ((int64_t)A.nRows + 15) / 16, whole = A.nRows / 16;
   const int ci = blockIdx.x - cta0;
   const int64_t b0 = nBlk * ci / nCta, b1 = nBlk * (ci + 1) / nCta;
-  // NB blocks per turn, their loads issued together: with few tiles a block is little work, and the left values come from
-  // L2 (500k x 200, 256 values, eight left rows, three tiles: 301 us with one block per turn, its loads one turn ahead)
-  constexpr int NB = NT <= 3 ? 4 : (NT <= 5 ? 2 : 1);
-  for (int64_t blk = b0 + warp * NB; blk < b1; blk += LR_W * NB) {
-    uint32_t id[NB][NT];
+  // NB blocks per turn, the next turn's loads in flight during this one's lookups: with few tiles a block is little work,
+  // and the left values come from L2
+  constexpr int NB = NT <= 4 ? 2 : 1;
+  uint32_t id[NB][NT];
+  double2 ya[NB], yb[NB];
+  auto load = [&](int64_t k0) {
+#pragma unroll
+    for (int n = 0; n < NB; n++) {
+      const int64_t k = min(k0 + n, nBlk - 1);
+#pragma unroll
+      for (int u = 0; u < NT; u++) id[n][u] = ids_at(u, k);
+      if (k < whole) {
+        ya[n] = __ldg((const double2*)(yr + k * 16));
+        yb[n] = __ldg((const double2*)(yr + k * 16) + 1);
+      }
+    }
+  };
+  int64_t blk = b0 + warp * NB;
+  if (blk < b1) load(blk);
+  for (; blk < b1; blk += LR_W * NB) {
+    uint32_t w[NB][NT];
     double yv[NB][4];
 #pragma unroll
     for (int n = 0; n < NB; n++) {
-      const int64_t k = blk + n;
-      const bool in = k < b1;
 #pragma unroll
-      for (int u = 0; u < NT; u++) id[n][u] = in ? ids_at(u, k) : 0u;
-#pragma unroll
-      for (int i = 0; i < 4; i++) yv[n][i] = 0.0;
-      if (in && k < whole) {
-        const double2 ya = __ldg((const double2*)(yr + k * 16)), yb = __ldg((const double2*)(yr + k * 16) + 1);
-        yv[n][0] = ya.x, yv[n][1] = ya.y, yv[n][2] = yb.x, yv[n][3] = yb.y;
-      }
+      for (int u = 0; u < NT; u++) w[n][u] = id[n][u];
+      yv[n][0] = ya[n].x, yv[n][1] = ya[n].y, yv[n][2] = yb[n].x, yv[n][3] = yb[n].y;
     }
+    if (blk + LR_W * NB < b1) load(blk + LR_W * NB);
 #pragma unroll
     for (int n = 0; n < NB; n++) {
       if (blk + n >= b1) break;
@@ -475,7 +619,7 @@ __device__ __forceinline__ void lmm_rows_body(const LmmRowsArgs& A, int chunk, i
         for (int u = 0; u < NT; u++) {
           double x[4];
 #pragma unroll
-          for (int i = 0; i < 4; i++) x[i] = lds_f64(entry_at(id[n][u], i, tb[u]));
+          for (int i = 0; i < 4; i++) x[i] = lds_f64(entry_at(w[n][u], i, tb[u]));
 #pragma unroll
           for (int i = 0; i < 4; i++) dmma884(c[u][0], c[u][1], yv[n][i], x[i]);
         }
@@ -487,7 +631,7 @@ __device__ __forceinline__ void lmm_rows_body(const LmmRowsArgs& A, int chunk, i
         for (int u = 0; u < NT; u++)
 #pragma unroll
           for (int i = 0; i < 4; i++)
-            dmma884(c[u][0], c[u][1], yv[n][i], r0 + i < A.nRows ? lds_f64(entry_at(id[n][u], i, tb[u])) : 0.0);
+            dmma884(c[u][0], c[u][1], yv[n][i], r0 + i < A.nRows ? lds_f64(entry_at(w[n][u], i, tb[u])) : 0.0);
       }
       if (A.constV) ys += (yv[n][0] + yv[n][1]) + (yv[n][2] + yv[n][3]);
     }
@@ -1578,11 +1722,37 @@ int64_t fast_lmm_vec(Matrix* m, const double* dY, double* dOut, cudaStream_t s) 
   return fp->partial ? 2 : 1;
 }
 
-// q = 2 .. 8 left rows (row i at y + i * pitch, 16-byte aligned) in one pass; same return values as fast_lmm_vec.
-int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* dOut, cudaStream_t s) {
-  FastPlan* fp = m->fast;
-  if (!fp || !fp->ok || ((uintptr_t)dY & 15) || (pitch & 1)) return 0;
-  if (q < 1 || q > 8) return fail(CLA_ERR_BAD_ARG, "fast_lmm_rows: up to 8 rows");
+// Q = 2 or 4 left rows (rows q of y at y + q * pitch, 16-byte aligned) in one pass; same return values as fast_lmm_vec.
+template <int Q>
+static int64_t fast_lmm_rows_t(Matrix* m, FastPlan* fp, const double* dY, size_t pitch, double* dOut, cudaStream_t s) {
+  int64_t rc;
+  const size_t partBytes = (size_t)fp->lmmGrid * Q * LMM_PART * 8;
+  if ((rc = ensure_scratch(m, partBytes + 256)) < 0) return rc;
+  double* partial = (double*)m->scratch;
+  CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)Q * m->nCols, s));
+  size_t smem = (size_t)LQ_W * Q * LMM_PART * 8;
+  for (auto& c : fp->lchunks) smem = std::max(smem, (size_t)c.tblDoubles * 8);
+  static bool attr[64] = {};  // per device
+  if (!attr[m->device & 63]) {
+    CLA_CUDA(cudaFuncSetAttribute(k_lmm_vecq_u8<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
+    attr[m->device & 63] = true;
+  }
+  prof_begin(m, s);
+  k_lmm_vecq_u8<Q><<<fp->lmmGrid, LQ_T, smem, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dLmmMaps, fp->nRB, fp->dLmmTables, dY,
+                                                  pitch, m->nRows, partial, m->dErr);
+  prof_end(m, s);
+  k_lmm_vecq_final<<<dim3((unsigned)fp->lchunks.size(), LMM_MAX_UNITS, Q), 512, 0, s>>>(fp->dLChunks, (int)fp->lchunks.size(),
+                                                                                       fp->dSlotCol, partial, dOut, Q, m->nCols);
+  m->stats.kernel_launches += 2;
+  if (m->hasConst)
+    for (int q = 0; q < Q; q++)
+      if ((rc = launch_lmm_const(m, dY + q * pitch, 1, dOut + (size_t)q * m->nCols, s)) < 0) return rc;
+  CLA_CUDA(cudaGetLastError());
+  return fp->partial ? 2 : 1;
+}
+// Up to eight left rows on the tensor core; NOT_HERE: k_lmm_vecq is the better one.
+constexpr int64_t NOT_HERE = 3;
+static int64_t lmm_rows_tensor(Matrix* m, FastPlan* fp, const double* dY, size_t pitch, int q, double* dOut, cudaStream_t s) {
   LmmRowsArgs A{};
   A.units = fp->dUnits;
   A.imaps = fp->dLmmMaps;
@@ -1608,6 +1778,7 @@ int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* 
   // Tiles per chunk: what fits, and by the same balance as lmm_chunk_units -- clocks per 16 rows 16 a tile and 10 for the
   // left values, 2 per tuple of a staged tile, at least one round of blocks.
   size_t smem = 0;
+  int fits = 0;
   double bestCost = 1e300;
   const int64_t nBlk = ((int64_t)m->nRows + 15) / 16;
   for (int U = 1; U <= LR_MAXT; U++) {
@@ -1617,6 +1788,7 @@ int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* 
     for (int c = 0; c < T.nChunks; c++) stage = std::max(stage, bytes_of(T.tile0(c), T.tile0(c + 1) - T.tile0(c)));
     most = std::max(most, stage);
     if (most > (size_t)LR_SMEM) continue;
+    fits = U;
     const double ctas = std::max(1.0, (double)m->smCount / T.nChunks), blocks = nBlk / ctas, waves = std::ceil((double)T.nChunks / m->smCount);
     const double cost = waves * (stage / 128.0 + std::max(blocks * (16.0 * U + 10.0), std::ceil(blocks / LR_W) * (700.0 + 60.0 * U)));
     if (cost < bestCost) {
@@ -1626,6 +1798,10 @@ int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* 
     }
   }
   if (A.nChunks == 0) return fail(CLA_ERR_STATE, "left product: a table does not fit shared memory");
+  // Up to four rows on deep tables: half of the products would be wasted, and with few tiles per CTA the left values are
+  // read too often for that (1M x 200, 256 values, 2 / 3 / 4 rows: 199 / 207 / 215 us here, 121 / 197 / 154 in passes of
+  // k_lmm_vecq; at 100 values and eight tiles, 100k x 500, three rows, 50 against 74).
+  if (q <= 4 && fits < 6 && A.nTiles > fits) return NOT_HERE;
   // at least one CTA for every chunk, however the shares round; no more than four blocks of rows justify
   const int64_t most = std::max<int64_t>((int64_t)2 * A.nChunks, ((nBlk + 3) / 4) * A.nChunks);
   const int grid = A.grid = (int)std::min<int64_t>(most, 2 * A.nChunks > m->smCount ? 2 * A.nChunks : m->smCount);
@@ -1657,6 +1833,26 @@ int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* 
       if ((rc = launch_lmm_const(m, dY + i * pitch, 1, dOut + (size_t)i * m->nCols, s)) < 0) return rc;
   CLA_CUDA(cudaGetLastError());
   return fp->partial ? 2 : 1;
+}
+
+// q left rows (row i at y + i * pitch, 16-byte aligned); same return values as fast_lmm_vec.
+int64_t fast_lmm_rows(Matrix* m, const double* dY, size_t pitch, int q, double* dOut, cudaStream_t s) {
+  FastPlan* fp = m->fast;
+  if (!fp || !fp->ok || ((uintptr_t)dY & 15) || (pitch & 1)) return 0;
+  int64_t rc = 0;
+  for (int i = 0; i < q;) {
+    const double* y = dY + (size_t)i * pitch;
+    double* o = dOut + (size_t)i * m->nCols;
+    int n = std::min(8, q - i);
+    rc = n == 1 ? NOT_HERE : lmm_rows_tensor(m, fp, y, pitch, n, o, s);
+    if (rc == NOT_HERE) {
+      n = n == 4 ? 4 : std::min(2, n);
+      rc = n == 4 ? fast_lmm_rows_t<4>(m, fp, y, pitch, o, s) : (n == 2 ? fast_lmm_rows_t<2>(m, fp, y, pitch, o, s) : fast_lmm_vec(m, y, o, s));
+    }
+    if (rc <= 0) return rc;
+    i += n;
+  }
+  return rc;
 }
 
 // Host-buffer t(y) %*% X with the upload of y overlapped with the product: y is copied in up to LMM_PIPE_MAX row ranges

@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(RR_T, 4) k_rest_rmm(const __grid_constant__ Re
 // --------------------------------------------------------------------------------------------------
 // Yt X
 // --------------------------------------------------------------------------------------------------
-constexpr int RL_WARPS = 8;     // two CTAs per SM
+constexpr int RL_WARPS = 8;     // two CTAs per SM (three or four, of 80 or 64 registers: 5 to 35 % slower)
 constexpr int RL_T = RL_WARPS * 32;
 constexpr int RL_TASKS = 320;   // columns per CTA of the first kind
 constexpr int RL_UC = 64;       // columns per CTA of the second
@@ -637,7 +637,7 @@ int64_t rest_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t
       const int slots = 2 * m->smCount;
       // CTAs of the two kinds: the block's bytes against the list walks, about 1 us of an SM per 350 columns and block
       const int nBlocks = (m->nRows + SKIP_ROWS - 1) / SKIP_ROWS;
-      const double wT = A.nTasks * 1.0, wU = A.gCols * 2.5;
+      const double wT = A.nTasks * 1.0, wU = A.gCols * 4.0;
       int nT = A.nTasks ? (A.gCols ? std::max(1, (int)(slots * wT / (wT + wU))) : slots) : 0;
       A.ctaTasks = A.nTasks ? std::max(1, std::min(nBlocks, nT / A.nChunks)) : 0;
       const int nU = std::max(1, slots - A.ctaTasks * A.nChunks);
