@@ -364,14 +364,14 @@ class Workload:
         """(bound, work per launch, unit scale, peak, unit, kernel): bytes for the HBM-bound products, flops for TSMM."""
         n, ib = self.n, self.index_bytes
         if self.idx == 0:
-            return "hbm", ib + n * 8 + 100 * 8, "k_rmm_vec_f"
+            return "hbm", ib + n * 8 + 100 * 8, "k_rmm_vec"
         if self.idx == 1:
-            return "hbm", ib + n * 8 + 200 * 8, "k_lmm_vec_u8"
+            return "hbm", ib + n * 8 + 200 * 8, "k_lmm_vec"
         if self.idx == 2:
-            return "hbm", ib + n * 64 * 8 + 500 * 64 * 8, "k_rmm_dmma3"
+            return "hbm", ib + n * 64 * 8 + 500 * 64 * 8, "k_rmm_wide"
         if self.idx == 3:
             return "tensor", 2.0 * n * 100 * 101 / 2, "k_tsmm_tri16"
-        return "hbm", 2 * ib + 2 * n * 8 + 2 * 1000 * 8, "k_rmm_vec_b + k_lmm_vec_u8"
+        return "hbm", 2 * ib + 2 * n * 8 + 2 * 1000 * 8, "k_rmm_vec + k_lmm_vec"
 
     # the same product through the host-buffer call (pinned operands prepared by e2e_prepare)
     def e2e_prepare(self, pinned=True):

@@ -64,8 +64,17 @@ struct WideChunk {
   int tblBytes;        // tables
   int64_t img;         // their image (doubles)
 };
+// A sparse table row (tuple of an SDC / RLE group of one column): its value and where its row of V lies.
+struct WideSv {
+  double val;
+  uint32_t at;  // bytes from the first sparse row of V in shared memory
+  uint32_t pad;
+};
 struct WidePlanNT {
   bool built = false;
+  int nSp = 0;                // rows of V kept for the SDC / RLE columns in the first chunk's CTAs; 0: tables P instead
+  int32_t* spCols = nullptr;  // [nSp] matrix columns
+  WideSv* sv = nullptr;       // [sparse table rows]
   std::vector<WideChunk> chunks;
   WideCol* cols = nullptr;
   double* image = nullptr;
@@ -86,6 +95,9 @@ struct WideArgs {
   const double* P;       // [table rows][vCols]
   const uint32_t *rowPtr, *rowItems, *fullPtr, *fullItems, *partPtr;
   const uint2* partItems;
+  int nSp;               // > 0: the sparse groups from values and rows of V in shared memory, not from P
+  const int32_t* spCols;
+  const WideSv* sv;
   const double* constRow;
   double* out;
   int32_t* err;
@@ -98,6 +110,13 @@ __global__ void k_wide_image(const WideCol* __restrict__ cols, int n, double* __
   const WideCol c = cols[blockIdx.x];
   if (c.imgAt < 0) return;
   for (int k = threadIdx.x; k < c.nVals; k += blockDim.x) image[c.imgAt + k] = c.src[(size_t)k * c.stride];
+}
+__global__ void k_wide_sv(const SparseVal* __restrict__ sv, int64_t nSv, const int32_t* __restrict__ slotOf, uint32_t rowBytes,
+                          WideSv* __restrict__ out) {
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < nSv; p += (int64_t)gridDim.x * blockDim.x) {
+    const int slot = sv[p].col >= 0 ? slotOf[sv[p].col] : -1;
+    out[p] = WideSv{sv[p].val, (uint32_t)max(slot, 0) * rowBytes, 0u};  // (groups without rows have no slot, and no items)
+  }
 }
 // P[p][j] for every sparse table row
 __global__ void k_wide_terms(const SparseVal* __restrict__ sv, int64_t nSv, const DevGroup* __restrict__ groups,
@@ -136,6 +155,8 @@ __global__ void __launch_bounds__(WD_T, 1) k_rmm_wide(const __grid_constant__ Wi
   double* Vs = (double*)(wsm + A.ch.tblBytes);
   const void** mapOf = (const void**)(Vs + (size_t)A.ch.nPad * LDB);
   uint32_t* tblOf = (uint32_t*)(mapOf + A.ch.nPad);
+  double* spV = (double*)(tblOf + ((A.ch.nPad + 3) & ~3));  // [nSp][LDB]
+  const char* spB = (const char*)spV;
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(wsm);
   if (A.ch.tblBytes) {
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&mbar);
@@ -156,6 +177,10 @@ __global__ void __launch_bounds__(WD_T, 1) k_rmm_wide(const __grid_constant__ Wi
     const int k = e / TN, n = e - k * TN;
     const int vr = A.cols[A.ch.col0 + k].vrow;
     Vs[k * LDB + n] = (vr >= 0 && n < vc) ? A.V[(size_t)vr * A.vCols + j0 + n] : 0.0;
+  }
+  for (int e = tid; e < A.nSp * TN; e += WD_T) {
+    const int k = e / TN, n = e - k * TN;
+    spV[k * LDB + n] = n < vc ? A.V[(size_t)A.spCols[k] * A.vCols + j0 + n] : 0.0;
   }
   for (int k = tid; k < A.ch.nPad; k += WD_T) {
     const WideCol& c = A.cols[A.ch.col0 + k];
@@ -181,7 +206,19 @@ __global__ void __launch_bounds__(WD_T, 1) k_rmm_wide(const __grid_constant__ Wi
   // windows are dealt to the SMs first, then to their warps: short matrices use every SM
   for (int w = warp * gridDim.x + blockIdx.x; w < nWin; w += gridDim.x * WD_WARPS) {
     double full[2] = {0.0, 0.0};  // runs over the whole window: lane = result column
-    if (A.fullPtr && lane < vc) {
+    if (A.fullPtr && A.nSp) {
+      const uint32_t q1 = A.fullPtr[w + 1];
+      for (uint32_t p = A.fullPtr[w]; p < q1; p += 32) {  // a lane per item, then every item by all lanes
+        WideSv mine = {0.0, 0u, 0u};
+        if (p + lane < q1) mine = A.sv[A.fullItems[p + lane]];
+        const int n = (int)min(32u, q1 - p);
+        for (int u = 0; u < n; u++) {
+          const double x = __shfl_sync(0xffffffffu, mine.val, u);
+          const uint32_t at = __shfl_sync(0xffffffffu, mine.at, u);
+          if (lane < TN) full[0] = fma(x, *(const double*)(spB + at + lane * 8), full[0]);
+        }
+      }
+    } else if (A.fullPtr && lane < vc) {
       const uint32_t q1 = A.fullPtr[w + 1];
       for (uint32_t p = A.fullPtr[w]; p < q1; p += 8) {
         double x[8];
@@ -296,7 +333,34 @@ __global__ void __launch_bounds__(WD_T, 1) k_rmm_wide(const __grid_constant__ Wi
         multiply(ks, x[0], x[1]);
       }
       // SDC: the listed tuples of the lane's rows; the four lanes of a row read 64 bytes of a table row per n
-      if (A.rowPtr) {
+      if (A.rowPtr && A.nSp) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int r = row + i;
+          uint32_t p = 0, p1 = 0;
+          if (r < A.nRows) {
+            p = A.rowPtr[r];
+            p1 = A.rowPtr[r + 1];
+          }
+          for (; p < p1; p += 4) {  // four items in flight
+            WideSv e[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) e[u] = p + u < p1 ? A.sv[A.rowItems[p + u]] : WideSv{0.0, 0u, 0u};
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+              if (p + u < p1) {
+                const char* q = spB + e[u].at + 2 * t * 8;
+#pragma unroll
+                for (int n = 0; n < NT; n++) {
+                  const double2 v = *(const double2*)(q + n * 64);
+                  double* d = &c[i >> 1][n][(i & 1) * 2];
+                  d[0] = fma(e[u].val, v.x, d[0]);
+                  d[1] = fma(e[u].val, v.y, d[1]);
+                }
+              }
+          }
+        }
+      } else if (A.rowPtr) {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
           const int r = row + i;
@@ -342,9 +406,18 @@ __global__ void __launch_bounds__(WD_T, 1) k_rmm_wide(const __grid_constant__ Wi
           const int ra = (int)(it.y & 0xFF) - half * 32, rb = (int)(it.y >> 8) - half * 32;
           if (rb <= 0 || ra >= 32) continue;
           const double* q = A.P + (size_t)it.x * A.vCols + j0 + 2 * t;
+          WideSv e = {0.0, 0u, 0u};
+          if (A.nSp) e = A.sv[it.x];
 #pragma unroll
           for (int n = 0; n < NT; n++) {
-            const double x = n * 8 + 2 * t < vc ? q[n * 8] : 0.0, y = n * 8 + 2 * t + 1 < vc ? q[n * 8 + 1] : 0.0;
+            double x, y;
+            if (A.nSp) {
+              const double2 v = *(const double2*)(spB + e.at + (2 * t + n * 8) * 8);
+              x = e.val * v.x, y = e.val * v.y;
+            } else {
+              x = n * 8 + 2 * t < vc ? q[n * 8] : 0.0;
+              y = n * 8 + 2 * t + 1 < vc ? q[n * 8 + 1] : 0.0;
+            }
 #pragma unroll
             for (int i = 0; i < 4; i++)
               if (4 * g + i >= ra && 4 * g + i < rb) {
@@ -426,7 +499,28 @@ static int64_t ensure_wide(Matrix* m, int NT, cudaStream_t s) {
   }
   const size_t perCol = (size_t)(NT * 8 + 4) * 8 + 12;
   auto cost = [&](const WideCol& c) { return perCol + (c.tbl >= 0 ? (((size_t)c.nVals * 8 + 15) & ~(size_t)15) : 0); };
-  size_t total = 0;
+  // Rows of V of the SDC / RLE columns, next to the first chunk, where they take at most half of it and every such group
+  // has one column: reading table rows P = D V (eight tuples and 64 columns: 4 KB a column) from L2 instead was 3.8 GB per
+  // product on 1M x 500 mixed, 64 columns of V (1.51 ms; 1.41 ms so).
+  std::vector<int32_t> spCols, slotOf(m->nCols, -1);
+  bool single = true;
+  for (size_t hi = 0; hi < m->hg.size(); hi++) {
+    const int gi = m->regToDev[hi];
+    if (gi < 0) continue;
+    const DevGroup& g = m->groups[gi];
+    if (!((g.type == GT_SDC && g.nOff > 0) || (g.type == GT_RLE && g.nRuns > 0))) continue;
+    single &= g.gCols == 1;
+    const int c = m->hg[hi].cols[0];
+    if (slotOf[c] < 0) {
+      slotOf[c] = (int)spCols.size();
+      spCols.push_back(c);
+    }
+  }
+  const size_t rowB = (size_t)(NT * 8 + 4) * 8;
+  if (!single || spCols.size() * rowB > WD_SMEM / 2) spCols.clear();
+  W.nSp = (int)spCols.size();
+  const size_t spBytes = spCols.size() * rowB;
+  size_t total = spBytes;
   for (auto& k : kind)
     for (auto& c : k) total += cost(c);
   // Kinds are padded to eights. A padding column of the first two kinds reads the map of the matrix' column of that kind
@@ -474,22 +568,35 @@ static int64_t ensure_wide(Matrix* m, int NT, cudaStream_t s) {
     img += tb / 8;
     W.chunks.push_back(ch);
   };
-  size_t used = 0;
+  size_t used = spBytes;
+  bool any = false;
   for (int k = 0; k < 4; k++)
     for (auto& c : kind[k]) {
       const size_t b = cost(c);
-      if (used > 0 && used + b > std::min(want, room)) {
+      if (any && used + b > std::min(want, room)) {
         flush();
         used = 0;
       }
       cur[k].push_back(c);
+      any = true;
       used += b;
     }
   flush();
-  for (auto& c : W.chunks) W.smem = std::max(W.smem, (size_t)c.tblBytes + (size_t)c.nPad * perCol + 64);
+  for (size_t i = 0; i < W.chunks.size(); i++)
+    W.smem = std::max(W.smem, (size_t)W.chunks[i].tblBytes + (size_t)W.chunks[i].nPad * perCol + (i == 0 ? spBytes : 0) + 64);
   void* d = nullptr;
   const size_t bc = (cols.size() * sizeof(WideCol) + 255) & ~(size_t)255;
-  if ((rc = plan_alloc(m, &d, bc + (size_t)img * 8)) < 0) return rc;
+  const size_t bi = ((size_t)img * 8 + 255) & ~(size_t)255, bs = ((size_t)W.nSp * 4 + 255) & ~(size_t)255;
+  const size_t bl = ((size_t)m->nCols * 4 + 255) & ~(size_t)255, bv = W.nSp ? (size_t)m->rows.nSv * sizeof(WideSv) : 0;
+  if ((rc = plan_alloc(m, &d, bc + bi + bs + bl + bv)) < 0) return rc;
+  W.spCols = (int32_t*)((char*)d + bc + bi);
+  W.sv = (WideSv*)((char*)d + bc + bi + bs + bl);
+  if (W.nSp) {
+    int32_t* slots = (int32_t*)((char*)d + bc + bi + bs);
+    CLA_CUDA(cudaMemcpyAsync(W.spCols, spCols.data(), spCols.size() * 4, cudaMemcpyHostToDevice, s));
+    CLA_CUDA(cudaMemcpyAsync(slots, slotOf.data(), slotOf.size() * 4, cudaMemcpyHostToDevice, s));
+    k_wide_sv<<<(unsigned)std::min<int64_t>(1024, (m->rows.nSv + 255) / 256), 256, 0, s>>>(m->rows.sv, m->rows.nSv, slots, (uint32_t)rowB, W.sv);
+  }
   W.cols = (WideCol*)d;
   W.image = (double*)((char*)d + bc);
   CLA_CUDA(cudaMemsetAsync(W.image, 0, (size_t)img * 8, s));
@@ -511,7 +618,7 @@ int64_t wide_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStrea
   const int slices = (vCols + 31) / 32, NT = ((vCols + slices - 1) / slices + 7) / 8;
   if ((rc = ensure_wide(m, NT, s)) < 0) return rc;
   const WidePlanNT& W = m->wide->nt[NT];
-  const bool sparse = L.nSdc > 0 || L.nRle > 0;
+  const bool sparse = (L.nSdc > 0 || L.nRle > 0) && W.nSp == 0;  // needs the tables P
   const size_t pBytes = sparse ? (((size_t)L.nSv * vCols * sizeof(double) + 255) & ~(size_t)255) : 0;
   if ((rc = ensure_scratch(m, pBytes + (size_t)vCols * sizeof(double) + 256)) < 0) return rc;
   WideArgs A{};
@@ -550,6 +657,9 @@ int64_t wide_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStrea
     A.ch = W.chunks[i];
     A.first = i == 0;
     A.last = i + 1 == W.chunks.size();
+    A.nSp = A.first ? W.nSp : 0;
+    A.spCols = W.spCols;
+    A.sv = W.sv;
     A.rowPtr = (A.first && L.nSdc) ? L.rowPtr : nullptr;
     A.rowItems = L.rowItems;
     A.fullPtr = (A.first && L.nRle) ? L.fullPtr : nullptr;

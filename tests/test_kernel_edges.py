@@ -137,16 +137,21 @@ def test_decompress_columns(nRows, nCols):
 
 
 @pytest.mark.parametrize("nRows", [4096, 4127, 4161])
-@pytest.mark.parametrize("kinds", ["bytes", "chars", "mixed", "sparse"])
+@pytest.mark.parametrize("kinds", ["bytes", "chars", "mixed", "sparse", "cocoded"])
 def test_wide_right_operand(nRows, kinds):
     """X %*% V around the tile widths (8, 16, 24, 32 columns, two slices) and row remainders: several chunks of columns,
-    padding columns of every kind, dictionaries too large to stay resident, odd column counts, no dense column at all."""
+    padding columns of every kind, dictionaries too large to stay resident, odd column counts, no dense column at all,
+    SDC and RLE groups of two columns (tables instead of rows of V)."""
     if kinds == "bytes":
         cmb = _ddc(nRows, [256] * 130 + [2, 2, 3], 3, const=True)
     elif kinds == "chars":
         cmb = _ddc(nRows, [300, 1000, 4096, 5000] * 3 + [9], 4)
     elif kinds == "mixed":
         cmb = datagen.random_cmb(nRows, nRows, datagen.KINDS + ("unc", "ddc2", "ddc_char", "rle", "sdcz"))
+    elif kinds == "cocoded":
+        rng = np.random.default_rng(nRows)
+        cmb = CompressedMatrixBlock(nRows, 9, [datagen.random_group(k, c, nRows, rng) for k, c in (
+            ("sdc", [0, 1]), ("rle", [2, 3]), ("sdcz", [4]), ("ddc", [5]), ("rle", [6]), ("sdcs", [7, 8]))])
     else:
         cmb = datagen.random_cmb(nRows, nRows, ("sdc", "sdcz", "rle", "sdcs", "const", "rle"))
     cmb.to_device()
