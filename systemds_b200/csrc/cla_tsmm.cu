@@ -8,6 +8,7 @@
 #include "cla_common.cuh"
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 namespace cla {
 
@@ -94,7 +95,8 @@ k_gemm_tn(const double* __restrict__ A, int aCols, int lda, const double* __rest
   const int s0 = (int)((int64_t)nSt * c / nCta), s1 = (int)((int64_t)nSt * (c + 1) / nCta);
   // The block's tiles are dealt to the warps in turn, so that they spread over the SM's four schedulers (by position in
   // the block, the triangle's tiles fell 1 : 2 : 3 : 4 on them and cost as much as a whole block); with eight tiles or
-  // fewer two warps share a tile, one for each eight rows of a stage.
+  // fewer two warps share a tile, one for each eight rows of a stage. Tiles on the diagonal do without the products of
+  // their lower left quarter and go to warps 0, 1, 4, 5: a triangle's ten tiles load the schedulers 2.5 : 2.5 : 2 : 2.
   const int ti = (min(GT_BLK, aCols - i0) + 31) / 32, tj = (min(GT_BLK, bCols - j0) + 31) / 32;
   const int nT = diag ? ti * (ti + 1) / 2 : ti * tj, split = nT <= GT_WARPS / 2 ? 2 : 1;
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(gts);
@@ -130,16 +132,19 @@ k_gemm_tn(const double* __restrict__ A, int aCols, int lda, const double* __rest
   };
   if (warp == 0)
     for (int i = 0; i < GT_STAGES - 2; i++) issue(s0 + i);
-  const int tile = split == 2 ? warp & (GT_WARPS / 2 - 1) : warp;
-  if (tile >= nT) return;
-  const int kBeg = split == 2 ? warp / (GT_WARPS / 2) * 8 : 0, kEnd = split == 2 ? kBeg + 8 : GT_KT;
-  int wi = 0, wj = tile;
-  if (diag) {
-    int rest = tile;
-    while (wi + 1 < ti && rest >= ti - wi) rest -= ti - wi, wi++;
-    wj = wi + rest;
-  } else
+  if (warp >= nT * split) return;
+  const int tile = warp % nT;
+  const int kBeg = split == 2 ? warp / nT * 8 : 0, kEnd = split == 2 ? kBeg + 8 : GT_KT;
+  int wi, wj;
+  if (!diag)
     wi = tile / tj, wj = tile - wi * tj;
+  else if (tile < 8 && !(tile & 2) && (tile & 1) + (tile >> 2) * 2 < ti)
+    wi = wj = (tile & 1) + (tile >> 2) * 2;
+  else {
+    int rest = tile - min(ti, min(tile, 2) + max(0, min(tile - 4, 2)));  // of the tiles above the diagonal
+    for (wi = 0; rest >= ti - 1 - wi; wi++) rest -= ti - 1 - wi;
+    wj = wi + 1 + rest;
+  }
   double acc[2][4][4];
 #pragma unroll
   for (int i = 0; i < 2; i++)
@@ -147,43 +152,48 @@ k_gemm_tn(const double* __restrict__ A, int aCols, int lda, const double* __rest
     for (int j = 0; j < 4; j++)
 #pragma unroll
       for (int u = 0; u < 4; u++) acc[i][j][u] = 0.0;
-  for (int st = s0; st < s1; st++) {
-    const int n = st - s0, b = n % GT_STAGES;
-    // four stages ahead, into the buffer of the stage before last: the other warps have long left that one
-    if (warp == 0 && !issue(st + GT_STAGES - 2)) {
-      if (lane == 0) atomicExch(err, 111);
-      return;
-    }
-    if (!gt_wait(full + 8 * b, (uint32_t)(n / GT_STAGES) & 1u)) {
-      if (lane == 0) atomicExch(err, 112);
-      return;
-    }
-    const double* sA = gts + (size_t)b * GT_STAGE + wi * 32 + g;
-    const double* sB = gts + (size_t)b * GT_STAGE + (diag ? 0 : GT_KT * GT_LD) + wj * 32 + g;
+  auto run = [&](auto onDiagonal) {  // (a product skipped by a predicate would still take its turn in the tensor pipe)
+    constexpr int J1 = decltype(onDiagonal)::value ? 2 : 0;
+    for (int st = s0; st < s1; st++) {
+      const int n = st - s0, b = n % GT_STAGES;
+      // four stages ahead, into the buffer of the stage before last: the other warps have long left that one
+      if (warp == 0 && !issue(st + GT_STAGES - 2)) {
+        if (lane == 0) atomicExch(err, 111);
+        return false;
+      }
+      if (!gt_wait(full + 8 * b, (uint32_t)(n / GT_STAGES) & 1u)) {
+        if (lane == 0) atomicExch(err, 112);
+        return false;
+      }
+      const double* sA = gts + (size_t)b * GT_STAGE + wi * 32 + g;
+      const double* sB = gts + (size_t)b * GT_STAGE + (diag ? 0 : GT_KT * GT_LD) + wj * 32 + g;
 #pragma unroll 1
-    for (int k = kBeg; k < kEnd; k += 8) {
-      double a[2][4], bb[4][2];
+      for (int k = kBeg; k < kEnd; k += 8) {
+        double a[2][4], bb[4][2];
 #pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const double* x = sA + (k + t) * GT_LD + i * 16;
-        a[i][0] = x[0];
-        a[i][1] = x[8];
-        a[i][2] = x[4 * GT_LD];
-        a[i][3] = x[4 * GT_LD + 8];
+        for (int i = 0; i < 2; i++) {
+          const double* x = sA + (k + t) * GT_LD + i * 16;
+          a[i][0] = x[0];
+          a[i][1] = x[8];
+          a[i][2] = x[4 * GT_LD];
+          a[i][3] = x[4 * GT_LD + 8];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          bb[j][0] = sB[(k + t) * GT_LD + j * 8];
+          bb[j][1] = sB[(k + 4 + t) * GT_LD + j * 8];
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int j = i * J1; j < 4; j++) dmma1688(acc[i][j], a[i][0], a[i][1], a[i][2], a[i][3], bb[j][0], bb[j][1]);
       }
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        bb[j][0] = sB[(k + t) * GT_LD + j * 8];
-        bb[j][1] = sB[(k + 4 + t) * GT_LD + j * 8];
-      }
-#pragma unroll
-      for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) dmma1688(acc[i][j], a[i][0], a[i][1], a[i][2], a[i][3], bb[j][0], bb[j][1]);
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * b) : "memory");
     }
-    __syncwarp();
-    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * b) : "memory");
-  }
+    return true;
+  };
+  if (!((SYRK && diag && wi == wj) ? run(std::true_type{}) : run(std::false_type{}))) return;
 #pragma unroll
   for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -215,7 +225,9 @@ static int64_t launch_gemm_tn(Matrix* m, const double* A, int aCols, int lda, co
       G.bj[G.n] = (int16_t)bj;
       const int ti = tiles(aCols, bi), tj = tiles(bCols, bj);
       const int nT = (SYRK && bi == bj) ? ti * (ti + 1) / 2 : ti * tj;
-      sum += w[G.n++] = nT <= 8 ? (nT + 1) / 2 * 2 : (nT + 3) / 4 * 4;  // what the busiest scheduler has to do
+      // tiles of the busiest scheduler
+      constexpr double DIAG[5] = {0.0, 0.375, 0.875, 1.375, 2.5};
+      sum += w[G.n++] = (SYRK && bi == bj) ? DIAG[ti] : nT <= 8 ? (nT + 1) / 2 * 0.5 : (nT + 3) / 4;
       if (++bj == nB) {
         bi++;
         bj = SYRK ? bi : 0;
