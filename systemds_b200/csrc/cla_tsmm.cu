@@ -49,18 +49,20 @@ __device__ __forceinline__ uint32_t ld_u16_here(const uint16_t* p) {
 // C [aCols x bCols] += A^T B for row-major chunks A [rows x lda], B [rows x ldb] of the same rows, on 128 x 128 blocks of C:
 // a CTA owns one block (or, on the diagonal of a self product, its upper triangle of 32 x 32 tiles) over a range of rows,
 // a warp one 32 x 32 tile in registers (eight m16n8k8 per eight rows from 16 fragment loads). 16-row stages arrive row by
-// row by TMA bulk copies in a ring of six, issued four stages ahead; full / empty mbarriers let the warps drift apart, so
+// row by TMA bulk copies in a ring of six; full / empty mbarriers let the warps drift apart, so
 // that one's fragment loads hide behind the others' products. Rows of a stage are 132 doubles apart (4 mod 16:
 // conflict-free fragment loads). The blocks get CTAs in proportion to their tiles.
-// Bound: the FP64 tensor pipe, 128 clocks per warp and eight rows against 32 wavefronts of the L1 data pipe; it is busy 73 %
-// of the time, 90 % being the most that the 3 : 3 : 2 : 2 split of a triangle's ten tiles allows. 98,304 rows x 250
-// columns: 308 us (64 x 64 blocks of m8n8k4 with the stage loaded through registers: 316 at 45 % and atomics four times as
-// often; with cp.async by all threads and a barrier per stage: 318 at 67 %).
+// Bound: the FP64 tensor pipe, 1024 clocks per tile and stage on a scheduler. 98,304 rows x 250 columns: 308 us with the
+// copies made by warp 0 between its products (64 x 64 blocks of m8n8k4 with the stage loaded through registers: 316 at 45 %
+// of the pipe and atomics four times as often; cp.async by all threads and a barrier per stage: 318); with warps for the
+// copies, 100,001 rows: 129 columns 508 -> 224 us, 200: 283 -> 230, 250: 350 -> 313 (every warp copying its row of each
+// stage: 319, 226, 326; one warp for all copies and 96 registers for the others: 352, 232, 317).
 constexpr int GT_KT = 16;
 constexpr int GT_BLK = 128;
 constexpr int GT_LD = GT_BLK + 4;
 constexpr int GT_WARPS = 16;
-constexpr int GT_T = GT_WARPS * 32;
+constexpr int GT_COPY = 4;  // warps that make the copies: a warpgroup, which hands its registers to the others
+constexpr int GT_T = (GT_WARPS + GT_COPY) * 32;
 constexpr int GT_STAGES = 6;
 constexpr int GT_STAGE = 2 * GT_KT * GT_LD;  // doubles
 constexpr size_t GT_SMEM = (size_t)GT_STAGES * GT_STAGE * sizeof(double) + 2 * GT_STAGES * sizeof(uint64_t);
@@ -110,28 +112,34 @@ k_gemm_tn(const double* __restrict__ A, int aCols, int lda, const double* __rest
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
-  // the copies, by warp 0: lane = row of the stage, lanes 0..15 A, lanes 16..31 B
-  const uint32_t wA = (uint32_t)min(GT_BLK, lda - i0) * 8u, wB = diag ? 0u : (uint32_t)min(GT_BLK, ldb - j0) * 8u;
-  const bool isB = lane >= GT_KT;
-  const uint32_t bytes = isB ? wB : wA;
-  const double* src = isB ? B + (size_t)(lane - GT_KT) * ldb + j0 : A + (size_t)lane * lda + i0;
-  const size_t step = (size_t)GT_KT * (isB ? ldb : lda);
-  auto issue = [&](int st) -> bool {
-    if (st >= s1) return true;
-    const int k = st - s0, b = k % GT_STAGES;
-    if (k >= GT_STAGES && !gt_wait(empty + 8 * b, (uint32_t)(k / GT_STAGES - 1) & 1u)) return false;
-    if (lane == 0)
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + 8 * b), "r"((wA + wB) * GT_KT) : "memory");
-    __syncwarp();
-    if (bytes)
-      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                       base + (uint32_t)(b * GT_STAGE + lane * GT_LD) * 8u),
-                   "l"(src + (size_t)st * step), "r"(bytes), "r"(full + 8 * b)
-                   : "memory");
-    return true;
-  };
-  if (warp == 0)
-    for (int i = 0; i < GT_STAGES - 2; i++) issue(s0 + i);
+  // The copies of a stage, 16 rows of A and of B, by four warps of their own that run ahead (a warp takes about as long
+  // for 32 copies as for a tile's products). Registers: 640 threads start with 96; 128 x 24 + 512 x 112 of them remain.
+  if (warp >= GT_WARPS) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+    const int row = (warp - GT_WARPS) * (GT_KT / GT_COPY) + (lane & 3);
+    const bool isB = lane >= GT_KT / GT_COPY;
+    const uint32_t wA = (uint32_t)min(GT_BLK, lda - i0) * 8u, wB = diag ? 0u : (uint32_t)min(GT_BLK, ldb - j0) * 8u;
+    const uint32_t bytes = lane >= 2 * (GT_KT / GT_COPY) ? 0u : isB ? wB : wA;
+    const size_t ld = isB ? ldb : lda;
+    const double* src = (isB ? B + j0 : A + i0) + ((size_t)s0 * GT_KT + row) * ld;
+    const uint32_t dst = base + (uint32_t)(row + (isB ? GT_KT : 0)) * GT_LD * 8u;
+    for (int k = 0; k < s1 - s0; k++, src += GT_KT * ld) {
+      const int b = k % GT_STAGES;
+      if (k >= GT_STAGES && !gt_wait(empty + 8 * b, (uint32_t)(k / GT_STAGES - 1) & 1u)) {
+        if (lane == 0) atomicExch(err, 111);
+        return;
+      }
+      if (warp == GT_WARPS && lane == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + 8 * b), "r"((wA + wB) * GT_KT) : "memory");
+      if (bytes)
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         dst + (uint32_t)(b * GT_STAGE) * 8u),
+                     "l"(src), "r"(bytes), "r"(full + 8 * b)
+                     : "memory");
+    }
+    return;
+  }
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
   if (warp >= nT * split) return;
   const int tile = warp % nT;
   const int kBeg = split == 2 ? warp / nT * 8 : 0, kEnd = split == 2 ? kBeg + 8 : GT_KT;
@@ -156,11 +164,6 @@ k_gemm_tn(const double* __restrict__ A, int aCols, int lda, const double* __rest
     constexpr int J1 = decltype(onDiagonal)::value ? 2 : 0;
     for (int st = s0; st < s1; st++) {
       const int n = st - s0, b = n % GT_STAGES;
-      // four stages ahead, into the buffer of the stage before last: the other warps have long left that one
-      if (warp == 0 && !issue(st + GT_STAGES - 2)) {
-        if (lane == 0) atomicExch(err, 111);
-        return false;
-      }
       if (!gt_wait(full + 8 * b, (uint32_t)(n / GT_STAGES) & 1u)) {
         if (lane == 0) atomicExch(err, 112);
         return false;
