@@ -205,12 +205,12 @@ __global__ void __launch_bounds__(RR_T, 4) k_rest_rmm(const __grid_constant__ Re
 // --------------------------------------------------------------------------------------------------
 constexpr int RL_WARPS = 8;     // two CTAs per SM (three or four, of 80 or 64 registers: 5 to 35 % slower)
 constexpr int RL_T = RL_WARPS * 32;
-constexpr int RL_TASKS = 320;   // columns per CTA of the first kind
+constexpr int RL_TASKS = 320;   // columns per CTA of the first kind, at most
 constexpr int RL_UC = 64;       // columns per CTA of the second
 constexpr int RL_WIN = SKIP_ROWS / WIN_ROWS;
 struct RestLmmArgs {
   const RestTask* tasks;
-  int nTasks, nChunks;       // chunks of RL_TASKS columns; the first nSparse are SDC / RLE columns
+  int nTasks, nChunks, per;  // chunks of per columns; the first nSparse are SDC / RLE columns
   int nSparse;
   int ctaTasks;              // CTAs per chunk
   const double* dense;       // uncompressed group (null: none), its width, chunks of RL_UC columns, CTAs per chunk
@@ -218,7 +218,7 @@ struct RestLmmArgs {
   int gCols, nUncChunks, ctaUnc;
   int nRows, q, nCols;
   const double* Yt;
-  double* partT;             // [nChunks][ctaTasks][RL_TASKS][QT]
+  double* partT;             // [nChunks][ctaTasks][per][QT]
   double* partU;             // [nUncChunks][ctaUnc][RL_UC][QT]
   double* out;
 };
@@ -230,7 +230,7 @@ __device__ __forceinline__ void rest_lmm_tasks(const RestLmmArgs& A, int chunk, 
   double* sums = ws + QT * RL_WIN;                  // [RL_TASKS][QT]
   RestTask* T = (RestTask*)(sums + RL_TASKS * QT);  // [RL_TASKS]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t0 = chunk * RL_TASKS, nt = min(RL_TASKS, A.nTasks - t0), nSparse = max(0, min(nt, A.nSparse - t0));
+  const int t0 = chunk * A.per, nt = min(A.per, A.nTasks - t0), nSparse = max(0, min(nt, A.nSparse - t0));
   for (int i = tid; i < nt; i += RL_T) T[i] = A.tasks[t0 + i];
   for (int i = tid; i < nt * QT; i += RL_T) sums[i] = 0.0;
   const int nBlocks = (A.nRows + SKIP_ROWS - 1) / SKIP_ROWS;
@@ -355,7 +355,7 @@ __device__ __forceinline__ void rest_lmm_tasks(const RestLmmArgs& A, int chunk, 
     }
   }
   __syncthreads();
-  double* o = A.partT + ((size_t)chunk * A.ctaTasks + cta) * RL_TASKS * QT;
+  double* o = A.partT + ((size_t)chunk * A.ctaTasks + cta) * A.per * QT;
   for (int i = tid; i < nt * QT; i += RL_T) o[i] = sums[i];
 }
 
@@ -430,12 +430,12 @@ __global__ void __launch_bounds__(256) k_rest_lmm_final(const __grid_constant__ 
   double s = 0.0;
   int col = -1, i = 0;
   if (e < nT) {
-    const int task = e / QT, chunk = task / RL_TASKS;
+    const int task = e / QT, chunk = task / A.per;
     i = e - task * QT;
     col = A.tasks[task].col;
-    const double* p = A.partT + (size_t)chunk * A.ctaTasks * RL_TASKS * QT + (task - chunk * RL_TASKS) * QT + i;
+    const double* p = A.partT + (size_t)chunk * A.ctaTasks * A.per * QT + (task - chunk * A.per) * QT + i;
 #pragma unroll 4
-    for (int k = sub; k < A.ctaTasks; k += 8) s += __ldcg(p + (size_t)k * RL_TASKS * QT);
+    for (int k = sub; k < A.ctaTasks; k += 8) s += __ldcg(p + (size_t)k * A.per * QT);
   } else if (e < nT + nU) {
     const int c = (e - nT) / QT, chunk = c / RL_UC;
     i = (e - nT) - c * QT;
@@ -624,7 +624,6 @@ int64_t rest_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t
         A.gCols = g.gCols;
       }
       if (A.nTasks == 0 && A.gCols == 0) break;
-      A.nChunks = (A.nTasks + RL_TASKS - 1) / RL_TASKS;
       A.nUncChunks = (A.gCols + RL_UC - 1) / RL_UC;
       A.nRows = m->nRows;
       A.q = qc;
@@ -639,10 +638,15 @@ int64_t rest_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t
       const int nBlocks = (m->nRows + SKIP_ROWS - 1) / SKIP_ROWS;
       const double wT = A.nTasks * 1.0, wU = A.gCols * 4.0;
       int nT = A.nTasks ? (A.gCols ? std::max(1, (int)(slots * wT / (wT + wU))) : slots) : 0;
+      // Few blocks: fewer columns per CTA until the CTAs fill the SMs, one per warp at least (320 always: 6,126 rows x 101
+      // columns of 16-bit maps took 140 us on 6 CTAs, 18 now).
+      const int64_t even = nT ? ((int64_t)A.nTasks * nBlocks + nT - 1) / nT : 0;
+      A.per = (int)std::max<int64_t>(RL_WARPS, std::min<int64_t>(RL_TASKS, (even + RL_WARPS - 1) / RL_WARPS * RL_WARPS));
+      A.nChunks = (A.nTasks + A.per - 1) / A.per;
       A.ctaTasks = A.nTasks ? std::max(1, std::min(nBlocks, nT / A.nChunks)) : 0;
       const int nU = std::max(1, slots - A.ctaTasks * A.nChunks);
       A.ctaUnc = A.gCols ? std::max(1, std::min((m->nRows + 255) / 256, nU / A.nUncChunks)) : 0;
-      const size_t bT = (size_t)A.nChunks * A.ctaTasks * RL_TASKS * QT * 8, bU = (size_t)A.nUncChunks * A.ctaUnc * RL_UC * QT * 8;
+      const size_t bT = (size_t)A.nChunks * A.ctaTasks * A.per * QT * 8, bU = (size_t)A.nUncChunks * A.ctaUnc * RL_UC * QT * 8;
       if ((rc = ensure_scratch(m, bT + bU + 256)) < 0) return rc;
       A.partT = (double*)m->scratch;
       A.partU = (double*)((char*)m->scratch + bT);
