@@ -260,12 +260,12 @@ static int64_t decompress_chunk(Matrix* m, int r0, int r1, double* X, int ld, cu
   return launch_decompress_range(m, r0, r1, X, s, (size_t)ld);
 }
 
-// Rows of a decompressed chunk: enough that the partial sums every CTA adds to the result at its end do not count, little
-// enough not to matter in 180 GB (200,000 x 250 mixed: 616 us with 192 MB, 603 with 512).
+// Rows of a decompressed chunk, about 192 MB in even parts: enough that the partial sums every CTA adds to the result at its
+// end do not count (200,000 x 250 mixed: 616 us with 192 MB and a third chunk for the last 3,392 rows, 600 with 512 MB),
+// little enough that the first call's allocation does not (512 MB: 0.9 ms more there).
 static int64_t chunk_rows(int64_t nRows, int64_t cols) {
-  int64_t chunk = (512ll << 20) / (cols * 8);
-  chunk = std::max<int64_t>(SKIP_ROWS, (chunk / SKIP_ROWS) * SKIP_ROWS);
-  return std::min<int64_t>(chunk, (nRows + SKIP_ROWS - 1) / SKIP_ROWS * SKIP_ROWS);
+  const int64_t parts = std::max<int64_t>(1, (nRows * cols * 8 + (96ll << 20)) / (192ll << 20));
+  return std::max<int64_t>(SKIP_ROWS, ((nRows + parts - 1) / parts + SKIP_ROWS - 1) / SKIP_ROWS * SKIP_ROWS);
 }
 
 // --------------------------------------------------------------------------------------------------
