@@ -59,7 +59,7 @@ DESCS = {
 }
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the dominant kernel, per matrix row, from ncu captures of
 # scaled-down cases (traffic grows in proportion to the rows); None = not captured
-TRAFFIC_PER_ROW = {0: 134.6, 1: 223.45, 2: 1846.0, 3: 202.95, 4: 2170.5}
+TRAFFIC_PER_ROW = {0: 64.7, 1: 219.4, 2: 1287.1, 3: 202.7, 4: 2171.5}
 
 
 def measured_peaks():
