@@ -183,12 +183,13 @@ struct RestTask {
   const double* src;   // dictionary + position of the column
   const void* a;       // SDC: items; RLE: runs; dense map: map
   const void* b;       // SDC: skip entries; RLE: first run of every block; dense map: high bytes
-  int64_t n;           // SDC: listed rows; RLE: runs
+  int64_t n;           // SDC: listed rows; RLE: runs; dense map: tuples
   int32_t kind, mapType, stride, col;
 };
 struct RestPlan {
   bool tried = false, ok = false;
   int nTasks = 0, nUnc = 0, nDense = 0;
+  int nTable = 0, tableVals = 0;  // 16-bit map columns whose tables fit shared memory (the last tasks), longest table
   RestTask* tasks = nullptr;      // SDC, RLE and remaining dense-map columns
   ColRef* dense = nullptr;        // the remaining dense-map columns, list order
   std::vector<int> unc;           // device group indices of the uncompressed groups

@@ -455,6 +455,95 @@ __global__ void __launch_bounds__(256) k_rest_lmm_final(const __grid_constant__ 
 // --------------------------------------------------------------------------------------------------
 // plan and launchers
 // --------------------------------------------------------------------------------------------------
+// --------------------------------------------------------------------------------------------------
+// Yt X over 16-bit maps from TL_ROWS rows on: a CTA keeps the tables of up to sixteen columns in shared memory and walks a
+// range of rows, a warp (or several, where long tables leave fewer columns) per column, lanes along the rows.
+// Bound: the L1 / shared data pipe. Per 32 cells two 128-byte accesses for the left values, one for the ids and about six for
+// random 8-byte reads of the table; from global memory, as the blockwise kernel reads them, each such read goes to its own
+// line. 1,000,003 rows x 300 columns of 500 tuples, one left row: 2393 -> 360 us; 27,362 x 391, eight: 511 -> 59.
+// --------------------------------------------------------------------------------------------------
+constexpr int TL_WARPS = 16;
+constexpr int TL_SMEM = 200 * 1024;
+constexpr int TL_VALS = TL_SMEM / 8 / 4;  // tuples of a table, at most: four columns per CTA
+constexpr int TL_ROWS = 16384;            // fewer rows: filling the tables is most of the time
+struct TableLmmArgs {
+  const RestTask* tasks;
+  int n, vals, C, parts;  // columns, longest table, columns per CTA, row ranges
+  int nRows, q, nCols;
+  const double* Yt;
+  double* part;  // [parts][n][QT]
+  double* out;
+};
+template <int QT>
+__global__ void __launch_bounds__(TL_WARPS * 32, 1) k_table_lmm(const __grid_constant__ TableLmmArgs A) {
+  extern __shared__ __align__(16) double tlsm[];  // [C][vals]
+  __shared__ double red[TL_WARPS][QT];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int chunk = blockIdx.x / A.parts, p = blockIdx.x - chunk * A.parts;
+  const int t0 = chunk * A.C, nt = min(A.C, A.n - t0), W = TL_WARPS / A.C, c = warp / W, sub = warp - c * W;
+  for (int k = 0; k < nt; k++) {
+    const RestTask& T = A.tasks[t0 + k];
+    for (int v = tid; v < (int)T.n; v += TL_WARPS * 32) tlsm[k * A.vals + v] = T.src[(size_t)v * T.stride];
+  }
+  __syncthreads();
+  double acc[QT];
+#pragma unroll
+  for (int i = 0; i < QT; i++) acc[i] = 0.0;
+  if (c < nt) {
+    const uint16_t* map = (const uint16_t*)A.tasks[t0 + c].a;
+    const double* tab = tlsm + c * A.vals;
+    const int r0 = (int)((int64_t)A.nRows * p / A.parts), r1 = (int)((int64_t)A.nRows * (p + 1) / A.parts);
+    constexpr int U = QT == 1 ? 8 : 4;
+    const double* y[QT];
+#pragma unroll
+    for (int i = 0; i < QT; i++) y[i] = A.Yt + (size_t)min(i, A.q - 1) * A.nRows;
+    int r = r0 + sub * 32 * U + lane;
+    for (; r - lane + 32 * U <= r1; r += W * 32 * U) {
+      uint32_t id[U];
+      double l[U][QT];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        id[u] = __ldg(map + r + 32 * u);
+#pragma unroll
+        for (int i = 0; i < QT; i++) l[u][i] = __ldg(y[i] + r + 32 * u);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const double x = tab[id[u]];
+#pragma unroll
+        for (int i = 0; i < QT; i++) acc[i] = fma(x, l[u][i], acc[i]);
+      }
+    }
+    for (int u = 0; u < U; u++, r += 32)  // the range's last rows (one warp of the column has some)
+      if (r < r1) {
+        const double x = tab[__ldg(map + r)];
+#pragma unroll
+        for (int i = 0; i < QT; i++) acc[i] = fma(x, __ldg(y[i] + r), acc[i]);
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < QT; i++) {
+    for (int d = 16; d; d >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], d);
+    if (lane == 0) red[warp][i] = acc[i];
+  }
+  __syncthreads();
+  if (c < nt && sub == 0 && lane < QT) {
+    double s = 0.0;
+    for (int k = 0; k < W; k++) s += red[warp + k][lane];
+    A.part[((size_t)p * A.n + t0 + c) * QT + lane] = s;
+  }
+}
+template <int QT>
+__global__ void __launch_bounds__(256) k_table_lmm_final(const __grid_constant__ TableLmmArgs A) {
+  const int lane = threadIdx.x & 31, e = blockIdx.x * 8 + (threadIdx.x >> 5);  // a warp per sum
+  if (e >= A.n * QT) return;
+  double s = 0.0;
+  for (int p = lane; p < A.parts; p += 32) s += A.part[(size_t)p * A.n * QT + e];
+  for (int d = 16; d; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+  const int task = e / QT, i = e - task * QT;
+  if (lane == 0 && i < A.q) atomicAdd(&A.out[(size_t)i * A.nCols + A.tasks[task].col], s);  // (several groups may hold a column)
+}
+
 static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
   RestPlan& R = m->rest;
   if (R.tried) return CLA_OK;
@@ -462,7 +551,7 @@ static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
   int64_t rc;
   if ((rc = ensure_row_lists(m, s)) < 0) return rc;
   if (!m->rows.ok) return CLA_OK;
-  std::vector<RestTask> sdc, rle, ddc;
+  std::vector<RestTask> sdc, rle, ddc, table;
   std::vector<ColRef> dense;
   for (size_t hi = 0; hi < m->hg.size(); hi++) {
     const int gi = m->regToDev[hi];
@@ -492,7 +581,12 @@ static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
       } else {
         t.a = g.map;
         t.b = g.mapHi;
-        ddc.push_back(t);
+        t.n = g.nVals;
+        if (g.mapType == CLA_MAP_CHAR && g.nVals <= TL_VALS) {
+          table.push_back(t);
+          R.tableVals = std::max(R.tableVals, g.nVals);
+        } else
+          ddc.push_back(t);
         dense.push_back(ColRef{g.map, g.mapHi, g.dict + j, GT_DDC, g.mapType, g.gCols, t.col, gi, 0});
       }
     }
@@ -500,6 +594,8 @@ static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
   std::vector<RestTask> all(sdc);
   all.insert(all.end(), rle.begin(), rle.end());
   all.insert(all.end(), ddc.begin(), ddc.end());
+  all.insert(all.end(), table.begin(), table.end());
+  R.nTable = (int)table.size();
   R.nTasks = (int)all.size();
   R.nDense = (int)dense.size();
   R.nUnc = (int)R.unc.size();
@@ -604,18 +700,58 @@ static int64_t rest_lmm_go(Matrix* m, RestLmmArgs& A, int grid, size_t smem, cud
   return CLA_OK;
 }
 
+template <int QT>
+static int64_t table_lmm_go(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s) {
+  static bool attrSet[64] = {};  // per device
+  if (!attrSet[m->device & 63]) {
+    CLA_CUDA(cudaFuncSetAttribute(k_table_lmm<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TL_SMEM));
+    attrSet[m->device & 63] = true;
+  }
+  const RestPlan& R = m->rest;
+  TableLmmArgs A{};
+  A.tasks = R.tasks + (R.nTasks - R.nTable);
+  A.n = R.nTable;
+  A.vals = R.tableVals;
+  for (A.C = TL_WARPS; A.C * A.vals * 8 > TL_SMEM; A.C /= 2) {
+  }
+  A.nRows = m->nRows;
+  A.q = q;
+  A.nCols = m->nCols;
+  const int chunks = (A.n + A.C - 1) / A.C;
+  A.parts = std::max(1, m->smCount / chunks);
+  A.Yt = dYt;
+  A.out = dOut;
+  int64_t rc;
+  if ((rc = ensure_scratch(m, (size_t)A.parts * A.n * QT * 8 + 256)) < 0) return rc;
+  A.part = (double*)m->scratch;
+  k_table_lmm<QT><<<chunks * A.parts, TL_WARPS * 32, (size_t)A.C * A.vals * 8, s>>>(A);
+  k_table_lmm_final<QT><<<(A.n * QT + 7) / 8, 256, 0, s>>>(A);
+  m->stats.kernel_launches += 2;
+  return CLA_OK;
+}
+
 // Adds the remaining groups' part of Yt X to dOut (which holds the specialised kernels' part, or zeros and constants).
 int64_t rest_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s) {
   int64_t rc;
   if ((rc = ensure_rest(m, s)) < 0) return rc;
   const RestPlan& R = m->rest;
   if (!R.ok) return 0;
+  const bool table = R.nTable > 0 && m->nRows >= TL_ROWS;
+  const int nTasks = R.nTasks - (table ? R.nTable : 0);
   for (int q0 = 0; q0 < q;) {
     const int left = q - q0, QT = left >= 5 ? 8 : (left >= 2 ? 4 : 1), qc = std::min(QT, left);
+    if (table) {
+      const double* y = dYt + (size_t)q0 * m->nRows;
+      double* o = dOut + (size_t)q0 * m->nCols;
+      if (nTasks == 0 && R.nUnc == 0) prof_begin(m, s);
+      rc = QT == 8 ? table_lmm_go<8>(m, y, qc, o, s) : (QT == 4 ? table_lmm_go<4>(m, y, qc, o, s) : table_lmm_go<1>(m, y, qc, o, s));
+      if (rc < 0) return rc;
+      if (nTasks == 0 && R.nUnc == 0) prof_end(m, s);
+    }
     for (int u = 0; u == 0 || u < R.nUnc; u++) {  // one uncompressed group per launch; the first takes the other groups too
       RestLmmArgs A{};
       A.tasks = R.tasks;
-      A.nTasks = u == 0 ? R.nTasks : 0;
+      A.nTasks = u == 0 ? nTasks : 0;
       A.nSparse = R.nTasks - R.nDense;
       if (u < R.nUnc) {
         const DevGroup& g = m->groups[R.unc[u]];
