@@ -474,6 +474,65 @@ struct TableLmmArgs {
   double* part;  // [parts][n][QT]
   double* out;
 };
+// X v over the same columns, where the rows of an SM outnumber half the longest table (every SM fills every table: 65,537 rows
+// x 300 columns of 2,000 tuples took 654 us) and from TL_XROWS rows on: a CTA owns a range of rows, lane = row, and takes the columns in turns,
+// the tables D v of up to sixteen in shared memory; a row's sum waits in the result between the turns. Per 32 cells one
+// 128-byte access for the ids and about six for the lookups. 1,000,003 x 300 columns of 500 tuples: 1618 -> 480 us.
+constexpr int TL_XROWS = 65536;  // 443 rows per SM, a step of nearly every warp
+struct TableRmmArgs {
+  const RestTask* tasks;
+  int n, vals, C, nRows, nCols, addTo;
+  const double *v, *constV, *rowScale;
+  double* out;
+};
+__global__ void __launch_bounds__(TL_WARPS * 32, 1) k_table_rmm(const __grid_constant__ TableRmmArgs A) {
+  extern __shared__ __align__(16) double tlsm[];  // [C][vals]
+  __shared__ const uint16_t* maps[TL_WARPS];
+  __shared__ double cred[TL_WARPS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, W = TL_WARPS / A.C;
+  const int nSteps = (A.nRows + 31) / 32;
+  const int s0 = (int)((int64_t)nSteps * blockIdx.x / gridDim.x), s1 = (int)((int64_t)nSteps * (blockIdx.x + 1) / gridDim.x);
+  double c0 = 0.0;
+  if (A.constV) {
+    for (int c = tid; c < A.nCols; c += TL_WARPS * 32) c0 = fma(A.constV[c], A.v[c], c0);
+    for (int d = 16; d; d >>= 1) c0 += __shfl_xor_sync(0xffffffffu, c0, d);
+    if (lane == 0) cred[warp] = c0;
+    __syncthreads();
+    c0 = 0.0;
+    for (int w = 0; w < TL_WARPS; w++) c0 += cred[w];
+  }
+  for (int k0 = 0; k0 < A.n; k0 += A.C) {
+    const int nt = min(A.C, A.n - k0), k = warp / W;
+    __syncthreads();  // the previous tables' readers are done
+    if (k < nt) {
+      const RestTask& T = A.tasks[k0 + k];
+      const double x = A.v[T.col];
+      if (lane == 0) maps[k] = (const uint16_t*)T.a;
+      const int n = (int)T.n, stride = T.stride;
+      const double* src = T.src;
+#pragma unroll 8
+      for (int i = (warp - k * W) * 32 + lane; i < n; i += W * 32) tlsm[k * A.vals + i] = src[(size_t)i * stride] * x;
+    }
+    __syncthreads();
+    const bool last = k0 + A.C >= A.n;
+    for (int st = s0 + warp; st < s1; st += TL_WARPS) {
+      const int r = min(st * 32 + lane, A.nRows - 1);
+      double acc = (k0 || A.addTo) ? A.out[r] : c0;
+      int c = 0;
+      for (; c + 8 <= nt; c += 8) {
+        uint32_t id[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) id[u] = __ldg(maps[c + u] + r);
+#pragma unroll
+        for (int u = 0; u < 8; u++) acc += tlsm[(c + u) * A.vals + id[u]];
+      }
+      for (; c < nt; c++) acc += tlsm[c * A.vals + __ldg(maps[c] + r)];
+      if (last && A.rowScale) acc *= A.rowScale[r];
+      if (st * 32 + lane < A.nRows) A.out[r] = acc;
+    }
+  }
+}
+
 template <int QT>
 __global__ void __launch_bounds__(TL_WARPS * 32, 1) k_table_lmm(const __grid_constant__ TableLmmArgs A) {
   extern __shared__ __align__(16) double tlsm[];  // [C][vals]
@@ -552,7 +611,7 @@ static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
   if ((rc = ensure_row_lists(m, s)) < 0) return rc;
   if (!m->rows.ok) return CLA_OK;
   std::vector<RestTask> sdc, rle, ddc, table;
-  std::vector<ColRef> dense;
+  std::vector<ColRef> dense, denseTable;
   for (size_t hi = 0; hi < m->hg.size(); hi++) {
     const int gi = m->regToDev[hi];
     if (gi < 0) continue;
@@ -582,12 +641,10 @@ static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
         t.a = g.map;
         t.b = g.mapHi;
         t.n = g.nVals;
-        if (g.mapType == CLA_MAP_CHAR && g.nVals <= TL_VALS) {
-          table.push_back(t);
-          R.tableVals = std::max(R.tableVals, g.nVals);
-        } else
-          ddc.push_back(t);
-        dense.push_back(ColRef{g.map, g.mapHi, g.dict + j, GT_DDC, g.mapType, g.gCols, t.col, gi, 0});
+        const bool tab = g.mapType == CLA_MAP_CHAR && g.nVals <= TL_VALS;
+        (tab ? table : ddc).push_back(t);
+        if (tab) R.tableVals = std::max(R.tableVals, g.nVals);
+        (tab ? denseTable : dense).push_back(ColRef{g.map, g.mapHi, g.dict + j, GT_DDC, g.mapType, g.gCols, t.col, gi, 0});
       }
     }
   }
@@ -596,6 +653,7 @@ static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
   all.insert(all.end(), ddc.begin(), ddc.end());
   all.insert(all.end(), table.begin(), table.end());
   R.nTable = (int)table.size();
+  dense.insert(dense.end(), denseTable.begin(), denseTable.end());
   R.nTasks = (int)all.size();
   R.nDense = (int)dense.size();
   R.nUnc = (int)R.unc.size();
@@ -614,6 +672,32 @@ static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
   return CLA_OK;
 }
 
+static int64_t table_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s, bool addTo) {
+  static bool attrSet[64] = {};  // per device
+  if (!attrSet[m->device & 63]) {
+    CLA_CUDA(cudaFuncSetAttribute(k_table_rmm, cudaFuncAttributeMaxDynamicSharedMemorySize, TL_SMEM));
+    attrSet[m->device & 63] = true;
+  }
+  const RestPlan& R = m->rest;
+  TableRmmArgs A{};
+  A.tasks = R.tasks + (R.nTasks - R.nTable);
+  A.n = R.nTable;
+  A.vals = R.tableVals;
+  for (A.C = TL_WARPS; A.C * A.vals * 8 > TL_SMEM; A.C /= 2) {
+  }
+  A.nRows = m->nRows;
+  A.nCols = m->nCols;
+  A.addTo = addTo ? 1 : 0;
+  A.v = dV;
+  A.constV = (!addTo && m->hasConst) ? m->dConstV : nullptr;
+  A.rowScale = dW;
+  A.out = dOut;
+  k_table_rmm<<<m->smCount, TL_WARPS * 32, (size_t)A.C * A.vals * 8, s>>>(A);
+  m->stats.kernel_launches++;
+  CLA_CUDA(cudaGetLastError());
+  return CLA_OK;
+}
+
 // addTo: dOut holds the specialised kernels' part (constants included)
 int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s, bool addTo) {
   int64_t rc;
@@ -621,6 +705,15 @@ int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cu
   const RestPlan& R = m->rest;
   const RowLists& L = m->rows;
   if (!R.ok) return 0;
+  const bool table = R.nTable > 0 && m->nRows >= TL_XROWS && (int64_t)m->nRows * 2 >= (int64_t)m->smCount * R.tableVals;
+  if (table) {
+    const bool all = R.nDense == R.nTable && R.nUnc == 0 && !L.nSdc && !L.nRle;
+    if (all) prof_begin(m, s);
+    if ((rc = table_rmm(m, dV, dOut, all ? dW : nullptr, s, addTo)) < 0) return rc;
+    if (all) prof_end(m, s);
+    if (all) return 1;
+    addTo = true;
+  }
   RestRmmArgs A{};
   A.sv = L.sv;
   A.svOff = L.svOff;
@@ -628,7 +721,7 @@ int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cu
   A.nSv = (L.nSdc || L.nRle) ? (int)L.nSv : 0;
   A.nRows = m->nRows;
   A.nCols = m->nCols;
-  A.nDense = R.nDense;
+  A.nDense = R.nDense - (table ? R.nTable : 0);
   A.dense = R.dense;
   A.rowPtr = L.nSdc ? L.rowPtr : nullptr;
   A.rowItems = L.rowItems;

@@ -159,10 +159,10 @@ def test_wide_right_operand(nRows, kinds):
     cmb.free()
 
 
-@pytest.mark.parametrize("nRows", [16384, 17001])
+@pytest.mark.parametrize("nRows", [16384, 17001, 74003, 120001])
 @pytest.mark.parametrize("longest", [257, 1601, 6400, 6401])
-def test_left_product_with_tables_of_16_bit_maps(nRows, longest):
+def test_products_with_tables_of_16_bit_maps(nRows, longest):
     """Sixteen, eight and four columns per CTA, a table that stays in global memory, co-coded and constant columns."""
     cmb = _ddc(nRows, [300, 1000, 257] * 6 + [longest, 9], longest, const=True, width=2 if longest == 1601 else 1).to_device()
-    _check(cmb, ks=(1,), qs=(1, 2, 5, 9), chain=False)
+    _check(cmb, ks=(1,), qs=(1, 2, 5, 9))
     cmb.free()
