@@ -104,6 +104,11 @@ int64_t cla_stats_get(cla_handle h, cla_stats* out);
  * product call brackets its dominant kernel with CUDA events on the launching stream; cla_stats_get
  * synchronises those events and adds them to main_kernel_ms / main_kernel_count. */
 int64_t cla_set_profile(cla_handle h, int32_t on);
+/* Device memory the handle may take for the plans its products build on first use (row lists, column records, tables
+ * laid out for a kernel); negative: no limit, the default. A plan that does not fit, here or on the device, is not built
+ * and not tried again: the products then take kernels that work on the registered arrays alone, with results within the
+ * same tolerance. Plans that exist already stay. */
+int64_t cla_set_plan_limit(cla_handle h, int64_t bytes);
 /* Diagnostics: sustained TFLOP/s of back-to-back FP64 tensor-core instructions (DMMA m8n8k4) and of FP64 FMA on
  * `device`, the denominators of the tensor-pipe and FMA fractions reported for the kernels. About 0.1 s. */
 int64_t cla_measure_fp64_peaks(int32_t device, double* dmmaTflops, double* dfmaTflops);

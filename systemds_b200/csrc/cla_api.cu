@@ -174,6 +174,12 @@ int64_t cla_set_profile(cla_handle h, int32_t on) {
   return CLA_OK;
 }
 
+int64_t cla_set_plan_limit(cla_handle h, int64_t bytes) {
+  GET_MATRIX(h);
+  m->planLimit = bytes < 0 ? -1 : bytes;
+  return CLA_OK;
+}
+
 static int64_t add_dict_group(Matrix* m, HostGroup& g, int type, const int32_t* colIdx, int32_t gCols,
                               const double* dict, int32_t nVals) {
   int64_t rc = check_cols(m, colIdx, gCols);
@@ -598,7 +604,8 @@ enum HostDirect {
 
 static int small_direct(Matrix* m, size_t vCells) {
   if (!small_block(m)) return HD_NONE;
-  if (cudaSetDevice(m->device) != cudaSuccess || ensure_col_plan(m) < 0 || ensure_row_lists(m, m->stream) < 0 || !m->rows.ok) return HD_NONE;
+  if (cudaSetDevice(m->device) != cudaSuccess || ensure_col_plan(m) < 0 || ensure_row_lists(m, m->stream) < 0 || !m->cols.ok || !m->rows.ok)
+    return HD_NONE;
   // every CTA of the right product reads V once over the bus: worth it while that is less than a copy's latency
   const bool in = vCells != SIZE_MAX && vCells * 8 * ((m->nRows + 31) / 32) <= 128 * 1024;
   return in ? HD_OUT | HD_IN : HD_OUT;

@@ -201,7 +201,7 @@ struct DecPlan {  // column-per-lane decompress (cla_generic.cu)
   size_t smem = 0;
 };
 struct ColPlan {
-  bool built = false;
+  bool tried = false, ok = false;
   int nDense = 0, nRefs = 0;
   ColRef* dense = nullptr;     // dense-map and uncompressed columns, list order
   ColRef* refs = nullptr;      // every column of every group, sorted by matrix column (list order within a column)
@@ -264,6 +264,7 @@ struct Matrix {
   bool hasConst = false;
   std::vector<void*> allocs;     // everything cudaMalloc'ed for the groups
   int64_t deviceBytes = 0, indexBytes = 0;
+  int64_t planBytes = 0, planLimit = -1;  // plans built on first use: bytes held, bytes allowed (-1: no limit)
   // growable scratch (value arenas, partial results, host staging)
   void* scratch = nullptr;
   size_t scratchBytes = 0;
@@ -335,12 +336,15 @@ int64_t device_to_host_staged(Matrix* m, void* host, const void* dSrc, size_t by
 void host_stage_free(Matrix* m);
 int64_t ensure_sparse_list(Matrix* m);  // Matrix::dSparseIdx (cla_generic.cu)
 
-int64_t ensure_col_plan(Matrix* m);                        // Matrix::cols
+int64_t ensure_col_plan(Matrix* m);                        // Matrix::cols; cols.ok tells whether it exists
 int64_t ensure_row_lists(Matrix* m, cudaStream_t s);       // Matrix::rows; rows.ok tells whether they exist
 // The groups the specialised kernels leave (cla_rest.cu): 1 = done, 0 = not covered (the general kernels then run)
 int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s, bool addTo);
 int64_t rest_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s);
-int64_t plan_alloc(Matrix* m, void** p, size_t bytes);
+// Device memory of a plan built on first use, kept until the handle goes. CLA_ERR_NOMEM where the device or the handle's
+// limit has no room: the product then takes the kernels that need no plan. `needed`: no kernel does without it, no limit.
+int64_t plan_alloc(Matrix* m, void** p, size_t bytes, bool needed = false);
+void plan_release(Matrix* m, void* p, size_t bytes);  // gives one back early; no stream may still use it
 int64_t wide_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStream_t s);  // cla_wide.cu: 1 = done, 0 = not covered
 void wide_plan_free(Matrix* m);
 // Short blocks (cla_small.cu): one kernel per product, every group type. 1 = done, 0 = not covered

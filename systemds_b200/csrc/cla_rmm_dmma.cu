@@ -1,5 +1,5 @@
 // X %*% V on any mix of groups, on the FP64 tensor cores: the always available form, for blocks whose row lists
-// (cla_rows.cu) do not exist because they would not fit 32-bit positions or device memory (cla_wide.cu otherwise).
+// or plan (cla_rows.cu, cla_wide.cu) do not exist: 32-bit positions, device memory or the handle's plan limit have no room.
 //
 // With many right-hand columns the per-row gather-add of the general tile kernel is bound by FP64 adds and
 // L1 traffic, not by HBM. Here a CTA owns 128 rows x 64 output columns and
@@ -208,7 +208,7 @@ static int64_t ensure_dense_cols(Matrix* m) {
     for (int j = 0; j < m->groups[gi].gCols; j++) dc.push_back(DenseCol{gi, j, m->hg[hi].cols[j], 0});
   }
   if (!dc.empty()) {
-    int64_t rc = plan_alloc(m, &m->dDenseCols, dc.size() * sizeof(DenseCol));
+    int64_t rc = plan_alloc(m, &m->dDenseCols, dc.size() * sizeof(DenseCol), true);
     if (rc < 0) return rc;
     CLA_CUDA(cudaMemcpy(m->dDenseCols, dc.data(), dc.size() * sizeof(DenseCol), cudaMemcpyHostToDevice));
   }

@@ -24,22 +24,33 @@ namespace cla {
 constexpr int RL_WIN = SKIP_ROWS / WIN_ROWS;  // windows per block
 constexpr int RL_THREADS = 256;
 
-int64_t plan_alloc(Matrix* m, void** p, size_t bytes) {
+int64_t plan_alloc(Matrix* m, void** p, size_t bytes, bool needed) {
   *p = nullptr;
+  if (!needed && m->planLimit >= 0 && m->planBytes + (int64_t)bytes > m->planLimit)
+    return fail(CLA_ERR_NOMEM, "the handle's plan limit has no room for " + std::to_string(bytes) + " bytes");
   cudaError_t e = dev_malloc(m, p, std::max<size_t>(bytes, 16));
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(CLA_ERR_NOMEM, std::string("cudaMalloc row plan: ") + cudaGetErrorString(e));
   }
   m->allocs.push_back(*p);
+  if (!needed) m->planBytes += (int64_t)bytes;
   m->deviceBytes += (int64_t)bytes;
   m->stats.device_bytes = m->deviceBytes;
   return CLA_OK;
 }
+void plan_release(Matrix* m, void* p, size_t bytes) {
+  m->allocs.erase(std::remove(m->allocs.begin(), m->allocs.end(), p), m->allocs.end());
+  dev_free(m, p);
+  m->planBytes -= (int64_t)bytes;
+  m->deviceBytes -= (int64_t)bytes;
+  m->stats.device_bytes = m->deviceBytes;
+}
 
 int64_t ensure_col_plan(Matrix* m) {
   ColPlan& cp = m->cols;
-  if (cp.built) return CLA_OK;
+  if (cp.tried) return CLA_OK;
+  cp.tried = true;
   std::vector<ColRef> dense, all;
   for (size_t hi = 0; hi < m->hg.size(); hi++) {
     const int gi = m->regToDev[hi];
@@ -71,15 +82,14 @@ int64_t ensure_col_plan(Matrix* m) {
   if (ba) memcpy(blob.data() + bd, all.data(), ba);
   memcpy(blob.data() + bd + ba, ptr.data(), bp);
   void* d = nullptr;
-  int64_t rc = plan_alloc(m, &d, blob.size());
-  if (rc < 0) return rc;
+  if (plan_alloc(m, &d, blob.size()) < 0) return CLA_OK;
   CLA_CUDA(cudaMemcpy(d, blob.data(), blob.size(), cudaMemcpyHostToDevice));
   cp.dense = (ColRef*)d;
   cp.refs = (ColRef*)((char*)d + bd);
   cp.refPtr = (int32_t*)((char*)d + bd + ba);
   cp.nDense = (int)dense.size();
   cp.nRefs = (int)all.size();
-  cp.built = true;
+  cp.ok = true;
   return CLA_OK;
 }
 
@@ -234,7 +244,8 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   cub::DeviceScan::ExclusiveSum(nullptr, tb2, (uint32_t*)nullptr, (uint32_t*)nullptr, (int)nWinPtr, s);
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   void* base = nullptr;
-  if (plan_alloc(m, &base, al(bBase) + al(bOff) + al(bList) + al(bSv) + al(bRow) + 2 * al(bWin) + std::max(tb1, tb2)) < 0) return CLA_OK;
+  const size_t bytes = al(bBase) + al(bOff) + al(bList) + al(bSv) + al(bRow) + 2 * al(bWin) + std::max(tb1, tb2);
+  if (plan_alloc(m, &base, bytes) < 0) return CLA_OK;
   char* p = (char*)base;
   L.svOff = (int32_t*)p; p += al(bOff);
   int64_t* dBase = (int64_t*)p; p += al(bBase);
@@ -270,7 +281,11 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   CLA_CUDA(cudaStreamSynchronize(s));
   void* items = nullptr;
   const size_t i0 = al((size_t)tot[0] * 4), i1 = al((size_t)tot[1] * 4), i2 = al((size_t)tot[2] * 8);
-  if (plan_alloc(m, &items, 2 * i0 + i1 + i2) < 0) return CLA_OK;
+  if (plan_alloc(m, &items, 2 * i0 + i1 + i2) < 0) {
+    plan_release(m, base, bytes);
+    L.svOff = nullptr, L.sv = nullptr, L.rowPtr = L.fullPtr = L.partPtr = nullptr;
+    return CLA_OK;
+  }
   L.sdcItems = (uint32_t*)((char*)items + i0 + i1 + i2);
   L.rowItems = (uint32_t*)items;
   L.fullItems = (uint32_t*)((char*)items + i0);

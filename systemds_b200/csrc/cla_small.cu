@@ -307,7 +307,7 @@ int64_t small_rmm(Matrix* m, const double* dV, int vCols, double* dOut, const do
   int64_t rc;
   if ((rc = ensure_col_plan(m)) < 0 || (rc = ensure_row_lists(m, s)) < 0) return rc;
   const RowLists& L = m->rows;
-  if (!L.ok) return 0;
+  if (!m->cols.ok || !L.ok) return 0;
   const int KT = vCols == 1 ? 1 : (vCols <= 4 ? 4 : 8);
   const bool vShared = (int64_t)m->nCols * KT <= SR_VMAX;
   const int warps = KT == 1 ? SmallRmm<1>::WARPS : SmallRmm<8>::WARPS;
@@ -353,6 +353,7 @@ int64_t small_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_
   if (!small_block(m) || q <= 0) return 0;
   int64_t rc;
   if ((rc = ensure_col_plan(m)) < 0) return rc;
+  if (!m->cols.ok) return 0;
   const int QT = q == 1 ? 1 : 4;
   const dim3 grid((m->nCols + SL_WARPS / SL_WPC - 1) / (SL_WARPS / SL_WPC), (q + QT - 1) / QT);
   auto kern = QT == 1 ? k_small_lmm<1> : k_small_lmm<4>;

@@ -71,7 +71,7 @@ struct WideSv {
   uint32_t pad;
 };
 struct WidePlanNT {
-  bool built = false;
+  bool tried = false, ok = false;
   int nSp = 0;                // rows of V kept for the SDC / RLE columns in the first chunk's CTAs; 0: tables P instead
   int32_t* spCols = nullptr;  // [nSp] matrix columns
   WideSv* sv = nullptr;       // [sparse table rows]
@@ -470,10 +470,10 @@ void wide_plan_free(Matrix* m) {
 
 static int64_t ensure_wide(Matrix* m, int NT, cudaStream_t s) {
   if (!m->wide) m->wide = new WidePlan();
-  WidePlanNT& W = m->wide->nt[NT];
-  if (W.built) return CLA_OK;
-  int64_t rc;
-  if ((rc = ensure_col_plan(m)) < 0) return rc;
+  if (m->wide->nt[NT].tried) return CLA_OK;
+  m->wide->nt[NT].tried = true;
+  WidePlanNT W;  // takes its place in the handle when it is complete
+  W.tried = true;
   std::vector<WideCol> kind[4];
   for (size_t hi = 0; hi < m->hg.size(); hi++) {
     const int gi = m->regToDev[hi];
@@ -588,7 +588,7 @@ static int64_t ensure_wide(Matrix* m, int NT, cudaStream_t s) {
   const size_t bc = (cols.size() * sizeof(WideCol) + 255) & ~(size_t)255;
   const size_t bi = ((size_t)img * 8 + 255) & ~(size_t)255, bs = ((size_t)W.nSp * 4 + 255) & ~(size_t)255;
   const size_t bl = ((size_t)m->nCols * 4 + 255) & ~(size_t)255, bv = W.nSp ? (size_t)m->rows.nSv * sizeof(WideSv) : 0;
-  if ((rc = plan_alloc(m, &d, bc + bi + bs + bl + bv)) < 0) return rc;
+  if (plan_alloc(m, &d, bc + bi + bs + bl + bv) < 0) return CLA_OK;
   W.spCols = (int32_t*)((char*)d + bc + bi);
   W.sv = (WideSv*)((char*)d + bc + bi + bs + bl);
   if (W.nSp) {
@@ -604,11 +604,12 @@ static int64_t ensure_wide(Matrix* m, int NT, cudaStream_t s) {
   if (!cols.empty()) k_wide_image<<<(unsigned)cols.size(), 128, 0, s>>>(W.cols, (int)cols.size(), W.image);
   CLA_CUDA(cudaGetLastError());
   CLA_CUDA(cudaStreamSynchronize(s));
-  W.built = true;
+  W.ok = true;
+  m->wide->nt[NT] = std::move(W);
   return CLA_OK;
 }
 
-// 1 = done, 0 = not covered (no row lists: the caller takes the general kernel)
+// 1 = done, 0 = not covered (no row lists or no plan: the caller takes the general kernel)
 int64_t wide_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStream_t s) {
   if (m->nRows == 0 || vCols == 0) return 1;
   int64_t rc;
@@ -618,6 +619,7 @@ int64_t wide_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStrea
   const int slices = (vCols + 31) / 32, NT = ((vCols + slices - 1) / slices + 7) / 8;
   if ((rc = ensure_wide(m, NT, s)) < 0) return rc;
   const WidePlanNT& W = m->wide->nt[NT];
+  if (!W.ok) return 0;
   const bool sparse = (L.nSdc > 0 || L.nRle > 0) && W.nSp == 0;  // needs the tables P
   const size_t pBytes = sparse ? (((size_t)L.nSv * vCols * sizeof(double) + 255) & ~(size_t)255) : 0;
   if ((rc = ensure_scratch(m, pBytes + (size_t)vCols * sizeof(double) + 256)) < 0) return rc;
