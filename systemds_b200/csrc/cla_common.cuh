@@ -44,6 +44,7 @@ struct DevGroup {
   int32_t inFast;  // 1: the specialised vector kernels cover this group (general kernels skip it on their request)
   int64_t mapSize, offLen, nOff, nRuns, dataLen;
   int64_t valOff;  // first row of this group's table in the per-call value arenas (sum of nVals before it)
+  int64_t listAt;  // SDC: first of its listed rows in Matrix::sdcItems (sum of nOff of the SDC groups before it)
   const int32_t* cols;
   const double* dict;  // effective dictionary (default tuple subtracted), [nVals x gCols]
   const double* dictRaw;  // the dictionary as registered (== dict unless a default tuple was folded into constV)
@@ -174,9 +175,6 @@ struct RowLists {
   uint32_t* fullItems = nullptr;
   uint32_t* partPtr = nullptr;      // runs that cover part of a window: table row, first row | end row << 8 in the window
   uint2* partItems = nullptr;
-  // the same listed rows group by group, element order: row in its 1024-row block | tuple << 10
-  uint32_t* sdcItems = nullptr;
-  std::vector<int64_t> sdcBase;     // [nDev] first item of a group
 };
 // One column of a group the column-per-lane kernels do not take, as the left product walks it (cla_rest.cu).
 struct RestTask {
@@ -195,9 +193,9 @@ struct RestPlan {
   std::vector<int> unc;           // device group indices of the uncompressed groups
 };
 struct DecPlan {  // column-per-lane decompress (cla_generic.cu)
-  bool tried = false;
-  void* cols = nullptr;
-  int warps = 0;
+  int warps = 0;  // of a CTA; 0: the tile kernel is the better one
+  bool again = false;    // the block has been decompressed before
+  void* cols = nullptr;  // records, built on first use
   size_t smem = 0;
 };
 struct ColPlan {
@@ -286,6 +284,9 @@ struct Matrix {
   cudaStream_t lastStream = nullptr;
   bool lastValid = false;
   FastPlan* fast = nullptr;
+  // listed rows of the SDC groups, group by group in element order: row in its 1024-row block | tuple << 10
+  uint32_t* sdcItems = nullptr;
+  bool sdcItemsOk = false;
   RowLists rows;
   ColPlan cols;
   RestPlan rest;
@@ -337,7 +338,9 @@ void host_stage_free(Matrix* m);
 int64_t ensure_sparse_list(Matrix* m);  // Matrix::dSparseIdx (cla_generic.cu)
 
 int64_t ensure_col_plan(Matrix* m);                        // Matrix::cols; cols.ok tells whether it exists
-int64_t ensure_row_lists(Matrix* m, cudaStream_t s);       // Matrix::rows; rows.ok tells whether they exist
+int64_t sdc_items_bytes(const Matrix* m);                  // size of Matrix::sdcItems; -1: they cannot exist
+int64_t fill_sdc_items(Matrix* m, uint32_t* items, cudaStream_t s);  // builds Matrix::sdcItems in `items`
+int64_t ensure_row_lists(Matrix* m, cudaStream_t s);       // Matrix::rows and sdcItems; rows.ok tells whether they exist
 // The groups the specialised kernels leave (cla_rest.cu): 1 = done, 0 = not covered (the general kernels then run)
 int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s, bool addTo);
 int64_t rest_lmm(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s);
@@ -371,6 +374,7 @@ int64_t launch_tmm(Matrix* left, Matrix* right, double* dOut, cudaStream_t s);  
 bool pairs_eligible(const Matrix* L, const Matrix* R, bool self);
 int64_t launch_pairs(Matrix* L, Matrix* R, bool self, double* dOut, cudaStream_t s);
 int64_t launch_decompress(Matrix* m, double* dOut, cudaStream_t s);
+void decomp_shape(Matrix* m, const int32_t* colSrc);  // Matrix::dec; colSrc: [nCols][2], host copy of Matrix::dColSrc
 // X %*% V kept compressed: fills `child` (fresh Matrix) with groups that alias m's index structures (cla_generic.cu)
 int64_t make_overlapping(Matrix* m, Matrix* child, const double* dV, int vCols, cudaStream_t s);
 int64_t init_device_state(Matrix* m);  // stream, events, error word of a Matrix whose device is set (cla_finalize.cu)

@@ -561,7 +561,7 @@ int64_t finalize_device(Matrix* m) {
   m->constV.assign(m->nCols, 0.0);
   m->regToDev.assign(m->hg.size(), -1);
   m->groups.clear();
-  int64_t valOff = 0;
+  int64_t valOff = 0, listAt = 0;
   m->colMin.assign(m->nCols, INFINITY);
   m->colMax.assign(m->nCols, -INFINITY);
   {
@@ -785,6 +785,8 @@ int64_t finalize_device(Matrix* m) {
     } else {
       g.valOff = valOff;
       valOff += g.nVals;
+      g.listAt = listAt;
+      if (g.type == GT_SDC) listAt += g.nOff;
     }
     m->regToDev[gi] = (int)m->groups.size();
     m->groups.push_back(g);
@@ -827,6 +829,7 @@ int64_t finalize_device(Matrix* m) {
     const int32_t* dcs = nullptr;
     if ((rc = upload(m, colSrc.data(), colSrc.size(), &dcs, false)) < 0) return rc;
     m->dColSrc = const_cast<int32_t*>(dcs);
+    if (m->colSrcValid) decomp_shape(m, colSrc.data());
   }
   if ((rc = flush_uploads(m)) < 0) return rc;
   CLA_CUDA(cudaStreamSynchronize(m->stream));

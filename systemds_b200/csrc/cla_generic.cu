@@ -526,8 +526,10 @@ k_decomp_block(const DevGroup* __restrict__ groups, const int32_t* __restrict__ 
 // small dense-map groups, the next listed row and its value for an SDC column, the current run for an RLE column, the dense
 // block itself for an uncompressed one. Each cell is formed in the register it is stored from, and the warps of a CTA
 // write whole stretches of a row at the same time. The tile kernel above builds every cell in shared memory and reads
-// it back, and finds its way into the offset streams by a scan. What is left is the latency of the chains item -> value and
-// run -> value. 250,001 x 500 mixed (1 GB): 482 -> 310 us, 3.2 TB/s written.
+// it back. What is left is the latency of the chains item -> value and run -> value.
+// The records and the items of a block are filled on the device in its first call, nothing is copied or waited for (row
+// lists, which hold the items too, take 350 us). 250,001 x 500 mixed (1 GB), tile kernel against this one: 495 -> 320 us, 3.1
+// TB/s written; first call on a block 539 -> 399 us, host time included.
 struct DecCol {
   const double* dict;  // dictionary (or dense block) + position in the group
   const void* a;       // byte / bit map; SDC items; RLE runs
@@ -539,9 +541,18 @@ struct DecCol {
   int32_t mapType, pad;
 };
 enum { DC_CONST = 0, DC_BYTES = 1, DC_BITS = 2, DC_MAP = 3, DC_SDC = 4, DC_RLE = 5, DC_UNC = 6 };
+__host__ __device__ inline int dc_kind(const DevGroup& g) {
+  if (g.type == GT_UNC) return DC_UNC;
+  if (g.type == GT_SDC) return g.nOff > 0 ? DC_SDC : DC_CONST;
+  if (g.type == GT_RLE) return g.nRuns > 0 ? DC_RLE : DC_CONST;
+  if (g.nVals > 256) return DC_MAP;
+  return g.mapType == CLA_MAP_UBYTE || g.mapType == CLA_MAP_BYTE ? DC_BYTES : (g.mapType == CLA_MAP_BIT ? DC_BITS : DC_MAP);
+}
 constexpr int DC_ROWS = 64;            // (256 / 128 / 64 rows on 250,001 x 500: 346 / 319 / 310 us)
+constexpr int DC_WARPS = 16;
+constexpr int64_t DC_CELLS = 4 << 20, DC_FIRST = 20 << 20;  // cells of a call; of the block, for its first call
 constexpr size_t DC_TBL = 100 * 1024;  // table bytes of a CTA
-__global__ void __launch_bounds__(512) k_decomp_cols(const DecCol* __restrict__ cols, double* __restrict__ out, size_t ld, int r0, int r1,
+__global__ void __launch_bounds__(DC_WARPS * 32) k_decomp_cols(const DecCol* __restrict__ cols, double* __restrict__ out, size_t ld, int r0, int r1,
                                                      int nRows, int nCols, int exactSdc) {
   extern __shared__ double dct[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nW = blockDim.x >> 5;
@@ -644,90 +655,91 @@ __global__ void __launch_bounds__(512) k_decomp_cols(const DecCol* __restrict__ 
   }
 }
 
-// Column records of k_decomp_cols; m->dec.warps tells how many warps a CTA has (0: the tile kernel is the better one).
-static int64_t ensure_dec(Matrix* m, cudaStream_t s) {
-  DecPlan& D = m->dec;
-  if (D.tried) return CLA_OK;
-  D.tried = true;
-  int64_t rc;
-  if ((rc = ensure_row_lists(m, s)) < 0) return rc;
-  if (!m->rows.ok) return CLA_OK;
-  std::vector<DecCol> cols(m->nCols);
-  for (int c = 0; c < m->nCols; c++) {
-    cols[c] = DecCol{};
-    cols[c].kind = DC_CONST;
-    cols[c].cst = m->hasConst ? m->constV[c] : 0.0;
-  }
-  int scattered = 0;
-  for (size_t hi = 0; hi < m->hg.size(); hi++) {
-    const int gi = m->regToDev[hi];
-    if (gi < 0) continue;
-    const DevGroup& g = m->groups[gi];
-    for (int j = 0; j < g.gCols; j++) {
-      DecCol& d = cols[m->hg[hi].cols[j]];
+// The records of k_decomp_cols, filled by CTAs of the shape it will have.
+__global__ void __launch_bounds__(DC_WARPS * 32)
+k_dec_cols(const DevGroup* __restrict__ groups, const int32_t* __restrict__ colSrc, const double* __restrict__ constV,
+           const uint32_t* __restrict__ sdcItems, DecCol* __restrict__ cols, int nCols, int exactSdc) {
+  __shared__ int deep[DC_WARPS];  // longest table of every 32 columns
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * blockDim.x + threadIdx.x;
+  DecCol d = {};
+  d.kind = DC_CONST;
+  if (c < nCols) {
+    d.cst = constV ? constV[c] : 0.0;
+    const int gi = colSrc[2 * c], j = colSrc[2 * c + 1];
+    if (gi >= 0) {
+      const DevGroup& g = groups[gi];
+      d.kind = dc_kind(g);
       d.stride = g.gCols;
       d.nVals = g.nVals;
       d.mapType = g.mapType;
-      d.dict = (g.type == GT_UNC ? g.dense : g.dict) + j;
-      if (g.type == GT_DDC) {
-        d.a = g.map;
-        d.b = g.mapHi;
-        d.kind = g.nVals > 256 ? DC_MAP
-                 : (g.mapType == CLA_MAP_UBYTE || g.mapType == CLA_MAP_BYTE ? DC_BYTES : (g.mapType == CLA_MAP_BIT ? DC_BITS : DC_MAP));
-        scattered += d.kind == DC_MAP;
-      } else if (g.type == GT_SDC) {
-        if (g.nOff == 0) continue;
-        d.kind = DC_SDC;
-        d.a = m->rows.sdcItems + m->rows.sdcBase[gi];
-        d.b = g.skip;
-        d.n = g.nOff;
-        if (!m->multiCover) d.dict = g.dictRaw + j;
-      } else if (g.type == GT_RLE) {
-        if (g.nRuns == 0) continue;
-        d.kind = DC_RLE;
-        d.a = g.runs;
-        d.b = g.runSkip;
-        d.n = g.nRuns;
-      } else
-        d.kind = DC_UNC;
+      d.dict = (d.kind == DC_UNC ? g.dense : (d.kind == DC_SDC && exactSdc ? g.dictRaw : g.dict)) + j;
+      d.a = d.kind == DC_SDC ? (const void*)(sdcItems + g.listAt) : (d.kind == DC_RLE ? (const void*)g.runs : g.map);
+      d.b = d.kind == DC_SDC ? (const void*)g.skip : (d.kind == DC_RLE ? (const void*)g.runSkip : g.mapHi);
+      d.n = d.kind == DC_SDC ? g.nOff : g.nRuns;
     }
+  }
+  const int most = __reduce_max_sync(0xffffffffu, d.kind == DC_BYTES || d.kind == DC_BITS ? d.nVals : 0);
+  if (lane == 0) deep[warp] = most;
+  __syncthreads();
+  for (int w = 0; w < warp; w++) d.tbl += deep[w] * 32;
+  if (c < nCols) cols[c] = d;
+}
+
+// Whether k_decomp_cols is the better kernel for the block's columns (m->dec.warps, 0: the tile kernel is) and how many
+// warps a CTA has. Part of the upload, whose pass over the columns has everything at hand: finding it out at the first call
+// took longer than that call saves on small blocks.
+void decomp_shape(Matrix* m, const int32_t* colSrc) {
+  int scattered = 0, kinds = 0;
+  std::vector<int> deep((m->nCols + 31) / 32, 0);
+  for (int c0 = 0; c0 < m->nCols; c0 += 32) {
+    unsigned seen = 0;
+    for (int c = c0; c < std::min(m->nCols, c0 + 32); c++) {
+      const int gi = colSrc[2 * c], k = gi < 0 ? DC_CONST : dc_kind(m->groups[gi]);
+      scattered += k == DC_MAP;
+      seen |= 1u << (k == DC_BITS ? DC_BYTES : k);
+      if (k == DC_BYTES || k == DC_BITS) deep[c0 / 32] = std::max(deep[c0 / 32], m->groups[gi].nVals);
+    }
+    kinds += __builtin_popcount(seen);
   }
   // A lane-private gather from a large dictionary touches 32 lines per row, and a warp whose columns are of several kinds
   // walks its rows once per kind: matrices with many such columns keep the tile kernel (1M x 60 with four kinds in two
   // warps: 280 us there, 342 here).
-  int kinds = 0;
-  for (int c0 = 0; c0 < m->nCols; c0 += 32) {
-    unsigned seen = 0;
-    for (int c = c0; c < std::min(m->nCols, c0 + 32); c++) seen |= 1u << (cols[c].kind == DC_BITS ? DC_BYTES : cols[c].kind);
-    kinds += __builtin_popcount(seen);
-  }
-  if (scattered * 16 > m->nCols || kinds * 5 > (m->nCols + 31) / 32 * 7) return CLA_OK;
+  if (scattered * 16 > m->nCols || kinds * 5 > (int)deep.size() * 7) return;
   // tables: 256 bytes per tuple of the deepest small dictionary of every 32 columns; fewer columns per CTA if they are deep
-  int warps = std::max(1, std::min(16, (m->nCols + 31) / 32));
-  size_t most = 0;
-  for (; warps >= 1; warps /= 2) {
-    most = 0;
-    for (int c0 = 0; c0 < m->nCols; c0 += warps * 32) {
+  for (int warps = std::min<int>(DC_WARPS, (int)deep.size()); warps >= 1; warps /= 2) {
+    size_t most = 0;
+    for (size_t w = 0; w < deep.size(); w += warps) {
       size_t b = 0;
-      for (int g0 = c0; g0 < std::min(m->nCols, c0 + warps * 32); g0 += 32) {
-        int deep = 0;
-        for (int c = g0; c < std::min(m->nCols, g0 + 32); c++)
-          if (cols[c].kind == DC_BYTES || cols[c].kind == DC_BITS) deep = std::max(deep, cols[c].nVals);
-        for (int c = g0; c < std::min(m->nCols, g0 + 32); c++) cols[c].tbl = (int)(b / 8);
-        b += (size_t)deep * 256;
-      }
+      for (size_t i = w; i < std::min(deep.size(), w + warps); i++) b += (size_t)deep[i] * 256;
       most = std::max(most, b);
     }
-    if (most <= DC_TBL) break;
+    if (most <= DC_TBL) {
+      m->dec.warps = warps;
+      m->dec.smem = most;
+      return;
+    }
   }
-  if (warps < 1) return CLA_OK;
+}
+
+// The records of k_decomp_cols and the items of the SDC columns; m->dec.warps becomes 0 where there is no room for them. Nothing
+// is copied or waited for: the device fills them.
+static int64_t ensure_dec(Matrix* m, cudaStream_t s) {
+  DecPlan& D = m->dec;
+  if (D.cols || D.warps == 0) return CLA_OK;
+  const int warps = D.warps;
+  const int64_t itemBytes = m->sdcItemsOk ? 0 : sdc_items_bytes(m);
+  const size_t at = ((size_t)m->nCols * sizeof(DecCol) + 255) & ~(size_t)255;
   void* p = nullptr;
-  if (plan_alloc(m, &p, cols.size() * sizeof(DecCol)) < 0) return CLA_OK;  // (the tile kernel needs none)
-  CLA_CUDA(cudaMemcpyAsync(p, cols.data(), cols.size() * sizeof(DecCol), cudaMemcpyHostToDevice, s));
-  CLA_CUDA(cudaStreamSynchronize(s));
+  D.warps = 0;
+  if (itemBytes < 0 || plan_alloc(m, &p, at + (size_t)itemBytes) < 0) return CLA_OK;
+  int64_t rc;
+  if (!m->sdcItemsOk && (rc = fill_sdc_items(m, (uint32_t*)((char*)p + at), s)) < 0) return rc;
+  k_dec_cols<<<(m->nCols + warps * 32 - 1) / (warps * 32), warps * 32, 0, s>>>(
+      m->dGroups, m->dColSrc, m->hasConst ? m->dConstV : nullptr, m->sdcItems, (DecCol*)p, m->nCols, m->multiCover ? 0 : 1);
+  m->stats.kernel_launches++;
+  CLA_CUDA(cudaGetLastError());
   D.cols = p;
   D.warps = warps;
-  D.smem = most;
   return CLA_OK;
 }
 
@@ -740,7 +752,14 @@ int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStr
     const int64_t rf = fast_decompress(m, r0, r1, dOut, s, ld);  // byte-map matrices: straight from the column-per-lane layout
     if (rf != 0) return rf < 0 ? rf : CLA_OK;
     int64_t rc;
-    const bool byCols = n >= (4 << 20);  // (below, too few of its warps are in flight)
+    // Below DC_CELLS both kernels take the same time (8,400 x 500: 32 us). Records and items cost a block's first call 25 to 40
+    // us, which its kernel makes up for from DC_FIRST on (12 million cells: 117 us against 96 with the tile kernel, 24: 143
+    // against 147, 125: 399 against 539); a smaller block gets them when it is decompressed again (12 million: 58 against 66).
+    bool byCols = n >= DC_CELLS;
+    if (byCols && !m->dec.cols) {
+      byCols = m->dec.again || (int64_t)m->nRows * m->nCols >= DC_FIRST;
+      m->dec.again = true;
+    }
     if (byCols && (rc = ensure_dec(m, s)) < 0) return rc;
     if (byCols && m->dec.warps > 0) {
       static bool decAttr[64] = {};  // per device

@@ -627,7 +627,7 @@ static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
       t.col = m->hg[hi].cols[j];
       if (g.type == GT_SDC) {
         if (g.nOff == 0) continue;
-        t.a = m->rows.sdcItems + m->rows.sdcBase[gi];
+        t.a = m->sdcItems + g.listAt;
         t.b = g.skip;
         t.n = g.nOff;
         sdc.push_back(t);

@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(RL_THREADS)
 k_row_lists(const DevGroup* __restrict__ groups, const int32_t* __restrict__ list, int nSdc, int nRle, int nRows,
             const int32_t* __restrict__ svOff, uint32_t* __restrict__ rowPtr, uint32_t* __restrict__ rowItems,
             uint32_t* __restrict__ fullPtr, uint32_t* __restrict__ fullItems, uint32_t* __restrict__ partPtr,
-            uint2* __restrict__ partItems, uint32_t* __restrict__ sdcItems, const int64_t* __restrict__ sdcBase) {
+            uint2* __restrict__ partItems, uint32_t* __restrict__ sdcItems) {
   __shared__ uint32_t cnt[SKIP_ROWS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int blk = blockIdx.x, b0 = blk * SKIP_ROWS, b1 = min(nRows, b0 + SKIP_ROWS);
@@ -128,7 +128,7 @@ k_row_lists(const DevGroup* __restrict__ groups, const int32_t* __restrict__ lis
         if (FILL) {
           const uint32_t id = (uint32_t)(g.single ? 0 : map_get(g.mapType, g.map, g.mapHi, e));
           rowItems[p] = o + id;
-          sdcItems[sdcBase[gi] + e] = (uint32_t)(row - b0) | (id << 10);
+          if (sdcItems) sdcItems[g.listAt + e] = (uint32_t)(row - b0) | (id << 10);
         }
       });
       __syncwarp();
@@ -195,6 +195,43 @@ k_row_lists(const DevGroup* __restrict__ groups, const int32_t* __restrict__ lis
     }
 }
 
+// The items alone, where nothing needs the rows' lists: a warp per group and 1024-row block. An item's place follows from
+// the group's element number, so nothing is counted and nothing waited for.
+constexpr int SDC_ITEM_VALS = 1 << 22;  // an item holds 22 bits of tuple
+__global__ void __launch_bounds__(RL_THREADS) k_sdc_items(const DevGroup* __restrict__ groups, int nDev, int nRows, uint32_t* __restrict__ items) {
+  const int perBlock = (nDev + RL_THREADS / 32 - 1) / (RL_THREADS / 32), blk = blockIdx.x / perBlock;
+  const int gi = (blockIdx.x - blk * perBlock) * (RL_THREADS / 32) + (threadIdx.x >> 5);
+  if (gi >= nDev || groups[gi].type != GT_SDC) return;
+  const DevGroup& g = groups[gi];
+  const int b0 = blk * SKIP_ROWS;
+  uint32_t* to = items + g.listAt;
+  sdc_walk_block(g, b0, min(nRows, b0 + SKIP_ROWS), [&](int row, int e) {
+    to[e] = (uint32_t)(row - b0) | ((uint32_t)(g.single ? 0 : map_get(g.mapType, g.map, g.mapHi, e)) << 10);
+  });
+}
+
+// -1: a group's tuples do not fit an item
+int64_t sdc_items_bytes(const Matrix* m) {
+  int64_t n = 0;
+  for (auto& g : m->groups)
+    if (g.type == GT_SDC && g.nOff > 0) {
+      if (g.nVals > SDC_ITEM_VALS) return -1;
+      n += g.nOff;
+    }
+  return n * 4;
+}
+int64_t fill_sdc_items(Matrix* m, uint32_t* items, cudaStream_t s) {
+  if (sdc_items_bytes(m) > 0) {
+    const unsigned grid = (unsigned)((m->nRows + SKIP_ROWS - 1) / SKIP_ROWS) * (unsigned)((m->nDev + RL_THREADS / 32 - 1) / (RL_THREADS / 32));
+    k_sdc_items<<<grid, RL_THREADS, 0, s>>>(m->dGroups, m->nDev, m->nRows, items);
+    m->stats.kernel_launches++;
+    CLA_CUDA(cudaGetLastError());
+  }
+  m->sdcItems = items;
+  m->sdcItemsOk = true;
+  return CLA_OK;
+}
+
 int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   RowLists& L = m->rows;
   if (L.tried) return CLA_OK;
@@ -228,14 +265,8 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   std::vector<int32_t> list(sdc);
   list.insert(list.end(), rle.begin(), rle.end());
   // pointers, group list, table-row numbering and values in one allocation
-  L.sdcBase.assign(m->nDev, 0);
-  int64_t nListed = 0;
-  for (int gi : sdc) {
-    L.sdcBase[gi] = nListed;
-    nListed += m->groups[gi].nOff;
-    if (m->groups[gi].nVals > (1 << 22)) return CLA_OK;  // an item holds 22 bits of tuple
-  }
-  const size_t bBase = (size_t)m->nDev * 8;
+  for (int gi : sdc)
+    if (m->groups[gi].nVals > SDC_ITEM_VALS) return CLA_OK;
   const size_t bOff = ((size_t)m->nDev * 4 + 15) & ~(size_t)15, bList = (list.size() * 4 + 15) & ~(size_t)15;
   const size_t bSv = (size_t)std::max<int64_t>(nSv, 1) * sizeof(SparseVal);
   const size_t bRow = (L.nSdc ? (size_t)nRowPtr * 4 : 0), bWin = (L.nRle ? (size_t)nWinPtr * 4 : 0);
@@ -244,11 +275,10 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   cub::DeviceScan::ExclusiveSum(nullptr, tb2, (uint32_t*)nullptr, (uint32_t*)nullptr, (int)nWinPtr, s);
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   void* base = nullptr;
-  const size_t bytes = al(bBase) + al(bOff) + al(bList) + al(bSv) + al(bRow) + 2 * al(bWin) + std::max(tb1, tb2);
+  const size_t bytes = al(bOff) + al(bList) + al(bSv) + al(bRow) + 2 * al(bWin) + std::max(tb1, tb2);
   if (plan_alloc(m, &base, bytes) < 0) return CLA_OK;
   char* p = (char*)base;
   L.svOff = (int32_t*)p; p += al(bOff);
-  int64_t* dBase = (int64_t*)p; p += al(bBase);
   int32_t* dList = (int32_t*)p; p += al(bList);
   L.sv = (SparseVal*)p; p += al(bSv);
   if (L.nSdc) L.rowPtr = (uint32_t*)p;
@@ -259,11 +289,10 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   p += al(bWin);
   void* tmp = p;
   CLA_CUDA(cudaMemcpyAsync(L.svOff, off.data(), (size_t)m->nDev * 4, cudaMemcpyHostToDevice, s));
-  CLA_CUDA(cudaMemcpyAsync(dBase, L.sdcBase.data(), bBase, cudaMemcpyHostToDevice, s));
   CLA_CUDA(cudaMemcpyAsync(dList, list.data(), list.size() * 4, cudaMemcpyHostToDevice, s));
   k_sparse_vals<<<m->nDev, 128, 0, s>>>(m->dGroups, L.svOff, L.sv);
   k_row_lists<false><<<nBlocks, RL_THREADS, 0, s>>>(m->dGroups, dList, L.nSdc, L.nRle, m->nRows, L.svOff, L.rowPtr, nullptr,
-                                                   L.fullPtr, nullptr, L.partPtr, nullptr, nullptr, nullptr);
+                                                   L.fullPtr, nullptr, L.partPtr, nullptr, nullptr);
   uint32_t tot[3] = {0, 0, 0};
   if (L.nSdc) {
     CLA_CUDA(cudaMemsetAsync(L.rowPtr + nRowPtr - 1, 0, 4, s));
@@ -281,19 +310,24 @@ int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {
   CLA_CUDA(cudaStreamSynchronize(s));
   void* items = nullptr;
   const size_t i0 = al((size_t)tot[0] * 4), i1 = al((size_t)tot[1] * 4), i2 = al((size_t)tot[2] * 8);
-  if (plan_alloc(m, &items, 2 * i0 + i1 + i2) < 0) {
+  const bool own = !m->sdcItemsOk;  // (the decompress may have built them already)
+  if (plan_alloc(m, &items, (own ? 2 : 1) * i0 + i1 + i2) < 0) {
     plan_release(m, base, bytes);
     L.svOff = nullptr, L.sv = nullptr, L.rowPtr = L.fullPtr = L.partPtr = nullptr;
     return CLA_OK;
   }
-  L.sdcItems = (uint32_t*)((char*)items + i0 + i1 + i2);
+  uint32_t* sdcItems = own ? (uint32_t*)((char*)items + i0 + i1 + i2) : nullptr;
   L.rowItems = (uint32_t*)items;
   L.fullItems = (uint32_t*)((char*)items + i0);
   L.partItems = (uint2*)((char*)items + i0 + i1);
   k_row_lists<true><<<nBlocks, RL_THREADS, 0, s>>>(m->dGroups, dList, L.nSdc, L.nRle, m->nRows, L.svOff, L.rowPtr, L.rowItems,
-                                                  L.fullPtr, L.fullItems, L.partPtr, L.partItems, L.sdcItems, dBase);
+                                                  L.fullPtr, L.fullItems, L.partPtr, L.partItems, sdcItems);
   CLA_CUDA(cudaGetLastError());
   CLA_CUDA(cudaStreamSynchronize(s));
+  if (own) {
+    m->sdcItems = sdcItems;
+    m->sdcItemsOk = true;
+  }
   L.ok = true;
   return CLA_OK;
 }

@@ -166,3 +166,69 @@ def test_products_with_tables_of_16_bit_maps(nRows, longest):
     cmb = _ddc(nRows, [300, 1000, 257] * 6 + [longest, 9], longest, const=True, width=2 if longest == 1601 else 1).to_device()
     _check(cmb, ks=(1,), qs=(1, 2, 5, 9))
     cmb.free()
+
+
+def _sdc(nRows, dens, card, default, seed, rows=None):
+    """An SDC column with listed rows of the given density (or exactly `rows`)."""
+    rng = np.random.default_rng(seed)
+    ids = np.full(nRows, -1, np.int32)
+    mask = rng.random(nRows) < dens if rows is None else np.isin(np.arange(nRows), rows)
+    ids[mask] = rng.integers(0, card, int(mask.sum()))
+    return lambda c: cg.sdc_from_row_ids([c], rng.standard_normal((card, 1)), ids, rng.standard_normal(1) if default else None)
+
+
+def _by_kind(nRows):
+    """A kind per 32 columns, as the decompress by columns wants them: offset streams with 8- and 16-bit deltas, gaps beyond
+    their range, dense lists, none, one or two listed rows (also at the edges of 64-row pieces), one tuple only; short and
+    long runs, rows without a run; byte and bit maps; dense columns; a few long tables and two-column groups."""
+    rng = np.random.default_rng(nRows)
+    groups, c = [], 0
+
+    def add(make, width=1):
+        nonlocal c
+        groups.append(make(c) if width == 1 else make(list(range(c, c + width))))
+        c += width
+
+    last = nRows - 1
+    for i, (dens, card) in enumerate([(0.05, 8), (0.0004, 8), (0.5, 3), (0.3, 300), (0.02, 1), (0.999, 2)] * 5):
+        add(_sdc(nRows, dens, card, i % 2, i))
+    add(_sdc(nRows, 0, 3, False, 1, rows=[63, 64, 1023, 1024, last]))
+    add(_sdc(nRows, 0, 3, True, 2, rows=[last - 1]))
+    for rows in ([0], [last], [0, last], [63, 64], [64], [1023, 1024], [5000, last], [2]):
+        add(_sdc(nRows, 0, 2, len(rows) == 1, 3, rows=rows))
+    for i in range(24):
+        add(_sdc(nRows, 0.05, 5, i % 2, 100 + i))
+    for i in range(32):
+        add(lambda c: datagen.random_group("rle", [c], nRows, rng))
+    for i in range(32):
+        add(lambda c: datagen.random_group("ddc_bit" if i % 3 else "ddc", [c], nRows, rng))
+    for i in range(16):
+        add(lambda cs: datagen.random_group("ddc2", cs, nRows, rng), 2)
+    for i in range(4):
+        add(lambda cs: datagen.random_group("unc", cs, nRows, rng), 8)
+    for i in range(31):
+        add(lambda c: datagen.random_group("const" if i % 2 else "empty", [c], nRows, rng))
+    for i in range(2):
+        add(lambda c: datagen.random_group("ddc_char", [c], nRows, rng))
+    return CompressedMatrixBlock(nRows, c, groups)
+
+
+@pytest.mark.parametrize("nRows", [18817, 19455, 70001, 93313])
+def test_decompress_by_columns(nRows):
+    """From four million cells on, columns sorted by kind; the first call on a block (by columns from 20 million cells on) and
+    a repeated one: the cells are the registered values, also in the row chunks of a self product, and the handle takes no
+    more memory than one word per listed row and a record per column."""
+    cmb = _by_kind(nRows)
+    assert nRows * cmb.clen >= 4 << 20
+    X = dense_of(cmb)
+    cmb.to_device()
+    held = cmb.stats()["device_bytes"]
+    for _ in range(2):
+        assert np.array_equal(np.array(CLALibDecompress.decompress(cmb)), X)
+    listed = sum(g._indexes.getSize() for g in cmb.getColGroups() if hasattr(g, "_indexes"))
+    assert cmb.stats()["device_bytes"] - held <= 4 * listed + 64 * cmb.clen + 256
+    got = CLALibTSMM.leftMultByTransposeSelf(cmb)
+    assert rel_err(got, X.T @ X, np.abs(X).T @ np.abs(X) + 1e-300) < TOL
+    _check(cmb, ks=(1, 3), chain=False)
+    assert np.array_equal(np.array(CLALibDecompress.decompress(cmb)), X)
+    cmb.free()
