@@ -9,6 +9,7 @@
 #include <string>
 #include <vector>
 #include "../../include/systemds_cla.h"
+#include "cla_once.h"
 
 namespace cla {
 
@@ -313,6 +314,16 @@ int64_t fail(int64_t code, const std::string& msg);
     if (e_ != cudaSuccess)                                                                          \
       return ::cla::fail(CLA_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_));         \
   } while (0)
+
+// Lets kernels take `bytes` of dynamic shared memory; `device` is the current device.
+template <class... K>
+inline int64_t allow_smem(OncePerDevice& once, int device, size_t bytes, K... kernels) {
+  return once(device, [&]() -> int64_t {
+    cudaError_t e = cudaSuccess;
+    ((e == cudaSuccess ? (void)(e = cudaFuncSetAttribute(kernels, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)) : (void)0), ...);
+    return e == cudaSuccess ? CLA_OK : fail(CLA_ERR_CUDA, std::string("shared memory of a kernel: ") + cudaGetErrorString(e));
+  });
+}
 
 // profiling brackets around the dominant kernel of a product call (no-ops unless m->profile)
 void prof_begin(Matrix* m, cudaStream_t s);

@@ -1505,14 +1505,9 @@ int64_t fast_plan_build(Matrix* m) {
     k_joint_interleave<<<m->smCount * 8, 256, 0, m->stream>>>(fp->dJSlots, (const uint8_t* const*)(base + oGMap), fp->nJU16 * 16,
                                                              m->nRows, fp->nRB, fp->dJMaps);
   CLA_CUDA(cudaStreamSynchronize(m->stream));
-  static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
-  if (!attrSet[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_lmm_vec, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
-    CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
-    CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
-    CLA_CUDA(cudaFuncSetAttribute(k_decomp_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 2048));
-    attrSet[m->device & 63] = true;
-  }
+  static OncePerDevice once, onceDecomp;
+  if ((rc = allow_smem(once, m->device, SMEM_MAX - 1024, k_lmm_vec, k_rmm_vec<false>, k_rmm_vec<true>)) < 0) return rc;
+  if ((rc = allow_smem(onceDecomp, m->device, SMEM_MAX - 2048, k_decomp_fast)) < 0) return rc;
   if (fp->partial) {  // tell the general kernels which groups are taken care of
     for (auto& x : sel) m->groups[x.dev].inFast = 1;
     CLA_CUDA(cudaMemcpy(m->dGroups, m->groups.data(), sizeof(DevGroup) * m->groups.size(), cudaMemcpyHostToDevice));
@@ -1686,12 +1681,8 @@ int64_t fast_chain(Matrix* m, const double* dV, const double* dW, double* dOut, 
   C.w = dW;
   C.u = dU;
   C.nCols = m->nCols;
-  static bool attrSet[64] = {};  // per device
-  if (!attrSet[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_chain_vec, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  SMEM_MAX - CH_STATIC));
-    attrSet[m->device & 63] = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, SMEM_MAX - CH_STATIC, k_chain_vec); e < 0) return e;
   prof_begin(m, s);
   k_chain_vec<<<grid, CH_T, smem, s>>>(C);
   m->stats.kernel_launches++;
@@ -1732,11 +1723,8 @@ static int64_t fast_lmm_rows_t(Matrix* m, FastPlan* fp, const double* dY, size_t
   CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)Q * m->nCols, s));
   size_t smem = (size_t)LQ_W * Q * LMM_PART * 8;
   for (auto& c : fp->lchunks) smem = std::max(smem, (size_t)c.tblDoubles * 8);
-  static bool attr[64] = {};  // per device
-  if (!attr[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_lmm_vecq_u8<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024));
-    attr[m->device & 63] = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, SMEM_MAX - 1024, k_lmm_vecq_u8<Q>); e < 0) return e;
   prof_begin(m, s);
   k_lmm_vecq_u8<Q><<<fp->lmmGrid, LQ_T, smem, s>>>(fp->dLChunks, (int)fp->lchunks.size(), fp->dLmmMaps, fp->nRB, fp->dLmmTables, dY,
                                                   pitch, m->nRows, partial, m->dErr);
@@ -1809,11 +1797,8 @@ static int64_t lmm_rows_tensor(Matrix* m, FastPlan* fp, const double* dY, size_t
   if ((rc = ensure_scratch(m, (size_t)grid * LR_PART * 8 + 256)) < 0) return rc;
   A.partial = (double*)m->scratch;
   if (A.addTo) CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)q * m->nCols, s));
-  static bool attr[64] = {};  // per device
-  if (!attr[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_lmm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, LR_SMEM));
-    attr[m->device & 63] = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, LR_SMEM, k_lmm_rows); e < 0) return e;
   prof_begin(m, s);
   k_lmm_rows<<<grid, LR_T, smem, s>>>(A);
   prof_end(m, s);

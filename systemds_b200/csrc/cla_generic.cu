@@ -236,12 +236,8 @@ int64_t launch_rmm(Matrix* m, const double* dV, const double* dW, double* dOut, 
     k_const_times_v<<<1, 128, 0, s>>>(m->dConstV, m->nCols, dV, 1, constRow);
     m->stats.kernel_launches++;
   }
-  static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
-  bool& attr = attrSet[m->device & 63];
-  if (!attr) {
-    CLA_CUDA(cudaFuncSetAttribute(k_rmm_vec_general, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RV_SMEM));
-    attr = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, RV_SMEM, k_rmm_vec_general); e < 0) return e;
   const int32_t* ddcIdx = afterFast ? m->dDdcRestIdx : m->dDdcIdx;
   const int nDdc = afterFast ? m->nDdcRest : m->nDdc;
   prof_begin(m, s);
@@ -762,11 +758,8 @@ int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStr
     }
     if (byCols && (rc = ensure_dec(m, s)) < 0) return rc;
     if (byCols && m->dec.warps > 0) {
-      static bool decAttr[64] = {};  // per device
-      if (!decAttr[m->device & 63]) {
-        CLA_CUDA(cudaFuncSetAttribute(k_decomp_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DC_TBL));
-        decAttr[m->device & 63] = true;
-      }
+      static OncePerDevice once;
+      if (const int64_t e = allow_smem(once, m->device, DC_TBL, k_decomp_cols); e < 0) return e;
       dim3 grid((r1 - r0 + DC_ROWS - 1) / DC_ROWS, (m->nCols + m->dec.warps * 32 - 1) / (m->dec.warps * 32));
       k_decomp_cols<<<grid, m->dec.warps * 32, m->dec.smem, s>>>((const DecCol*)m->dec.cols, dOut, ld, r0, r1, m->nRows, m->nCols,
                                                                 m->multiCover ? 0 : 1);
@@ -775,12 +768,8 @@ int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStr
       return CLA_OK;
     }
     const size_t smem = (size_t)DB_COLS * DB_LD * sizeof(double);
-    static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
-    bool& attr = attrSet[m->device & 63];
-    if (!attr) {
-      CLA_CUDA(cudaFuncSetAttribute(k_decomp_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      attr = true;
-    }
+    static OncePerDevice once;
+    if (const int64_t e = allow_smem(once, m->device, smem, k_decomp_block); e < 0) return e;
     dim3 grid((r1 - r0 + DB_ROWS - 1) / DB_ROWS, (m->nCols + DB_COLS - 1) / DB_COLS);
     k_decomp_block<<<grid, DB_WARPS * 32, smem, s>>>(m->dGroups, m->dColSrc, m->hasConst ? m->dConstV : nullptr, dOut, ld, r0, r1, m->nCols,
                                            m->multiCover ? 0 : 1);

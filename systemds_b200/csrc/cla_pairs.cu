@@ -206,13 +206,8 @@ int64_t launch_pairs(Matrix* L, Matrix* R, bool self, double* dOut, cudaStream_t
   if (!pairs.empty()) CLA_CUDA(cudaMemcpyAsync(dPairs, pairs.data(), pairs.size() * sizeof(PairDesc), cudaMemcpyHostToDevice, s));
   CLA_CUDA(cudaStreamSynchronize(s));  // the host vectors above go out of scope with this call
 
-  static bool attrSet[64] = {};
-  bool& attr = attrSet[L->device & 63];
-  if (!attr) {
-    CLA_CUDA(cudaFuncSetAttribute(k_hist1, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_MAX_CELLS * 4));
-    CLA_CUDA(cudaFuncSetAttribute(k_hist2, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_MAX_CELLS * 4));
-    attr = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, L->device, PAIR_MAX_CELLS * 4, k_hist1, k_hist2); e < 0) return e;
   const int nRows = L->nRows;
   // row chunks: enough CTAs to fill the GPU a few times over, at least 16K rows each
   auto chunking = [&](int64_t units, int* rowsPerChunk) {

@@ -673,11 +673,8 @@ static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
 }
 
 static int64_t table_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s, bool addTo) {
-  static bool attrSet[64] = {};  // per device
-  if (!attrSet[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_table_rmm, cudaFuncAttributeMaxDynamicSharedMemorySize, TL_SMEM));
-    attrSet[m->device & 63] = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, TL_SMEM, k_table_rmm); e < 0) return e;
   const RestPlan& R = m->rest;
   TableRmmArgs A{};
   A.tasks = R.tasks + (R.nTasks - R.nTable);
@@ -737,11 +734,8 @@ int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cu
     m->stats.kernel_launches++;
     A.P = (const double*)m->scratch;
   }
-  static bool attrSet[64] = {};  // per device
-  if (!attrSet[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_rest_rmm, cudaFuncAttributeMaxDynamicSharedMemorySize, (RR_PMAX + RR_UCOLS) * (int)sizeof(double)));
-    attrSet[m->device & 63] = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, (RR_PMAX + RR_UCOLS) * sizeof(double), k_rest_rmm); e < 0) return e;
   int u0 = 0;
   prof_begin(m, s);
   do {  // uncompressed groups up to RR_UNC and RR_UCOLS columns at a time; the first launch adds everything else
@@ -773,11 +767,8 @@ int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cu
 
 template <int QT>
 static int64_t rest_lmm_go(Matrix* m, RestLmmArgs& A, int grid, size_t smem, cudaStream_t s) {
-  static bool attrSet[64] = {};  // per device
-  if (!attrSet[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_rest_lmm<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
-    attrSet[m->device & 63] = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, 112 * 1024, k_rest_lmm<QT>); e < 0) return e;
   k_rest_lmm<QT><<<grid, RL_T, smem, s>>>(A);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)std::max(1, (int)(((int64_t)A.nTasks * QT + (int64_t)A.gCols * QT + 31) / 32)));
@@ -795,11 +786,8 @@ static int64_t rest_lmm_go(Matrix* m, RestLmmArgs& A, int grid, size_t smem, cud
 
 template <int QT>
 static int64_t table_lmm_go(Matrix* m, const double* dYt, int q, double* dOut, cudaStream_t s) {
-  static bool attrSet[64] = {};  // per device
-  if (!attrSet[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_table_lmm<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TL_SMEM));
-    attrSet[m->device & 63] = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, TL_SMEM, k_table_lmm<QT>); e < 0) return e;
   const RestPlan& R = m->rest;
   TableLmmArgs A{};
   A.tasks = R.tasks + (R.nTasks - R.nTable);

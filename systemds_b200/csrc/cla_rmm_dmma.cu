@@ -243,12 +243,8 @@ int64_t launch_rmm_dmma(Matrix* m, const double* dV, int vCols, double* dOut, cu
     m->stats.kernel_launches++;
   }
   const size_t smem = std::max((size_t)(GM_KC * GM_LDA + GM_KC * GM_LDB), (size_t)(GM_TR * GM_LDC + GM_TN)) * sizeof(double);
-  static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
-  bool& attr = attrSet[m->device & 63];
-  if (!attr) {
-    CLA_CUDA(cudaFuncSetAttribute(k_rmm_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, smem, k_rmm_dmma); e < 0) return e;
   prof_begin(m, s);
   dim3 grid((m->nRows + GM_TR - 1) / GM_TR, (vCols + GM_TN - 1) / GM_TN);
   k_rmm_dmma<<<grid, GM_THREADS, smem, s>>>(m->dGroups, m->nDev, (const DenseCol*)m->dDenseCols, m->nDenseCols, m->nRows, dV, vCols, P,

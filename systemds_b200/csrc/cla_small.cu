@@ -312,14 +312,11 @@ int64_t small_rmm(Matrix* m, const double* dV, int vCols, double* dOut, const do
   const bool vShared = (int64_t)m->nCols * KT <= SR_VMAX;
   const int warps = KT == 1 ? SmallRmm<1>::WARPS : SmallRmm<8>::WARPS;
   const size_t smem = ((size_t)warps * KT * 33 + (vShared ? (size_t)m->nCols * KT : 0)) * sizeof(double);
-  static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
-  if (!attrSet[m->device & 63]) {
-    const int most = (int)((16 * 8 * 33 + SR_VMAX) * sizeof(double));
-    CLA_CUDA(cudaFuncSetAttribute(k_small_rmm<1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    CLA_CUDA(cudaFuncSetAttribute(k_small_rmm<4, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    CLA_CUDA(cudaFuncSetAttribute(k_small_rmm<8, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    attrSet[m->device & 63] = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, (16 * 8 * 33 + SR_VMAX) * sizeof(double), k_small_rmm<1, 0>,
+                                         k_small_rmm<4, 0>, k_small_rmm<8, 0>);
+      e < 0)
+    return e;
   const dim3 grid((m->nRows + 31) / 32, (vCols + KT - 1) / KT);
   prof_begin(m, s);
 #define SMALL_RMM(K, N, ARG)                                                                                                   \

@@ -211,11 +211,8 @@ k_gemm_tn(const double* __restrict__ A, int aCols, int lda, const double* __rest
 template <bool SYRK>
 static int64_t launch_gemm_tn(Matrix* m, const double* A, int aCols, int lda, const double* B, int bCols, int ldb, int rows, double* C,
                               cudaStream_t s) {
-  static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
-  if (!attrSet[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_gemm_tn<SYRK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM));
-    attrSet[m->device & 63] = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, GT_SMEM, k_gemm_tn<SYRK>); e < 0) return e;
   const int nA = (aCols + GT_BLK - 1) / GT_BLK, nB = (bCols + GT_BLK - 1) / GT_BLK, nSt = (rows + GT_KT - 1) / GT_KT;
   auto tiles = [](int cols, int b) { return (std::min(GT_BLK, cols - b * GT_BLK) + 31) / 32; };
   int bi = 0, bj = 0;
@@ -727,12 +724,8 @@ int64_t launch_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
   bool denseOnly = m->colSrcValid;
   for (auto& g : m->groups) denseOnly &= (g.type == GT_DDC || g.type == GT_UNC);
   const size_t tri16Smem = (size_t)((n + 15) / 16 * 16) * (4 * TT_LDB * sizeof(double) + sizeof(TsmmCol) + 28) + 4 * sizeof(uint64_t);
-  static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
-  bool& attr = attrSet[m->device & 63];
-  if (!attr) {
-    if ((rc = tri16_set_smem(128 * (4 * TT_LDB * 8 + (int)sizeof(TsmmCol) + 28) + 32)) < 0) return rc;
-    attr = true;
-  }
+  static OncePerDevice once;
+  if ((rc = once(m->device, [&] { return tri16_set_smem(128 * (4 * TT_LDB * 8 + (int)sizeof(TsmmCol) + 28) + 32); })) < 0) return rc;
   if (tri && denseOnly) {  // one launch over all rows, decoding as it goes
     const int64_t nStages = ((int64_t)m->nRows + TT_KT - 1) / TT_KT;
     // one map width for every column (and every column held by a dense-map group): the specialised decode

@@ -643,14 +643,8 @@ int64_t wide_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStrea
     k_wide_const<<<vCols, 32, 0, s>>>(m->dConstV, m->nCols, dV, vCols, (double*)A.constRow);
     m->stats.kernel_launches++;
   }
-  static bool attrSet[64] = {};  // per device: function attributes belong to the device's context
-  if (!attrSet[m->device & 63]) {
-    CLA_CUDA(cudaFuncSetAttribute(k_rmm_wide<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WD_SMEM + 1024));
-    CLA_CUDA(cudaFuncSetAttribute(k_rmm_wide<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WD_SMEM + 1024));
-    CLA_CUDA(cudaFuncSetAttribute(k_rmm_wide<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WD_SMEM + 1024));
-    CLA_CUDA(cudaFuncSetAttribute(k_rmm_wide<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WD_SMEM + 1024));
-    attrSet[m->device & 63] = true;
-  }
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, WD_SMEM + 1024, k_rmm_wide<1>, k_rmm_wide<2>, k_rmm_wide<3>, k_rmm_wide<4>); e < 0) return e;
   const int gridY = (vCols + NT * 8 - 1) / (NT * 8), nWin = (m->nRows + WIN_ROWS - 1) / WIN_ROWS;
   const dim3 grid((unsigned)std::max(1, std::min(nWin, m->smCount / gridY)), gridY);
   auto kern = NT == 1 ? k_rmm_wide<1> : (NT == 2 ? k_rmm_wide<2> : (NT == 3 ? k_rmm_wide<3> : k_rmm_wide<4>));
