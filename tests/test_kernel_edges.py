@@ -232,3 +232,26 @@ def test_decompress_by_columns(nRows):
     _check(cmb, ks=(1, 3), chain=False)
     assert np.array_equal(np.array(CLALibDecompress.decompress(cmb)), X)
     cmb.free()
+
+
+@pytest.mark.parametrize("nCols", [128, 129, 300, 448, 449])
+@pytest.mark.parametrize("nRows", [77, 1000])
+def test_short_blocks_with_v_in_the_launch(nRows, nCols):
+    """A host-buffer product whose V travels with the launch: the last count of the small argument, the first and last of
+    the large one, and the first that is read from the mailbox instead."""
+    cmb = _ddc(nRows, [5] * (nCols - 1), nCols, const=True).to_device()
+    assert cmb.clen == nCols
+    _check(cmb, qs=(1,))
+    cmb.free()
+
+
+@pytest.mark.parametrize("longest", [6400, 6401])
+@pytest.mark.parametrize("extra", [-1, 0, 33])
+def test_right_product_with_the_longest_tables(longest, extra):
+    """X %*% v with tables of four columns per CTA: taken from half a table's rows per SM on, which the longest table that
+    fits needs most rows for; one tuple more, and the column stays with the other kernel."""
+    import torch
+    nRows = torch.cuda.get_device_properties(0).multi_processor_count * 3200 + extra
+    cmb = _ddc(nRows, [longest, 300, 257, longest, 1000, 512], longest + extra, const=True).to_device()
+    _check(cmb, ks=(1,), qs=(1, 2))
+    cmb.free()
