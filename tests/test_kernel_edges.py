@@ -7,7 +7,7 @@ from systemds_b200 import CompressedMatrixBlock, datagen
 from systemds_b200 import colgroup as cg
 from systemds_b200.cmb import CHAIN_XtwXv, CLALibDecompress, CLALibLeftMultBy, CLALibMMChain, CLALibRightMultBy, CLALibTSMM
 from systemds_b200.mapping import MapToFactory
-from tests.util import TOL, dense_of, rel_err
+from tests.util import TOL, abs_dense_of, dense_of, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -231,6 +231,27 @@ def test_decompress_by_columns(nRows):
     assert rel_err(got, X.T @ X, np.abs(X).T @ np.abs(X) + 1e-300) < TOL
     _check(cmb, ks=(1, 3), chain=False)
     assert np.array_equal(np.array(CLALibDecompress.decompress(cmb)), X)
+    cmb.free()
+
+
+def test_decompress_by_columns_with_references():
+    """Columns held by a group and by the constant group of its reference tuple: a cell is the sum of both. Such a block adds
+    the folded constants in every column: c + (d - c) for an SDC column with default c. The difference and the sum round
+    once each, so a cell is off by at most eps / 2 times |d - c| + |d| <= eps (|d| + |c|)."""
+    nRows, rng = 18817, np.random.default_rng(3)
+    cmb = _by_kind(nRows)
+    groups, c = list(cmb.getColGroups()), cmb.clen
+    for i in range(63):
+        groups.append(datagen.random_group("sdcfor" if i < 32 else "ddcfor", [c], nRows, rng))
+        c += 1
+    cmb = CompressedMatrixBlock(nRows, c, groups)
+    X, scale = dense_of(cmb), abs_dense_of(cmb) + 1e-300
+    for g in groups:
+        if getattr(g, "_defaultTuple", None) is not None:
+            scale[:, g.getColIndices()] += np.abs(g._defaultTuple)
+    cmb.to_device()
+    for _ in range(2):
+        assert rel_err(np.array(CLALibDecompress.decompress(cmb)), X, scale) <= 1.01 * np.finfo(float).eps
     cmb.free()
 
 

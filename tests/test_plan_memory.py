@@ -6,7 +6,7 @@ import pytest
 from systemds_b200 import CompressedMatrixBlock, datagen, native
 from systemds_b200.cmb import CLALibDecompress, CLALibTSMM
 from systemds_b200.native import check
-from tests.test_kernel_edges import _check, _ddc
+from tests.test_kernel_edges import _by_kind, _check, _ddc
 from tests.util import TOL, dense_of, rel_err
 
 
@@ -30,7 +30,8 @@ BLOCKS = {
     "cocoded": lambda: _cocoded(4161),
     "wide dense": lambda: _wide_dense(4127),
     "16-bit maps": lambda: _ddc(17001, [300, 1000, 5000, 257], 3, const=True),
-    "tall": lambda: datagen.random_cmb(9, 70001, ("ddc", "sdcz", "rle", "unc") * 16),  # decompress by columns from 4 million cells
+    "mixed kinds side by side": lambda: datagen.random_cmb(9, 70001, ("ddc", "sdcz", "rle", "unc") * 16),
+    "a kind per 32 columns": lambda: _by_kind(18817),  # decompress by columns
 }
 
 
