@@ -194,8 +194,9 @@ constexpr int VSTEP = 32;  // rows of a warp step: one 16-row block per half-war
 // dependent launch), and stores the result: nothing to clear beforehand. (Left to the last CTA of a chunk, without a second
 // launch: 18.2 instead of 14.3 us for the chain on 50,000 x 100, 17.6 instead of 14.2 for t(y) X on 250,000 x 40 -- one
 // CTA reads 148 partial rows too slowly.)
-// Measured (10M x 200, 256 values): 644 us, 3.2 TB/s; the one-row-step form before, with three instructions per address,
-// a clear, a separately launched sum, 670 us. 100,000 x 500: 36.9 -> 30.5 us, 5000 x 500: 15.4 -> 10.4.
+// Measured (10M x 200, 256 values): 634 us, 3.3 TB/s, on a box where the one-row-step form before, with three instructions
+// per address, a clear and a separately launched sum, took 685 (670 and 697 on another box).
+// 100,000 x 500: 36.9 -> 30.5 us, 5000 x 500: 15.4 -> 10.4.
 // --------------------------------------------------------------------------------------------------
 struct LmmArgs {
   const int2* units;           // {table offset / 16, depth}
@@ -370,7 +371,7 @@ __global__ void __launch_bounds__(LMM_T, 1) k_lmm_vec(const __grid_constant__ Lm
 
 // --------------------------------------------------------------------------------------------------
 // LMM with Q left rows at once (Q = 2 or 4; the reference's left-multiply blocks four rows too,
-// lib/CLALibLeftMultBy.java:731-819). Same layout and lookups as k_lmm_vec_u8, but a dictionary value fetched for a
+// lib/CLALibLeftMultBy.java:731-819). Same layout and lookups as k_lmm_vec, but a dictionary value fetched for a
 // cell multiplies the cell's Q left values: one pass over the maps and one lookup per cell serve Q rows, where Q
 // passes of the one-row kernel would fetch each value Q times. partial: [gridDim.x][Q][LMM_PART].
 // --------------------------------------------------------------------------------------------------
@@ -711,7 +712,7 @@ __global__ void __launch_bounds__(512) k_lmm_rows_final(const __grid_constant__ 
 // --------------------------------------------------------------------------------------------------
 // Decompress from the column-per-lane layout.
 //
-// Same chunks, interleaved maps and table images as k_lmm_vec_u8: lane s of a half-warp owns column slot s of a
+// Interleaved maps and table images of k_lmm_vec, chunks of units fixed at plan time: lane s of a half-warp owns column slot s of a
 // unit, loads 16 rows of its ids with one 128-bit load, reads each value from its own bank pair of the unit's
 // table and stores it. The 16 slots of a unit are 16 neighbouring output columns (the plan orders the slots by
 // column), so a warp store writes two full 128-byte pieces of two rows: no transposition through shared memory,

@@ -1,14 +1,14 @@
-// General product kernels: they accept every group type, any number of right-hand columns / left
-// rows, and overlapping groups. The specialised kernels in cla_fast.cu take over for the shapes
-// they cover; everything else runs here.
+// Decompress, X %*% V kept compressed, and the general product kernels: every group type, any number of left rows,
+// overlapping groups, from the registered arrays alone. The products come here where the kernels of cla_fast.cu,
+// cla_rest.cu and cla_small.cu cannot run because their row lists or plans do not exist: 32-bit positions, device memory or
+// the handle's plan limit have no room.
 //
 //   RMM  (CLALibRightMultBy.RMM, lib/CLALibRightMultBy.java:208-258)
 //        1. k_dict_times_v : P_g = D_g * V[cols_g, :] for every dictionary group
 //                            (ADictBasedColGroup.rightMultByMatrix, colgroup/ADictBasedColGroup.java:246-275)
 //        2. k_rmm_vec_general : one right-hand column; a CTA owns a block of output rows and sums
 //                            P_g[id_g(r)] over all groups, then adds constV * v (the decompress-and-sum of
-//                            lib/CLALibDecompress.java:310-357). Wider right-hand sides run on the FP64
-//                            tensor cores (cla_rmm_dmma.cu) or, for a few columns, once per column.
+//                            lib/CLALibDecompress.java:310-357). More right-hand columns: cla_rmm_dmma.cu.
 //   LMM  (CLALibLeftMultBy.LMM, lib/CLALibLeftMultBy.java:286-346)
 //        1. k_lmm_preagg   : A_g[i, k] = sum of Yt[i, r] over rows r holding tuple k
 //                            (APreAgg.preAggregateDense, colgroup/APreAgg.java:137)

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(RL_T, 2) k_rest_lmm(const __grid_constant__ Re
   extern __shared__ __align__(16) unsigned char rlsm[];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int nA = A.nChunks * A.ctaTasks;
-  // the two kinds are interleaved so that both are resident from the start
+  // (the launcher aims at no more CTAs than are resident at once, so that the second kind does not wait for the first)
   int b = blockIdx.x;
   if (b < nA) rest_lmm_tasks<QT>(A, b / A.ctaTasks, b % A.ctaTasks, rlsm);
   else {
@@ -452,9 +452,6 @@ __global__ void __launch_bounds__(256) k_rest_lmm_final(const __grid_constant__ 
   }
 }
 
-// --------------------------------------------------------------------------------------------------
-// plan and launchers
-// --------------------------------------------------------------------------------------------------
 // --------------------------------------------------------------------------------------------------
 // Yt X over 16-bit maps from TL_ROWS rows on: a CTA keeps the tables of up to sixteen columns in shared memory and walks a
 // range of rows, a warp (or several, where long tables leave fewer columns) per column, lanes along the rows.
@@ -603,6 +600,9 @@ __global__ void __launch_bounds__(256) k_table_lmm_final(const __grid_constant__
   if (lane == 0 && i < A.q) atomicAdd(&A.out[(size_t)i * A.nCols + A.tasks[task].col], s);  // (several groups may hold a column)
 }
 
+// --------------------------------------------------------------------------------------------------
+// plan and launchers
+// --------------------------------------------------------------------------------------------------
 static int64_t ensure_rest(Matrix* m, cudaStream_t s) {
   RestPlan& R = m->rest;
   if (R.tried) return CLA_OK;

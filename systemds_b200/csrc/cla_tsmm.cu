@@ -659,9 +659,8 @@ int64_t measure_fp64_peaks(int device, double* dmmaTflops, double* dfmaTflops) {
   return CLA_OK;
 }
 
-// The 16-warp kernel is instantiated for the map widths the decode specialises on and, by tile slots per warp, for
-// 3, 6 and 9 slots of 8 x 8 tiles (up to 48, 104 and 128 columns; rows read from a decompressed chunk) and for 2 and 5
-// slots of 16 x 8 tiles (up to 64 and 128 columns; decoded on the fly).
+// The 16-warp kernel is instantiated for the map widths the decode specialises on and for 2, 4 and 5 slots of 16 x 8 tiles
+// per warp (up to 80, 120 and 128 columns), decoded on the fly or read from a decompressed chunk.
 template <int TPW>
 static void tri16_go(bool fused, int mt, int simple, int grid, size_t smem, cudaStream_t s, const DevGroup* groups,
                      const int32_t* colSrc, const double* constV, const double* X, int rows, int n, double* dOut, int32_t* err) {
