@@ -350,7 +350,7 @@ int64_t ensure_sparse_list(Matrix* m);  // Matrix::dSparseIdx (cla_generic.cu)
 
 int64_t ensure_col_plan(Matrix* m);                        // Matrix::cols; cols.ok tells whether it exists
 int64_t sdc_items_bytes(const Matrix* m);                  // size of Matrix::sdcItems; -1: they cannot exist
-int64_t fill_sdc_items(Matrix* m, uint32_t* items, cudaStream_t s);  // builds Matrix::sdcItems in `items`
+void launch_sdc_items(Matrix* m, uint32_t* items, cudaStream_t s);  // fills them into `items`
 int64_t ensure_row_lists(Matrix* m, cudaStream_t s);       // Matrix::rows and sdcItems; rows.ok tells whether they exist
 // The groups the specialised kernels leave (cla_rest.cu): 1 = done, 0 = not covered (the general kernels then run)
 int64_t rest_rmm(Matrix* m, const double* dV, double* dOut, const double* dW, cudaStream_t s, bool addTo);

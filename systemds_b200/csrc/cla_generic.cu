@@ -523,9 +523,9 @@ k_decomp_block(const DevGroup* __restrict__ groups, const int32_t* __restrict__ 
 // block itself for an uncompressed one. Each cell is formed in the register it is stored from, and the warps of a CTA
 // write whole stretches of a row at the same time. The tile kernel above builds every cell in shared memory and reads
 // it back. What is left is the latency of the chains item -> value and run -> value.
-// The records and the items of a block are filled on the device in its first call, nothing is copied or waited for (row
-// lists, which hold the items too, take 350 us). 250,001 x 500 mixed (1 GB), tile kernel against this one: 495 -> 320 us, 3.1
-// TB/s written; first call on a block 539 -> 399 us, host time included.
+// The records and the items of a block are filled on the device in its first call, without a copy (row lists, which hold the
+// items too, take 350 us). 250,001 x 500 mixed (1 GB), tile kernel against this one: 495 -> 320 us, 3.1
+// TB/s written; first call on a block 534 -> 403 us, host time included.
 struct DecCol {
   const double* dict;  // dictionary (or dense block) + position in the group
   const void* a;       // byte / bit map; SDC items; RLE runs
@@ -717,23 +717,34 @@ void decomp_shape(Matrix* m, const int32_t* colSrc) {
   }
 }
 
-// The records of k_decomp_cols and the items of the SDC columns; m->dec.warps becomes 0 where there is no room for them. Nothing
-// is copied or waited for: the device fills them.
+// The records of k_decomp_cols and the items of the SDC columns, m->dec.cols; without them the tile kernel runs. m->dec.warps becomes 0
+// where there is no room for them. The device fills them, no host copy; they are complete when the handle has them, so that a
+// call on any stream may use them.
 static int64_t ensure_dec(Matrix* m, cudaStream_t s) {
   DecPlan& D = m->dec;
   if (D.cols || D.warps == 0) return CLA_OK;
   const int warps = D.warps;
+  // (a call that is being captured runs nothing yet, so it cannot build a plan)
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) {
+    cudaGetLastError();
+    return CLA_OK;
+  }
+  if (capture != cudaStreamCaptureStatusNone) return CLA_OK;
   const int64_t itemBytes = m->sdcItemsOk ? 0 : sdc_items_bytes(m);
   const size_t at = ((size_t)m->nCols * sizeof(DecCol) + 255) & ~(size_t)255;
   void* p = nullptr;
   D.warps = 0;
   if (itemBytes < 0 || plan_alloc(m, &p, at + (size_t)itemBytes) < 0) return CLA_OK;
-  int64_t rc;
-  if (!m->sdcItemsOk && (rc = fill_sdc_items(m, (uint32_t*)((char*)p + at), s)) < 0) return rc;
+  uint32_t* items = m->sdcItemsOk ? m->sdcItems : (uint32_t*)((char*)p + at);
+  if (!m->sdcItemsOk) launch_sdc_items(m, items, s);
   k_dec_cols<<<(m->nCols + warps * 32 - 1) / (warps * 32), warps * 32, 0, s>>>(
-      m->dGroups, m->dColSrc, m->hasConst ? m->dConstV : nullptr, m->sdcItems, (DecCol*)p, m->nCols, m->multiCover ? 0 : 1);
+      m->dGroups, m->dColSrc, m->hasConst ? m->dConstV : nullptr, items, (DecCol*)p, m->nCols, m->multiCover ? 0 : 1);
   m->stats.kernel_launches++;
   CLA_CUDA(cudaGetLastError());
+  CLA_CUDA(cudaStreamSynchronize(s));
+  m->sdcItems = items;
+  m->sdcItemsOk = true;
   D.cols = p;
   D.warps = warps;
   return CLA_OK;
@@ -748,16 +759,16 @@ int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStr
     const int64_t rf = fast_decompress(m, r0, r1, dOut, s, ld);  // byte-map matrices: straight from the column-per-lane layout
     if (rf != 0) return rf < 0 ? rf : CLA_OK;
     int64_t rc;
-    // Below DC_CELLS both kernels take the same time (8,400 x 500: 32 us). Records and items cost a block's first call 25 to 40
-    // us, which its kernel makes up for from DC_FIRST on (12 million cells: 117 us against 96 with the tile kernel, 24: 143
-    // against 147, 125: 399 against 539); a smaller block gets them when it is decompressed again (12 million: 58 against 66).
+    // Below DC_CELLS both kernels take the same time (8,400 x 500: 32 us). Records and items cost a call 30 to 40 us,
+    // which a block's first call makes up for from DC_FIRST on (24 million cells: 147 us as with the tile kernel, 33: 177 against
+    // 183, 125: 403 against 534); a smaller block gets them when it is decompressed again (12 million: 58 against 66 from then on).
     bool byCols = n >= DC_CELLS;
     if (byCols && !m->dec.cols) {
       byCols = m->dec.again || (int64_t)m->nRows * m->nCols >= DC_FIRST;
       m->dec.again = true;
     }
     if (byCols && (rc = ensure_dec(m, s)) < 0) return rc;
-    if (byCols && m->dec.warps > 0) {
+    if (byCols && m->dec.cols) {
       static OncePerDevice once;
       if (const int64_t e = allow_smem(once, m->device, DC_TBL, k_decomp_cols); e < 0) return e;
       dim3 grid((r1 - r0 + DC_ROWS - 1) / DC_ROWS, (m->nCols + m->dec.warps * 32 - 1) / (m->dec.warps * 32));

@@ -50,7 +50,6 @@ void plan_release(Matrix* m, void* p, size_t bytes) {
 int64_t ensure_col_plan(Matrix* m) {
   ColPlan& cp = m->cols;
   if (cp.tried) return CLA_OK;
-  cp.tried = true;
   std::vector<ColRef> dense, all;
   for (size_t hi = 0; hi < m->hg.size(); hi++) {
     const int gi = m->regToDev[hi];
@@ -82,14 +81,17 @@ int64_t ensure_col_plan(Matrix* m) {
   if (ba) memcpy(blob.data() + bd, all.data(), ba);
   memcpy(blob.data() + bd + ba, ptr.data(), bp);
   void* d = nullptr;
-  if (plan_alloc(m, &d, blob.size()) < 0) return CLA_OK;
+  if (plan_alloc(m, &d, blob.size()) < 0) {
+    cp.tried = true;
+    return CLA_OK;
+  }
   CLA_CUDA(cudaMemcpy(d, blob.data(), blob.size(), cudaMemcpyHostToDevice));
   cp.dense = (ColRef*)d;
   cp.refs = (ColRef*)((char*)d + bd);
   cp.refPtr = (int32_t*)((char*)d + bd + ba);
   cp.nDense = (int)dense.size();
   cp.nRefs = (int)all.size();
-  cp.ok = true;
+  cp.tried = cp.ok = true;
   return CLA_OK;
 }
 
@@ -196,7 +198,7 @@ k_row_lists(const DevGroup* __restrict__ groups, const int32_t* __restrict__ lis
 }
 
 // The items alone, where nothing needs the rows' lists: a warp per group and 1024-row block. An item's place follows from
-// the group's element number, so nothing is counted and nothing waited for.
+// the group's element number, so there is no counting pass.
 constexpr int SDC_ITEM_VALS = 1 << 22;  // an item holds 22 bits of tuple
 __global__ void __launch_bounds__(RL_THREADS) k_sdc_items(const DevGroup* __restrict__ groups, int nDev, int nRows, uint32_t* __restrict__ items) {
   const int perBlock = (nDev + RL_THREADS / 32 - 1) / (RL_THREADS / 32), blk = blockIdx.x / perBlock;
@@ -220,16 +222,11 @@ int64_t sdc_items_bytes(const Matrix* m) {
     }
   return n * 4;
 }
-int64_t fill_sdc_items(Matrix* m, uint32_t* items, cudaStream_t s) {
-  if (sdc_items_bytes(m) > 0) {
-    const unsigned grid = (unsigned)((m->nRows + SKIP_ROWS - 1) / SKIP_ROWS) * (unsigned)((m->nDev + RL_THREADS / 32 - 1) / (RL_THREADS / 32));
-    k_sdc_items<<<grid, RL_THREADS, 0, s>>>(m->dGroups, m->nDev, m->nRows, items);
-    m->stats.kernel_launches++;
-    CLA_CUDA(cudaGetLastError());
-  }
-  m->sdcItems = items;
-  m->sdcItemsOk = true;
-  return CLA_OK;
+void launch_sdc_items(Matrix* m, uint32_t* items, cudaStream_t s) {
+  if (sdc_items_bytes(m) <= 0) return;
+  const unsigned grid = (unsigned)((m->nRows + SKIP_ROWS - 1) / SKIP_ROWS) * (unsigned)((m->nDev + RL_THREADS / 32 - 1) / (RL_THREADS / 32));
+  k_sdc_items<<<grid, RL_THREADS, 0, s>>>(m->dGroups, m->nDev, m->nRows, items);
+  m->stats.kernel_launches++;
 }
 
 int64_t ensure_row_lists(Matrix* m, cudaStream_t s) {

@@ -471,8 +471,7 @@ void wide_plan_free(Matrix* m) {
 static int64_t ensure_wide(Matrix* m, int NT, cudaStream_t s) {
   if (!m->wide) m->wide = new WidePlan();
   if (m->wide->nt[NT].tried) return CLA_OK;
-  m->wide->nt[NT].tried = true;
-  WidePlanNT W;  // takes its place in the handle when it is complete
+  WidePlanNT W;  // takes its place in the handle when it is complete (after an error the next call tries again)
   W.tried = true;
   std::vector<WideCol> kind[4];
   for (size_t hi = 0; hi < m->hg.size(); hi++) {
@@ -588,7 +587,10 @@ static int64_t ensure_wide(Matrix* m, int NT, cudaStream_t s) {
   const size_t bc = (cols.size() * sizeof(WideCol) + 255) & ~(size_t)255;
   const size_t bi = ((size_t)img * 8 + 255) & ~(size_t)255, bs = ((size_t)W.nSp * 4 + 255) & ~(size_t)255;
   const size_t bl = ((size_t)m->nCols * 4 + 255) & ~(size_t)255, bv = W.nSp ? (size_t)m->rows.nSv * sizeof(WideSv) : 0;
-  if (plan_alloc(m, &d, bc + bi + bs + bl + bv) < 0) return CLA_OK;
+  if (plan_alloc(m, &d, bc + bi + bs + bl + bv) < 0) {
+    m->wide->nt[NT].tried = true;
+    return CLA_OK;
+  }
   W.spCols = (int32_t*)((char*)d + bc + bi);
   W.sv = (WideSv*)((char*)d + bc + bi + bs + bl);
   if (W.nSp) {

@@ -255,6 +255,28 @@ def test_decompress_by_columns_with_references():
     cmb.free()
 
 
+def test_decompress_first_called_in_a_capture():
+    """A captured call leaves no plan that only its replay would fill: direct calls and replays after it are right."""
+    import torch
+    from systemds_b200 import native
+    cmb = _by_kind(93313)
+    X = torch.from_numpy(dense_of(cmb)).cuda()
+    cmb.to_device()
+    lib, h = native.lib(), cmb.handle()
+    out, stream, graph = torch.empty_like(X), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        native.check(lib.cla_decompress_dev(h, out.data_ptr(), stream.cuda_stream))
+    with torch.cuda.stream(stream):
+        for call in (lambda: native.check(lib.cla_decompress_dev(h, out.data_ptr(), stream.cuda_stream)), graph.replay) * 2:
+            out.zero_()
+            call()
+            stream.synchronize()
+            assert torch.equal(out, X)
+    del graph
+    cmb.free()
+
+
 @pytest.mark.parametrize("nCols", [128, 129, 300, 448, 449])
 @pytest.mark.parametrize("nRows", [77, 1000])
 def test_short_blocks_with_v_in_the_launch(nRows, nCols):
