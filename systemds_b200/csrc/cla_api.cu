@@ -867,8 +867,8 @@ int64_t cla_unary_agg(cla_handle h, int32_t op, double* out) {
   if (op >= CLA_AGG_COL_MINS) {
     CLA_CUDA(cudaSetDevice(m->device));
     std::vector<double> lo, hi;
-    int64_t rc = col_minmax(m, lo, hi, m->stream);
-    if (rc < 0) return rc;
+    int64_t rc = order_begin(m, m->stream);  // its scratch may be in use by a call on another stream
+    if (rc < 0 || (rc = col_minmax(m, lo, hi, m->stream)) < 0) return rc;
     if ((rc = check_errword(m)) < 0) return rc;
     const bool wantMax = (op == CLA_AGG_COL_MAXS || op == CLA_AGG_MAX);
     const std::vector<double>& v = wantMax ? hi : lo;
