@@ -54,16 +54,24 @@ constexpr int JS_MAX = 8;
 struct JointSlot {
   int32_t n;              // groups (0: unused slot)
   int32_t total;          // joint tuples
+  int32_t split, nLo;     // groups 0..split-1 are the low part of the joint id, nLo tuples
   int32_t group[JS_MAX];  // device group indices
   int32_t nv[JS_MAX];
 };
-struct JointGroup {  // the i-th group of a slot, what its table is built from
-  const double* dict;
-  const int32_t* cols;
-  int32_t nv, gCols, col, pad;
+// One term D_g[a] v of a slot's table, its groups one after the other: a value times v[col], or for a group of several
+// columns (gCols > 0) the tuple at dict.
+struct JointTerm {
+  union {
+    double val;
+    const double* dict;
+  };
+  union {
+    int64_t col;  // -1: behind the slot's last term
+    const int32_t* cols;
+  };
 };
-constexpr int JS_TERMS = 132;   // terms of a slot with two or more groups: at most 2 + 128
-constexpr int JOINT_UNITS = 6;  // units per chunk: their tables and two units' terms fit shared memory
+constexpr int JOINT_UNITS = 6;  // units per chunk, at most
+constexpr int JOINT_TAIL = 4;   // so many slots behind the last whole unit go by rows instead of taking a unit
 struct FastPlan {
   bool ok = false;
   bool partial = false;      // only some groups are covered; the general kernels add the rest
@@ -86,8 +94,12 @@ struct FastPlan {
   size_t imageDoubles = 0;
   // X v on joint slots
   int nJU16 = 0;                       // 0: not worth it, the column slots serve X v too
+  int jTail = 0;                       // slots of the last unit that go by rows (0: it is a unit like the others)
+  int jParts = 0;                      // sums of parts of a slot, at most
   JointSlot* dJSlots = nullptr;        // [nJU16 * 16]
-  JointGroup* dJGroups = nullptr;      // [nJU16 * 16][JS_MAX]
+  JointTerm* dJTerms = nullptr;        // [nJU16][jTerms][16]
+  int* dJTermCols = nullptr;           // the same places: columns of the group, 0: one
+  int jTerms = 0, jJoinTerms = 0;      // terms of a slot, of one of two or more groups, at most
   std::vector<int> jNk;
   int2* dJUnits = nullptr;
   uint8_t* dJMaps = nullptr;
@@ -165,6 +177,11 @@ __device__ __forceinline__ bool tma_reload(void* dst, const void* src, uint32_t 
         : "memory");
   }
   return __syncthreads_and(done != 0) != 0;
+}
+
+// bytes (a multiple of 16) from p (aligned to 16) to L2
+__device__ __forceinline__ void l2_fetch(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes));
 }
 
 __device__ __forceinline__ double lds_f64(uint32_t addr) {
@@ -845,22 +862,24 @@ __device__ __forceinline__ double one_if(int a, int b) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, %2;\n\tselp.f64 %0, 0d3FF0000000000000, 0d0000000000000000, p;\n\t}" : "=d"(r) : "r"(a), "r"(b));
   return r;
 }
-// Sums acc[i] over the 16 lanes of each half-warp: lane 4 g returns the sums of row g of the lower half-warp (s0) and of
-// the upper one (s1); the other lanes return nothing of use.
-__device__ __forceinline__ void half_warp_sums(const double (&acc)[8], double& s0, double& s1) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  // C[m][n] = sum over the four lanes of quad n of acc[m]: B = acc[i], A_i = 1 in row i (two chains of four products)
-  double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+// Sums acc[i] over the 16 lanes of each half-warp, over quads of lanes by products with 0 / 1 matrices (C[m][n] = sum over the four
+// lanes of quad n of acc[m]: B = acc[i], A_i = 1 in row i; the lower half-warp's quads are 0..3) and over two pairs of quads by one shuffle: lane
+// 4 g + t returns row g of the lower half-warp where t < 2, of the upper one otherwise.
+__device__ __forceinline__ double half_warp_sums(const double (&acc)[8]) {
+  const int g = (threadIdx.x & 31) >> 2;
+  double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};  // two chains of four products
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     dmma884(c[0][0], c[0][1], one_if(g, i), acc[i]);
     dmma884(c[1][0], c[1][1], one_if(g, i + 4), acc[i + 4]);
   }
-  // quads 0..3 are the lower half-warp: sum C over n into column 0 for them and into column 1 for the others
-  const double sel = one_if(g, t >> 1);
-  s0 = s1 = 0.0;
-  dmma884(s0, s1, c[0][0] + c[1][0], sel);
-  dmma884(s0, s1, c[0][1] + c[1][1], sel);
+  const double s = (c[0][0] + c[0][1]) + (c[1][0] + c[1][1]);
+  return s + __shfl_xor_sync(0xffffffffu, s, 1);
+}
+// The row of a step of 32 whose sum this lane holds afterwards: t odd for the second eight rows of a block.
+__device__ __forceinline__ int sum_row() {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  return (t >> 1) * 16 + (t & 1) * 8 + g;
 }
 
 struct RmmArgs {
@@ -870,7 +889,12 @@ struct RmmArgs {
   const double* tables;    // column slots
   const int* slotCol;
   const JointSlot* joint;  // joint slots
-  const JointGroup* jointGroups;
+  const JointTerm* terms;
+  const int* termCols;     // null: all groups have one column
+  int nTerms, joinTerms;   // terms of a slot, of one of two or more groups, at most
+  int U;                   // units per chunk
+  int tail;                // slots behind them that go by rows
+  int partRows, pairs;     // see joint_tables: rows of 32 slots before their tables, at most; pairs of units that have room for them
   const double* v;
   const double* constV;    // null: none
   int nCols;
@@ -881,88 +905,67 @@ struct RmmArgs {
   int32_t* err;
 };
 
-// The sums of step `st` again, for a warp that saw an Inf or NaN: every row by itself, with shuffles. Lane 4 g + t, t < 2,
-// returns rows 8 t + g of the two blocks.
-__device__ __noinline__ double2 rmm_step_by_rows(const uint8_t* mp, size_t ustr, const int2* units, const int* slotCol,
-                                                 const double* v, int64_t stride, int nu, uint32_t table0) {
-  const int lane = threadIdx.x & 31, slot = lane & 15, g = lane >> 2, t = lane & 3;
-  double2 r = make_double2(0.0, 0.0);
+// The sums of step `st` again, for a warp that saw an Inf or NaN: every row by itself, with shuffles. v null: joint slots.
+__device__ __noinline__ double rmm_step_by_rows(const uint8_t* mp, size_t ustr, const int2* units, const int* slotCol,
+                                                const double* v, int64_t stride, int nu, uint32_t table0) {
+  const int lane = threadIdx.x & 31, slot = lane & 15, row = sum_row();
+  double r = 0.0;
   for (int i = 0; i < 16; i++) {
     double a = 0.0;
     for (int u = 0; u < nu; u++) {
-      const int col = slotCol[u * 16 + slot];
-      if (col >= 0)
-        a = fma(lds_f64(table0 + (uint32_t)(units[u].x - units[0].x) * 128u + slot * 8 + 128u * mp[u * ustr + i]), v[col * stride], a);
+      const double x = lds_f64(table0 + (uint32_t)(units[u].x - units[0].x) * 128u + slot * 8 + 128u * mp[u * ustr + i]);
+      if (!v) a += x;
+      else if (const int col = slotCol[u * 16 + slot]; col >= 0) a = fma(x, v[col * stride], a);
     }
     for (int d = 1; d < 16; d <<= 1) a += __shfl_xor_sync(0xffffffffu, a, d);
     const double other = __shfl_xor_sync(0xffffffffu, a, 16);
-    if (i == (t & 1) * 8 + g) r = lane < 16 ? make_double2(a, other) : make_double2(other, a);
+    if (i == (row & 15)) r = (lane >> 4) == (row >> 4) ? a : other;
   }
   return r;
 }
 
-// Row sums of one step from its id words: lane 4 g + t, t < 2, returns those of rows 8 t + g of the two half-warps' blocks.
-// JOINT: the terms are the table entries themselves, and the reduction is one of shuffles -- with four units or so per
-// step the products with 0 / 1 matrices would keep the FP64 pipe as long as the lookups take (1M x 100, 16 values:
-// 43.6 us with products).
+// Row sums of one step from its id words, this lane's as sum_row says. JOINT: the terms are the table entries themselves.
+// (Joint slots with a reduction of shuffles alone: 30 of the 150 wavefronts of a step of three units; 40.4 against 38.0 us for 1M x 100 of
+// 16 values, cold.)
 template <int NU, bool JOINT, int UNROLL_ROWS>
-__device__ __forceinline__ void step_sums(const uint4 (&m)[NU], const uint32_t (&tb)[NU], const double (&v)[NU], double& r0, double& r1) {
-  const int lane = threadIdx.x & 31;
-  if constexpr (JOINT) {
-    const int slot = lane & 15;
-    double acc[16];
+__device__ __forceinline__ double step_sums(const uint4 (&m)[NU], const uint32_t (&tb)[NU], const double (&v)[NU]) {
+  double r = 0.0;
+#pragma unroll UNROLL_ROWS
+  for (int h = 0; h < 2; h++) {  // rows 0..7 and 8..15 of each half-warp's block
+    double acc[8];
 #pragma unroll
-    for (int i = 0; i < 16; i++) acc[i] = 0.0;
+    for (int i = 0; i < 8; i++) acc[i] = 0.0;
 #pragma unroll
     for (int u = 0; u < NU; u++) {
-      const uint32_t ww[4] = {m[u].x, m[u].y, m[u].z, m[u].w};
+      const uint32_t w0 = h ? m[u].z : m[u].x, w1 = h ? m[u].w : m[u].y;
 #pragma unroll
-      for (int i = 0; i < 16; i++) acc[i] += lds_f64(entry_at(ww[i >> 2], i & 3, tb[u]));
-    }
-    // reduce-scatter over the half-warp: after the stage with distance d, a lane keeps the rows whose bit d equals its
-    // own slot bit
-#pragma unroll
-    for (int d = 8; d >= 1; d >>= 1) {
-      const bool up = (slot & d) != 0;
-#pragma unroll
-      for (int i = 0; i < d; i++) {
-        const double lo = acc[i], hi = acc[i + d];
-        const double recv = __shfl_xor_sync(0xffffffffu, up ? lo : hi, d);
-        acc[i] = (up ? hi : lo) + recv;
+      for (int i = 0; i < 8; i++) {
+        const double x = lds_f64(entry_at(i < 4 ? w0 : w1, i & 3, tb[u]));
+        acc[i] = JOINT ? acc[i] + x : fma(x, v[u], acc[i]);
       }
     }
-    r0 = acc[0];  // lane s of a half-warp holds row s of its block
-    r1 = 0.0;
-  } else {
-    const int t = lane & 3;
-#pragma unroll UNROLL_ROWS
-    for (int h = 0; h < 2; h++) {  // rows 0..7 and 8..15 of each half-warp's block
-      double acc[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) acc[i] = 0.0;
-#pragma unroll
-      for (int u = 0; u < NU; u++) {
-        const uint32_t w0 = h ? m[u].z : m[u].x, w1 = h ? m[u].w : m[u].y;
-#pragma unroll
-        for (int i = 0; i < 8; i++) acc[i] = fma(lds_f64(entry_at(i < 4 ? w0 : w1, i & 3, tb[u])), v[u], acc[i]);
-      }
-      double d0, d1;
-      half_warp_sums(acc, d0, d1);
-      if (h == 0) r0 = d0, r1 = d1;
-      else {  // rows 8..15 go to the lanes t = 1
-        d0 = __shfl_up_sync(0xffffffffu, d0, 1);
-        d1 = __shfl_up_sync(0xffffffffu, d1, 1);
-        if (t == 1) r0 = d0, r1 = d1;
-      }
-    }
+    const double s = half_warp_sums(acc);
+    if ((threadIdx.x & 1) == h) r = s;
   }
+  return r;
 }
+
+// Ids of units [unit0, unit0 + nu) for the steps [from, from + n), clipped to s1, to L2: warp u takes unit u.
+__device__ __forceinline__ void rmm_fetch(const RmmArgs& A, int unit0, int nu, int64_t from, int64_t n, int64_t s1) {
+  const int warp = threadIdx.x >> 5;
+  n = min(n, s1 - from);
+  if (warp < nu && (threadIdx.x & 31) == 0 && n > 0)
+    l2_fetch(A.imaps + ((size_t)(unit0 + warp) * A.nRB + (size_t)from * 2) * 256, (uint32_t)n * 512u);
+}
+// Turns of the warps whose ids are on their way to L2: about 200 KB per SM, more than the memory's latency takes. (625,000 x 1000: 255 us
+// without, 236 with.)
+__host__ __device__ constexpr int rmm_ahead(int nu) { return 24 / nu; }
 
 template <int NU, bool JOINT>
 __device__ __forceinline__ void rmm_rows(const RmmArgs& A, int unit0, int64_t s0, int64_t s1, double init, bool first, bool last,
-                                         uint32_t table0) {
+                                         uint32_t table0, uint32_t tail0) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int slot = lane & 15, half = lane >> 4, g = lane >> 2, t = lane & 3;
+  const int slot = lane & 15, half = lane >> 4, rowOf = sum_row();
   uint32_t tb[NU];
   double v[NU];
 #pragma unroll
@@ -981,86 +984,111 @@ __device__ __forceinline__ void rmm_rows(const RmmArgs& A, int unit0, int64_t s0
     uint4 m[NU];
 #pragma unroll
     for (int u = 0; u < NU; u++) m[u] = __ldg((const uint4*)(mp + u * ustr + st * 512));
-    const int64_t row = st * VSTEP + (JOINT ? lane : (t & 1) * 8 + g);
-    const bool mine0 = (JOINT || t < 2) && row < A.nRows, mine1 = !JOINT && t < 2 && row + 16 < A.nRows;
-    double o0 = init, o1 = init;  // what these rows hold from the chunks before
-    if (!first) {
-      o0 = mine0 ? A.out[row * A.stride] : 0.0;
-      o1 = mine1 ? A.out[(row + 16) * A.stride] : 0.0;
-    }
-    double r0, r1;
-    step_sums<NU, JOINT, 2>(m, tb, v, r0, r1);
-    if (!JOINT && __any_sync(0xffffffffu, t < 2 && !(isfinite(r0) && isfinite(r1)))) {
-      const double2 r = rmm_step_by_rows(mp + st * 512, ustr, A.units + unit0, A.slotCol + unit0 * 16, A.v, A.stride, NU, table0);
-      r0 = r.x, r1 = r.y;
-    }
-    r0 += o0;
-    r1 += o1;
-    if (last && A.rowScale) {
-      if (mine0) r0 *= A.rowScale[row];
-      if (mine1) r1 *= A.rowScale[row + 16];
-    }
-    if (mine0) A.out[row * A.stride] = r0;
-    if (mine1) A.out[(row + 16) * A.stride] = r1;
+    rmm_fetch(A, unit0, NU, st - warp + rmm_ahead(NU) * RB_W, RB_W, s1);
+    const int64_t row = st * VSTEP + rowOf;
+    const bool mine = row < A.nRows;
+    uint32_t tailId[JOINT_TAIL];
+    if (JOINT && last)
+#pragma unroll
+      for (int b = 0; b < JOINT_TAIL; b++)
+        if (b < A.tail) tailId[b] = __ldg(A.imaps + ((size_t)(unit0 + NU) * A.nRB + (size_t)st * 2 + (rowOf >> 4)) * 256 + b * 16 + (rowOf & 15));
+    double o = init;  // what this row holds from the chunks before
+    if (!first) o = mine ? A.out[row * A.stride] : 0.0;
+    double r = step_sums<NU, JOINT, 2>(m, tb, v);
+    if (__any_sync(0xffffffffu, !isfinite(r)))
+      r = rmm_step_by_rows(mp + st * 512, ustr, A.units + unit0, A.slotCol + unit0 * 16, JOINT ? nullptr : A.v, A.stride, NU, table0);
+    if (JOINT && last)
+#pragma unroll
+      for (int b = 0; b < JOINT_TAIL; b++)
+        if (b < A.tail) r += lds_f64(tail0 + (uint32_t)b * 2048u + tailId[b] * 8u);
+    r += o;
+    if (last && A.rowScale && mine) r *= A.rowScale[row];
+    if (mine) A.out[row * A.stride] = r;
   }
 }
 
-// Tables of the joint slots of `nu` units, two units at a time: first the terms P_g = D_g v of their groups, then the
-// tables by adding one group after the other (T[k + n a] = T[k] + P[a] for the n joint tuples so far). A lane works for
-// one slot, its entries are spread over the warps. (With every entry taking its id apart by divisions and reading the
-// dictionaries through the group records, this was 40 of the 70 us of a 1M x 100 product.)
+// Tables of the joint slots of `nu` units, and of `tail` slots behind them whose entries lie side by side (tailTbl): first the terms
+// D_g v of their groups, then the sums of the low and of the high groups of every slot, then the tables as sums of the two. A lane works
+// for one slot, its entries are spread over warps; as many pairs of units at once as have room for what comes before the tables.
+// Bound: the latency of the first loads. (Group after group with a barrier after each, two units at a time, each term behind the load of its
+// group's record: 1M x 100 of 16 values, inputs changing from call to call, 43.0 us; 34.9 now, with the slots by rows and the ids brought to L2;
+// 41.5 with the ids asked for before the terms.)
 constexpr int RB_T = RB_W * 32;
-__device__ __forceinline__ void joint_tables(const RmmArgs& A, int unit0, int nu, double* tbl, double* terms) {
-  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
-  double* P = terms + lane * JS_TERMS;
-  for (int u0 = 0; u0 < nu; u0 += 2) {
-    const int u = unit0 + min(u0 + (lane >> 4), nu - 1), slot = u * 16 + (lane & 15);
-    const bool on = u0 + (lane >> 4) < nu;
-    const JointSlot& js = A.joint[slot];
-    const int depth = A.units[u].y, n = on ? js.n : 0;
-    double* T = tbl + (size_t)(A.units[u].x - A.units[unit0].x) * 16 + (lane & 15);
-    int off = 0, nvs[JS_MAX];
+template <class F>
+__device__ __forceinline__ void joint_tables(const RmmArgs& A, int unit0, int nu, int tail, double* tbl, double* tailTbl, double* parts, F&& loaded) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, all = nu + (tail > 0), nPairs = (all + 1) / 2;
+  for (int p0 = 0; p0 < nPairs; p0 += A.pairs) {
+    const int np = min(A.pairs, nPairs - p0), wp = RB_W / np;  // warps per pair
+    const int pair = p0 + warp / wp, r = warp % wp, u = 2 * pair + (lane >> 4), sl = lane & 15, slot = (unit0 + u) * 16 + sl;
+    const bool on = warp < wp * np && u < all && (u < nu || sl < tail);
+    JointSlot js;
+    js.n = 0;
+    if (on) js = A.joint[slot];
+    const int n = js.n;
+    double* P = parts + (size_t)(pair - p0) * A.partRows * 32 + lane;
+    double* T = u < nu ? tbl + (size_t)(on ? A.units[unit0 + u].x - A.units[unit0].x : 0) * 16 + sl : tailTbl + sl * 256;
+    const int str = u < nu ? 16 : 1, depth = on && u < nu ? A.units[unit0 + u].y : 0;
+    // (the records of the terms lie side by side, so that nothing but v hangs on a load before)
+    if (on) {
+      const size_t at = ((size_t)(unit0 + u) * A.nTerms) * 16 + sl;
+#pragma unroll 4
+      for (int e = r; e < A.nTerms; e += wp) {
+        const JointTerm t = A.terms[at + (size_t)e * 16];
+        const int gc = A.termCols ? A.termCols[at + (size_t)e * 16] : 0;
+        double x = 0.0;
+        if (gc > 0)
+          for (int h = 0; h < gc; h++) x += t.dict[h] * A.v[t.cols[h] * A.stride];
+        else if (t.col >= 0) x = t.val * A.v[t.col * A.stride];
+        if (n > 1 && e < A.joinTerms) P[(size_t)e * 32] = x;
+        else if (n == 1 && e < js.total) T[(size_t)e * str] = x;
+      }
+    }
+    for (int k = (n > 0 ? js.total : 0) + r; k < depth; k += wp) T[(size_t)k * str] = 0.0;
+    __syncthreads();
+    if (p0 == 0) loaded();
+    // low and high part: the terms themselves where it is one group, behind the terms otherwise
+    const int nLo = n > 1 ? js.nLo : 0, nHi = n > 1 ? js.total / js.nLo : 0;
+    const double *L = P, *H = P;
+    if (n > 1) {
+      int at = 0;
 #pragma unroll
-    for (int i = 0; i < JS_MAX; i++) {
-      nvs[i] = 0;
-      if (i < n) {
-        const JointGroup G = A.jointGroups[slot * JS_MAX + i];
-        nvs[i] = G.nv;
-        for (int a = r; a < G.nv; a += RB_W) {
+      for (int i = 0; i < JS_MAX; i++)
+        if (i < js.split) at += js.nv[i];
+      H = P + (size_t)at * 32;  // first term of the high groups
+      double* free = P + (size_t)A.joinTerms * 32;
+      auto sums = [&](const double* src, int g0, int g1, int count) {
+        for (int e = r; e < count; e += wp) {
+          const double* q = src;
           double x = 0.0;
-          if (G.gCols == 1) x = G.dict[a] * A.v[G.col * A.stride];
-          else
-            for (int h = 0; h < G.gCols; h++) x += G.dict[(size_t)a * G.gCols + h] * A.v[G.cols[h] * A.stride];
-          if (i == 0) T[(size_t)a * 16] = x;
-          else P[off + a] = x;
-        }
-        if (i > 0) off += G.nv;
-      }
-    }
-    int cur = n > 0 ? nvs[0] : 0;
-    off = 0;
+          int k = e;
 #pragma unroll
-    for (int i = 1; i < JS_MAX; i++) {
-      if (!__syncthreads_or(i < n)) break;
-      if (i < n) {
-        // the tuples so far are split over the warps; few tuples: the values of the new group as well
-        const int parts = max(1, RB_W / cur), k0 = cur >= RB_W ? r : r % cur, a0 = cur >= RB_W ? 1 : 1 + r / cur;
-        if (a0 <= parts)
-          for (int k = k0; k < cur; k += RB_W) {
-            const double x = T[(size_t)k * 16];
-            for (int a = a0; a < nvs[i]; a += parts) T[(size_t)(k + cur * a) * 16] = x + P[off + a];
-          }
-      }
-      __syncthreads();
-      if (i < n) {
-        const double p0 = P[off];
-        for (int k = r; k < cur; k += RB_W) T[(size_t)k * 16] += p0;
-        off += nvs[i];
-        cur *= nvs[i];
-      }
+          for (int i = 0; i < JS_MAX; i++)
+            if (i >= g0 && i < g1) {
+              const int d = (int)(((float)k + 0.5f) / (float)js.nv[i]);  // k / nv: half a step from any whole number
+              x += q[(size_t)(k - d * js.nv[i]) * 32];
+              q += (size_t)js.nv[i] * 32;
+              k = d;
+            }
+          free[(size_t)e * 32] = x;
+        }
+        const double* res = free;
+        free += (size_t)count * 32;
+        return res;
+      };
+      if (js.split > 1) L = sums(P, 0, js.split, nLo);
+      if (n - js.split > 1) H = sums(H, js.split, n, nHi);
     }
-    if (on)
-      for (int k = cur + r; k < depth; k += RB_W) T[(size_t)k * 16] = 0.0;
+    __syncthreads();
+    if (n > 1) {
+      // few low tuples: warps side by side along the high ones
+      const int side = max(1, wp / nLo), l0 = nLo >= wp ? r : r % nLo, h0 = nLo >= wp ? 0 : r / nLo;
+      if (h0 < side)
+        for (int k = l0; k < nLo; k += wp) {
+          const double x = L[(size_t)k * 32];
+#pragma unroll 4
+          for (int h = h0; h < nHi; h += side) T[(size_t)(k + nLo * h) * str] = x + H[(size_t)h * 32];
+        }
+    }
     __syncthreads();
   }
 }
@@ -1082,13 +1110,20 @@ __global__ void __launch_bounds__(RB_T, 1) k_rmm_vec(const __grid_constant__ Rmm
     for (int w = 0; w < RB_W; w++) init += cred[w];
   }
   tma_barrier_init(&mbar);
-  const int most = JOINT ? JOINT_UNITS : LMM_MAX_UNITS, nChunks = (A.nU16 + most - 1) / most, U = (A.nU16 + nChunks - 1) / nChunks;
+  const int U = A.U;
   for (int unit0 = 0, c = 0; unit0 < A.nU16; unit0 += U, c++) {
     const int nu = min(U, A.nU16 - unit0);
+    const bool last = unit0 + nu == A.nU16;
+    uint32_t tail0 = 0;
+    auto fetch = [&] { rmm_fetch(A, unit0, nu, s0, rmm_ahead(nu) * RB_W, s1); };
+    if (!JOINT) fetch();
     __syncthreads();  // everyone is done with the previous chunk's tables
     if (JOINT) {
       const int rows = A.units[unit0 + nu - 1].x + A.units[unit0 + nu - 1].y - A.units[unit0].x;
-      joint_tables(A, unit0, nu, (double*)smraw, (double*)smraw + (size_t)rows * 16);
+      double* tails = (double*)smraw + (size_t)rows * 16;
+      const int tail = last ? A.tail : 0;
+      tail0 = smem_u32(tails);
+      joint_tables(A, unit0, nu, tail, (double*)smraw, tails, tails + tail * 256, fetch);  // (the ids behind the terms, which the tables wait for)
     } else {
       const int2 f = A.units[unit0], l = A.units[unit0 + nu - 1];
       if (!tma_reload(smraw, A.tables + (size_t)f.x * 16, (uint32_t)(l.x + l.y - f.x) * 128u, &mbar, (uint32_t)(c & 1))) {
@@ -1096,12 +1131,11 @@ __global__ void __launch_bounds__(RB_T, 1) k_rmm_vec(const __grid_constant__ Rmm
         return;
       }
     }
-    const bool last = unit0 + nu == A.nU16;
     const uint32_t t0 = smem_u32(smraw);
-#define RB_CASE(N) case N: rmm_rows<N, JOINT>(A, unit0, s0, s1, init, c == 0, last, t0); break;
+#define RB_CASE(N) case N: rmm_rows<N, JOINT>(A, unit0, s0, s1, init, c == 0, last, t0, tail0); break;
     switch (nu) {
       RB_CASE(1) RB_CASE(2) RB_CASE(3) RB_CASE(4) RB_CASE(5) RB_CASE(6)
-      default: rmm_rows<7, JOINT>(A, unit0, s0, s1, init, c == 0, last, t0); break;
+      default: rmm_rows<7, JOINT>(A, unit0, s0, s1, init, c == 0, last, t0, tail0); break;
     }
 #undef RB_CASE
   }
@@ -1129,7 +1163,7 @@ template <int NU>
 __device__ __forceinline__ void chain_body(const ChainArgs& C, unsigned char* smraw, uint64_t* mbar, double* ubuf, double init) {
   const LmmArgs& A = C.L;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int slot = lane & 15, half = lane >> 4, g = lane >> 2, t = lane & 3;
+  const int slot = lane & 15, half = lane >> 4, rowOf = sum_row();
   double* mine = A.partial + (size_t)blockIdx.x * (LMM_PART + 1);
   const int2 first = A.units[0], last = A.units[NU - 1];
   if (!tma_load_to_smem(smraw, A.tables, (uint32_t)(last.x + last.y - first.x) * 128u, mbar)) {
@@ -1155,29 +1189,14 @@ __device__ __forceinline__ void chain_body(const ChainArgs& C, unsigned char* sm
     uint4 m[NU];
 #pragma unroll
     for (int u = 0; u < NU; u++) m[u] = __ldg((const uint4*)(mp + u * ustr + st * 512));
-    const int64_t row = st * VSTEP + (t & 1) * 8 + g;
-    const bool mine0 = t < 2 && row < A.nRows, mine1 = t < 2 && row + 16 < A.nRows;
-    double w0 = 1.0, w1 = 1.0;
-    if (C.w) {
-      w0 = mine0 ? C.w[row] : 0.0;
-      w1 = mine1 ? C.w[row + 16] : 0.0;
-    }
-    double r0, r1;
-    step_sums<NU, false, 1>(m, tb, v, r0, r1);
-    if (__any_sync(0xffffffffu, t < 2 && !(isfinite(r0) && isfinite(r1)))) {
-      const double2 r = rmm_step_by_rows(mp + st * 512, ustr, A.units, A.slotCol, C.v, 1, NU, table0);
-      r0 = r.x, r1 = r.y;
-    }
-    r0 = (r0 + init) * w0;
-    r1 = (r1 + init) * w1;
-    if (C.u) {
-      if (mine0) C.u[row] = r0;
-      if (mine1) C.u[row + 16] = r1;
-    }
-    if (t < 2) {
-      ub[t * 8 + g] = r0;
-      ub[16 + t * 8 + g] = r1;
-    }
+    const int64_t row = st * VSTEP + rowOf;
+    const bool in = row < A.nRows;
+    const double wt = C.w && in ? C.w[row] : 1.0;
+    double r = step_sums<NU, false, 1>(m, tb, v);
+    if (__any_sync(0xffffffffu, !isfinite(r))) r = rmm_step_by_rows(mp + st * 512, ustr, A.units, A.slotCol, C.v, 1, NU, table0);
+    r = (r + init) * wt;
+    if (C.u && in) C.u[row] = r;
+    ub[rowOf] = r;
     __syncwarp();
     if (st * VSTEP + VSTEP <= A.nRows) {
 #pragma unroll 1
@@ -1442,10 +1461,7 @@ int64_t fast_plan_build(Matrix* m) {
     std::stable_sort(byNv.begin(), byNv.end(), [&](int a, int b) { return G(a).nVals < G(b).nVals; });
     for (int i : byNv) {
       const int nv = G(i).nVals;
-      int terms = nv;
-      if (!js.empty())
-        for (int k = 0; k < js.back().n; k++) terms += js.back().nv[k];
-      if (js.empty() || js.back().n == JS_MAX || js.back().total * nv > 256 || terms > JS_TERMS) {
+      if (js.empty() || js.back().n == JS_MAX || js.back().total * nv > 256) {
         JointSlot s{};
         s.total = 1;
         js.push_back(s);
@@ -1458,18 +1474,48 @@ int64_t fast_plan_build(Matrix* m) {
     }
     // a second copy of the maps pays from a quarter fewer lookups on
     if (js.size() * 4 > (size_t)fp->nUnits * 3) js.clear();
+    for (auto& x : js) {  // low and high part: the split with the fewest terms
+      x.split = x.n;
+      x.nLo = x.total;
+      int lo = 1, best = x.total + 1;
+      for (int k = 1; k < x.n; k++) {
+        lo *= x.nv[k - 1];
+        const int hi = x.total / lo;
+        if (lo + hi < best) best = lo + hi, x.split = k, x.nLo = lo;
+      }
+      if (x.n > 1) {
+        fp->jParts = std::max(fp->jParts, (x.split > 1 ? x.nLo : 0) + (x.n - x.split > 1 ? x.total / x.nLo : 0));
+      }
+      int terms = 0;
+      for (int k = 0; k < x.n; k++) terms += x.nv[k];
+      fp->jTerms = std::max(fp->jTerms, terms);
+      if (x.n > 1) fp->jJoinTerms = std::max(fp->jJoinTerms, terms);
+    }
     std::stable_sort(js.begin(), js.end(), [](const JointSlot& a, const JointSlot& b) { return a.total > b.total; });
     fp->nJU16 = (int)(js.size() + 15) / 16;
+    fp->jTail = js.size() > 16 && js.size() % 16 <= JOINT_TAIL ? (int)(js.size() % 16) : 0;
     js.resize((size_t)fp->nJU16 * 16, JointSlot{});
   }
-  std::vector<JointGroup> jg(js.size() * JS_MAX, JointGroup{});
+  std::vector<JointTerm> jt(js.size() * fp->jTerms);
+  std::vector<int> jtCols, regOf(m->nDev, 0);
+  for (auto& x : sel) regOf[x.dev] = x.reg;
+  for (auto& t : jt) t.val = 0.0, t.col = -1;
   for (size_t i = 0; i < js.size(); i++)
-    for (int k = 0; k < js[i].n; k++) {
+    for (int k = 0, e = 0; k < js[i].n; k++) {
       const DevGroup& g = m->groups[js[i].group[k]];
-      int col = 0;
-      for (auto& x : sel)
-        if (x.dev == js[i].group[k]) col = m->hg[x.reg].cols[0];
-      jg[i * JS_MAX + k] = JointGroup{g.dict, g.cols, js[i].nv[k], g.gCols, col, 0};
+      const HostGroup* hg = &m->hg[regOf[js[i].group[k]]];
+      for (int a = 0; a < js[i].nv[k]; a++, e++) {
+        const size_t at = ((i / 16) * fp->jTerms + e) * 16 + i % 16;
+        if (g.gCols == 1) {  // (an OLE group's extra "no tuple" entry is zero)
+          jt[at].val = a < (int)hg->dict.size() ? hg->dict[a] : 0.0;
+          jt[at].col = hg->cols[0];
+        } else {
+          jt[at].dict = g.dict + (size_t)a * g.gCols;
+          jt[at].cols = g.cols;
+          jtCols.resize(jt.size(), 0);
+          jtCols[at] = g.gCols;
+        }
+      }
     }
   std::vector<int2> jRec(fp->nJU16);
   fp->jNk.assign(fp->nJU16, 1);
@@ -1483,7 +1529,7 @@ int64_t fast_plan_build(Matrix* m) {
   PlanBlob blob;
   const size_t oChunks = blob.add(fp->lchunks), oMap = blob.add(slotMap), oCol = blob.add(slotCol), oBare = blob.add(bare);
   const size_t oUnits = blob.add(unitRec), oImage = blob.add(image);
-  const size_t oJs = blob.add(js), oJg = blob.add(jg), oJRec = blob.add(jRec), oGMap = blob.add(groupMap);
+  const size_t oJs = blob.add(js), oJt = blob.add(jt), oJtCols = blob.add(jtCols), oJRec = blob.add(jRec), oGMap = blob.add(groupMap);
   const size_t mapBytes = (size_t)fp->nSlots * fp->nRB * 16, jMapBytes = (size_t)fp->nJU16 * 16 * fp->nRB * 16;
   void *d = nullptr, *maps = nullptr;
   if ((rc = plan_malloc(m, fp, &d, blob.host.size())) < 0 || (rc = plan_malloc(m, fp, &maps, mapBytes + jMapBytes)) < 0) return rc;
@@ -1496,7 +1542,8 @@ int64_t fast_plan_build(Matrix* m) {
   fp->dUnits = (int2*)(base + oUnits);
   fp->dLmmTables = (double*)(base + oImage);
   fp->dJSlots = (JointSlot*)(base + oJs);
-  fp->dJGroups = (JointGroup*)(base + oJg);
+  fp->dJTerms = (JointTerm*)(base + oJt);
+  fp->dJTermCols = jtCols.empty() ? nullptr : (int*)(base + oJtCols);
   fp->dJUnits = (int2*)(base + oJRec);
   fp->dLmmMaps = (uint8_t*)maps;
   fp->dJMaps = (uint8_t*)maps + mapBytes;
@@ -1552,7 +1599,10 @@ int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW
   A.tables = fp->dLmmTables;
   A.slotCol = fp->dSlotCol;
   A.joint = fp->dJSlots;
-  A.jointGroups = fp->dJGroups;
+  A.terms = fp->dJTerms;
+  A.termCols = fp->dJTermCols;
+  A.nTerms = fp->jTerms;
+  A.joinTerms = fp->jJoinTerms;
   A.v = dV;
   A.constV = m->hasConst ? m->dConstV : nullptr;
   A.nCols = m->nCols;
@@ -1563,14 +1613,27 @@ int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW
   A.out = dOut;
   A.err = m->dErr;
   const std::vector<int>& nk = joint ? fp->jNk : fp->unitNk;
-  const int most = joint ? JOINT_UNITS : LMM_MAX_UNITS, nChunks = (A.nU16 + most - 1) / most, U = (A.nU16 + nChunks - 1) / nChunks;
-  size_t smem = 1024;
-  for (int q = 0; q < A.nU16; q += U) {
-    size_t b = 0;
-    for (int i = q; i < std::min(A.nU16, q + U); i++) b += (size_t)nk[i] * 128;
-    smem = std::max(smem, b);
+  if (joint && fp->jTail) {
+    A.tail = fp->jTail;
+    A.nU16--;
   }
-  if (joint) smem += 32 * JS_TERMS * sizeof(double);
+  // units per chunk, evenly: what fits, the joint slots' with room for what comes before the tables of a pair of units
+  A.partRows = std::max(1, fp->jJoinTerms + fp->jParts);
+  const size_t parts = joint ? (size_t)A.partRows * 256 : 0, tails = (size_t)A.tail * 2048, room = SMEM_MAX - 1024;
+  size_t tables = 1024;
+  for (int most = joint ? JOINT_UNITS : LMM_MAX_UNITS; most >= 1; most--) {
+    const int nChunks = (A.nU16 + most - 1) / most;
+    A.U = (A.nU16 + nChunks - 1) / nChunks;
+    tables = 1024;
+    for (int q = 0; q < A.nU16; q += A.U) {
+      size_t b = 0;
+      for (int i = q; i < std::min(A.nU16, q + A.U); i++) b += (size_t)nk[i] * 128;
+      tables = std::max(tables, b);
+    }
+    if (tables + tails + parts <= room) break;
+  }
+  A.pairs = joint ? std::max(1, std::min((A.U + 2) / 2, (int)((room - tables - tails) / parts))) : 1;
+  const size_t smem = tables + tails + A.pairs * parts;
   const int64_t nSteps = ((int64_t)m->nRows + VSTEP - 1) / VSTEP;
   const int grid = (int)std::min<int64_t>(m->smCount, nSteps);
   prof_begin(m, s);

@@ -84,6 +84,33 @@ def test_joint_slots_of_uneven_dictionaries():
         cmb.free()
 
 
+@pytest.mark.parametrize("cards", [[16] * 33, [16] * 40, [16] * 42, [6] * 51, [2] * 144, [16] * 195, [200] * 20 + [16] * 40, [2, 128] * 20])
+def test_joint_slots_behind_the_last_unit(cards):
+    """Joint slots by rows: one, four and none behind the last whole unit; parts of one and of several groups; several chunks;
+    slots of one group. Inf and NaN entries stay in their rows, also those of the slots that go by rows."""
+    cmb = _ddc(300001, cards, len(cards)).to_device()
+    _check(cmb, chain=False)
+    cmb.free()
+    rng = np.random.default_rng(3)
+    groups = []
+    for c, k in enumerate(cards):
+        d = rng.standard_normal((k, 1))
+        ids = rng.integers(0, k - 1, 300001)
+        if c % 16 in (0, 7):
+            d[k - 1] = np.inf if c % 2 else np.nan
+            ids[rng.integers(0, 300001, 20)] = k - 1
+        groups.append(cg.ColGroupDDC([c], d, MapToFactory.create_from(ids, k)))
+    cmb = CompressedMatrixBlock(300001, len(cards), groups).to_device()
+    X = dense_of(cmb)
+    v = rng.standard_normal(len(cards))
+    got = np.asarray(CLALibRightMultBy.rightMultByMatrix(cmb, v)).ravel()
+    fine = np.isfinite(X).all(axis=1)
+    assert 0 < fine.sum() < 300001
+    assert np.array_equal(np.isfinite(got), fine)
+    assert rel_err(got[fine], X[fine] @ v, np.abs(X[fine]) @ np.abs(v)) < TOL
+    cmb.free()
+
+
 @pytest.mark.parametrize("nRows", [5000, 300007])
 def test_non_finite_values_stay_in_their_rows(nRows):
     """Inf and NaN dictionary entries reach the rows that hold them and no other (the row sums of neighbouring rows are
