@@ -202,17 +202,26 @@ __device__ __forceinline__ uint32_t byte_x128(uint32_t w, int i) {  // (byte i o
   return i == 0 ? (w << 7) & 0x7F80u : (i == 3 ? (w >> 17) & 0x7F80u : (w >> (8 * i - 7)) & 0x7F80u);
 }
 
+__device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
 constexpr int VSTEP = 32;  // rows of a warp step: one 16-row block per half-warp
 
 // --------------------------------------------------------------------------------------------------
-// LMM: t(y) X. The grid is cut into chunks of U units; a chunk's CTAs split the rows. y is loaded with 128-bit loads
-// that are uniform per half-warp and multiplied into NU accumulators per lane. The CTA's partial sums go to `partial`.
+// LMM: t(y) X. The grid is cut into chunks of U units; a chunk's CTAs split the rows. A lane needs the y of every row of its
+// half-warp's block, multiplied into NU accumulators. It loads those of the rows 4 j + t and the FP64 tensor core, idle otherwise, hands them
+// round: m8n8k4 with A[m][k] = y of row 4 j + k of the half-warp of m and a 0 / 1 matrix that picks two k's gives two rows to every lane.
+// Eight bytes to 32 lanes are two wavefronts of the pipe that bounds this kernel, so loads of every row (128 bits, uniform per
+// half-warp) were 32 of the 284 wavefronts of a step of seven units, eight now. The CTA's partial sums go to `partial`.
 // k_lmm_final adds them up in a fixed order, a CTA per 16 columns, resident before the last CTA ends (programmatic
 // dependent launch), and stores the result: nothing to clear beforehand. (Left to the last CTA of a chunk, without a second
 // launch: 18.2 instead of 14.3 us for the chain on 50,000 x 100, 17.6 instead of 14.2 for t(y) X on 250,000 x 40 -- one
 // CTA reads 148 partial rows too slowly.)
-// Measured (10M x 200, 256 values): 634 us, 3.3 TB/s, on a box where the one-row-step form before, with three instructions
-// per address, a clear and a separately launched sum, took 685 (670 and 697 on another box).
+// Measured (10M x 200, 256 values): 577 us, 3.6 TB/s; 634 with y loaded row by row, 685 for the one-row-step form before that, with
+// three instructions per address, a clear and a separately launched sum. 625,000 x 1000: 208 -> 187.
 // 100,000 x 500: 36.9 -> 30.5 us, 5000 x 500: 15.4 -> 10.4.
 // --------------------------------------------------------------------------------------------------
 struct LmmArgs {
@@ -315,40 +324,56 @@ __device__ __forceinline__ void lmm_vec_body(const LmmArgs& A, int chunk, int ct
     const int64_t nSteps = A.stepEnd - A.stepBegin;
     const int c = blockIdx.x - cta0;
     const int64_t s0 = A.stepBegin + nSteps * c / nCta, s1 = A.stepBegin + nSteps * (c + 1) / nCta;
+    const int g = lane >> 2, t = lane & 3;
+    const double even = t == (g & 1) ? 1.0 : 0.0, odd = t == 2 + (g & 1) ? 1.0 : 0.0;  // rows 0, 1 and 2, 3 of four
     uint4 m[NU];
+    double y[4];
+    auto load_y = [&](int64_t k) {  // rows 4 j + t of this half-warp's block
+      const double* ys = A.y + k * VSTEP + half * 16 + t;
+#pragma unroll
+      for (int j = 0; j < 4; j++) y[j] = k * VSTEP + VSTEP <= A.nRows ? __ldg(ys + 4 * j) : 0.0;
+    };
     int64_t st = s0 + warp;
     if (st < s1) {
 #pragma unroll
       for (int u = 0; u < NU; u++) m[u] = __ldg((const uint4*)(mp + u * ustr + st * 512));
+      load_y(st);
     }
     for (; st < s1; st += LMM_W) {
-      const int64_t r0 = st * VSTEP + half * 16, nxt = st + LMM_W;
-      if (st * VSTEP + VSTEP <= A.nRows) {
+      const int64_t nxt = st + LMM_W;
+      const double four = (y[0] + y[1]) + (y[2] + y[3]);
+      // (a product with 0 would carry an Inf or NaN into other rows: such steps go row by row, like the ragged last one)
+      if (st * VSTEP + VSTEP <= A.nRows && !__any_sync(0xffffffffu, !isfinite(four))) {
+        ysum += four;
         double yv[16];
-        const double2* ys = (const double2*)(A.y + r0);
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const double2 t = __ldg(ys + i);
-          yv[2 * i] = t.x;
-          yv[2 * i + 1] = t.y;
+        for (int i = 0; i < 16; i++) yv[i] = 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          dmma884(yv[4 * j], yv[4 * j + 1], y[j], even);
+          dmma884(yv[4 * j + 2], yv[4 * j + 3], y[j], odd);
         }
-        if (A.constV)
-#pragma unroll
-          for (int i = 0; i < 16; i++) ysum += yv[i];
+        if (nxt < s1) load_y(nxt);  // in flight until the next step, and the ids likewise
 #pragma unroll
         for (int u = 0; u < NU; u++) {
           const uint4 w = m[u];
-          if (nxt < s1) m[u] = __ldg((const uint4*)(mp + u * ustr + nxt * 512));  // in flight until the next step
+          if (nxt < s1) m[u] = __ldg((const uint4*)(mp + u * ustr + nxt * 512));
           const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
           for (int i = 0; i < 16; i++) acc[u] = fma(yv[i], lds_f64(entry_at(ww[i >> 2], i & 3, tb[u])), acc[u]);
         }
-      } else {  // ragged last step
+      } else {
+        const int64_t r0 = st * VSTEP + half * 16;
         for (int i = 0; i < 16 && r0 + i < A.nRows; i++) {
           const double yy = A.y[r0 + i];
-          ysum += yy;
+          if (t == 0) ysum += yy;
 #pragma unroll
           for (int u = 0; u < NU; u++) acc[u] = fma(yy, lds_f64(tb[u] + 128u * mp[u * ustr + st * 512 + i]), acc[u]);
+        }
+        if (nxt < s1) {
+#pragma unroll
+          for (int u = 0; u < NU; u++) m[u] = __ldg((const uint4*)(mp + u * ustr + nxt * 512));
+          load_y(nxt);
         }
       }
     }
@@ -361,7 +386,7 @@ __device__ __forceinline__ void lmm_vec_body(const LmmArgs& A, int chunk, int ct
       a += __shfl_xor_sync(0xffffffffu, a, 16);
       if (half == 0) red[warp * (NU * 16 + 1) + u * 16 + slot] = a;
     }
-    ysum += __shfl_xor_sync(0xffffffffu, ysum, 16);
+    for (int d = 1; d < 32; d = d == 2 ? 16 : 2 * d) ysum += __shfl_xor_sync(0xffffffffu, ysum, d);  // (a lane's rows are those of its t)
     if (lane == 0) red[warp * (NU * 16 + 1) + NU * 16] = ysum;
     __syncthreads();
     for (int u = tid; u <= NU * 16; u += LMM_T) {
@@ -530,11 +555,6 @@ __global__ void k_lmm_vecq_final(const LmmChunk* __restrict__ chunks, int nChunk
 // wasted), against 8 for the lookups, 1 for the ids and 8 for the left values of all the CTA's slots. (FMA on scalar
 // accumulators, four left rows per lookup, took 47 us per pass of four rows over 500k x 100 columns of four tuples.)
 // --------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
 constexpr int LR_W = 16;
 constexpr int LR_T = LR_W * 32;
 constexpr int LR_MAXT = 8;                    // tiles of eight slots per CTA
@@ -1647,7 +1667,8 @@ int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW
 
 // Units per chunk of k_lmm_vec: with few rows per CTA, staging the tables (32 KB per unit) costs more than the rows, so
 // the columns are spread over more CTAs; with many, wide chunks read y less often. Clocks, from the pipe's
-// wavefronts: 512 per unit staged, 1.13 per unit and 1 for y per row, and at least one round of steps.
+// wavefronts: 512 per unit staged, 1.13 per unit and row and 1 for the rest, and at least one round of steps. (0.3 for the rest, what y takes
+// there now, changes little but 100,000 x 200: 18.9 instead of 16.8 us.)
 static int lmm_chunk_units(const FastPlan* fp, int nRows, int sm) {
   int best = 1;
   double bestCost = 1e300;

@@ -138,6 +138,22 @@ def test_non_finite_values_stay_in_their_rows(nRows):
     cmb.free()
 
 
+@pytest.mark.parametrize("nRows", [4127, 40001])
+def test_left_product_of_non_finite_values(nRows):
+    """Inf in the left vector makes Inf, not NaN, of columns of one sign, whichever rows share its products with zeros; NaN
+    and the ragged last rows likewise."""
+    rng = np.random.default_rng(nRows)
+    groups = [cg.ColGroupDDC([c], rng.uniform(0.5, 1.0, (9, 1)), MapToFactory.create_from(rng.integers(0, 9, nRows), 9)) for c in range(40)]
+    cmb = CompressedMatrixBlock(nRows, 40, groups).to_device()
+    for row in (0, 3, 18, nRows - 1, nRows - 40):
+        for value in (np.inf, -np.inf, np.nan):
+            y = rng.standard_normal((1, nRows))
+            y[0, row] = value
+            got = np.asarray(CLALibLeftMultBy.leftMultByMatrix(cmb, y)).ravel()
+            assert np.isnan(got).all() if np.isnan(value) else (got == value).all()
+    cmb.free()
+
+
 @pytest.mark.parametrize("nRows", [33, 5000])
 @pytest.mark.parametrize("nCols", [127, 129, 160, 257])
 def test_self_product_blocks(oracle, nRows, nCols):
