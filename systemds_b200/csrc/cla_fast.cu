@@ -33,9 +33,10 @@ constexpr int FAST_MIN_ROWS = 4096;
 constexpr int SMEM_MAX = 227 * 1024;
 
 // ---- plan ----
-// Warps per CTA (one CTA per SM).
-constexpr int LMM_W = 16;
-constexpr int LMM_T = LMM_W * 32;
+// Warps per CTA (one CTA per SM). k_lmm_vec: 12 where a CTA has five units or more (10M x 200, 7 + 6 units: 8 / 10 / 12 / 14 / 16 warps
+// 615 / 609 / 562 / 658 / 577 us; 16 and 14 leave 128 registers), 16 where fewer (300,001 x 60, 4 units: 16.4 against 17.0 with 12).
+__host__ __device__ constexpr int lmm_warps(int units) { return units > 4 ? 12 : 16; }
+constexpr int LMM_MAXW = 16;
 constexpr int RB_W = 16;              // k_rmm_vec
 constexpr int LMM_MAX_UNITS = 7;      // 16-column table units per CTA (7 x 32 KB at 256 tuples)
 constexpr int LMM_PART = LMM_MAX_UNITS * 16;  // partial sums a CTA writes
@@ -244,23 +245,24 @@ struct LmmArgs {
   int32_t* err;
 };
 
-// Adds up the partial sums of unit `u` of a chunk, by one CTA of LMM_T threads: 32 groups of 16 lanes (a lane per
+// Adds up the partial sums of unit `u` of a chunk, by one CTA of LMM_FT threads: 32 groups of 16 lanes (a lane per
 // column) take every 32nd partial sum, then a tree over the groups: a fixed order.
-constexpr int LMM_FIN = (LMM_T / 16) * 17 + LMM_T / 32;  // doubles of shared memory it needs
+constexpr int LMM_FT = 512;
+constexpr int LMM_FIN = (LMM_FT / 16) * 17 + LMM_FT / 32;  // doubles of shared memory it needs
 __device__ __forceinline__ void lmm_finish(const LmmArgs& A, int chunk, int cta0, int nCta, int grid, int u, bool withBare,
                                            double* sm) {
   double(*red)[17] = (double(*)[17])sm;
-  double* yred = sm + (LMM_T / 16) * 17;
+  double* yred = sm + (LMM_FT / 16) * 17;
   const int tid = threadIdx.x, col = tid & 15, sub = tid >> 4;
   const int n = A.parts * nCta;
   double s = 0.0, ys = 0.0;
-  for (int i = sub; i < n; i += LMM_T / 16) {
+  for (int i = sub; i < n; i += LMM_FT / 16) {
     const int p = i / nCta, b = i - p * nCta;
     s += __ldcg(A.partial + ((size_t)p * grid + cta0 + b) * (LMM_PART + 1) + u * 16 + col);
   }
   red[sub][col] = s;
   if (A.constV) {
-    for (int i = tid; i < n; i += LMM_T) {
+    for (int i = tid; i < n; i += LMM_FT) {
       const int p = i / nCta, b = i - p * nCta;
       ys += __ldcg(A.partial + ((size_t)p * grid + cta0 + b) * (LMM_PART + 1) + LMM_PART);
     }
@@ -268,13 +270,13 @@ __device__ __forceinline__ void lmm_finish(const LmmArgs& A, int chunk, int cta0
     if ((tid & 31) == 0) yred[tid >> 5] = ys;
   }
   __syncthreads();
-  for (int h = LMM_T / 32; h; h >>= 1) {
+  for (int h = LMM_FT / 32; h; h >>= 1) {
     if (sub < h) red[sub][col] += red[sub + h][col];
     __syncthreads();
   }
   if (A.constV) {
     ys = 0.0;
-    for (int w = 0; w < LMM_T / 32; w++) ys += yred[w];
+    for (int w = 0; w < LMM_FT / 32; w++) ys += yred[w];
   }
   if (tid < 16) {
     const int c = A.slotCol[(chunk * A.U + u) * 16 + tid];
@@ -284,22 +286,23 @@ __device__ __forceinline__ void lmm_finish(const LmmArgs& A, int chunk, int cta0
     }
   }
   if (withBare && chunk == 0 && !A.addTo)  // columns of constant groups, and those the general kernels will add to
-    for (int i = tid; i < A.nBare; i += LMM_T) {
+    for (int i = tid; i < A.nBare; i += LMM_FT) {
       const int c = A.bareCols[i];
       A.out[c] = A.constV ? ys * A.constV[c] : 0.0;
     }
 }
 
 // grid: units
-__global__ void __launch_bounds__(LMM_T) k_lmm_final(const __grid_constant__ LmmArgs A, int grid) {
+__global__ void __launch_bounds__(LMM_FT) k_lmm_final(const __grid_constant__ LmmArgs A, int grid) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int chunk = blockIdx.x / A.U, u = blockIdx.x - chunk * A.U;
   __shared__ double sm[LMM_FIN];
   lmm_finish(A, chunk, chunk * A.ctaFull, chunk == A.nChunks - 1 ? A.ctaLast : A.ctaFull, grid, u, u == 0, sm);
 }
 
-template <int NU>
+template <int NU, int LMM_W>
 __device__ __forceinline__ void lmm_vec_body(const LmmArgs& A, int chunk, int cta0, int nCta, unsigned char* smraw, uint64_t* mbar) {
+  constexpr int LMM_T = LMM_W * 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int slot = lane & 15, half = lane >> 4;
   const int unit0 = chunk * A.U;
@@ -397,16 +400,16 @@ __device__ __forceinline__ void lmm_vec_body(const LmmArgs& A, int chunk, int ct
   }
 }
 
-__global__ void __launch_bounds__(LMM_T, 1) k_lmm_vec(const __grid_constant__ LmmArgs A) {
+template <int W>
+__global__ void __launch_bounds__(W * 32, 1) k_lmm_vec(const __grid_constant__ LmmArgs A) {
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ __align__(8) uint64_t mbar;
   const int chunk = min((int)blockIdx.x / A.ctaFull, A.nChunks - 1), cta0 = chunk * A.ctaFull;
   const int nCta = chunk == A.nChunks - 1 ? A.ctaLast : A.ctaFull;
   if (A.parts) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#define LMM_CASE(N) case N: lmm_vec_body<N>(A, chunk, cta0, nCta, smraw, &mbar); break;
+#define LMM_CASE(N) case N: if constexpr (lmm_warps(N) >= W) lmm_vec_body<N, W>(A, chunk, cta0, nCta, smraw, &mbar); break;
   switch (min(A.U, A.nU16 - chunk * A.U)) {
-    LMM_CASE(1) LMM_CASE(2) LMM_CASE(3) LMM_CASE(4) LMM_CASE(5) LMM_CASE(6)
-    default: lmm_vec_body<7>(A, chunk, cta0, nCta, smraw, &mbar); break;
+    LMM_CASE(1) LMM_CASE(2) LMM_CASE(3) LMM_CASE(4) LMM_CASE(5) LMM_CASE(6) LMM_CASE(7)
   }
 #undef LMM_CASE
 }
@@ -977,9 +980,9 @@ __device__ __forceinline__ void rmm_fetch(const RmmArgs& A, int unit0, int nu, i
   if (warp < nu && (threadIdx.x & 31) == 0 && n > 0)
     l2_fetch(A.imaps + ((size_t)(unit0 + warp) * A.nRB + (size_t)from * 2) * 256, (uint32_t)n * 512u);
 }
-// Turns of the warps whose ids are on their way to L2: about 200 KB per SM, more than the memory's latency takes. (625,000 x 1000: 255 us
-// without, 236 with.)
-__host__ __device__ constexpr int rmm_ahead(int nu) { return 24 / nu; }
+// Turns of the warps whose ids are on their way to L2: about 100 KB per SM, what the memory's latency takes. (1,250,000 x 1000: 430 us
+// without, 409 with, 413 and 433 with two and four times as many.)
+__host__ __device__ constexpr int rmm_ahead(int nu) { return 14 / nu; }
 
 template <int NU, bool JOINT>
 __device__ __forceinline__ void rmm_rows(const RmmArgs& A, int unit0, int64_t s0, int64_t s1, double init, bool first, bool last,
@@ -1574,7 +1577,7 @@ int64_t fast_plan_build(Matrix* m) {
                                                              m->nRows, fp->nRB, fp->dJMaps);
   CLA_CUDA(cudaStreamSynchronize(m->stream));
   static OncePerDevice once, onceDecomp;
-  if ((rc = allow_smem(once, m->device, SMEM_MAX - 1024, k_lmm_vec, k_rmm_vec<false>, k_rmm_vec<true>)) < 0) return rc;
+  if ((rc = allow_smem(once, m->device, SMEM_MAX - 1024, k_lmm_vec<12>, k_lmm_vec<16>, k_rmm_vec<false>, k_rmm_vec<true>)) < 0) return rc;
   if ((rc = allow_smem(onceDecomp, m->device, SMEM_MAX - 2048, k_decomp_fast)) < 0) return rc;
   if (fp->partial) {  // tell the general kernels which groups are taken care of
     for (auto& x : sel) m->groups[x.dev].inFast = 1;
@@ -1676,7 +1679,7 @@ static int lmm_chunk_units(const FastPlan* fp, int nRows, int sm) {
     const int nChunks = (fp->nU16 + U - 1) / U, u = (fp->nU16 + nChunks - 1) / nChunks;
     if (nChunks > sm && U < LMM_MAX_UNITS) continue;
     const double ctas = std::max(1.0, (double)sm / nChunks), rows = nRows / ctas, waves = std::ceil((double)nChunks / sm);
-    const double rounds = std::ceil(rows / (VSTEP * LMM_W));
+    const double rounds = std::ceil(rows / (VSTEP * lmm_warps(u)));
     const double cost = waves * (512.0 * u + std::max(rows * (1.13 * u + 1.0), rounds * (600.0 + 40.0 * u)));
     if (cost < bestCost) bestCost = cost, best = u;
   }
@@ -1709,7 +1712,7 @@ static size_t lmm_args(Matrix* m, FastPlan* fp, LmmArgs& A, int* grid) {
   if (A.nChunks > 1 && A.ctaFull * (A.nChunks - 1) >= m->smCount) A.ctaFull = std::max(1, (m->smCount - 1) / (A.nChunks - 1));
   A.ctaLast = std::max(1, std::min(steps, m->smCount - A.ctaFull * (A.nChunks - 1)));
   *grid = A.ctaFull * (A.nChunks - 1) + A.ctaLast;
-  size_t smem = (size_t)LMM_W * (LMM_PART + 1) * 8;
+  size_t smem = (size_t)LMM_MAXW * (LMM_PART + 1) * 8;
   for (int q = 0; q < fp->nU16; q += A.U) {
     size_t b = 0;
     for (int i = q; i < std::min(fp->nU16, q + A.U); i++) b += (size_t)fp->unitNk[i] * 128;
@@ -1722,7 +1725,7 @@ static size_t lmm_args(Matrix* m, FastPlan* fp, LmmArgs& A, int* grid) {
 static int64_t launch_lmm_final(Matrix* m, const LmmArgs& A, int grid, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)A.nU16);
-  cfg.blockDim = dim3(LMM_T);
+  cfg.blockDim = dim3(LMM_FT);
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1735,7 +1738,9 @@ static int64_t launch_lmm_final(Matrix* m, const LmmArgs& A, int grid, cudaStrea
 }
 // The product's last (or only) launch of k_lmm_vec and what finishes it
 static int64_t launch_lmm_vec(Matrix* m, const LmmArgs& A, int grid, size_t smem, cudaStream_t s) {
-  k_lmm_vec<<<grid, LMM_T, smem, s>>>(A);
+  const int W = lmm_warps(A.U);
+  if (W == 12) k_lmm_vec<12><<<grid, 12 * 32, smem, s>>>(A);
+  else k_lmm_vec<16><<<grid, 16 * 32, smem, s>>>(A);
   m->stats.kernel_launches++;
   if (A.parts) return launch_lmm_final(m, A, grid, s);
   return CLA_OK;
