@@ -222,6 +222,7 @@ struct Finish {
   uint32_t seq = 0;
 };
 struct WidePlan;  // plan of the wide right product (cla_wide.cu)
+struct SplitPlan; // of the self product in 8-bit digits (cla_split.cu)
 struct HostStage; // pinned ring for operands in pageable host memory (cla_hostcopy.cu)
 
 struct Matrix;
@@ -293,6 +294,7 @@ struct Matrix {
   RestPlan rest;
   DecPlan dec;
   WidePlan* wide = nullptr;
+  SplitPlan* split = nullptr;
   HostStage* hostStage = nullptr;
   char* mail = nullptr;          // pinned: Mailbox, inputs, outputs (small host-buffer calls)
   unsigned long long* dFin = nullptr;  // device counters of Finish
@@ -361,6 +363,12 @@ int64_t plan_alloc(Matrix* m, void** p, size_t bytes, bool needed = false);
 void plan_release(Matrix* m, void* p, size_t bytes);  // gives one back early; no stream may still use it
 int64_t wide_rmm(Matrix* m, const double* dV, int vCols, double* dOut, cudaStream_t s);  // cla_wide.cu: 1 = done, 0 = not covered
 void wide_plan_free(Matrix* m);
+// t(X) X of many columns in 8-bit digits (cla_split.cu): 1 = done, 0 = not covered
+int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s);
+void split_plan_free(Matrix* m);
+// Rows [r0, r1) straight to digit planes, a thread per column (cla_generic.cu); whether the block's columns suit that
+bool split_cols_covers(Matrix* m, cudaStream_t s);
+int64_t launch_split_cols(Matrix* m, int r0, int r1, const int32_t* expo, int64_t halves, uint8_t* planes, unsigned long long* check, cudaStream_t s);
 // Short blocks (cla_small.cu): one kernel per product, every group type. 1 = done, 0 = not covered
 bool small_block(const Matrix* m);
 int64_t small_rmm(Matrix* m, const double* dV, int vCols, double* dOut, const double* dW, cudaStream_t s, const Finish& fin,

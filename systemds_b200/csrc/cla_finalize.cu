@@ -857,6 +857,7 @@ void release(Matrix* m) {
   if (m->stream) cudaDeviceSynchronize();  // nothing on any stream uses the handle's memory any more
   fast_plan_free(m);
   wide_plan_free(m);
+  split_plan_free(m);
   for (void* p : m->allocs) dev_free(m, p);
   m->allocs.clear();
   for (void* p : {m->scratch, m->scratch2, m->io, m->small_, (void*)m->dErr}) dev_free(m, p);

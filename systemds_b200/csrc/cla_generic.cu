@@ -16,6 +16,7 @@
 //        3. k_lmm_unc      : uncompressed groups, direct product (ColGroupUncompressed.java:429-539)
 //        4. k_lmm_const    : out += rowSums(Yt) (x) constV  (lib/CLALibLeftMultBy.java:530-629)
 #include "cla_common.cuh"
+#include "cla_split.cuh"
 #include <algorithm>
 #include <climits>
 
@@ -651,6 +652,126 @@ __global__ void __launch_bounds__(DC_WARPS * 32) k_decomp_cols(const DecCol* __r
   }
 }
 
+// The same walk, sixteen rows at a time, into digit planes (cla_split.cu) instead of doubles: tables hold the digits, and a value is split
+// where it changes. halves: of 16 rows, those behind the last row are zeros. 200,000 x 250 mixed: 136 us against 272 for
+// k_decomp_cols and a pass over the doubles; what is left is the latency of the same chains.
+template <bool CHECK>
+__global__ void __launch_bounds__(DC_WARPS * 32)
+k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, int64_t halves, uint8_t* __restrict__ planes, int r0, int r1,
+             int nRows, int nCols, int exactSdc, unsigned long long* __restrict__ check) {
+  extern __shared__ double dct[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nW = blockDim.x >> 5;
+  const int c = (blockIdx.y * nW + warp) * 32 + lane;
+  if (c >= nCols) return;
+  const int rb = r0 + blockIdx.x * DC_ROWS, re = min(r1, rb + DC_ROWS), blk = rb / SKIP_ROWS, nBlocks = (nRows + SKIP_ROWS - 1) / SKIP_ROWS;
+  const DecCol d = cols[c];
+  const double cst = d.cst, scale = split_scale(expo[c]);
+  uint8_t* o = planes + ((size_t)(c / SP_COLS) * halves + (size_t)blockIdx.x * (DC_ROWS / 16)) * SP_HALF;
+  SplitCheck<CHECK> seen;
+  const unsigned long long base = split_pack(cst, scale, seen);
+  auto value = [&](size_t k) {
+    const double x = d.dict[k * d.stride];
+    return split_pack(d.kind == DC_SDC && exactSdc ? x : cst + x, scale, seen);
+  };
+  unsigned long long v[16];
+  // the groups of 16 rows; cell(i, row) gives the digits
+  auto walk = [&](auto&& cell) {
+    for (int g = 0; g < DC_ROWS / 16; g++) {
+      const int r = rb + g * 16;
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = r + i < re ? cell(r + i) : 0ull;
+      split_store(o + (size_t)g * SP_HALF, c, v, seen);
+    }
+  };
+  if (rb >= r1) walk([&](int) { return 0ull; });
+  else if (d.kind == DC_BYTES || d.kind == DC_BITS) {
+    unsigned long long* T = (unsigned long long*)dct + d.tbl + lane;
+    for (int k = 0; k < d.nVals; k++) T[k * 32] = value(k);
+    for (int g = 0; g < DC_ROWS / 16; g++) {
+      const int r = rb + g * 16;
+      if (r + 16 <= re) {
+        uint32_t w[4];
+        if (d.kind == DC_BYTES) {
+          const uint4 q = __ldg((const uint4*)((const uint8_t*)d.a + r));
+          w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
+        } else {
+          const uint32_t bits = (uint32_t)(((const unsigned long long*)d.a)[r >> 6] >> (r & 63));
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const uint32_t x = bits >> (4 * q);
+            w[q] = (x & 1u) | ((x & 2u) << 7) | ((x & 4u) << 14) | ((x & 8u) << 21);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = T[((w[i >> 2] >> (8 * (i & 3))) & 0xFF) * 32];
+      } else
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = r + i < re ? T[map_get(d.mapType, d.a, nullptr, r + i) * 32] : 0ull;
+      split_store(o + (size_t)g * SP_HALF, c, v, seen);
+    }
+  } else if (d.kind == DC_UNC) {
+    const double* x = d.dict + (size_t)rb * d.stride;
+    const size_t xs = d.stride;
+    for (int g = 0; g < DC_ROWS / 16; g++, x += 16 * xs) {
+      double y[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) y[i] = rb + g * 16 + i < re ? __ldcs(x + i * xs) : 0.0;
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = rb + g * 16 + i < re ? split_pack(cst + y[i], scale, seen) : 0ull;
+      split_store(o + (size_t)g * SP_HALF, c, v, seen);
+    }
+  } else if (d.kind == DC_SDC) {
+    const uint32_t* items = (const uint32_t*)d.a;
+    const SdcSkip* sk = (const SdcSkip*)d.b;
+    const int64_t end = blk + 1 < nBlocks ? (int64_t)sk[blk + 1].elem : d.n;
+    int64_t p = sk[blk].elem, hi = end;
+    const uint32_t first = (uint32_t)(rb & (SKIP_ROWS - 1));
+    while (p < hi) {  // first item at or behind row rb
+      const int64_t mid = (p + hi) >> 1;
+      if ((items[mid] & 1023u) < first) p = mid + 1;
+      else hi = mid;
+    }
+    const int at = blk * SKIP_ROWS;
+    uint32_t it = p < end ? items[p] : 0u, ahead = p + 1 < end ? items[p + 1] : 0u;
+    int row = p < end ? at + (int)(it & 1023u) : INT_MAX;
+    unsigned long long val = p < end ? value(it >> 10) : 0ull;
+    walk([&](int r) {
+      unsigned long long x = base;
+      if (r == row) {
+        x = val;
+        p++;
+        row = p < end ? at + (int)(ahead & 1023u) : INT_MAX;
+        if (p < end) val = value(ahead >> 10);
+        ahead = p + 1 < end ? items[p + 1] : 0u;
+      }
+      return x;
+    });
+  } else if (d.kind == DC_RLE) {
+    const RleRun* runs = (const RleRun*)d.a;
+    int64_t ri = ((const int32_t*)d.b)[blk];
+    int start = INT_MAX, end = INT_MAX;  // the current or next run
+    unsigned long long val = 0;
+    auto next = [&]() {
+      if (ri < d.n) {
+        const RleRun run = runs[ri++];
+        start = run.start;
+        end = run.start + (int)run.len;
+        val = value(run.k);
+      } else
+        start = end = INT_MAX;
+    };
+    next();
+    walk([&](int r) {
+      while (end <= r) next();
+      return r >= start ? val : base;
+    });
+  } else if (d.kind == DC_MAP) {
+    walk([&](int r) { return value(map_get(d.mapType, d.a, d.b, r)); });
+  } else
+    walk([&](int) { return base; });
+  seen.report(check, c);
+}
+
 // The records of k_decomp_cols, filled by CTAs of the shape it will have.
 __global__ void __launch_bounds__(DC_WARPS * 32)
 k_dec_cols(const DevGroup* __restrict__ groups, const int32_t* __restrict__ colSrc, const double* __restrict__ constV,
@@ -801,6 +922,23 @@ int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStr
       k_decomp_rle<<<64, 256, 0, s>>>(g, dOut, r0, r1, ld);
     m->stats.kernel_launches++;
   }
+  CLA_CUDA(cudaGetLastError());
+  return CLA_OK;
+}
+
+bool split_cols_covers(Matrix* m, cudaStream_t s) {
+  // (fewer warps than four a CTA: deep tables, better read once to doubles)
+  return m->colSrcValid && m->dec.warps >= 4 && ensure_dec(m, s) >= 0 && m->dec.cols;
+}
+int64_t launch_split_cols(Matrix* m, int r0, int r1, const int32_t* expo, int64_t halves, uint8_t* planes, unsigned long long* check, cudaStream_t s) {
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, DC_TBL, k_split_cols<false>, k_split_cols<true>); e < 0) return e;
+  dim3 grid((unsigned)((halves * 16 + DC_ROWS - 1) / DC_ROWS), (m->nCols + m->dec.warps * 32 - 1) / (m->dec.warps * 32));
+  const DecCol* cols = (const DecCol*)m->dec.cols;
+  const int exact = m->multiCover ? 0 : 1, threads = m->dec.warps * 32;
+  if (check) k_split_cols<true><<<grid, threads, m->dec.smem, s>>>(cols, expo, halves, planes, r0, r1, m->nRows, m->nCols, exact, check);
+  else k_split_cols<false><<<grid, threads, m->dec.smem, s>>>(cols, expo, halves, planes, r0, r1, m->nRows, m->nCols, exact, nullptr);
+  m->stats.kernel_launches++;
   CLA_CUDA(cudaGetLastError());
   return CLA_OK;
 }

@@ -1,0 +1,474 @@
+// t(X) X of more than 128 columns on the 8-bit tensor cores, in exact integer arithmetic.
+//
+// Every cell is split into seven signed base-256 digits relative to its column's largest magnitude (56 bits with the
+// sign: x = 2^e * sum of d_i 2^(-8 i - 7)), the digits are multiplied by tcgen05.mma (kind::i8) with 32-bit sums in tensor memory,
+// and the products of the same weight i + j are added up as 64-bit integers: no rounding, no order. Kept are the products with
+// i + j <= 7, so that what is lost is what lies behind a cell's 55 bits below 2^e, 2^-56 of 2^e at most, and 2^-60 of the product of two columns'
+// powers of two per row: against 64 bits the results are nearer than the FP64 sums are (six kinds of column, 20,011 x 250: 2e-17 of the
+// product of the columns' norms in the mean square and 3e-16 at most, against 4e-16 and 1e-14). The FP64 tensor core, which does the same sums at 37 TFLOP/s with a rounding per four rows,
+// stays for blocks in whose columns a few values stand out so far that this would not hold for the others: a column's
+// largest magnitude may be at most SP_SPREAD times the root mean square of its cells other than zero, and every value must be finite.
+//
+//  * k_split: decompressed rows -> planes [block of 128 columns][16 rows][digit][column][16 bytes], which is at once the layout of
+//    the operands in shared memory (K-major, no swizzle: a core matrix is 8 columns x 16 rows), so that a stage is copied as it lies.
+//  * k_syrk_i8: a CTA takes one pair of column blocks, half of the weights and a range of rows: bulk copies in a ring of
+//    four stages, one thread issues the products, four warps take the sums out of tensor memory at the end.
+//  * k_syrk_final: the integers to doubles, both triangles.
+#include "cla_common.cuh"
+#include "cla_split.cuh"
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+namespace cla {
+
+constexpr int SP_STAGES = 4;
+constexpr int SP_RING = 224 * 1024;
+constexpr int SP_T = 288;                               // four warps that take sums out, one that copies, four that multiply
+constexpr int SP_BLOCKS = 16;                           // 2048 columns
+constexpr int SP_ITEMS = SP_BLOCKS * (SP_BLOCKS - 1) + 3 * SP_BLOCKS;
+// rows whose sums stay below 2^31: seven products of 2^14 a row and weight
+constexpr int SP_ROWS = 16384;
+constexpr int SP_PAD = 24;                              // halves: whole stages of every set
+// What a CTA multiplies: a set of products d_i d_j whose sums fit tensor memory, four of 128 columns. Two sets for a pair of
+// different blocks (weights 0..3 and 4..7), three for a block with itself, where i < j stands for j < i too: those sums D are kept apart
+// from the E of i = j.
+struct SplitSet {
+  int products, digits, steps;  // steps of 32 rows in a stage
+  int clocks;                   // measured, of a step: what the CTAs are dealt by
+};
+__host__ __device__ constexpr SplitSet sp_set(int t) {
+  return t == 0 ? SplitSet{10, 4, 2, 770} : t == 1 ? SplitSet{24, 7, 1, 1690} : t == 2 ? SplitSet{4, 3, 4, 380} : t == 3 ? SplitSet{5, 5, 3, 470}
+                                                                                                          : SplitSet{10, 7, 2, 755};
+}
+// The sum (0..3) that product i, j of set t goes to, -1: not in the set
+__host__ __device__ constexpr int sp_sum(int t, int i, int j) {
+  const int w = i + j;
+  if (t == 0) return w <= 3 ? w : -1;
+  if (t == 1) return w >= 4 && w <= 7 ? w - 4 : -1;
+  if (i > j) return -1;
+  if (t == 2) return w == 0 ? 0 : w == 1 ? 1 : w == 2 ? (i < j ? 2 : 3) : -1;          // E0 D1 D2 E2
+  if (t == 3) return w == 3 ? 0 : w == 4 ? (i < j ? 1 : 2) : -1;                       // D3 D4 E4
+  return w == 5 ? 0 : w == 6 ? (i < j ? 1 : 2) : w == 7 ? 3 : -1;                       // D5 D6 E6 D7
+}
+// Whether it is the first of its sum, products in the order of i
+__host__ __device__ constexpr bool sp_first(int t, int i, int j) {
+  for (int a = 0; a < i; a++)
+    for (int b = 0; b < SP_DIG; b++)
+      if (sp_sum(t, a, b) == sp_sum(t, i, j)) return false;
+  for (int b = 0; b < j; b++)
+    if (sp_sum(t, i, b) == sp_sum(t, i, j)) return false;
+  return true;
+}
+constexpr double SP_SPREAD = 16.0;
+// Below these the FP64 products are as fast (us, FP64 / digits): 200,000 x 130 370 / 376, 200,000 x 150 320 / 353, 100,000 x 180 235 / 229; 2,500 x 250
+// 42 / 42, 5,000 x 250 44 / 44, 9,000 x 250 54 / 48, 12,000 x 180 47 / 47, 5,000 x 800 225 / 108.
+constexpr int SP_MIN_COLS = 176, SP_MIN_ROWS = 4096;
+constexpr int64_t SP_MIN_CELLS = 2000000;
+constexpr size_t SP_CHUNK = 192ull << 20;  // bytes of a chunk of rows (200,000 x 250: 303 us in one chunk of 358 MB, 317 in two)
+constexpr size_t SP_SMEM = (size_t)SP_RING + 1024;
+
+struct SplitPlan {
+  bool tried = false, ok = false;
+  int32_t* expo = nullptr;                // [nCols] e of every column
+  unsigned long long* check = nullptr;    // what the first call looks at: [0] cells that have no digits, [1 + column] cells other than zero
+};
+
+// --------------------------------------------------------------------------------------------------
+// A thread per column and 16 rows; rows behind the last one count as zeros. Bound: the two streams (8 bytes in, 7 out).
+template <bool CHECK>
+__global__ void __launch_bounds__(128) k_split(const double* __restrict__ X, size_t ld, int rows, int n, const int32_t* __restrict__ expo,
+                                               int64_t halves, uint8_t* __restrict__ planes, unsigned long long* __restrict__ check) {
+  const int c = blockIdx.y * SP_COLS + threadIdx.x;
+  if (c >= n) return;
+  const double scale = split_scale(expo[c]);
+  SplitCheck<CHECK> seen;
+  for (int64_t h = blockIdx.x; h < halves; h += gridDim.x) {
+    unsigned long long v[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = split_pack(h * 16 + i < rows ? __ldcs(X + (size_t)(h * 16 + i) * ld + c) : 0.0, scale, seen);
+    split_store(planes + ((size_t)blockIdx.y * halves + h) * SP_HALF, c, v, seen);
+  }
+  seen.report(check, c);
+}
+
+// --------------------------------------------------------------------------------------------------
+struct SyrkArgs {
+  const uint8_t* planes;
+  int64_t halves;               // of every block: 16 rows each, even
+  int nBlocks, lastN;           // columns of the last block, a multiple of 16
+  int nItems;
+  int16_t cta0[SP_ITEMS + 1];   // first CTA of an item: pairs of blocks row by row of the upper triangle, their sets in order
+  long long* sums;              // [pairs of blocks][weights 0..3, weights 4..7][column][row]
+  int32_t* err;
+};
+
+__device__ __forceinline__ uint32_t sp_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool sp_wait(uint32_t bar, uint32_t parity) {
+  uint32_t done = 0;
+  for (int it = 0; it < (1 << 22) && !done; it++) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  }
+  return done != 0;
+}
+// Operand of one digit of a stage: no swizzle, K-major; core matrices 128 bytes apart along the columns, `half` along the rows
+__device__ __forceinline__ uint64_t sp_desc(uint32_t addr, uint32_t half) {
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)(half >> 4) << 16 | (uint64_t)(128 >> 4) << 32 | (uint64_t)1 << 46;
+}
+__device__ __forceinline__ void sp_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b),
+               "r"(idesc), "r"((uint32_t)add)
+               : "memory");
+}
+// The products of one stage that go to one sum
+template <int T, int SUM, int P = 0>
+__device__ __forceinline__ void sp_products(uint32_t sum, uint64_t a, uint64_t b, uint32_t idesc, bool fresh) {
+  if constexpr (P < SP_DIG * SP_DIG) {
+    constexpr int i = P / SP_DIG, j = P % SP_DIG;
+    if constexpr (sp_sum(T, i, j) == SUM) {
+      constexpr uint64_t DIG = SP_PLANE >> 4;
+      sp_mma(sum, a + i * DIG, b + j * DIG, idesc, !(fresh && sp_first(T, i, j)));
+    }
+    sp_products<T, SUM, P + 1>(sum, a, b, idesc, fresh);
+  }
+}
+// One lane of the warp, the same each time: the loops around stay uniform
+__device__ __forceinline__ bool sp_elect() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+__device__ __forceinline__ void sp_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// Bound: the tensor pipe, 64 clocks a product of 128 x 128 x 32, next to the shared memory it reads its operands from, 8 KB a product, and
+// the stages are written to. A set of products is what four sums of 128 columns leave of tensor memory (SplitSet). 200,000 x 250 in one
+// launch: 150 us, tensor pipe 71 % active; 485 us for the FP64 products. On the way (one launch, some with fewer products): 338 with
+// stages of 32 rows, whose waits cost sets of few products more than their products; 328 with the CTAs of an item in row ranges of
+// their own, which read the planes from memory three times.
+__global__ void __launch_bounds__(SP_T, 1) k_syrk_i8(const __grid_constant__ SyrkArgs A) {
+  extern __shared__ __align__(1024) unsigned char spsm[];
+  __shared__ __align__(8) uint64_t full[SP_STAGES], empty[SP_STAGES], sumFull, sumEmpty;
+  __shared__ uint32_t tmemAt;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int item = 0;
+  for (int lo = 0, hi = A.nItems; lo < hi;) {  // the last item that starts at or before this CTA
+    const int mid = (lo + hi) / 2;
+    if (A.cta0[mid] <= (int)blockIdx.x) item = mid, lo = mid + 1;
+    else hi = mid;
+  }
+  int I = 0, J = 0, pair = 0, set = 0;
+  for (int it = 0; it + (I == J ? 3 : 2) <= item; pair++) {
+    it += I == J ? 3 : 2;
+    set = it;
+    if (++J == A.nBlocks) J = ++I;
+  }
+  set = item - set + (I == J ? 2 : 0);
+  const int N = J == A.nBlocks - 1 ? A.lastN : SP_COLS;
+  const int part = blockIdx.x - A.cta0[item], parts = A.cta0[item + 1] - A.cta0[item];
+  const int digits = sp_set(set).digits, nSums = set == 3 ? 3 : 4;
+  const uint32_t smem = (sp_smem(spsm) + 1023u) & ~1023u;
+  // A stage: the item's digits of 16 rows and of the next 16, so many times, of the first block and then of the second. The CTAs of an
+  // item take stages in turn, so that all items go down the rows together and the planes come from memory once.
+  const int R = sp_set(set).steps, nStages = (int)(A.halves / (2 * R)), mine = part < nStages ? (nStages - part + parts - 1) / parts : 0;
+  const uint32_t half = (uint32_t)digits * SP_PLANE, block = half * 2 * R, step = block * (I == J ? 1 : 2);
+  const int stages = min(SP_STAGES, SP_RING / (int)step);
+  if (warp == 5) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(sp_smem(&tmemAt)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    for (int i = 0; i < SP_STAGES; i++) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sp_smem(full + i)));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sp_smem(empty + i)), "r"(nSums));
+    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sp_smem(&sumFull)), "r"(nSums));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;" ::"r"(sp_smem(&sumEmpty)));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmemAt;
+  const int PIECE = SP_ROWS / 32 / R, pieces = (mine + PIECE - 1) / PIECE;  // stages between two times the sums are taken out
+  bool ok = true;
+  if (warp == 4) {
+    const uint8_t* a = A.planes + (size_t)I * A.halves * SP_HALF;
+    const uint8_t* b = A.planes + (size_t)J * A.halves * SP_HALF;
+    int s = 0;
+    uint32_t ph = 1;
+    for (int n = 0; n < mine; n++) {
+      ok = sp_wait(sp_smem(empty + s), ph);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      if (sp_elect()) {
+        const uint32_t bar = sp_smem(full + s), dst = smem + (uint32_t)s * step;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(step) : "memory");
+        const size_t at = (size_t)(part + (int64_t)n * parts) * (2 * R) * SP_HALF;
+        for (int h = 0; h < 2 * R; h++) {
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst + h * half),
+                       "l"(a + at + (size_t)h * SP_HALF), "r"(half), "r"(bar)
+                       : "memory");
+          if (I != J)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst + block + h * half),
+                         "l"(b + at + (size_t)h * SP_HALF), "r"(half), "r"(bar)
+                         : "memory");
+        }
+      }
+      __syncwarp();
+      if (++s == stages) s = 0, ph ^= 1;
+    }
+  } else if (warp >= 5) {
+    // A warp per sum: what a stage costs beside its products (waits, commit, operands to uniform registers: 400 clocks against 64 a product) it
+    // costs one warp while the others' products run.
+    const uint32_t sum = tmem + (warp - 5) * SP_COLS;
+    // 32-bit sums of signed bytes, both operands K-major, N x 128
+    const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(SP_COLS >> 4) << 24);
+    int s = 0, done = 0, at = 0;
+    uint32_t ph = 0;
+    for (int n = 0; n < (warp - 5 < nSums ? mine : 0); n++) {
+      ok = true;
+      if (at == 0 && n > 0) {  // the sums have been taken out
+        ok = sp_wait(sp_smem(&sumEmpty), (uint32_t)(done - 1) & 1u);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      ok = ok && sp_wait(sp_smem(full + s), ph);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      const uint32_t base = smem + (uint32_t)s * step;
+      uint64_t a = sp_desc(base, half), b = sp_desc(I == J ? base : base + block, half);
+      const bool out = at == PIECE - 1 || n + 1 == mine;
+      if (sp_elect()) {
+        for (int r = 0; r < R; r++, a += half >> 3, b += half >> 3)
+#define SP_CASE(T, SUM) case T * 4 + SUM: sp_products<T, SUM>(sum, a, b, idesc, at == 0 && r == 0); break;
+        switch (set * 4 + warp - 5) {
+          SP_CASE(0, 0) SP_CASE(0, 1) SP_CASE(0, 2) SP_CASE(0, 3) SP_CASE(1, 0) SP_CASE(1, 1) SP_CASE(1, 2) SP_CASE(1, 3)
+          SP_CASE(2, 0) SP_CASE(2, 1) SP_CASE(2, 2) SP_CASE(2, 3) SP_CASE(3, 0) SP_CASE(3, 1) SP_CASE(3, 2)
+          SP_CASE(4, 0) SP_CASE(4, 1) SP_CASE(4, 2) SP_CASE(4, 3)
+        }
+#undef SP_CASE
+        sp_commit(sp_smem(empty + s));
+        if (out) sp_commit(sp_smem(&sumFull));
+      }
+      __syncwarp();
+      at = out ? 0 : at + 1;
+      done += out;
+      if (++s == stages) s = 0, ph ^= 1;
+    }
+  } else {
+    long long* hi = A.sums + (size_t)pair * 2 * SP_COLS * SP_COLS + warp * 32 + lane;
+    long long* lo = hi + SP_COLS * SP_COLS;
+    const uint32_t t0 = tmem + ((uint32_t)warp << 21);
+    for (int p = 0; p < pieces && ok; p++) {
+      ok = sp_wait(sp_smem(&sumFull), (uint32_t)p & 1u);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int c = 0; c < N; c += 8) {
+        int32_t v[4][8];
+#pragma unroll
+        for (int w = 0; w < 4; w++)
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                       : "=r"(v[w][0]), "=r"(v[w][1]), "=r"(v[w][2]), "=r"(v[w][3]), "=r"(v[w][4]), "=r"(v[w][5]), "=r"(v[w][6]), "=r"(v[w][7])
+                       : "r"(t0 + min(w, nSums - 1) * SP_COLS + c)
+                       : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int w = 0; w < 4; w++)  // (nothing reads the registers before the wait)
+          asm volatile("" : "+r"(v[w][0]), "+r"(v[w][1]), "+r"(v[w][2]), "+r"(v[w][3]), "+r"(v[w][4]), "+r"(v[w][5]), "+r"(v[w][6]), "+r"(v[w][7]));
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          // in units of weight 3 and of weight 7; of a block with itself 2 D + E, whose mean with its mirror image is D + D' + E
+          const long long x = v[0][i], y = v[1][i], z = v[2][i], u = v[3][i];
+          unsigned long long* h = (unsigned long long*)(hi + (size_t)(c + i) * SP_COLS);
+          unsigned long long* l = (unsigned long long*)(lo + (size_t)(c + i) * SP_COLS);
+          if (set < 2) atomicAdd(set == 0 ? h : l, (unsigned long long)(((x * 256 + y) * 256 + z) * 256 + u));
+          else if (set == 2) atomicAdd(h, (unsigned long long)(((x * 256 + 2 * y) * 256 + 2 * z + u) * 256));
+          else if (set == 3) {
+            atomicAdd(h, (unsigned long long)(2 * x));
+            atomicAdd(l, (unsigned long long)((2 * y + z) * (1 << 24)));
+          } else atomicAdd(l, (unsigned long long)((2 * x * 256 + 2 * y + z) * 256 + 2 * u));
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sp_smem(&sumEmpty)) : "memory");
+    }
+  }
+  if (!ok) atomicExch(A.err, 106);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  __syncwarp();
+  if (warp == 5) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+  }
+}
+
+// Cells of the upper triangle's blocks from their two sums, to both triangles. grid: (pairs of blocks, rows of a block)
+__global__ void __launch_bounds__(SP_COLS) k_syrk_final(const long long* __restrict__ sums, int nBlocks, int n, const int32_t* __restrict__ expo,
+                                                        double* __restrict__ out, const int32_t* __restrict__ err) {
+  int I = 0, first = 0;
+  while (first + nBlocks - I <= (int)blockIdx.x) first += nBlocks - I++;
+  const int J = I + blockIdx.x - first, r = I * SP_COLS + threadIdx.x, c = J * SP_COLS + blockIdx.y;
+  if (r >= n || c >= n) return;
+  const long long* p = sums + (size_t)blockIdx.x * 2 * SP_COLS * SP_COLS + blockIdx.y * SP_COLS + threadIdx.x;
+  long long hi = p[0], lo = p[SP_COLS * SP_COLS];
+  if (I == J) {  // the mean with the mirror image
+    const long long* q = sums + (size_t)blockIdx.x * 2 * SP_COLS * SP_COLS + threadIdx.x * SP_COLS + blockIdx.y;
+    hi = (hi + q[0]) / 2;
+    lo = (lo + q[SP_COLS * SP_COLS]) / 2;
+  }
+  // in units of weights 3 and 7: 2^72 and 2^40, times 2^(e + e' - 110)
+  const double h = (double)hi, rest = (double)(hi - (long long)h);
+  double x = scalbn(h + fma((double)lo, 0x1p-32, rest), expo[r] + expo[c] - 38);
+  if (*err) x = __longlong_as_double(0x7ff8000000000000ll);  // (a kernel gave up: visible in the result as well)
+  out[(size_t)r * n + c] = x;
+  out[(size_t)c * n + r] = x;
+}
+
+// --------------------------------------------------------------------------------------------------
+static int blocks_of(const Matrix* m) { return (m->nCols + SP_COLS - 1) / SP_COLS; }
+// Rows of a chunk, in even parts of about SP_CHUNK bytes, a multiple of SKIP_ROWS; dense: it is decompressed first
+static int64_t split_chunk(const Matrix* m, bool dense) {
+  const double row = (dense ? ((m->nCols + 1) & ~1) * 8.0 : 0.0) + (double)blocks_of(m) * SP_COLS * SP_DIG;
+  const int64_t parts = std::max<int64_t>(1, (int64_t)(m->nRows * row / SP_CHUNK + 0.5));
+  return std::max<int64_t>(SKIP_ROWS, ((m->nRows + parts - 1) / parts + SKIP_ROWS - 1) / SKIP_ROWS * SKIP_ROWS);
+}
+
+// The columns' exponents, from the extrema (a bound on the cells is enough)
+static int64_t ensure_split(Matrix* m, cudaStream_t s) {
+  SplitPlan& P = *m->split;
+  if (P.tried) return CLA_OK;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return CLA_OK;  // (a call that is being captured runs nothing yet: no plan from it)
+  }
+  const int n = m->nCols;
+  std::vector<double> lo, hi;
+  int64_t rc;
+  if ((rc = col_minmax(m, lo, hi, s)) < 0) return rc;
+  P.tried = true;
+  std::vector<int32_t> e(n, 0);
+  for (int c = 0; c < n; c++) {
+    const double M = std::max(std::fabs(lo[c]), std::fabs(hi[c]));
+    if (M == 0.0) continue;
+    if (!(M < 1e140 && M > 1e-140)) return CLA_OK;  // the scale or the sums would leave the range of doubles
+    int x;
+    if (std::frexp(M, &x) > 0.99) x++;  // the leading digit stays within a byte when the others carry
+    e[c] = x;
+  }
+  const size_t expoBytes = ((size_t)n * 4 + 255) & ~(size_t)255, checkBytes = ((size_t)n + 1) * 8;
+  void* p = nullptr;
+  if (plan_alloc(m, &p, expoBytes + checkBytes) < 0) return CLA_OK;
+  CLA_CUDA(cudaMemcpyAsync(p, e.data(), (size_t)n * 4, cudaMemcpyHostToDevice, s));
+  CLA_CUDA(cudaMemsetAsync((char*)p + expoBytes, 0, checkBytes, s));
+  CLA_CUDA(cudaStreamSynchronize(s));
+  P.expo = (int32_t*)p;
+  P.check = (unsigned long long*)((char*)p + expoBytes);
+  P.ok = true;
+  return CLA_OK;
+}
+// After the first product: whether its columns are such that digits were the better way. The sums of squares are on its diagonal.
+static int64_t check_split(Matrix* m, const double* dOut, cudaStream_t s) {
+  SplitPlan& P = *m->split;
+  const int n = m->nCols;
+  std::vector<unsigned long long> seen(n + 1);
+  std::vector<double> squares(n);
+  std::vector<int32_t> e(n);
+  CLA_CUDA(cudaMemcpyAsync(seen.data(), P.check, ((size_t)n + 1) * 8, cudaMemcpyDeviceToHost, s));
+  CLA_CUDA(cudaMemcpyAsync(e.data(), P.expo, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
+  CLA_CUDA(cudaMemcpy2DAsync(squares.data(), 8, dOut, ((size_t)n + 1) * 8, 8, n, cudaMemcpyDeviceToHost, s));
+  CLA_CUDA(cudaStreamSynchronize(s));
+  P.check = nullptr;
+  if (seen[0]) P.ok = false;
+  for (int c = 0; c < n; c++)
+    if (std::ldexp(1.0, e[c]) > 2.0 * SP_SPREAD * std::sqrt(squares[c] / std::max<double>(1.0, (double)seen[c + 1])) && squares[c] > 0.0) P.ok = false;
+  return CLA_OK;
+}
+
+bool split_covers(const Matrix* m) {
+  return m->nCols >= SP_MIN_COLS && m->nCols <= SP_BLOCKS * SP_COLS && m->nRows >= SP_MIN_ROWS && (int64_t)m->nRows * m->nCols >= SP_MIN_CELLS && m->colSrcValid && !m->overlapping;
+}
+
+int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
+  if (!split_covers(m)) return 0;
+  if (!m->split) m->split = new SplitPlan();
+  if (m->split->tried && !m->split->ok) return 0;
+  const int n = m->nCols, nb = blocks_of(m), pairs = nb * (nb + 1) / 2;
+  const size_t ld = (size_t)((n + 1) & ~1);
+  int64_t rc;
+  if ((rc = ensure_split(m, s)) < 0) return rc;
+  if (!m->split->ok) return 0;
+  const bool direct = split_cols_covers(m, s);
+  const int64_t chunk = split_chunk(m, !direct);
+  const size_t denseBytes = direct ? 0 : (size_t)chunk * ld * 8, planeBytes = (size_t)nb * (chunk / 16 + SP_PAD) * SP_HALF;
+  const size_t sumBytes = (size_t)pairs * 2 * SP_COLS * SP_COLS * 8;
+  if ((rc = ensure_scratch2(m, denseBytes + planeBytes + sumBytes)) < 0) return rc;
+  double* X = (double*)m->scratch2;
+  uint8_t* planes = (uint8_t*)m->scratch2 + denseBytes;
+  long long* sums = (long long*)(planes + planeBytes);
+  static OncePerDevice once;
+  if (const int64_t e = allow_smem(once, m->device, SP_SMEM, k_syrk_i8); e < 0) return e;
+  CLA_CUDA(cudaMemsetAsync(sums, 0, sumBytes, s));
+  SyrkArgs A{};
+  A.planes = planes;
+  A.nBlocks = nb;
+  A.lastN = (n - (nb - 1) * SP_COLS + 15) / 16 * 16;
+  A.nItems = pairs * 2 + nb;
+  A.sums = sums;
+  A.err = m->dErr;
+  // CTAs in proportion to the products of an item
+  {
+    double total = 0.0, at = 0.0;
+    auto each = [&](auto&& f) {
+      int it = 0;
+      for (int I = 0; I < nb; I++)
+        for (int J = I; J < nb; J++)
+          for (int t = I == J ? 2 : 0; t < (I == J ? 5 : 2); t++, it++) {
+            const SplitSet S = sp_set(t);
+            f(it, J == nb - 1 ? std::max(S.clocks * A.lastN / (double)SP_COLS, S.clocks * 0.6) : S.clocks);
+          }
+    };
+    each([&](int, double c) { total += c; });
+    const int ctas = std::max(m->smCount, A.nItems);
+    each([&](int it, double c) {
+      const int want = (int)(at / total * ctas + 0.5);
+      A.cta0[it] = (int16_t)std::min(std::max(want, it == 0 ? 0 : A.cta0[it - 1] + 1), ctas - (A.nItems - it));
+      at += c;
+    });
+    A.cta0[A.nItems] = (int16_t)ctas;
+  }
+  for (int64_t r0 = 0; r0 < m->nRows; r0 += chunk) {
+    const int r1 = (int)std::min<int64_t>(m->nRows, r0 + chunk), rows = r1 - (int)r0;
+    A.halves = ((int64_t)rows + 16 * SP_PAD - 1) / (16 * SP_PAD) * SP_PAD;
+    if (direct) {
+      if ((rc = launch_split_cols(m, (int)r0, r1, m->split->expo, A.halves, planes, m->split->check, s)) < 0) return rc;
+    } else if ((rc = launch_decompress_range(m, (int)r0, r1, X, s, ld)) < 0) return rc;
+    if (!direct) {
+      const dim3 grid((unsigned)std::min<int64_t>(A.halves, 16 * m->smCount / nb), nb);
+      if (m->split->check) k_split<true><<<grid, SP_COLS, 0, s>>>(X, ld, rows, n, m->split->expo, A.halves, planes, m->split->check);
+      else k_split<false><<<grid, SP_COLS, 0, s>>>(X, ld, rows, n, m->split->expo, A.halves, planes, nullptr);
+    }
+    if (r0 == 0) prof_begin(m, s);
+    k_syrk_i8<<<A.cta0[A.nItems], SP_T, SP_SMEM, s>>>(A);
+    if (r0 == 0) prof_end(m, s);
+    m->stats.kernel_launches += direct ? 1 : 2;
+  }
+  k_syrk_final<<<dim3(pairs, SP_COLS), SP_COLS, 0, s>>>(sums, nb, n, m->split->expo, dOut, m->dErr);
+  m->stats.kernel_launches++;
+  CLA_CUDA(cudaGetLastError());
+  if (m->split->check && (rc = check_split(m, dOut, s)) < 0) return rc;
+  return m->split->ok ? 1 : 0;
+}
+
+void split_plan_free(Matrix* m) {
+  delete m->split;
+  m->split = nullptr;
+}
+
+}  // namespace cla

@@ -716,9 +716,10 @@ int64_t launch_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
     CLA_CUDA(cudaGetLastError());
     return CLA_OK;
   }
+  int64_t rc;
+  if ((rc = split_tsmm(m, dOut, s)) != 0) return rc < 0 ? rc : CLA_OK;
   CLA_CUDA(cudaMemsetAsync(dOut, 0, sizeof(double) * (size_t)n * n, s));
   if (m->nRows == 0) return CLA_OK;
-  int64_t rc;
   const bool tri = n <= 128;
   bool denseOnly = m->colSrcValid;
   for (auto& g : m->groups) denseOnly &= (g.type == GT_DDC || g.type == GT_UNC);

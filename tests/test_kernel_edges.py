@@ -7,6 +7,7 @@ from systemds_b200 import CompressedMatrixBlock, datagen
 from systemds_b200 import colgroup as cg
 from systemds_b200.cmb import CHAIN_XtwXv, CLALibDecompress, CLALibLeftMultBy, CLALibMMChain, CLALibRightMultBy, CLALibTSMM
 from systemds_b200.mapping import MapToFactory
+from systemds_b200.offset import OffsetFactory
 from tests.util import TOL, abs_dense_of, dense_of, rel_err
 
 pytestmark = pytest.mark.gpu
@@ -165,6 +166,92 @@ def test_self_product_blocks(oracle, nRows, nCols):
         assert rel_err(got, oracle.dense_tsmm_ld(X), np.abs(X).T @ np.abs(X) + 1e-300) < TOL
         assert np.array_equal(got, got.T)
         cmb.free()
+
+
+def _six_kinds(nRows, nCols, by_kind):
+    """Byte and wide maps, listed rows without and with a default tuple, runs, dense columns; all of them of modest spread."""
+    rng = np.random.default_rng(nCols)
+    kinds = ["ddc", "sdc", "default", "rle", "unc", "wide"]
+    groups = []
+    for c in range(nCols):
+        k = kinds[c * 6 // nCols if by_kind else c % 6]
+        if k == "ddc":
+            n = int(rng.integers(2, 40))
+            groups.append(cg.ColGroupDDC([c], rng.standard_normal((n, 1)), MapToFactory.create_from(rng.integers(0, n, nRows), n)))
+        elif k == "wide":
+            groups.append(cg.ColGroupDDC([c], rng.uniform(-1, 1, (400, 1)), MapToFactory.create_from(rng.integers(0, 400, nRows), 400)))
+        elif k in ("sdc", "default"):
+            rows = np.flatnonzero(rng.random(nRows) < 0.1)
+            ids = MapToFactory.create_from(rng.integers(0, 5, rows.size), 5)
+            d, off = rng.standard_normal((5, 1)), OffsetFactory.createOffset(rows)
+            groups.append(cg.ColGroupSDCZeros([c], nRows, d, off, ids) if k == "sdc" else
+                          cg.ColGroupSDC([c], nRows, d, np.array([0.3]), off, ids))
+        elif k == "rle":
+            ends = np.minimum(np.cumsum(rng.geometric(0.01, size=nRows // 30)), nRows)
+            starts = np.concatenate([[0], ends[:-1]])
+            keep = ends > starts
+            starts, ends = starts[keep], ends[keep]
+            ends[-1] = nRows
+            groups.append(cg.ColGroupRLE.from_runs([c], rng.standard_normal((9, 1)), starts, ends - starts, rng.integers(0, 9, starts.size), nRows))
+        else:
+            groups.append(cg.ColGroupUncompressed([c], rng.standard_normal((nRows, 1))))
+    return CompressedMatrixBlock(nRows, nCols, groups)
+
+
+@pytest.mark.parametrize("nRows,nCols", [(11364, 176), (8193, 255), (20011, 257), (40001, 384), (4096, 500)])
+@pytest.mark.parametrize("by_kind", [True, False])
+def test_self_product_in_digits(oracle, nRows, nCols, by_kind):
+    """t(X) X by 8-bit digits, straight from the columns and from decompressed rows: smallest sizes, blocks of 128 columns with
+    few and many left over, row remainders. What is lost lies 55 bits behind a column's power of two 2^e (2^-56 of it
+    per cell at most) and behind weight 7 (five products of digits below 2^14 in units of 2^-78, and what follows); then the
+    result is rounded. Integers: the same bits from every call."""
+    cmb = _six_kinds(nRows, nCols, by_kind).to_device()
+    X = dense_of(cmb)
+    got = np.array(CLALibTSMM.leftMultByTransposeSelf(cmb))
+    want = oracle.dense_tsmm_ld(X)
+    e = np.exp2(np.ceil(np.log2(np.abs(X).max(axis=0) / 0.99)))
+    a = np.abs(X).sum(axis=0)
+    lost = 2.0**-56 * (np.outer(e, a) + np.outer(a, e)) + nRows * 2.0**-60 * np.outer(e, e)
+    oracles = nRows * 2.0**-64 * (np.abs(X).T @ np.abs(X))  # long double, one sum after the other
+    assert (np.abs(got - want) <= lost + oracles + 2.0**-52 * np.abs(want)).all()
+    norms = np.sqrt(np.outer(np.diag(want), np.diag(want)))
+    assert (np.abs(got - want) / norms).max() < 1e-15  # (the FP64 products: 4e-15 to 2e-14)
+    assert np.array_equal(got, got.T)
+    assert np.array_equal(got, np.array(CLALibTSMM.leftMultByTransposeSelf(cmb)))
+    cmb.free()
+
+
+def test_self_product_of_integers_in_digits():
+    """Integers of up to 24 bits: nothing is lost, to the last bit of sums below 2^53."""
+    rng = np.random.default_rng(2)
+    groups = [cg.ColGroupDDC([c], rng.integers(-2**16, 2**16, (9, 1)).astype(float) * (2.0**8 if c % 3 else 2.0**-20),
+                             MapToFactory.create_from(rng.integers(0, 9, 12000), 9)) for c in range(200)]
+    cmb = CompressedMatrixBlock(12000, 200, groups).to_device()
+    X = dense_of(cmb)
+    s = np.where(np.arange(200) % 3, 2.0**-8, 2.0**20)
+    Z = (X * s).astype(np.int64)
+    assert np.array_equal(np.array(CLALibTSMM.leftMultByTransposeSelf(cmb)), (Z.T @ Z).astype(float) / np.outer(s, s))
+    cmb.free()
+
+
+@pytest.mark.parametrize("values", [[1e6] + [1.0] * 8, [np.inf] + [1.0] * 8, [np.nan] + [1.0] * 8, [1e-200, 2e-200] + [1e-200] * 7, [0.0] * 9])
+def test_self_product_without_digits(values):
+    """One column whose values stand out too far, are not finite or too small, or all zero: the products in double precision, or
+    digits that are all zero."""
+    rng = np.random.default_rng(1)
+    groups = [cg.ColGroupDDC([c], rng.standard_normal((9, 1)), MapToFactory.create_from(rng.integers(0, 9, 12000), 9)) for c in range(199)]
+    ids = rng.integers(1, 9, 12000)
+    ids[17] = 0
+    groups.append(cg.ColGroupDDC([199], np.array(values).reshape(-1, 1), MapToFactory.create_from(ids, 9)))
+    cmb = CompressedMatrixBlock(12000, 200, groups).to_device()
+    X = dense_of(cmb)
+    got = np.array(CLALibTSMM.leftMultByTransposeSelf(cmb))
+    with np.errstate(invalid="ignore"):
+        want, s = X.T @ X, np.abs(X).T @ np.abs(X)
+    fine = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), fine)
+    assert (np.abs(got - want)[fine] <= TOL * s[fine] + 1e-320).all()
+    cmb.free()
 
 
 @pytest.mark.parametrize("nRows", [1, 255, 257, 1040, 5001])
