@@ -9,7 +9,7 @@
 // stays for blocks in whose columns a few values stand out so far that this would not hold for the others: a column's
 // largest magnitude may be at most SP_SPREAD times the root mean square of its cells other than zero, and every value must be finite.
 //
-//  * k_split: decompressed rows -> planes [block of 128 columns][16 rows][digit][column][16 bytes], which is at once the layout of
+//  * k_split_maps, k_split_cols (cla_generic.cu), k_split: dense maps, other columns by kind, decompressed rows -> planes [block of 128 columns][16 rows][digit][column][16 bytes], which is at once the layout of
 //    the operands in shared memory (K-major, no swizzle: a core matrix is 8 columns x 16 rows), so that a stage is copied as it lies.
 //  * k_syrk_i8: a CTA takes one pair of column blocks, half of the weights and a range of rows: bulk copies in a ring of
 //    four stages, one thread issues the products, four warps take the sums out of tensor memory at the end.
@@ -28,6 +28,7 @@ constexpr int SP_RING = 224 * 1024;
 constexpr int SP_T = 288;                               // four warps that take sums out, one that copies, four that multiply
 constexpr int SP_BLOCKS = 16;                           // 2048 columns
 constexpr int SP_ITEMS = SP_BLOCKS * (SP_BLOCKS - 1) + 3 * SP_BLOCKS;
+constexpr int64_t SP_TOTAL = 4 << 20;                   // rows whose 64-bit sums are safe: five products of 2^14 in units of 2^24 a row, with room
 // rows whose sums stay below 2^31: seven products of 2^14 a row and weight
 constexpr int SP_ROWS = 16384;
 constexpr int SP_PAD = 24;                              // halves: whole stages of every set
@@ -66,6 +67,7 @@ constexpr double SP_SPREAD = 16.0;
 // 42 / 42, 5,000 x 250 44 / 44, 9,000 x 250 54 / 48, 12,000 x 180 47 / 47, 5,000 x 800 225 / 108.
 constexpr int SP_MIN_COLS = 176, SP_MIN_ROWS = 4096;
 constexpr int64_t SP_MIN_CELLS = 2000000;
+constexpr int SP_MAPS_COLS = 129;  // where k_split_maps takes the block (200,000 x 130 bytes 319 / 222, 1000 values 359 / 260; 16,000 x 130 47 / 38)
 constexpr size_t SP_CHUNK = 192ull << 20;  // bytes of a chunk of rows (200,000 x 250: 303 us in one chunk of 358 MB, 317 in two)
 constexpr size_t SP_SMEM = (size_t)SP_RING + 1024;
 
@@ -91,6 +93,66 @@ __global__ void __launch_bounds__(128) k_split(const double* __restrict__ X, siz
     split_store(planes + ((size_t)blockIdx.y * halves + h) * SP_HALF, c, v, seen);
   }
   seen.report(check, c);
+}
+
+// Dense maps straight to planes: a CTA owns 16 columns, their tables of digits in shared memory (entry k of slot s at k * 16 + s, so that a
+// lane stays in its banks), and a range of rows; a lane takes 16 rows of its column.
+// Bound: the latency of the maps' loads, a sector a lane, next to the planes written (7 bytes a cell). The self product of 160,000 x 250 of 1000 values
+// took 421 us with the rows decompressed and split, 232 with this (256 values: 380 and 211).
+constexpr int SM_W = 16;
+constexpr int SM_VALS = 1600;  // tuples, at most: 200 KB
+template <bool CHECK>
+__global__ void __launch_bounds__(SM_W * 32, 1) k_split_maps(const DevGroup* __restrict__ groups, const int32_t* __restrict__ colSrc, const double* __restrict__ constV,
+                                                             const int32_t* __restrict__ expo, int n, int r0, int r1, int64_t halves,
+                                                             uint8_t* __restrict__ planes, unsigned long long* __restrict__ check) {
+  extern __shared__ unsigned long long smt[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.y * 16 + (lane & 15), up = lane >> 4;
+  const bool on = c < n;
+  const DevGroup& g = groups[colSrc[2 * (on ? c : 0)]];
+  const int nv = g.nVals, mt = g.mapType;
+  unsigned long long* T = smt + (lane & 15);
+  SplitCheck<CHECK> seen;
+  if (on) {
+    const double* dict = g.dict + colSrc[2 * c + 1];
+    const double cst = constV ? constV[c] : 0.0, scale = split_scale(expo[c]);
+    const int gc = g.gCols;
+#pragma unroll 4
+    for (int k = warp * 2 + up; k < nv; k += SM_W * 2) T[k * 16] = split_pack(cst + dict[(size_t)k * gc], scale, seen);
+  }
+  __syncthreads();
+  uint8_t* o = planes + (size_t)(c / SP_COLS) * halves * SP_HALF;
+  const int64_t h0 = halves * blockIdx.x / gridDim.x, h1 = halves * (blockIdx.x + 1) / gridDim.x;
+  const void* map = g.map;
+  // the ids of a lane's next 16 rows are under way while it works on these
+  uint4 a0 = make_uint4(0, 0, 0, 0), b0 = a0;
+  auto load = [&](int64_t h) {
+    const int64_t r = r0 + h * 16;
+    if (h >= h1 || r + 16 > r1 || !on) return;
+    if (mt == CLA_MAP_CHAR) {
+      a0 = __ldg((const uint4*)((const uint16_t*)map + r));
+      b0 = __ldg((const uint4*)((const uint16_t*)map + r) + 1);
+    } else if (mt != CLA_MAP_BIT) a0 = __ldg((const uint4*)((const uint8_t*)map + r));
+  };
+  load(h0 + warp * 2 + up);
+  for (int64_t h = h0 + warp * 2 + up; h < h1; h += SM_W * 2) {
+    if (!on) continue;
+    const int64_t r = r0 + h * 16;
+    const uint32_t w[8] = {a0.x, a0.y, a0.z, a0.w, b0.x, b0.y, b0.z, b0.w};
+    load(h + SM_W * 2);
+    unsigned long long v[16];
+    if (r + 16 <= r1 && mt == CLA_MAP_CHAR) {
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = T[(i & 1 ? w[i >> 1] >> 16 : w[i >> 1] & 0xFFFFu) * 16];
+    } else if (r + 16 <= r1 && mt != CLA_MAP_BIT) {
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = T[((w[i >> 2] >> (8 * (i & 3))) & 0xFFu) * 16];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = r + i < r1 ? T[map_get(mt, map, nullptr, r + i) * 16] : 0ull;
+    }
+    split_store(o + (size_t)h * SP_HALF, c, v, seen);
+  }
+  if (on) seen.report(check, c);
 }
 
 // --------------------------------------------------------------------------------------------------
@@ -310,7 +372,7 @@ __global__ void __launch_bounds__(SP_T, 1) k_syrk_i8(const __grid_constant__ Syr
 
 // Cells of the upper triangle's blocks from their two sums, to both triangles. grid: (pairs of blocks, rows of a block)
 __global__ void __launch_bounds__(SP_COLS) k_syrk_final(const long long* __restrict__ sums, int nBlocks, int n, const int32_t* __restrict__ expo,
-                                                        double* __restrict__ out, const int32_t* __restrict__ err) {
+                                                        double* __restrict__ out, int add, const int32_t* __restrict__ err) {
   int I = 0, first = 0;
   while (first + nBlocks - I <= (int)blockIdx.x) first += nBlocks - I++;
   const int J = I + blockIdx.x - first, r = I * SP_COLS + threadIdx.x, c = J * SP_COLS + blockIdx.y;
@@ -319,13 +381,15 @@ __global__ void __launch_bounds__(SP_COLS) k_syrk_final(const long long* __restr
   long long hi = p[0], lo = p[SP_COLS * SP_COLS];
   if (I == J) {  // the mean with the mirror image
     const long long* q = sums + (size_t)blockIdx.x * 2 * SP_COLS * SP_COLS + threadIdx.x * SP_COLS + blockIdx.y;
-    hi = (hi + q[0]) / 2;
-    lo = (lo + q[SP_COLS * SP_COLS]) / 2;
+    hi = hi / 2 + q[0] / 2 + (hi % 2 + q[0] % 2) / 2;
+    lo = lo / 2 + q[SP_COLS * SP_COLS] / 2 + (lo % 2 + q[SP_COLS * SP_COLS] % 2) / 2;
   }
   // in units of weights 3 and 7: 2^72 and 2^40, times 2^(e + e' - 110)
   const double h = (double)hi, rest = (double)(hi - (long long)h);
   double x = scalbn(h + fma((double)lo, 0x1p-32, rest), expo[r] + expo[c] - 38);
   if (*err) x = __longlong_as_double(0x7ff8000000000000ll);  // (a kernel gave up: visible in the result as well)
+  if (I == J && c < r) return;  // (written from the other side)
+  if (add) x += out[(size_t)r * n + c];
   out[(size_t)r * n + c] = x;
   out[(size_t)c * n + r] = x;
 }
@@ -391,12 +455,27 @@ static int64_t check_split(Matrix* m, const double* dOut, cudaStream_t s) {
   return CLA_OK;
 }
 
-bool split_covers(const Matrix* m) {
-  return m->nCols >= SP_MIN_COLS && m->nCols <= SP_BLOCKS * SP_COLS && m->nRows >= SP_MIN_ROWS && (int64_t)m->nRows * m->nCols >= SP_MIN_CELLS && m->colSrcValid && !m->overlapping;
+// Every column in a dense map of bits, bytes or 16 bits whose table fits: k_split_maps; the longest table, 0: no
+static int split_maps_vals(const Matrix* m) {
+  if (!m->colSrcValid || m->multiCover) return 0;
+  int64_t covered = 0;
+  int vals = 0;
+  for (auto& g : m->groups) {
+    if (g.type != GT_DDC || g.nVals > SM_VALS) return 0;
+    if (g.mapType != CLA_MAP_BIT && g.mapType != CLA_MAP_BYTE && g.mapType != CLA_MAP_UBYTE && g.mapType != CLA_MAP_CHAR) return 0;
+    covered += g.gCols;
+    vals = std::max(vals, g.nVals);
+  }
+  return covered == m->nCols ? vals : 0;
+}
+static bool split_covers(const Matrix* m, bool maps) {
+  const int64_t cells = (int64_t)m->nRows * m->nCols;
+  return m->nCols >= (maps ? SP_MAPS_COLS : SP_MIN_COLS) && m->nCols <= SP_BLOCKS * SP_COLS && m->nRows >= SP_MIN_ROWS && cells >= SP_MIN_CELLS && m->colSrcValid && !m->overlapping;
 }
 
 int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
-  if (!split_covers(m)) return 0;
+  const int vals = split_maps_vals(m);
+  if (!split_covers(m, vals > 0)) return 0;
   if (!m->split) m->split = new SplitPlan();
   if (m->split->tried && !m->split->ok) return 0;
   const int n = m->nCols, nb = blocks_of(m), pairs = nb * (nb + 1) / 2;
@@ -404,9 +483,11 @@ int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
   int64_t rc;
   if ((rc = ensure_split(m, s)) < 0) return rc;
   if (!m->split->ok) return 0;
-  const bool direct = split_cols_covers(m, s);
-  const int64_t chunk = split_chunk(m, !direct);
-  const size_t denseBytes = direct ? 0 : (size_t)chunk * ld * 8, planeBytes = (size_t)nb * (chunk / 16 + SP_PAD) * SP_HALF;
+  const int32_t* expo = m->split->expo;
+  unsigned long long* check = m->split->check;
+  const bool cols = !vals && split_cols_covers(m, s), dense = !vals && !cols;
+  const int64_t chunk = split_chunk(m, dense);
+  const size_t denseBytes = dense ? (size_t)chunk * ld * 8 : 0, planeBytes = (size_t)nb * (chunk / 16 + SP_PAD) * SP_HALF;
   const size_t sumBytes = (size_t)pairs * 2 * SP_COLS * SP_COLS * 8;
   if ((rc = ensure_scratch2(m, denseBytes + planeBytes + sumBytes)) < 0) return rc;
   double* X = (double*)m->scratch2;
@@ -414,7 +495,8 @@ int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
   long long* sums = (long long*)(planes + planeBytes);
   static OncePerDevice once;
   if (const int64_t e = allow_smem(once, m->device, SP_SMEM, k_syrk_i8); e < 0) return e;
-  CLA_CUDA(cudaMemsetAsync(sums, 0, sumBytes, s));
+  static OncePerDevice onceMaps;
+  if (const int64_t e = allow_smem(onceMaps, m->device, (size_t)SM_VALS * 128, k_split_maps<false>, k_split_maps<true>); e < 0) return e;
   SyrkArgs A{};
   A.planes = planes;
   A.nBlocks = nb;
@@ -422,7 +504,7 @@ int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
   A.nItems = pairs * 2 + nb;
   A.sums = sums;
   A.err = m->dErr;
-  // CTAs in proportion to the products of an item
+  // CTAs by the time of an item
   {
     double total = 0.0, at = 0.0;
     auto each = [&](auto&& f) {
@@ -443,26 +525,42 @@ int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
     });
     A.cta0[A.nItems] = (int16_t)ctas;
   }
+  int64_t summed = 0;  // rows in the 64-bit sums
+  bool add = false;
   for (int64_t r0 = 0; r0 < m->nRows; r0 += chunk) {
     const int r1 = (int)std::min<int64_t>(m->nRows, r0 + chunk), rows = r1 - (int)r0;
+    if (summed == 0) CLA_CUDA(cudaMemsetAsync(sums, 0, sumBytes, s));
     A.halves = ((int64_t)rows + 16 * SP_PAD - 1) / (16 * SP_PAD) * SP_PAD;
-    if (direct) {
-      if ((rc = launch_split_cols(m, (int)r0, r1, m->split->expo, A.halves, planes, m->split->check, s)) < 0) return rc;
-    } else if ((rc = launch_decompress_range(m, (int)r0, r1, X, s, ld)) < 0) return rc;
-    if (!direct) {
+    if (vals) {
+      const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(A.halves / (SM_W * 2) + 1, m->smCount / ((n + 15) / 16))), (n + 15) / 16);
+      const double* constV = m->hasConst ? m->dConstV : nullptr;
+      const size_t smem = (size_t)vals * 128;
+      if (check) k_split_maps<true><<<grid, SM_W * 32, smem, s>>>(m->dGroups, m->dColSrc, constV, expo, n, (int)r0, r1, A.halves, planes, check);
+      else k_split_maps<false><<<grid, SM_W * 32, smem, s>>>(m->dGroups, m->dColSrc, constV, expo, n, (int)r0, r1, A.halves, planes, nullptr);
+      m->stats.kernel_launches++;
+    } else if (cols) {
+      if ((rc = launch_split_cols(m, (int)r0, r1, expo, A.halves, planes, check, s)) < 0) return rc;
+    } else {
+      if ((rc = launch_decompress_range(m, (int)r0, r1, X, s, ld)) < 0) return rc;
       const dim3 grid((unsigned)std::min<int64_t>(A.halves, 16 * m->smCount / nb), nb);
-      if (m->split->check) k_split<true><<<grid, SP_COLS, 0, s>>>(X, ld, rows, n, m->split->expo, A.halves, planes, m->split->check);
-      else k_split<false><<<grid, SP_COLS, 0, s>>>(X, ld, rows, n, m->split->expo, A.halves, planes, nullptr);
+      if (check) k_split<true><<<grid, SP_COLS, 0, s>>>(X, ld, rows, n, expo, A.halves, planes, check);
+      else k_split<false><<<grid, SP_COLS, 0, s>>>(X, ld, rows, n, expo, A.halves, planes, nullptr);
+      m->stats.kernel_launches++;
     }
     if (r0 == 0) prof_begin(m, s);
     k_syrk_i8<<<A.cta0[A.nItems], SP_T, SP_SMEM, s>>>(A);
     if (r0 == 0) prof_end(m, s);
-    m->stats.kernel_launches += direct ? 1 : 2;
+    m->stats.kernel_launches++;
+    summed += rows;
+    if (r1 == m->nRows || summed + chunk > SP_TOTAL) {
+      k_syrk_final<<<dim3(pairs, SP_COLS), SP_COLS, 0, s>>>(sums, nb, n, expo, dOut, add ? 1 : 0, m->dErr);
+      m->stats.kernel_launches++;
+      summed = 0;
+      add = true;
+    }
   }
-  k_syrk_final<<<dim3(pairs, SP_COLS), SP_COLS, 0, s>>>(sums, nb, n, m->split->expo, dOut, m->dErr);
-  m->stats.kernel_launches++;
   CLA_CUDA(cudaGetLastError());
-  if (m->split->check && (rc = check_split(m, dOut, s)) < 0) return rc;
+  if (check && (rc = check_split(m, dOut, s)) < 0) return rc;
   return m->split->ok ? 1 : 0;
 }
 

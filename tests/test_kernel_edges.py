@@ -221,6 +221,50 @@ def test_self_product_in_digits(oracle, nRows, nCols, by_kind):
     cmb.free()
 
 
+def _self_product_in_digits(oracle, cmb):
+    X = dense_of(cmb)
+    got = np.array(CLALibTSMM.leftMultByTransposeSelf(cmb))
+    want = oracle.dense_tsmm_ld(X)
+    norms = np.sqrt(np.outer(np.diag(want), np.diag(want)))
+    assert (np.abs(got - want) / norms).max() < 1e-15
+    assert np.array_equal(got, got.T)
+    assert np.array_equal(got, np.array(CLALibTSMM.leftMultByTransposeSelf(cmb)))
+
+
+@pytest.mark.parametrize("nRows", [16384, 16399, 20001])
+@pytest.mark.parametrize("cards,width", [([7] * 129, 1), ([2, 256, 100] * 50, 1), ([400, 1600, 3] * 48, 1), ([9, 300] * 40, 2)])
+def test_self_product_of_dense_maps_in_digits(oracle, nRows, cards, width):
+    """Bit, byte and 16-bit maps, the longest tables, co-coded columns, a lane's last rows, part units of 16 columns."""
+    cmb = _ddc(nRows, cards, nRows + len(cards), width=width).to_device()
+    _self_product_in_digits(oracle, cmb)
+    cmb.free()
+
+
+def test_self_product_in_digits_of_many_rows():
+    """More rows than one round of 64-bit sums takes: 1' (X'X) 1 = |X 1|^2, and the square sums of single columns."""
+    torch = pytest.importorskip("torch")
+    from systemds_b200.mapping import MAP_BYTE, DeviceMap
+    n, cols = 5_000_017, 130
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(4)
+    rng = np.random.default_rng(4)
+    groups, ones, squares = [], torch.zeros(n, dtype=torch.float64, device="cuda"), []
+    for c in range(cols):
+        ids = torch.randint(0, 50, (n,), dtype=torch.uint8, device="cuda", generator=gen)
+        d = rng.standard_normal((50, 1))
+        x = torch.from_numpy(d.ravel()).cuda()[ids.long()]
+        ones += x
+        squares.append(float((x * x).sum()))
+        groups.append(cg.ColGroupDDC([c], d, DeviceMap(MAP_BYTE, n, 50, ids.data_ptr(), n, owner=ids)))
+    torch.cuda.synchronize()
+    cmb = CompressedMatrixBlock(n, cols, groups).to_device()
+    got = np.array(CLALibTSMM.leftMultByTransposeSelf(cmb))
+    assert np.allclose(np.diag(got), squares, rtol=1e-12, atol=0)
+    assert abs(got.sum() - float((ones * ones).sum())) <= 1e-12 * np.abs(got).sum()
+    assert np.array_equal(got, got.T)
+    cmb.free()
+
+
 def test_self_product_of_integers_in_digits():
     """Integers of up to 24 bits: nothing is lost, to the last bit of sums below 2^53."""
     rng = np.random.default_rng(2)
@@ -250,7 +294,7 @@ def test_self_product_without_digits(values):
         want, s = X.T @ X, np.abs(X).T @ np.abs(X)
     fine = np.isfinite(want)
     assert np.array_equal(np.isfinite(got), fine)
-    assert (np.abs(got - want)[fine] <= TOL * s[fine] + 1e-320).all()
+    assert (np.abs(got[fine] - want[fine]) <= TOL * s[fine] + 1e-320).all()
     cmb.free()
 
 
