@@ -52,20 +52,31 @@ void minmax_of_group(const HostGroup& hg, int nRows, std::vector<double>& colMin
     for (int j = 0; j < gc; j++) add(j, 0.0);
 }
 
-// X: [rows x n] row-major. grid (column tiles of 128, row splits); partial extrema per split.
-__global__ void k_dense_col_minmax(const double* __restrict__ X, int64_t rows, int n, int64_t rowsPerSplit,
-                                   double* __restrict__ pMin, double* __restrict__ pMax) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
+// X: [rows x n] row-major. grid (column tiles of 128, row splits); partial extrema per split. A narrow tile's rows are shared out
+// to as many groups of threads as it leaves room for, four rows of each in flight.
+constexpr int MM_T = 512;
+__global__ void __launch_bounds__(MM_T) k_dense_col_minmax(const double* __restrict__ X, int64_t rows, int n, int64_t rowsPerSplit,
+                                                           double* __restrict__ pMin, double* __restrict__ pMax) {
+  __shared__ double sLo[MM_T], sHi[MM_T];
+  const int c0 = blockIdx.x * 128, w = min(128, n - c0), groups = MM_T / w, g = threadIdx.x / w, c = c0 + threadIdx.x % w;
   const int64_t r0 = blockIdx.y * rowsPerSplit, r1 = min(rows, r0 + rowsPerSplit);
   double lo = INFINITY, hi = -INFINITY;
-  for (int64_t r = r0; r < r1; r++) {
-    const double v = X[r * n + c];
-    lo = fmin(lo, v);
-    hi = fmax(hi, v);
+  if (g < groups) {
+#pragma unroll 4
+    for (int64_t r = r0 + g; r < r1; r += groups) {
+      const double v = X[r * n + c];
+      lo = fmin(lo, v);
+      hi = fmax(hi, v);
+    }
   }
-  pMin[(size_t)blockIdx.y * n + c] = lo;
-  pMax[(size_t)blockIdx.y * n + c] = hi;
+  sLo[threadIdx.x] = lo;
+  sHi[threadIdx.x] = hi;
+  __syncthreads();
+  if (g == 0) {
+    for (int k = 1; k < groups; k++) lo = fmin(lo, sLo[k * w + threadIdx.x]), hi = fmax(hi, sHi[k * w + threadIdx.x]);
+    pMin[(size_t)blockIdx.y * n + c] = lo;
+    pMax[(size_t)blockIdx.y * n + c] = hi;
+  }
 }
 
 // a warp per row
@@ -85,14 +96,14 @@ __global__ void k_dense_row_minmax(const double* __restrict__ X, int64_t rows, i
 static int64_t dense_col_minmax(Matrix* m, const double* X, int64_t rows, int n, std::vector<double>& lo,
                                 std::vector<double>& hi, cudaStream_t s) {
   if (rows <= 0 || n <= 0) return CLA_OK;
-  const int splits = (int)std::max<int64_t>(1, std::min<int64_t>(4 * m->smCount, rows / 64));
+  const int splits = (int)std::max<int64_t>(1, std::min<int64_t>(m->smCount, rows / 64));  // (the host looks at each)
   const int64_t rps = (rows + splits - 1) / splits;
   int64_t rc = ensure_small(m, (size_t)2 * splits * n * sizeof(double) + 256);
   if (rc < 0) return rc;
   double* pMin = (double*)m->small_;
   double* pMax = pMin + (size_t)splits * n;
   dim3 grid((n + 127) / 128, splits);
-  k_dense_col_minmax<<<grid, 128, 0, s>>>(X, rows, n, rps, pMin, pMax);
+  k_dense_col_minmax<<<grid, MM_T, 0, s>>>(X, rows, n, rps, pMin, pMax);
   m->stats.kernel_launches++;
   std::vector<double> h((size_t)2 * splits * n);
   CLA_CUDA(cudaMemcpyAsync(h.data(), pMin, h.size() * sizeof(double), cudaMemcpyDeviceToHost, s));

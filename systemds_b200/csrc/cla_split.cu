@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(128) k_split(const double* __restrict__ X, siz
 // lane stays in its banks), and a range of rows; a lane takes 16 rows of its column.
 // Bound: the latency of the maps' loads, a sector a lane, next to the planes written (7 bytes a cell). The self product of 160,000 x 250 of 1000 values
 // took 421 us with the rows decompressed and split, 232 with this (256 values: 380 and 211).
-constexpr int SM_W = 16;
+constexpr int SM_W = 24;        // (16: 160,000 x 250 of 256 values 211 us instead of 205)
 constexpr int SM_VALS = 1600;  // tuples, at most: 200 KB
 template <bool CHECK>
 __global__ void __launch_bounds__(SM_W * 32, 1) k_split_maps(const DevGroup* __restrict__ groups, const int32_t* __restrict__ colSrc, const double* __restrict__ constV,
