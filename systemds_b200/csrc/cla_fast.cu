@@ -37,7 +37,10 @@ constexpr int SMEM_MAX = 227 * 1024;
 // 615 / 609 / 562 / 658 / 577 us; 16 and 14 leave 128 registers), 16 where fewer (300,001 x 60, 4 units: 16.4 against 17.0 with 12).
 __host__ __device__ constexpr int lmm_warps(int units) { return units > 4 ? 12 : 16; }
 constexpr int LMM_MAXW = 16;
-constexpr int RB_W = 16;              // k_rmm_vec
+// k_rmm_vec: 8 warps, whose 255 registers hold the next step's ids as well (1,250,000 x 1000: 402 us; 16 warps without them 409, 10 / 12 / 16 with
+// them 679 / 474 / 563, they spill; 2M x 112: 72.9, 77.3 with 16). On joint slots 16 warps (1M x 100 of 16 values: 32 us; with the next
+// step's ids 39).
+constexpr int RB_W = 8, RBJ_W = 16;
 constexpr int LMM_MAX_UNITS = 7;      // 16-column table units per CTA (7 x 32 KB at 256 tuples)
 constexpr int LMM_PART = LMM_MAX_UNITS * 16;  // partial sums a CTA writes
 constexpr int LMM_STEP = 64;          // rows per warp step (32 per half-warp)
@@ -950,8 +953,8 @@ __device__ __noinline__ double rmm_step_by_rows(const uint8_t* mp, size_t ustr, 
 // Row sums of one step from its id words, this lane's as sum_row says. JOINT: the terms are the table entries themselves.
 // (Joint slots with a reduction of shuffles alone: 30 of the 150 wavefronts of a step of three units; 40.4 against 38.0 us for 1M x 100 of
 // 16 values, cold.)
-template <int NU, bool JOINT, int UNROLL_ROWS>
-__device__ __forceinline__ double step_sums(const uint4 (&m)[NU], const uint32_t (&tb)[NU], const double (&v)[NU]) {
+template <int NU, bool JOINT, int UNROLL_ROWS, class F>
+__device__ __forceinline__ double step_sums(const uint4 (&m)[NU], const uint32_t (&tb)[NU], const double (&v)[NU], F&& used) {
   double r = 0.0;
 #pragma unroll UNROLL_ROWS
   for (int h = 0; h < 2; h++) {  // rows 0..7 and 8..15 of each half-warp's block
@@ -966,6 +969,7 @@ __device__ __forceinline__ double step_sums(const uint4 (&m)[NU], const uint32_t
         const double x = lds_f64(entry_at(i < 4 ? w0 : w1, i & 3, tb[u]));
         acc[i] = JOINT ? acc[i] + x : fma(x, v[u], acc[i]);
       }
+      if (h == 1) used(u);
     }
     const double s = half_warp_sums(acc);
     if ((threadIdx.x & 1) == h) r = s;
@@ -980,7 +984,7 @@ __device__ __forceinline__ void rmm_fetch(const RmmArgs& A, int unit0, int nu, i
   if (warp < nu && (threadIdx.x & 31) == 0 && n > 0)
     l2_fetch(A.imaps + ((size_t)(unit0 + warp) * A.nRB + (size_t)from * 2) * 256, (uint32_t)n * 512u);
 }
-// Turns of the warps whose ids are on their way to L2: about 100 KB per SM, what the memory's latency takes. (1,250,000 x 1000: 430 us
+// Turns of the warps whose ids are on their way to L2: about 100 KB per SM, what the memory's latency takes. (1,250,000 x 1000, 16 warps: 430 us
 // without, 409 with, 413 and 433 with two and four times as many.)
 __host__ __device__ constexpr int rmm_ahead(int nu) { return 14 / nu; }
 
@@ -1002,12 +1006,19 @@ __device__ __forceinline__ void rmm_rows(const RmmArgs& A, int unit0, int64_t s0
   }
   const uint8_t* mp = A.imaps + (size_t)unit0 * A.nRB * 256 + half * 256 + slot * 16;
   const size_t ustr = (size_t)A.nRB * 256;
-  for (int64_t st = s0 + warp; st < s1; st += RB_W) {
-    // (loading the ids a step ahead costs the registers of a second set, i.e. spills or fewer warps: slower either way)
-    uint4 m[NU];
+  constexpr int W = JOINT ? RBJ_W : RB_W;
+  uint4 m[NU];
+  auto load = [&](int64_t st) {
 #pragma unroll
     for (int u = 0; u < NU; u++) m[u] = __ldg((const uint4*)(mp + u * ustr + st * 512));
-    rmm_fetch(A, unit0, NU, st - warp + rmm_ahead(NU) * RB_W, RB_W, s1);
+  };
+  if (!JOINT && s0 + warp < s1) load(s0 + warp);
+  for (int64_t st = s0 + warp; st < s1; st += W) {
+    if (JOINT) load(st);
+    auto used = [&](int u) {  // a unit's ids of the next step, as soon as this step's are used up
+      if (!JOINT && st + W < s1) m[u] = __ldg((const uint4*)(mp + u * ustr + (st + W) * 512));
+    };
+    rmm_fetch(A, unit0, NU, st - warp + rmm_ahead(NU) * W, W, s1);
     const int64_t row = st * VSTEP + rowOf;
     const bool mine = row < A.nRows;
     uint32_t tailId[JOINT_TAIL];
@@ -1017,7 +1028,7 @@ __device__ __forceinline__ void rmm_rows(const RmmArgs& A, int unit0, int64_t s0
         if (b < A.tail) tailId[b] = __ldg(A.imaps + ((size_t)(unit0 + NU) * A.nRB + (size_t)st * 2 + (rowOf >> 4)) * 256 + b * 16 + (rowOf & 15));
     double o = init;  // what this row holds from the chunks before
     if (!first) o = mine ? A.out[row * A.stride] : 0.0;
-    double r = step_sums<NU, JOINT, 2>(m, tb, v);
+    double r = step_sums<NU, JOINT, 2>(m, tb, v, used);
     if (__any_sync(0xffffffffu, !isfinite(r)))
       r = rmm_step_by_rows(mp + st * 512, ustr, A.units + unit0, A.slotCol + unit0 * 16, JOINT ? nullptr : A.v, A.stride, NU, table0);
     if (JOINT && last)
@@ -1036,12 +1047,11 @@ __device__ __forceinline__ void rmm_rows(const RmmArgs& A, int unit0, int64_t s0
 // Bound: the latency of the first loads. (Group after group with a barrier after each, two units at a time, each term behind the load of its
 // group's record: 1M x 100 of 16 values, inputs changing from call to call, 43.0 us; 34.9 now, with the slots by rows and the ids brought to L2;
 // 41.5 with the ids asked for before the terms.)
-constexpr int RB_T = RB_W * 32;
 template <class F>
 __device__ __forceinline__ void joint_tables(const RmmArgs& A, int unit0, int nu, int tail, double* tbl, double* tailTbl, double* parts, F&& loaded) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, all = nu + (tail > 0), nPairs = (all + 1) / 2;
   for (int p0 = 0; p0 < nPairs; p0 += A.pairs) {
-    const int np = min(A.pairs, nPairs - p0), wp = RB_W / np;  // warps per pair
+    const int np = min(A.pairs, nPairs - p0), wp = RBJ_W / np;  // warps per pair
     const int pair = p0 + warp / wp, r = warp % wp, u = 2 * pair + (lane >> 4), sl = lane & 15, slot = (unit0 + u) * 16 + sl;
     const bool on = warp < wp * np && u < all && (u < nu || sl < tail);
     JointSlot js;
@@ -1117,20 +1127,21 @@ __device__ __forceinline__ void joint_tables(const RmmArgs& A, int unit0, int nu
 }
 
 template <bool JOINT>
-__global__ void __launch_bounds__(RB_T, 1) k_rmm_vec(const __grid_constant__ RmmArgs A) {
+__global__ void __launch_bounds__((JOINT ? RBJ_W : RB_W) * 32, 1) k_rmm_vec(const __grid_constant__ RmmArgs A) {
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ __align__(8) uint64_t mbar;
-  __shared__ double cred[RB_W];
+  constexpr int W = JOINT ? RBJ_W : RB_W;
+  __shared__ double cred[W];
   const int64_t nSteps = ((int64_t)A.nRows + VSTEP - 1) / VSTEP;
   const int64_t s0 = nSteps * blockIdx.x / gridDim.x, s1 = nSteps * (blockIdx.x + 1) / gridDim.x;
   double init = 0.0;
   if (A.constV) {
-    for (int c = threadIdx.x; c < A.nCols; c += RB_T) init = fma(A.constV[c], A.v[c * A.stride], init);
+    for (int c = threadIdx.x; c < A.nCols; c += W * 32) init = fma(A.constV[c], A.v[c * A.stride], init);
     for (int d = 16; d; d >>= 1) init += __shfl_xor_sync(0xffffffffu, init, d);
     if ((threadIdx.x & 31) == 0) cred[threadIdx.x >> 5] = init;
     __syncthreads();
     init = 0.0;
-    for (int w = 0; w < RB_W; w++) init += cred[w];
+    for (int w = 0; w < W; w++) init += cred[w];
   }
   tma_barrier_init(&mbar);
   const int U = A.U;
@@ -1138,7 +1149,7 @@ __global__ void __launch_bounds__(RB_T, 1) k_rmm_vec(const __grid_constant__ Rmm
     const int nu = min(U, A.nU16 - unit0);
     const bool last = unit0 + nu == A.nU16;
     uint32_t tail0 = 0;
-    auto fetch = [&] { rmm_fetch(A, unit0, nu, s0, rmm_ahead(nu) * RB_W, s1); };
+    auto fetch = [&] { rmm_fetch(A, unit0, nu, s0, rmm_ahead(nu) * W, s1); };
     if (!JOINT) fetch();
     __syncthreads();  // everyone is done with the previous chunk's tables
     if (JOINT) {
@@ -1215,7 +1226,7 @@ __device__ __forceinline__ void chain_body(const ChainArgs& C, unsigned char* sm
     const int64_t row = st * VSTEP + rowOf;
     const bool in = row < A.nRows;
     const double wt = C.w && in ? C.w[row] : 1.0;
-    double r = step_sums<NU, false, 1>(m, tb, v);
+    double r = step_sums<NU, false, 1>(m, tb, v, [](int) {});
     if (__any_sync(0xffffffffu, !isfinite(r))) r = rmm_step_by_rows(mp + st * 512, ustr, A.units, A.slotCol, C.v, 1, NU, table0);
     r = (r + init) * wt;
     if (C.u && in) C.u[row] = r;
@@ -1660,8 +1671,8 @@ int64_t fast_rmm_vec(Matrix* m, const double* dV, double* dOut, const double* dW
   const int64_t nSteps = ((int64_t)m->nRows + VSTEP - 1) / VSTEP;
   const int grid = (int)std::min<int64_t>(m->smCount, nSteps);
   prof_begin(m, s);
-  if (joint) k_rmm_vec<true><<<grid, RB_T, smem, s>>>(A);
-  else k_rmm_vec<false><<<grid, RB_T, smem, s>>>(A);
+  if (joint) k_rmm_vec<true><<<grid, RBJ_W * 32, smem, s>>>(A);
+  else k_rmm_vec<false><<<grid, RB_W * 32, smem, s>>>(A);
   prof_end(m, s);
   m->stats.kernel_launches++;
   CLA_CUDA(cudaGetLastError());
