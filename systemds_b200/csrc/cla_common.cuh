@@ -197,7 +197,7 @@ struct DecPlan {  // column-per-lane decompress (cla_generic.cu)
   int warps = 0;  // of a CTA; 0: the tile kernel is the better one
   bool again = false;    // the block has been decompressed before
   void* cols = nullptr;  // records, built on first use
-  size_t smem = 0;
+  size_t tables = 0, smem = 0;  // bytes of tables, and with the cells behind them
 };
 struct ColPlan {
   bool tried = false, ok = false;

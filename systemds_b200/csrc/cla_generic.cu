@@ -520,13 +520,16 @@ k_decomp_block(const DevGroup* __restrict__ groups, const int32_t* __restrict__ 
 
 // Decompress, column per lane: a warp owns 32 neighbouring columns and DC_ROWS rows and walks down the rows, every lane
 // in its own column: 16 ids per load and a table in shared memory (entry k of lane l at k * 32 + l: no bank conflicts) for
-// small dense-map groups, the next listed row and its value for an SDC column, the current run for an RLE column, the dense
-// block itself for an uncompressed one. Each cell is formed in the register it is stored from, and the warps of a CTA
-// write whole stretches of a row at the same time. The tile kernel above builds every cell in shared memory and reads
-// it back. What is left is the latency of the chains item -> value and run -> value.
+// small dense-map groups, the listed rows and their values for an SDC column, the runs for an RLE column, the dense
+// block itself for an uncompressed one. The warps of a CTA write whole stretches of a row at the same time. The tile kernel
+// above builds every cell in shared memory and reads it back. What is left is the latency of the chains item -> value and run
+// -> value, so lists and runs go sixteen rows at a time: a lane puts its next entries into its own sixteen cells of shared memory, as
+// many steps as the fullest column of the warp has entries there, and the sixteen stores then follow without a branch. Row by row,
+// with a test for an entry and its loads in each, a warp took sixteen divergent steps: 250,001 x 500 mixed 312 us, 284 with cells for lists,
+// 287 -> 273 with CTAs of eight warps. Of runs only the starts and ends go to cells, with a bit set for each (291 against 293 us).
 // The records and the items of a block are filled on the device in its first call, without a copy (row lists, which hold the
-// items too, take 350 us). 250,001 x 500 mixed (1 GB), tile kernel against this one: 495 -> 320 us, 3.1
-// TB/s written; first call on a block 534 -> 403 us, host time included.
+// items too, take 350 us). 250,001 x 500 mixed (1 GB), tile kernel against this one: 495 -> 273 us, 3.7
+// TB/s written.
 struct DecCol {
   const double* dict;  // dictionary (or dense block) + position in the group
   const void* a;       // byte / bit map; SDC items; RLE runs
@@ -549,8 +552,10 @@ constexpr int DC_ROWS = 64;            // (256 / 128 / 64 rows on 250,001 x 500:
 constexpr int DC_WARPS = 16;
 constexpr int64_t DC_CELLS = 4 << 20, DC_FIRST = 20 << 20;  // cells of a call; of the block, for its first call
 constexpr size_t DC_TBL = 100 * 1024;  // table bytes of a CTA
-__global__ void __launch_bounds__(DC_WARPS * 32) k_decomp_cols(const DecCol* __restrict__ cols, double* __restrict__ out, size_t ld, int r0, int r1,
-                                                     int nRows, int nCols, int exactSdc) {
+constexpr size_t DC_CELLBUF = 16 * 32 * 8;  // and of a warp with lists or runs to walk, sixteen rows of a column per lane
+constexpr size_t DC_SMEM = 113 * 1024;      // of both, for two CTAs on an SM
+__global__ void __launch_bounds__(DC_WARPS * 32, 2) k_decomp_cols(const DecCol* __restrict__ cols, double* __restrict__ out, size_t ld, int r0, int r1,
+                                                     int nRows, int nCols, int exactSdc, int cellsAt) {
   extern __shared__ double dct[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nW = blockDim.x >> 5;
   const int c = (blockIdx.y * nW + warp) * 32 + lane;
@@ -615,16 +620,20 @@ __global__ void __launch_bounds__(DC_WARPS * 32) k_decomp_cols(const DecCol* __r
     uint32_t it = p < end ? items[p] : 0u, ahead = p + 1 < end ? items[p + 1] : 0u;
     int row = p < end ? base + (int)(it & 1023u) : INT_MAX;
     double val = p < end ? value(it) : 0.0;
-    for (int r = rb; r < re; r++, o += ld) {
-      double v = cst;
-      if (r == row) {
-        v = val;
-        p++;
-        row = p < end ? base + (int)(ahead & 1023u) : INT_MAX;
-        if (p < end) val = value(ahead);
-        ahead = p + 1 < end ? items[p + 1] : 0u;
-      }
-      *o = v;
+    auto advance = [&]() {
+      p++;
+      row = p < end ? base + (int)(ahead & 1023u) : INT_MAX;
+      if (p < end) val = value(ahead);
+      ahead = p + 1 < end ? items[p + 1] : 0u;
+    };
+    double* cells = dct + cellsAt + warp * 512 + lane;
+    for (int r = rb; r < re; r += 16) {
+#pragma unroll
+      for (int i = 0; i < 16; i++) cells[i * 32] = cst;
+      for (; (uint32_t)(row - r) < 16u; advance()) cells[(row - r) * 32] = val;
+#pragma unroll
+      for (int i = 0; i < 16; i++, o += ld)
+        if (r + i < re) *o = cells[i * 32];
     }
   } else if (d.kind == DC_RLE) {
     const RleRun* runs = (const RleRun*)d.a;
@@ -641,9 +650,25 @@ __global__ void __launch_bounds__(DC_WARPS * 32) k_decomp_cols(const DecCol* __r
         start = end = INT_MAX;
     };
     next();
-    for (int r = rb; r < re; r++, o += ld) {
-      while (end <= r) next();
-      *o = r >= start ? val : cst;
+    double* cells = dct + cellsAt + warp * 512 + lane;
+    for (int r = rb; r < re; r += 16) {
+      uint32_t set = 0;
+      auto change = [&](int i, double x) {
+        cells[i * 32] = x;
+        set |= 1u << i;
+      };
+      for (; start - r < 16; next())
+        if (end > r) {
+          change(max(start - r, 0), val);
+          if (end - r > 16) break;
+          if (end - r < 16) change(end - r, cst);
+        }
+      double v = cst;
+#pragma unroll
+      for (int i = 0; i < 16; i++, o += ld) {
+        if (set >> i & 1) v = cells[i * 32];
+        if (r + i < re) *o = v;
+      }
     }
   } else if (d.kind == DC_MAP) {
     for (int r = rb; r < re; r++, o += ld) *o = cst + d.dict[(size_t)map_get(d.mapType, d.a, d.b, r) * d.stride];
@@ -653,12 +678,12 @@ __global__ void __launch_bounds__(DC_WARPS * 32) k_decomp_cols(const DecCol* __r
 }
 
 // The same walk, sixteen rows at a time, into digit planes (cla_split.cu) instead of doubles: tables hold the digits, and a value is split
-// where it changes. halves: of 16 rows, those behind the last row are zeros. 200,000 x 250 mixed: 136 us against 272 for
-// k_decomp_cols and a pass over the doubles; what is left is the latency of the same chains.
+// where it changes. halves: of 16 rows, those behind the last row are zeros. Two CTAs of sixteen warps' worth of registers on an SM
+// hide more of the chains than the 75 registers it would take (t(X) X of 200,000 x 250 mixed 297 -> 290 us, of 50,000 x 400 260 -> 237).
 template <bool CHECK>
-__global__ void __launch_bounds__(DC_WARPS * 32)
+__global__ void __launch_bounds__(DC_WARPS * 32, 2)
 k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, int64_t halves, uint8_t* __restrict__ planes, int r0, int r1,
-             int nRows, int nCols, int exactSdc, unsigned long long* __restrict__ check) {
+             int nRows, int nCols, int exactSdc, int cellsAt, unsigned long long* __restrict__ check) {
   extern __shared__ double dct[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nW = blockDim.x >> 5;
   const int c = (blockIdx.y * nW + warp) * 32 + lane;
@@ -735,17 +760,24 @@ k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, 
     uint32_t it = p < end ? items[p] : 0u, ahead = p + 1 < end ? items[p + 1] : 0u;
     int row = p < end ? at + (int)(it & 1023u) : INT_MAX;
     unsigned long long val = p < end ? value(it >> 10) : 0ull;
-    walk([&](int r) {
-      unsigned long long x = base;
-      if (r == row) {
-        x = val;
-        p++;
-        row = p < end ? at + (int)(ahead & 1023u) : INT_MAX;
-        if (p < end) val = value(ahead >> 10);
-        ahead = p + 1 < end ? items[p + 1] : 0u;
+    auto advance = [&]() {
+      p++;
+      row = p < end ? at + (int)(ahead & 1023u) : INT_MAX;
+      if (p < end) val = value(ahead >> 10);
+      ahead = p + 1 < end ? items[p + 1] : 0u;
+    };
+    unsigned long long* cells = (unsigned long long*)dct + cellsAt + warp * 512 + lane;  // (see k_decomp_cols)
+    for (int g = 0; g < DC_ROWS / 16; g++) {
+      const int r = rb + g * 16;
+      uint32_t set = 0;
+      for (; (uint32_t)(row - r) < 16u; advance()) {
+        cells[(row - r) * 32] = val;
+        set |= 1u << (row - r);
       }
-      return x;
-    });
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = set >> i & 1 ? cells[i * 32] : (r + i < re ? base : 0ull);
+      split_store(o + (size_t)g * SP_HALF, c, v, seen);
+    }
   } else if (d.kind == DC_RLE) {
     const RleRun* runs = (const RleRun*)d.a;
     int64_t ri = ((const int32_t*)d.b)[blk];
@@ -761,10 +793,28 @@ k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, 
         start = end = INT_MAX;
     };
     next();
-    walk([&](int r) {
-      while (end <= r) next();
-      return r >= start ? val : base;
-    });
+    unsigned long long* cells = (unsigned long long*)dct + cellsAt + warp * 512 + lane;
+    for (int g = 0; g < DC_ROWS / 16; g++) {
+      const int r = rb + g * 16;
+      uint32_t set = 0;
+      auto change = [&](int i, unsigned long long x) {
+        cells[i * 32] = x;
+        set |= 1u << i;
+      };
+      for (; start - r < 16; next())
+        if (end > r) {
+          change(max(start - r, 0), val);
+          if (end - r > 16) break;
+          if (end - r < 16) change(end - r, base);
+        }
+      unsigned long long x = base;
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        if (set >> i & 1) x = cells[i * 32];
+        v[i] = r + i < re ? x : 0ull;
+      }
+      split_store(o + (size_t)g * SP_HALF, c, v, seen);
+    }
   } else if (d.kind == DC_MAP) {
     walk([&](int r) { return value(map_get(d.mapType, d.a, d.b, r)); });
   } else
@@ -802,17 +852,34 @@ k_dec_cols(const DevGroup* __restrict__ groups, const int32_t* __restrict__ colS
   if (c < nCols) cols[c] = d;
 }
 
+// Warps of a CTA for n stretches of 32 columns. CTAs of five to eight warps overlap better than wider ones, whose warps all wait for
+// the slowest walk (250,001 x 500, 16 stretches: 273 us in two CTAs of eight, 292 in one; 200,003 x 384: 162 against 178 us),
+// as long as few of them are left without columns: warps that end at once hold their CTA's registers (100,000 x 350, 11 stretches in
+// two CTAs of six: 112 us, in one of eleven 104). A wide CTA counts as 6 % idle.
+static int dec_warps(int n) {
+  int best = n;
+  double cost = n > DC_WARPS ? 1.0 : (n > 8 ? 0.06 : 0.0);
+  for (int w = std::min(n, DC_WARPS); w >= 5; w--) {
+    const int all = (n + w - 1) / w * w;
+    const double c = (double)(all - n) / all + (w > 8 ? 0.06 : 0.0);
+    if (c < cost) best = w, cost = c;
+  }
+  return best;
+}
+
 // Whether k_decomp_cols is the better kernel for the block's columns (m->dec.warps, 0: the tile kernel is) and how many
 // warps a CTA has. Part of the upload, whose pass over the columns has everything at hand: finding it out at the first call
 // took longer than that call saves on small blocks.
 void decomp_shape(Matrix* m, const int32_t* colSrc) {
   int scattered = 0, kinds = 0;
+  bool walks = false;
   std::vector<int> deep((m->nCols + 31) / 32, 0);
   for (int c0 = 0; c0 < m->nCols; c0 += 32) {
     unsigned seen = 0;
     for (int c = c0; c < std::min(m->nCols, c0 + 32); c++) {
       const int gi = colSrc[2 * c], k = gi < 0 ? DC_CONST : dc_kind(m->groups[gi]);
       scattered += k == DC_MAP;
+      walks |= k == DC_SDC || k == DC_RLE;
       seen |= 1u << (k == DC_BITS ? DC_BYTES : k);
       if (k == DC_BYTES || k == DC_BITS) deep[c0 / 32] = std::max(deep[c0 / 32], m->groups[gi].nVals);
     }
@@ -823,16 +890,18 @@ void decomp_shape(Matrix* m, const int32_t* colSrc) {
   // warps: 280 us there, 342 here).
   if (scattered * 16 > m->nCols || kinds * 5 > (int)deep.size() * 7) return;
   // tables: 256 bytes per tuple of the deepest small dictionary of every 32 columns; fewer columns per CTA if they are deep
-  for (int warps = std::min<int>(DC_WARPS, (int)deep.size()); warps >= 1; warps /= 2) {
+  for (int warps = dec_warps((int)deep.size()); warps >= 1; warps /= 2) {
+    const size_t cells = walks ? warps * DC_CELLBUF : 0;
     size_t most = 0;
     for (size_t w = 0; w < deep.size(); w += warps) {
       size_t b = 0;
       for (size_t i = w; i < std::min(deep.size(), w + warps); i++) b += (size_t)deep[i] * 256;
       most = std::max(most, b);
     }
-    if (most <= DC_TBL) {
+    if (most <= DC_TBL && (warps <= 4 || most + cells <= DC_SMEM)) {
       m->dec.warps = warps;
-      m->dec.smem = most;
+      m->dec.tables = most;
+      m->dec.smem = most + cells;
       return;
     }
   }
@@ -891,10 +960,10 @@ int64_t launch_decompress_range(Matrix* m, int r0, int r1, double* dOut, cudaStr
     if (byCols && (rc = ensure_dec(m, s)) < 0) return rc;
     if (byCols && m->dec.cols) {
       static OncePerDevice once;
-      if (const int64_t e = allow_smem(once, m->device, DC_TBL, k_decomp_cols); e < 0) return e;
+      if (const int64_t e = allow_smem(once, m->device, DC_TBL + 4 * DC_CELLBUF, k_decomp_cols); e < 0) return e;
       dim3 grid((r1 - r0 + DC_ROWS - 1) / DC_ROWS, (m->nCols + m->dec.warps * 32 - 1) / (m->dec.warps * 32));
-      k_decomp_cols<<<grid, m->dec.warps * 32, m->dec.smem, s>>>((const DecCol*)m->dec.cols, dOut, ld, r0, r1, m->nRows, m->nCols,
-                                                                m->multiCover ? 0 : 1);
+      k_decomp_cols<<<grid, m->dec.warps * 32, m->dec.smem, s>>>(
+          (const DecCol*)m->dec.cols, dOut, ld, r0, r1, m->nRows, m->nCols, m->multiCover ? 0 : 1, (int)(m->dec.tables / 8));
       m->stats.kernel_launches++;
       CLA_CUDA(cudaGetLastError());
       return CLA_OK;
@@ -932,12 +1001,12 @@ bool split_cols_covers(Matrix* m, cudaStream_t s) {
 }
 int64_t launch_split_cols(Matrix* m, int r0, int r1, const int32_t* expo, int64_t halves, uint8_t* planes, unsigned long long* check, cudaStream_t s) {
   static OncePerDevice once;
-  if (const int64_t e = allow_smem(once, m->device, DC_TBL, k_split_cols<false>, k_split_cols<true>); e < 0) return e;
+  if (const int64_t e = allow_smem(once, m->device, DC_TBL + 4 * DC_CELLBUF, k_split_cols<false>, k_split_cols<true>); e < 0) return e;
   dim3 grid((unsigned)((halves * 16 + DC_ROWS - 1) / DC_ROWS), (m->nCols + m->dec.warps * 32 - 1) / (m->dec.warps * 32));
   const DecCol* cols = (const DecCol*)m->dec.cols;
   const int exact = m->multiCover ? 0 : 1, threads = m->dec.warps * 32;
-  if (check) k_split_cols<true><<<grid, threads, m->dec.smem, s>>>(cols, expo, halves, planes, r0, r1, m->nRows, m->nCols, exact, check);
-  else k_split_cols<false><<<grid, threads, m->dec.smem, s>>>(cols, expo, halves, planes, r0, r1, m->nRows, m->nCols, exact, nullptr);
+  if (check) k_split_cols<true><<<grid, threads, m->dec.smem, s>>>(cols, expo, halves, planes, r0, r1, m->nRows, m->nCols, exact, (int)(m->dec.tables / 8), check);
+  else k_split_cols<false><<<grid, threads, m->dec.smem, s>>>(cols, expo, halves, planes, r0, r1, m->nRows, m->nCols, exact, (int)(m->dec.tables / 8), nullptr);
   m->stats.kernel_launches++;
   CLA_CUDA(cudaGetLastError());
   return CLA_OK;

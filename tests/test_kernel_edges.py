@@ -428,6 +428,41 @@ def test_decompress_by_columns_with_references():
         assert rel_err(np.array(CLALibDecompress.decompress(cmb)), X, scale) <= 1.01 * np.finfo(float).eps
     cmb.free()
 
+def _runs_and_lists(nRows, nCols):
+    """Runs and lists whose entries lie at the edges of sixteen rows: single rows, neighbouring runs, runs over many groups of
+    sixteen, full and empty groups, entries in the last row."""
+    rng = np.random.default_rng(nRows)
+    groups = []
+    for c in range(nCols):
+        if c < nCols // 2:
+            cuts = np.unique(np.concatenate([np.arange(16, nRows, 16) + rng.integers(-1, 2, (nRows - 1) // 16), np.arange(64 * (c % 5), 64 * (c % 5) + 40),
+                                             [0, nRows - 1, nRows]]))
+            cuts = cuts[(cuts == 0) | (cuts >= nRows - 1) | (rng.random(cuts.size) < [1.0, 0.5, 0.05][c % 3])]
+            starts, ends = cuts[:-1], cuts[1:]
+            keep = rng.random(starts.size) < [1.0, 0.7][c % 2]
+            keep[-1] = True
+            starts, lens = starts[keep], (ends - starts)[keep]
+            groups.append(cg.ColGroupRLE.from_runs([c], rng.standard_normal((9, 1)), starts, lens, rng.integers(0, 9, starts.size), nRows))
+        else:
+            p = np.repeat(rng.choice([0.0, 0.06, 0.5, 1.0], nRows // 16 + 1), 16)[:nRows]
+            rows = np.flatnonzero((rng.random(nRows) < p) | np.isin(np.arange(nRows), [0, 15, 16, nRows - 1]))
+            ids, d = MapToFactory.create_from(rng.integers(0, 5, rows.size), 5), rng.standard_normal((5, 1))
+            off = OffsetFactory.createOffset(rows)
+            groups.append(cg.ColGroupSDCZeros([c], nRows, d, off, ids) if c % 2 else cg.ColGroupSDC([c], nRows, d, np.array([0.3]), off, ids))
+    return CompressedMatrixBlock(nRows, nCols, groups)
+
+
+@pytest.mark.parametrize("nRows,nCols", [(33001, 192), (16384, 289), (14001, 350), (9999, 576)])
+def test_runs_and_lists_by_sixteen_rows(oracle, nRows, nCols):
+    """Decompress copies values, so it is exact; t(X) X then reads the same walks as digits. CTAs of 6, 5, 11 and 6 warps."""
+    cmb = _runs_and_lists(nRows, nCols)
+    X = dense_of(cmb)
+    cmb.to_device()
+    for _ in range(2):
+        assert np.array_equal(np.array(CLALibDecompress.decompress(cmb)), X)
+    _self_product_in_digits(oracle, cmb)
+    cmb.free()
+
 
 def test_decompress_first_called_in_a_capture():
     """A captured call leaves no plan that only its replay would fill: direct calls and replays after it are right."""
