@@ -366,9 +366,10 @@ void wide_plan_free(Matrix* m);
 // t(X) X of many columns in 8-bit digits (cla_split.cu): 1 = done, 0 = not covered
 int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s);
 void split_plan_free(Matrix* m);
-// Rows [r0, r1) straight to digit planes, a thread per column (cla_generic.cu); whether the block's columns suit that
+// Rows [r0, r1) straight to digit planes, a thread per column (cla_generic.cu); whether the block's columns suit that. refused: the
+// planes are the guard's, and the word is set where a value has no digits
 bool split_cols_covers(Matrix* m, cudaStream_t s);
-int64_t launch_split_cols(Matrix* m, int r0, int r1, const int32_t* expo, int64_t halves, uint8_t* planes, unsigned long long* check, cudaStream_t s);
+int64_t launch_split_cols(Matrix* m, int r0, int r1, const int32_t* expo, int64_t halves, uint8_t* planes, int32_t* refused, cudaStream_t s);
 // Short blocks (cla_small.cu): one kernel per product, every group type. 1 = done, 0 = not covered
 bool small_block(const Matrix* m);
 int64_t small_rmm(Matrix* m, const double* dV, int vCols, double* dOut, const double* dW, cudaStream_t s, const Finish& fin,

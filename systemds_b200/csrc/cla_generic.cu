@@ -680,10 +680,10 @@ __global__ void __launch_bounds__(DC_WARPS * 32, 2) k_decomp_cols(const DecCol* 
 // The same walk, sixteen rows at a time, into digit planes (cla_split.cu) instead of doubles: tables hold the digits, and a value is split
 // where it changes. halves: of 16 rows, those behind the last row are zeros. Two CTAs of sixteen warps' worth of registers on an SM
 // hide more of the chains than the 75 registers it would take (t(X) X of 200,000 x 250 mixed 297 -> 290 us, of 50,000 x 400 260 -> 237).
-template <bool CHECK>
+template <bool GUARD>
 __global__ void __launch_bounds__(DC_WARPS * 32, 2)
 k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, int64_t halves, uint8_t* __restrict__ planes, int r0, int r1,
-             int nRows, int nCols, int exactSdc, int cellsAt, unsigned long long* __restrict__ check) {
+             int nRows, int nCols, int exactSdc, int cellsAt, int32_t* __restrict__ refused) {
   extern __shared__ double dct[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nW = blockDim.x >> 5;
   const int c = (blockIdx.y * nW + warp) * 32 + lane;
@@ -692,11 +692,11 @@ k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, 
   const DecCol d = cols[c];
   const double cst = d.cst, scale = split_scale(expo[c]);
   uint8_t* o = planes + ((size_t)(c / SP_COLS) * halves + (size_t)blockIdx.x * (DC_ROWS / 16)) * SP_HALF;
-  SplitCheck<CHECK> seen;
-  const unsigned long long base = split_pack(cst, scale, seen);
+  bool bad = false;
+  const unsigned long long base = split_pack<GUARD>(cst, scale, bad);
   auto value = [&](size_t k) {
     const double x = d.dict[k * d.stride];
-    return split_pack(d.kind == DC_SDC && exactSdc ? x : cst + x, scale, seen);
+    return split_pack<GUARD>(d.kind == DC_SDC && exactSdc ? x : cst + x, scale, bad);
   };
   unsigned long long v[16];
   // the groups of 16 rows; cell(i, row) gives the digits
@@ -705,7 +705,7 @@ k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, 
       const int r = rb + g * 16;
 #pragma unroll
       for (int i = 0; i < 16; i++) v[i] = r + i < re ? cell(r + i) : 0ull;
-      split_store(o + (size_t)g * SP_HALF, c, v, seen);
+      split_store<GUARD>(o + (size_t)g * SP_HALF, c, v);
     }
   };
   if (rb >= r1) walk([&](int) { return 0ull; });
@@ -732,7 +732,7 @@ k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, 
       } else
 #pragma unroll
         for (int i = 0; i < 16; i++) v[i] = r + i < re ? T[map_get(d.mapType, d.a, nullptr, r + i) * 32] : 0ull;
-      split_store(o + (size_t)g * SP_HALF, c, v, seen);
+      split_store<GUARD>(o + (size_t)g * SP_HALF, c, v);
     }
   } else if (d.kind == DC_UNC) {
     const double* x = d.dict + (size_t)rb * d.stride;
@@ -742,8 +742,8 @@ k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, 
 #pragma unroll
       for (int i = 0; i < 16; i++) y[i] = rb + g * 16 + i < re ? __ldcs(x + i * xs) : 0.0;
 #pragma unroll
-      for (int i = 0; i < 16; i++) v[i] = rb + g * 16 + i < re ? split_pack(cst + y[i], scale, seen) : 0ull;
-      split_store(o + (size_t)g * SP_HALF, c, v, seen);
+      for (int i = 0; i < 16; i++) v[i] = rb + g * 16 + i < re ? split_pack<GUARD>(cst + y[i], scale, bad) : 0ull;
+      split_store<GUARD>(o + (size_t)g * SP_HALF, c, v);
     }
   } else if (d.kind == DC_SDC) {
     const uint32_t* items = (const uint32_t*)d.a;
@@ -776,7 +776,7 @@ k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, 
       }
 #pragma unroll
       for (int i = 0; i < 16; i++) v[i] = set >> i & 1 ? cells[i * 32] : (r + i < re ? base : 0ull);
-      split_store(o + (size_t)g * SP_HALF, c, v, seen);
+      split_store<GUARD>(o + (size_t)g * SP_HALF, c, v);
     }
   } else if (d.kind == DC_RLE) {
     const RleRun* runs = (const RleRun*)d.a;
@@ -813,13 +813,13 @@ k_split_cols(const DecCol* __restrict__ cols, const int32_t* __restrict__ expo, 
         if (set >> i & 1) x = cells[i * 32];
         v[i] = r + i < re ? x : 0ull;
       }
-      split_store(o + (size_t)g * SP_HALF, c, v, seen);
+      split_store<GUARD>(o + (size_t)g * SP_HALF, c, v);
     }
   } else if (d.kind == DC_MAP) {
     walk([&](int r) { return value(map_get(d.mapType, d.a, d.b, r)); });
   } else
     walk([&](int) { return base; });
-  seen.report(check, c);
+  if (GUARD && bad) *refused = 1;
 }
 
 // The records of k_decomp_cols, filled by CTAs of the shape it will have.
@@ -999,13 +999,13 @@ bool split_cols_covers(Matrix* m, cudaStream_t s) {
   // (fewer warps than four a CTA: deep tables, better read once to doubles)
   return m->colSrcValid && m->dec.warps >= 4 && ensure_dec(m, s) >= 0 && m->dec.cols;
 }
-int64_t launch_split_cols(Matrix* m, int r0, int r1, const int32_t* expo, int64_t halves, uint8_t* planes, unsigned long long* check, cudaStream_t s) {
+int64_t launch_split_cols(Matrix* m, int r0, int r1, const int32_t* expo, int64_t halves, uint8_t* planes, int32_t* refused, cudaStream_t s) {
   static OncePerDevice once;
   if (const int64_t e = allow_smem(once, m->device, DC_TBL + 4 * DC_CELLBUF, k_split_cols<false>, k_split_cols<true>); e < 0) return e;
   dim3 grid((unsigned)((halves * 16 + DC_ROWS - 1) / DC_ROWS), (m->nCols + m->dec.warps * 32 - 1) / (m->dec.warps * 32));
   const DecCol* cols = (const DecCol*)m->dec.cols;
   const int exact = m->multiCover ? 0 : 1, threads = m->dec.warps * 32;
-  if (check) k_split_cols<true><<<grid, threads, m->dec.smem, s>>>(cols, expo, halves, planes, r0, r1, m->nRows, m->nCols, exact, (int)(m->dec.tables / 8), check);
+  if (refused) k_split_cols<true><<<grid, threads, m->dec.smem, s>>>(cols, expo, halves, planes, r0, r1, m->nRows, m->nCols, exact, (int)(m->dec.tables / 8), refused);
   else k_split_cols<false><<<grid, threads, m->dec.smem, s>>>(cols, expo, halves, planes, r0, r1, m->nRows, m->nCols, exact, (int)(m->dec.tables / 8), nullptr);
   m->stats.kernel_launches++;
   CLA_CUDA(cudaGetLastError());

@@ -2,18 +2,24 @@
 //
 // Every cell is split into seven signed base-256 digits relative to its column's largest magnitude (56 bits with the
 // sign: x = 2^e * sum of d_i 2^(-8 i - 7)), the digits are multiplied by tcgen05.mma (kind::i8) with 32-bit sums in tensor memory,
-// and the products of the same weight i + j are added up as 64-bit integers: no rounding, no order. Kept are the products with
-// i + j <= 7, so that what is lost is what lies behind a cell's 55 bits below 2^e, 2^-56 of 2^e at most, and 2^-60 of the product of two columns'
-// powers of two per row: against 64 bits the results are nearer than the FP64 sums are (six kinds of column, 20,011 x 250: 2e-17 of the
-// product of the columns' norms in the mean square and 3e-16 at most, against 4e-16 and 1e-14). The FP64 tensor core, which does the same sums at 37 TFLOP/s with a rounding per four rows,
-// stays for blocks in whose columns a few values stand out so far that this would not hold for the others: a column's
-// largest magnitude may be at most SP_SPREAD times the root mean square of its cells other than zero, and every value must be finite.
+// and the products of the same weight i + j are added up as 64-bit integers: no rounding, no order (the scheme of Ozaki and others for
+// integer matrix units). Kept are the products with i + j <= 7. So a cell is off by 2^-56 of its column's 2^e at most, whatever its own
+// size, and a row's product by 2^-61.6 of the two columns' 2^e. That is little for an entry whose cells come near their columns' largest
+// magnitudes, and all of it for one whose cells are small where the other column is not zero. The guard, which a block's first product
+// runs before it (k_split_guard), therefore bounds the error of every entry of the result against the sum of its terms' magnitudes, and
+// takes the digits only where all of them stay within SP_LOSS = 2^-50 of it, whatever the order of the rows; else, and where a value
+// is not finite, the FP64 tensor core does the sums (k_gemm_tn, 37 TFLOP/s), whose own bound is a rounding of 2^-53 per four rows.
+// Measured, error over the sum of the terms' magnitudes, mean square and largest (FP64 products beside it): 200,000 x 250 of lists, runs,
+// small dictionaries and normal values 1.2e-17 and 1.1e-16 (1.6e-15 and 4.8e-14), 20,011 x 257 of six kinds 2.0e-17 and 2.7e-16 (1.2e-15
+// and 1.6e-14), 8,000 x 250 1.8e-17 and 2.9e-16 (2.8e-16 and 4.1e-15), 4,096 x 500 2.2e-17 and 3.2e-16 (4.0e-16 and 9.1e-15).
 //
 //  * k_split_maps, k_split_cols (cla_generic.cu), k_split: dense maps, other columns by kind, decompressed rows -> planes [block of 128 columns][16 rows][digit][column][16 bytes], which is at once the layout of
 //    the operands in shared memory (K-major, no swizzle: a core matrix is 8 columns x 16 rows), so that a stage is copied as it lies.
 //  * k_syrk_i8: a CTA takes one pair of column blocks, half of the weights and a range of rows: bulk copies in a ring of
 //    four stages, one thread issues the products, four warps take the sums out of tensor memory at the end.
 //  * k_syrk_final: the integers to doubles, both triangles.
+//  * k_split_guard: the verdict over the guard's sums, which the same kernels form: planes of two digits a cell, "not zero" u and the
+//    leading seven bits of the magnitude a, and their four products.
 #include "cla_common.cuh"
 #include "cla_split.cuh"
 #include <algorithm>
@@ -41,13 +47,16 @@ struct SplitSet {
 };
 __host__ __device__ constexpr SplitSet sp_set(int t) {
   return t == 0 ? SplitSet{10, 4, 2, 770} : t == 1 ? SplitSet{24, 7, 1, 1690} : t == 2 ? SplitSet{4, 3, 4, 380} : t == 3 ? SplitSet{5, 5, 3, 470}
-                                                                                                          : SplitSet{10, 7, 2, 755};
+                                                                                                 : t == 4 ? SplitSet{10, 7, 2, 755}
+                                                                                                          : SplitSet{4, 2, 3, 400};
 }
+constexpr int SP_GUARD = 5;  // the guard's set, of any pair of blocks: u u', u a', a u', a a' (its clocks: all items are alike)
 // The sum (0..3) that product i, j of set t goes to, -1: not in the set
 __host__ __device__ constexpr int sp_sum(int t, int i, int j) {
   const int w = i + j;
   if (t == 0) return w <= 3 ? w : -1;
   if (t == 1) return w >= 4 && w <= 7 ? w - 4 : -1;
+  if (t == SP_GUARD) return i < 2 && j < 2 ? 2 * i + j : -1;
   if (i > j) return -1;
   if (t == 2) return w == 0 ? 0 : w == 1 ? 1 : w == 2 ? (i < j ? 2 : 3) : -1;          // E0 D1 D2 E2
   if (t == 3) return w == 3 ? 0 : w == 4 ? (i < j ? 1 : 2) : -1;                       // D3 D4 E4
@@ -62,7 +71,10 @@ __host__ __device__ constexpr bool sp_first(int t, int i, int j) {
     if (sp_sum(t, i, b) == sp_sum(t, i, j)) return false;
   return true;
 }
-constexpr double SP_SPREAD = 16.0;
+// Error of an entry over the sum of its terms' magnitudes, at most. With 2^-50 columns of the usual distributions are taken (bounds
+// found: 200,000 x 250 of lists, runs, small dictionaries and normal values 2^-51.3, six kinds of column on 4,096 to 40,001 rows 2^-51,
+// exponentially distributed values up to 2^e = 16 times their mean), some blocks whose lists have only a few rows in common are not.
+constexpr int SP_LOSS = -50;
 // Below these the FP64 products are as fast (us, FP64 / digits): 200,000 x 130 370 / 376, 200,000 x 150 320 / 353, 100,000 x 180 235 / 229; 2,500 x 250
 // 42 / 42, 5,000 x 250 44 / 44, 9,000 x 250 54 / 48, 12,000 x 180 47 / 47, 5,000 x 800 225 / 108.
 constexpr int SP_MIN_COLS = 176, SP_MIN_ROWS = 4096;
@@ -72,27 +84,26 @@ constexpr size_t SP_CHUNK = 192ull << 20;  // bytes of a chunk of rows (200,000 
 constexpr size_t SP_SMEM = (size_t)SP_RING + 1024;
 
 struct SplitPlan {
-  bool tried = false, ok = false;
-  int32_t* expo = nullptr;                // [nCols] e of every column
-  unsigned long long* check = nullptr;    // what the first call looks at: [0] cells that have no digits, [1 + column] cells other than zero
+  bool tried = false, ok = false;  // ok: the guard has let the block pass
+  int32_t* expo = nullptr;         // [nCols] e of every column
 };
 
 // --------------------------------------------------------------------------------------------------
 // A thread per column and 16 rows; rows behind the last one count as zeros. Bound: the two streams (8 bytes in, 7 out).
-template <bool CHECK>
+template <bool GUARD>
 __global__ void __launch_bounds__(128) k_split(const double* __restrict__ X, size_t ld, int rows, int n, const int32_t* __restrict__ expo,
-                                               int64_t halves, uint8_t* __restrict__ planes, unsigned long long* __restrict__ check) {
+                                               int64_t halves, uint8_t* __restrict__ planes, int32_t* __restrict__ refused) {
   const int c = blockIdx.y * SP_COLS + threadIdx.x;
   if (c >= n) return;
   const double scale = split_scale(expo[c]);
-  SplitCheck<CHECK> seen;
+  bool bad = false;
   for (int64_t h = blockIdx.x; h < halves; h += gridDim.x) {
     unsigned long long v[16];
 #pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = split_pack(h * 16 + i < rows ? __ldcs(X + (size_t)(h * 16 + i) * ld + c) : 0.0, scale, seen);
-    split_store(planes + ((size_t)blockIdx.y * halves + h) * SP_HALF, c, v, seen);
+    for (int i = 0; i < 16; i++) v[i] = split_pack<GUARD>(h * 16 + i < rows ? __ldcs(X + (size_t)(h * 16 + i) * ld + c) : 0.0, scale, bad);
+    split_store<GUARD>(planes + ((size_t)blockIdx.y * halves + h) * SP_HALF, c, v);
   }
-  seen.report(check, c);
+  if (GUARD && bad) *refused = 1;
 }
 
 // Dense maps straight to planes: a CTA owns 16 columns, their tables of digits in shared memory (entry k of slot s at k * 16 + s, so that a
@@ -101,23 +112,23 @@ __global__ void __launch_bounds__(128) k_split(const double* __restrict__ X, siz
 // took 421 us with the rows decompressed and split, 232 with this (256 values: 380 and 211).
 constexpr int SM_W = 24;        // (16: 160,000 x 250 of 256 values 211 us instead of 205)
 constexpr int SM_VALS = 1600;  // tuples, at most: 200 KB
-template <bool CHECK>
+template <bool GUARD>
 __global__ void __launch_bounds__(SM_W * 32, 1) k_split_maps(const DevGroup* __restrict__ groups, const int32_t* __restrict__ colSrc, const double* __restrict__ constV,
                                                              const int32_t* __restrict__ expo, int n, int r0, int r1, int64_t halves,
-                                                             uint8_t* __restrict__ planes, unsigned long long* __restrict__ check) {
+                                                             uint8_t* __restrict__ planes, int32_t* __restrict__ refused) {
   extern __shared__ unsigned long long smt[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.y * 16 + (lane & 15), up = lane >> 4;
   const bool on = c < n;
   const DevGroup& g = groups[colSrc[2 * (on ? c : 0)]];
   const int nv = g.nVals, mt = g.mapType;
   unsigned long long* T = smt + (lane & 15);
-  SplitCheck<CHECK> seen;
+  bool bad = false;
   if (on) {
     const double* dict = g.dict + colSrc[2 * c + 1];
     const double cst = constV ? constV[c] : 0.0, scale = split_scale(expo[c]);
     const int gc = g.gCols;
 #pragma unroll 4
-    for (int k = warp * 2 + up; k < nv; k += SM_W * 2) T[k * 16] = split_pack(cst + dict[(size_t)k * gc], scale, seen);
+    for (int k = warp * 2 + up; k < nv; k += SM_W * 2) T[k * 16] = split_pack<GUARD>(cst + dict[(size_t)k * gc], scale, bad);
   }
   __syncthreads();
   uint8_t* o = planes + (size_t)(c / SP_COLS) * halves * SP_HALF;
@@ -150,9 +161,9 @@ __global__ void __launch_bounds__(SM_W * 32, 1) k_split_maps(const DevGroup* __r
 #pragma unroll
       for (int i = 0; i < 16; i++) v[i] = r + i < r1 ? T[map_get(mt, map, nullptr, r + i) * 16] : 0ull;
     }
-    split_store(o + (size_t)h * SP_HALF, c, v, seen);
+    split_store<GUARD>(o + (size_t)h * SP_HALF, c, v);
   }
-  if (on) seen.report(check, c);
+  if (GUARD && bad) *refused = 1;
 }
 
 // --------------------------------------------------------------------------------------------------
@@ -214,6 +225,8 @@ __device__ __forceinline__ void sp_commit(uint32_t bar) {
 // launch: 150 us, tensor pipe 71 % active; 485 us for the FP64 products. On the way (one launch, some with fewer products): 338 with
 // stages of 32 rows, whose waits cost sets of few products more than their products; 328 with the CTAs of an item in row ranges of
 // their own, which read the planes from memory three times.
+// GUARD: an item per pair, the guard's set.
+template <bool GUARD>
 __global__ void __launch_bounds__(SP_T, 1) k_syrk_i8(const __grid_constant__ SyrkArgs A) {
   extern __shared__ __align__(1024) unsigned char spsm[];
   __shared__ __align__(8) uint64_t full[SP_STAGES], empty[SP_STAGES], sumFull, sumEmpty;
@@ -226,12 +239,12 @@ __global__ void __launch_bounds__(SP_T, 1) k_syrk_i8(const __grid_constant__ Syr
     else hi = mid;
   }
   int I = 0, J = 0, pair = 0, set = 0;
-  for (int it = 0; it + (I == J ? 3 : 2) <= item; pair++) {
-    it += I == J ? 3 : 2;
+  for (int it = 0; it + (GUARD ? 1 : I == J ? 3 : 2) <= item; pair++) {
+    it += GUARD ? 1 : I == J ? 3 : 2;
     set = it;
     if (++J == A.nBlocks) J = ++I;
   }
-  set = item - set + (I == J ? 2 : 0);
+  set = GUARD ? SP_GUARD : item - set + (I == J ? 2 : 0);
   const int N = J == A.nBlocks - 1 ? A.lastN : SP_COLS;
   const int part = blockIdx.x - A.cta0[item], parts = A.cta0[item + 1] - A.cta0[item];
   const int digits = sp_set(set).digits, nSums = set == 3 ? 3 : 4;
@@ -308,7 +321,8 @@ __global__ void __launch_bounds__(SP_T, 1) k_syrk_i8(const __grid_constant__ Syr
       if (sp_elect()) {
         for (int r = 0; r < R; r++, a += half >> 3, b += half >> 3)
 #define SP_CASE(T, SUM) case T * 4 + SUM: sp_products<T, SUM>(sum, a, b, idesc, at == 0 && r == 0); break;
-        switch (set * 4 + warp - 5) {
+        if (GUARD) switch (set * 4 + warp - 5) { SP_CASE(5, 0) SP_CASE(5, 1) SP_CASE(5, 2) SP_CASE(5, 3) }
+        else switch (set * 4 + warp - 5) {
           SP_CASE(0, 0) SP_CASE(0, 1) SP_CASE(0, 2) SP_CASE(0, 3) SP_CASE(1, 0) SP_CASE(1, 1) SP_CASE(1, 2) SP_CASE(1, 3)
           SP_CASE(2, 0) SP_CASE(2, 1) SP_CASE(2, 2) SP_CASE(2, 3) SP_CASE(3, 0) SP_CASE(3, 1) SP_CASE(3, 2)
           SP_CASE(4, 0) SP_CASE(4, 1) SP_CASE(4, 2) SP_CASE(4, 3)
@@ -348,7 +362,10 @@ __global__ void __launch_bounds__(SP_T, 1) k_syrk_i8(const __grid_constant__ Syr
           const long long x = v[0][i], y = v[1][i], z = v[2][i], u = v[3][i];
           unsigned long long* h = (unsigned long long*)(hi + (size_t)(c + i) * SP_COLS);
           unsigned long long* l = (unsigned long long*)(lo + (size_t)(c + i) * SP_COLS);
-          if (set < 2) atomicAdd(set == 0 ? h : l, (unsigned long long)(((x * 256 + y) * 256 + z) * 256 + u));
+          if (GUARD) {  // a a', and what the error is bounded by (k_split_guard)
+            atomicAdd(h, (unsigned long long)u);
+            atomicAdd(l, (unsigned long long)(y + z + 5 * x));
+          } else if (set < 2) atomicAdd(set == 0 ? h : l, (unsigned long long)(((x * 256 + y) * 256 + z) * 256 + u));
           else if (set == 2) atomicAdd(h, (unsigned long long)(((x * 256 + 2 * y) * 256 + 2 * z + u) * 256));
           else if (set == 3) {
             atomicAdd(h, (unsigned long long)(2 * x));
@@ -394,6 +411,21 @@ __global__ void __launch_bounds__(SP_COLS) k_syrk_final(const long long* __restr
   out[(size_t)c * n + r] = x;
 }
 
+// Whether an entry of the result could be off by more than 2^SP_LOSS of the sum of its terms' magnitudes. In units of 2^(e + e') a row's
+// product is off by 2^-56 |y| + 2^-56 |x| (the cells' last digits, where the other cell is not zero) and 2^-61.6 (the products left out) at
+// most. With |x| < (a + 1) 2^-7 that is 2^-63 (u a' + a u' + 5 u u'); the magnitudes add up to 2^-14 a a' at least. grid: (pairs of blocks, rows
+// of a block)
+__global__ void __launch_bounds__(SP_COLS) k_split_guard(const long long* __restrict__ sums, int nBlocks, int n, const int32_t* __restrict__ err,
+                                                         int32_t* __restrict__ refused) {
+  int I = 0, first = 0;
+  while (first + nBlocks - I <= (int)blockIdx.x) first += nBlocks - I++;
+  const int J = I + blockIdx.x - first, r = I * SP_COLS + threadIdx.x, c = J * SP_COLS + blockIdx.y;
+  if (r >= n || c >= n) return;
+  const long long* p = sums + (size_t)blockIdx.x * 2 * SP_COLS * SP_COLS + blockIdx.y * SP_COLS + threadIdx.x;
+  const long long magnitudes = p[0], lost = p[SP_COLS * SP_COLS];
+  if ((lost << (-49 - SP_LOSS)) > magnitudes || *err) *refused = 1;
+}
+
 // --------------------------------------------------------------------------------------------------
 static int blocks_of(const Matrix* m) { return (m->nCols + SP_COLS - 1) / SP_COLS; }
 // Rows of a chunk, in even parts of about SP_CHUNK bytes, a multiple of SKIP_ROWS; dense: it is decompressed first
@@ -401,58 +433,6 @@ static int64_t split_chunk(const Matrix* m, bool dense) {
   const double row = (dense ? ((m->nCols + 1) & ~1) * 8.0 : 0.0) + (double)blocks_of(m) * SP_COLS * SP_DIG;
   const int64_t parts = std::max<int64_t>(1, (int64_t)(m->nRows * row / SP_CHUNK + 0.5));
   return std::max<int64_t>(SKIP_ROWS, ((m->nRows + parts - 1) / parts + SKIP_ROWS - 1) / SKIP_ROWS * SKIP_ROWS);
-}
-
-// The columns' exponents, from the extrema (a bound on the cells is enough)
-static int64_t ensure_split(Matrix* m, cudaStream_t s) {
-  SplitPlan& P = *m->split;
-  if (P.tried) return CLA_OK;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return CLA_OK;  // (a call that is being captured runs nothing yet: no plan from it)
-  }
-  const int n = m->nCols;
-  std::vector<double> lo, hi;
-  int64_t rc;
-  if ((rc = col_minmax(m, lo, hi, s)) < 0) return rc;
-  P.tried = true;
-  std::vector<int32_t> e(n, 0);
-  for (int c = 0; c < n; c++) {
-    const double M = std::max(std::fabs(lo[c]), std::fabs(hi[c]));
-    if (M == 0.0) continue;
-    if (!(M < 1e140 && M > 1e-140)) return CLA_OK;  // the scale or the sums would leave the range of doubles
-    int x;
-    if (std::frexp(M, &x) > 0.99) x++;  // the leading digit stays within a byte when the others carry
-    e[c] = x;
-  }
-  const size_t expoBytes = ((size_t)n * 4 + 255) & ~(size_t)255, checkBytes = ((size_t)n + 1) * 8;
-  void* p = nullptr;
-  if (plan_alloc(m, &p, expoBytes + checkBytes) < 0) return CLA_OK;
-  CLA_CUDA(cudaMemcpyAsync(p, e.data(), (size_t)n * 4, cudaMemcpyHostToDevice, s));
-  CLA_CUDA(cudaMemsetAsync((char*)p + expoBytes, 0, checkBytes, s));
-  CLA_CUDA(cudaStreamSynchronize(s));
-  P.expo = (int32_t*)p;
-  P.check = (unsigned long long*)((char*)p + expoBytes);
-  P.ok = true;
-  return CLA_OK;
-}
-// After the first product: whether its columns are such that digits were the better way. The sums of squares are on its diagonal.
-static int64_t check_split(Matrix* m, const double* dOut, cudaStream_t s) {
-  SplitPlan& P = *m->split;
-  const int n = m->nCols;
-  std::vector<unsigned long long> seen(n + 1);
-  std::vector<double> squares(n);
-  std::vector<int32_t> e(n);
-  CLA_CUDA(cudaMemcpyAsync(seen.data(), P.check, ((size_t)n + 1) * 8, cudaMemcpyDeviceToHost, s));
-  CLA_CUDA(cudaMemcpyAsync(e.data(), P.expo, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
-  CLA_CUDA(cudaMemcpy2DAsync(squares.data(), 8, dOut, ((size_t)n + 1) * 8, 8, n, cudaMemcpyDeviceToHost, s));
-  CLA_CUDA(cudaStreamSynchronize(s));
-  P.check = nullptr;
-  if (seen[0]) P.ok = false;
-  for (int c = 0; c < n; c++)
-    if (std::ldexp(1.0, e[c]) > 2.0 * SP_SPREAD * std::sqrt(squares[c] / std::max<double>(1.0, (double)seen[c + 1])) && squares[c] > 0.0) P.ok = false;
-  return CLA_OK;
 }
 
 // Every column in a dense map of bits, bytes or 16 bits whose table fits: k_split_maps; the longest table, 0: no
@@ -473,35 +453,44 @@ static bool split_covers(const Matrix* m, bool maps) {
   return m->nCols >= (maps ? SP_MAPS_COLS : SP_MIN_COLS) && m->nCols <= SP_BLOCKS * SP_COLS && m->nRows >= SP_MIN_ROWS && cells >= SP_MIN_CELLS && m->colSrcValid && !m->overlapping;
 }
 
-int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
-  const int vals = split_maps_vals(m);
-  if (!split_covers(m, vals > 0)) return 0;
-  if (!m->split) m->split = new SplitPlan();
-  if (m->split->tried && !m->split->ok) return 0;
+// How the rows get to planes, and what of scratch2 that and the sums take
+struct SplitShape {
+  int vals;          // k_split_maps, its longest table; 0: not
+  bool cols, dense;  // k_split_cols; k_split of decompressed rows
+  int64_t chunk;
+  size_t ld, denseBytes, planeBytes, sumBytes;
+};
+static SplitShape split_shape(Matrix* m, int vals, cudaStream_t s) {
+  SplitShape S{};
+  const int nb = blocks_of(m), pairs = nb * (nb + 1) / 2;
+  S.vals = vals;
+  S.cols = !vals && split_cols_covers(m, s);
+  S.dense = !vals && !S.cols;
+  S.chunk = split_chunk(m, S.dense);
+  S.ld = (size_t)((m->nCols + 1) & ~1);
+  S.denseBytes = S.dense ? (size_t)S.chunk * S.ld * 8 : 0;
+  S.planeBytes = (size_t)nb * (S.chunk / 16 + SP_PAD) * SP_HALF;
+  S.sumBytes = (size_t)pairs * 2 * SP_COLS * SP_COLS * 8;
+  return S;
+}
+// All rows through planes and products. refused: the guard's planes, sums and verdict (set, or left), dOut null; else the product.
+static int64_t split_run(Matrix* m, const SplitShape& S, const int32_t* expo, double* dOut, int32_t* refused, cudaStream_t s) {
   const int n = m->nCols, nb = blocks_of(m), pairs = nb * (nb + 1) / 2;
-  const size_t ld = (size_t)((n + 1) & ~1);
+  const bool guard = refused != nullptr;
   int64_t rc;
-  if ((rc = ensure_split(m, s)) < 0) return rc;
-  if (!m->split->ok) return 0;
-  const int32_t* expo = m->split->expo;
-  unsigned long long* check = m->split->check;
-  const bool cols = !vals && split_cols_covers(m, s), dense = !vals && !cols;
-  const int64_t chunk = split_chunk(m, dense);
-  const size_t denseBytes = dense ? (size_t)chunk * ld * 8 : 0, planeBytes = (size_t)nb * (chunk / 16 + SP_PAD) * SP_HALF;
-  const size_t sumBytes = (size_t)pairs * 2 * SP_COLS * SP_COLS * 8;
-  if ((rc = ensure_scratch2(m, denseBytes + planeBytes + sumBytes)) < 0) return rc;
+  if ((rc = ensure_scratch2(m, S.denseBytes + S.planeBytes + S.sumBytes)) < 0) return rc;
   double* X = (double*)m->scratch2;
-  uint8_t* planes = (uint8_t*)m->scratch2 + denseBytes;
-  long long* sums = (long long*)(planes + planeBytes);
+  uint8_t* planes = (uint8_t*)m->scratch2 + S.denseBytes;
+  long long* sums = (long long*)(planes + S.planeBytes);
   static OncePerDevice once;
-  if (const int64_t e = allow_smem(once, m->device, SP_SMEM, k_syrk_i8); e < 0) return e;
+  if (const int64_t e = allow_smem(once, m->device, SP_SMEM, k_syrk_i8<false>, k_syrk_i8<true>); e < 0) return e;
   static OncePerDevice onceMaps;
   if (const int64_t e = allow_smem(onceMaps, m->device, (size_t)SM_VALS * 128, k_split_maps<false>, k_split_maps<true>); e < 0) return e;
   SyrkArgs A{};
   A.planes = planes;
   A.nBlocks = nb;
   A.lastN = (n - (nb - 1) * SP_COLS + 15) / 16 * 16;
-  A.nItems = pairs * 2 + nb;
+  A.nItems = guard ? pairs : pairs * 2 + nb;
   A.sums = sums;
   A.err = m->dErr;
   // CTAs by the time of an item
@@ -511,9 +500,9 @@ int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
       int it = 0;
       for (int I = 0; I < nb; I++)
         for (int J = I; J < nb; J++)
-          for (int t = I == J ? 2 : 0; t < (I == J ? 5 : 2); t++, it++) {
-            const SplitSet S = sp_set(t);
-            f(it, J == nb - 1 ? std::max(S.clocks * A.lastN / (double)SP_COLS, S.clocks * 0.6) : S.clocks);
+          for (int t = guard ? SP_GUARD : I == J ? 2 : 0; t < (guard ? SP_GUARD + 1 : I == J ? 5 : 2); t++, it++) {
+            const SplitSet set = sp_set(t);
+            f(it, J == nb - 1 ? std::max(set.clocks * A.lastN / (double)SP_COLS, set.clocks * 0.6) : set.clocks);
           }
     };
     each([&](int, double c) { total += c; });
@@ -527,41 +516,97 @@ int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
   }
   int64_t summed = 0;  // rows in the 64-bit sums
   bool add = false;
-  for (int64_t r0 = 0; r0 < m->nRows; r0 += chunk) {
-    const int r1 = (int)std::min<int64_t>(m->nRows, r0 + chunk), rows = r1 - (int)r0;
-    if (summed == 0) CLA_CUDA(cudaMemsetAsync(sums, 0, sumBytes, s));
+  for (int64_t r0 = 0; r0 < m->nRows; r0 += S.chunk) {
+    const int r1 = (int)std::min<int64_t>(m->nRows, r0 + S.chunk), rows = r1 - (int)r0;
+    if (summed == 0) CLA_CUDA(cudaMemsetAsync(sums, 0, S.sumBytes, s));
     A.halves = ((int64_t)rows + 16 * SP_PAD - 1) / (16 * SP_PAD) * SP_PAD;
-    if (vals) {
+    if (S.vals) {
       const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(A.halves / (SM_W * 2) + 1, m->smCount / ((n + 15) / 16))), (n + 15) / 16);
       const double* constV = m->hasConst ? m->dConstV : nullptr;
-      const size_t smem = (size_t)vals * 128;
-      if (check) k_split_maps<true><<<grid, SM_W * 32, smem, s>>>(m->dGroups, m->dColSrc, constV, expo, n, (int)r0, r1, A.halves, planes, check);
+      const size_t smem = (size_t)S.vals * 128;
+      if (guard) k_split_maps<true><<<grid, SM_W * 32, smem, s>>>(m->dGroups, m->dColSrc, constV, expo, n, (int)r0, r1, A.halves, planes, refused);
       else k_split_maps<false><<<grid, SM_W * 32, smem, s>>>(m->dGroups, m->dColSrc, constV, expo, n, (int)r0, r1, A.halves, planes, nullptr);
       m->stats.kernel_launches++;
-    } else if (cols) {
-      if ((rc = launch_split_cols(m, (int)r0, r1, expo, A.halves, planes, check, s)) < 0) return rc;
+    } else if (S.cols) {
+      if ((rc = launch_split_cols(m, (int)r0, r1, expo, A.halves, planes, refused, s)) < 0) return rc;
     } else {
-      if ((rc = launch_decompress_range(m, (int)r0, r1, X, s, ld)) < 0) return rc;
+      if ((rc = launch_decompress_range(m, (int)r0, r1, X, s, S.ld)) < 0) return rc;
       const dim3 grid((unsigned)std::min<int64_t>(A.halves, 16 * m->smCount / nb), nb);
-      if (check) k_split<true><<<grid, SP_COLS, 0, s>>>(X, ld, rows, n, expo, A.halves, planes, check);
-      else k_split<false><<<grid, SP_COLS, 0, s>>>(X, ld, rows, n, expo, A.halves, planes, nullptr);
+      if (guard) k_split<true><<<grid, SP_COLS, 0, s>>>(X, S.ld, rows, n, expo, A.halves, planes, refused);
+      else k_split<false><<<grid, SP_COLS, 0, s>>>(X, S.ld, rows, n, expo, A.halves, planes, nullptr);
       m->stats.kernel_launches++;
     }
-    if (r0 == 0) prof_begin(m, s);
-    k_syrk_i8<<<A.cta0[A.nItems], SP_T, SP_SMEM, s>>>(A);
-    if (r0 == 0) prof_end(m, s);
+    if (r0 == 0 && !guard) prof_begin(m, s);
+    if (guard) k_syrk_i8<true><<<A.cta0[A.nItems], SP_T, SP_SMEM, s>>>(A);
+    else k_syrk_i8<false><<<A.cta0[A.nItems], SP_T, SP_SMEM, s>>>(A);
+    if (r0 == 0 && !guard) prof_end(m, s);
     m->stats.kernel_launches++;
     summed += rows;
-    if (r1 == m->nRows || summed + chunk > SP_TOTAL) {
+    if (guard) continue;  // (its sums are safe for any number of rows: below 2^14 a row)
+    if (r1 == m->nRows || summed + S.chunk > SP_TOTAL) {
       k_syrk_final<<<dim3(pairs, SP_COLS), SP_COLS, 0, s>>>(sums, nb, n, expo, dOut, add ? 1 : 0, m->dErr);
       m->stats.kernel_launches++;
       summed = 0;
       add = true;
     }
   }
+  if (guard) {
+    k_split_guard<<<dim3(pairs, SP_COLS), SP_COLS, 0, s>>>(sums, nb, n, m->dErr, refused);
+    m->stats.kernel_launches++;
+  }
   CLA_CUDA(cudaGetLastError());
-  if (check && (rc = check_split(m, dOut, s)) < 0) return rc;
-  return m->split->ok ? 1 : 0;
+  return CLA_OK;
+}
+
+// The columns' exponents, from the extrema (a bound on the cells is enough), and the guard's verdict, which the host waits for: once per
+// block, in its first product (200,000 x 250 mixed: that product 658 us, the others 300).
+static int64_t ensure_split(Matrix* m, const SplitShape& S, cudaStream_t s) {
+  SplitPlan& P = *m->split;
+  const int n = m->nCols;
+  std::vector<double> lo, hi;
+  int64_t rc;
+  if ((rc = col_minmax(m, lo, hi, s)) < 0) return rc;
+  P.tried = true;
+  std::vector<int32_t> e(n + 1, 0);
+  for (int c = 0; c < n; c++) {
+    const double M = std::max(std::fabs(lo[c]), std::fabs(hi[c]));
+    if (M == 0.0) continue;
+    if (!(M < 1e140 && M > 1e-140)) return CLA_OK;  // the scale or the sums would leave the range of doubles
+    int x;
+    if (std::frexp(M, &x) > 0.99) x++;  // the leading digit stays within a byte when the others carry
+    e[c] = x;
+  }
+  void* p = nullptr;
+  if (plan_alloc(m, &p, ((size_t)n + 1) * 4) < 0) return CLA_OK;
+  P.expo = (int32_t*)p;
+  int32_t* refused = P.expo + n;
+  CLA_CUDA(cudaMemcpyAsync(p, e.data(), ((size_t)n + 1) * 4, cudaMemcpyHostToDevice, s));
+  if ((rc = split_run(m, S, P.expo, nullptr, refused, s)) < 0) return rc;
+  int32_t no = 1;
+  CLA_CUDA(cudaMemcpyAsync(&no, refused, 4, cudaMemcpyDeviceToHost, s));
+  CLA_CUDA(cudaStreamSynchronize(s));
+  P.ok = no == 0;
+  return CLA_OK;
+}
+
+int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
+  const int vals = split_maps_vals(m);
+  if (!split_covers(m, vals > 0)) return 0;
+  if (!m->split) m->split = new SplitPlan();
+  if (m->split->tried && !m->split->ok) return 0;
+  if (!m->split->tried) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return 0;  // (a call that is being captured runs nothing yet: no plan from it)
+    }
+  }
+  const SplitShape S = split_shape(m, vals, s);
+  int64_t rc;
+  if (!m->split->tried && (rc = ensure_split(m, S, s)) < 0) return rc;
+  if (!m->split->ok) return 0;
+  if ((rc = split_run(m, S, m->split->expo, dOut, nullptr, s)) < 0) return rc;
+  return 1;
 }
 
 void split_plan_free(Matrix* m) {

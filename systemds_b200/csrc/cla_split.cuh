@@ -10,29 +10,16 @@ constexpr int SP_PLANE = SP_COLS * 16;    // bytes of a digit of 16 rows
 constexpr int SP_HALF = SP_DIG * SP_PLANE;  // all digits of 16 rows
 
 __device__ __forceinline__ double split_scale(int e) { return scalbn(1.0, 55 - e); }
-// What a thread saw of its column: cells other than zero, and values that have no digits (not finite, or beyond the bound). ON: the
-// first product looks, the others do not (its registers cost a third of the warps: 200,000 x 250 as a whole 367 us instead of 317).
-template <bool ON>
-struct SplitCheck {
-  unsigned count = 0;
-  bool bad = false;
-  __device__ __forceinline__ void value(double y) {
-    if (ON) bad |= !(fabs(y) <= 0x1p55);
-  }
-  __device__ __forceinline__ void cell(unsigned long long v) {
-    if (ON) count += v != 0;
-  }
-  __device__ __forceinline__ void report(unsigned long long* check, int c) const {
-    if (!ON) return;
-    if (count) atomicAdd(check + 1 + c, (unsigned long long)count);
-    if (bad) atomicAdd(check, 1ull);
-  }
-};
-// The digits of x, |x| <= 0.99 * 2^e, the last one in byte 0
-template <bool ON>
-__device__ __forceinline__ unsigned long long split_pack(double x, double scale, SplitCheck<ON>& seen) {
+// The digits of x, |x| <= 0.99 * 2^e, the last one in byte 0. GUARD: what the guard multiplies in their place, digit 0 whether the
+// cell differs from zero (the cell itself, not its digits) and digit 1 its magnitude's leading seven bits, rounded down; bad: a value
+// that has no digits (not finite, or beyond the bound).
+template <bool GUARD>
+__device__ __forceinline__ unsigned long long split_pack(double x, double scale, bool& bad) {
   const double y = x * scale;
-  seen.value(y);
+  if (GUARD) {
+    bad |= !(fabs(y) <= 0x1p55);
+    return (unsigned long long)(x != 0.0) << 48 | (unsigned long long)min((int)(fabs(y) * 0x1p-48), 126) << 40;
+  }
   // + 128 in every byte makes the bytes the digits + 128
   return ((unsigned long long)__double2ll_rn(y) + 0x80808080808080ull) ^ 0x80808080808080ull;
 }
@@ -46,10 +33,8 @@ __device__ __forceinline__ void transpose4(uint32_t a, uint32_t b, uint32_t c, u
   o[3] = __byte_perm(AB, CD, 0x7632);
 }
 // 16 rows of column c to their place: p points at the 16 rows' first plane of the column's block
-template <bool ON>
-__device__ __forceinline__ void split_store(uint8_t* p, int c, const unsigned long long (&v)[16], SplitCheck<ON>& seen) {
-#pragma unroll
-  for (int i = 0; i < 16; i++) seen.cell(v[i]);
+template <bool GUARD>
+__device__ __forceinline__ void split_store(uint8_t* p, int c, const unsigned long long (&v)[16]) {
   uint32_t w[SP_DIG][4];
 #pragma unroll
   for (int q = 0; q < 4; q++) {
@@ -63,7 +48,7 @@ __device__ __forceinline__ void split_store(uint8_t* p, int c, const unsigned lo
   }
   p += (c % SP_COLS) * 16;
 #pragma unroll
-  for (int d = 0; d < SP_DIG; d++) *(uint4*)(p + (size_t)d * SP_PLANE) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
+  for (int d = 0; d < (GUARD ? 2 : SP_DIG); d++) *(uint4*)(p + (size_t)d * SP_PLANE) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
 }
 
 }  // namespace cla

@@ -298,6 +298,77 @@ def test_self_product_without_digits(values):
     cmb.free()
 
 
+def _two_scales(nRows, small, kinds, by_kind):
+    """200 columns, of every kind some a that are about 1 in the first half of the rows and about `small` in the others, and some b
+    that are about 1 in the others alone; small = 0: a is 1 in one row and 1e-18 in the others, b not zero in the others."""
+    rng = np.random.default_rng(nRows)
+    first = np.arange(nRows) < (nRows // 2 if small else 1)
+    groups = []
+    for c in range(200):
+        k = kinds[c * len(kinds) // 200 if by_kind else c % len(kinds)]
+        d = np.concatenate([rng.uniform(0.9, 1.1, 3), rng.uniform(0.9, 1.1, 3) * (small or 1e-18)] if c % 20 < 10 else [[0.0], rng.uniform(0.9, 1.1, 5)])
+        if c % 20 >= 10:
+            ids = np.where(first, 0, rng.integers(1, 6, nRows))
+        elif small:
+            ids = np.where(first, rng.integers(0, 3, nRows), rng.integers(3, 6, nRows))
+        else:
+            d[:3] = 1.0
+            ids = np.where(first, 0, rng.integers(3, 6, nRows))
+        d = d.reshape(-1, 1)
+        if k == "ddc":
+            groups.append(cg.ColGroupDDC([c], d, MapToFactory.create_from(ids, 6)))
+        elif k == "unc":
+            groups.append(cg.ColGroupUncompressed([c], d[ids]))
+        elif k == "sdc":  # the value of the first rows is the default
+            rows = np.flatnonzero(~first)
+            off, m = OffsetFactory.createOffset(rows), MapToFactory.create_from(ids[rows], 6)
+            groups.append(cg.ColGroupSDCZeros([c], nRows, d, off, m) if d[0, 0] == 0.0 else
+                          cg.ColGroupSDC([c], nRows, d, d[0].copy(), off, m))
+        else:
+            ids = np.where(first, ids[0], np.repeat(ids[::-1][:nRows // 50 + 1], 50)[:nRows][::-1])
+            starts = np.flatnonzero(np.diff(ids, prepend=-1))
+            groups.append(cg.ColGroupRLE.from_runs([c], d, starts, np.diff(starts, append=nRows), ids[starts], nRows))
+    return CompressedMatrixBlock(nRows, 200, groups)
+
+
+@pytest.mark.parametrize("small", [1e-6, 1e-9, 1e-12, 1e-18, 0])
+@pytest.mark.parametrize("kinds,by_kind", [(["ddc"], True), (["ddc", "sdc", "rle", "unc"], True), (["ddc", "sdc", "rle", "unc"], False)])
+def test_self_product_of_columns_of_two_scales(oracle, small, kinds, by_kind):
+    """Entries whose terms are far below their columns' largest magnitudes, as precise as the others: dense maps, columns by kind,
+    decompressed rows. The bound is the sum's, a rounding of 2^-53 per four rows, and the oracle's."""
+    nRows = 20011
+    cmb = _two_scales(nRows, small, kinds, by_kind)
+    X = dense_of(cmb)
+    cmb.to_device()
+    want, s = oracle.dense_tsmm_ld(X), np.abs(X).T @ np.abs(X)
+    for _ in range(2):
+        got = np.array(CLALibTSMM.leftMultByTransposeSelf(cmb))
+        assert (np.abs(got - want) <= nRows * 2.0**-55 * s).all(), (np.abs(got - want) / (s + 1e-300)).max()
+    cmb.free()
+
+
+@pytest.mark.parametrize("i,j", [(0, 1), (7, 131), (127, 128), (130, 259), (258, 259)])
+@pytest.mark.parametrize("row", [0, 16383, 50002])
+def test_self_product_with_one_small_term(i, j, row):
+    """One entry of the result has a single term, far below what its columns hold elsewhere: the product itself, wherever the
+    pair of columns and the row lie."""
+    rng = np.random.default_rng(i + j)
+    n, groups = 50003, []
+    for c in range(260):
+        ids, d = rng.integers(1, 9, n), rng.uniform(0.5, 1.0, 9)
+        ids[row], d[0] = 0, 0.7
+        if c == i:
+            d[0] = 3.3e-17
+        elif c == j:
+            d[1:] = 0.0
+        groups.append(cg.ColGroupDDC([c], d.reshape(-1, 1), MapToFactory.create_from(ids, 9)))
+    cmb = CompressedMatrixBlock(n, 260, groups).to_device()
+    for _ in range(2):
+        got = np.array(CLALibTSMM.leftMultByTransposeSelf(cmb))
+        assert got[i, j] == got[j, i] == 3.3e-17 * 0.7
+    cmb.free()
+
+
 @pytest.mark.parametrize("nRows", [1, 255, 257, 1040, 5001])
 @pytest.mark.parametrize("nCols", [31, 33, 530])
 def test_decompress_columns(nRows, nCols):
