@@ -565,8 +565,8 @@ static int64_t ensure_split(Matrix* m, const SplitShape& S, cudaStream_t s) {
   const int n = m->nCols;
   std::vector<double> lo, hi;
   int64_t rc;
+  P.tried = true;  // (whatever comes: not again)
   if ((rc = col_minmax(m, lo, hi, s)) < 0) return rc;
-  P.tried = true;
   std::vector<int32_t> e(n + 1, 0);
   for (int c = 0; c < n; c++) {
     const double M = std::max(std::fabs(lo[c]), std::fabs(hi[c]));
@@ -602,11 +602,13 @@ int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
     }
   }
   const SplitShape S = split_shape(m, vals, s);
-  int64_t rc;
-  if (!m->split->tried && (rc = ensure_split(m, S, s)) < 0) return rc;
-  if (!m->split->ok) return 0;
-  if ((rc = split_run(m, S, m->split->expo, dOut, nullptr, s)) < 0) return rc;
-  return 1;
+  int64_t rc = m->split->tried ? CLA_OK : ensure_split(m, S, s);
+  if (rc == CLA_OK && !m->split->ok) return 0;
+  if (rc == CLA_OK) rc = split_run(m, S, m->split->expo, dOut, nullptr, s);
+  if (rc != CLA_ERR_NOMEM) return rc < 0 ? rc : 1;
+  // Planes and sums can take more scratch than the FP64 products' chunk (100,000 x 130: 216 MiB against 124): no room, no digits from now on
+  m->split->ok = false;
+  return 0;
 }
 
 void split_plan_free(Matrix* m) {

@@ -5,6 +5,8 @@ import pytest
 
 from systemds_b200 import CompressedMatrixBlock, datagen, native
 from systemds_b200.cmb import CLALibDecompress, CLALibTSMM
+from systemds_b200 import colgroup as cg
+from systemds_b200.mapping import MapToFactory
 from systemds_b200.native import check
 from tests.test_kernel_edges import _by_kind, _check, _ddc
 from tests.util import TOL, dense_of, rel_err
@@ -67,6 +69,50 @@ def test_products_without_room_for_plans(kind):
         _use(cmb)
         # (what no kernel does without, a record per column, is not counted)
         assert _plan_bytes(cmb) - before <= limit + 64 * cmb.clen
+        cmb.free()
+
+
+@pytest.mark.gpu
+def test_self_product_where_device_memory_is_short():
+    """t(X) X in digits can need more scratch than the FP64 products: where only theirs fits, the call works all the same, and
+    so does the next one."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(3)
+    n, cols = 100_000, 130
+    groups = [cg.ColGroupDDC([c], rng.standard_normal((9, 1)), MapToFactory.create_from(rng.integers(0, 9, n), 9)) for c in range(cols)]
+    block = CompressedMatrixBlock(n, cols, groups)
+    X = torch.from_numpy(dense_of(block)).cuda()
+    want, s = (X.T @ X).cpu().numpy(), (X.abs().T @ X.abs()).cpu().numpy()
+    del X
+    out = torch.empty((cols, cols), dtype=torch.float64, device="cuda")
+    lib = native.lib()
+
+    def product(cmb):
+        out.zero_()
+        rc = lib.cla_tsmm_dev(cmb.handle(), out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        return rc, rel_err(out.cpu().numpy(), want, s + 1e-300)
+
+    for limit in (-1, 0):  # enough memory; both sides' kernels are loaded
+        cmb = block.to_device()
+        check(lib.cla_set_plan_limit(cmb.handle(), limit))
+        rc, err = product(cmb)
+        assert rc >= 0 and err < TOL
+        cmb.free()
+    # scratch of the FP64 products: n x 130 doubles and a quarter, 124 MiB; of the digits: planes of 256 columns x 7 bytes, 216
+    for left in (130, 150, 180, 260):
+        torch.cuda.empty_cache()
+        cmb = block.to_device()
+        rest = torch.cuda.mem_get_info()[0] - (left << 20)
+        hold = [torch.empty(1 << 28, dtype=torch.uint8, device="cuda") for _ in range(rest >> 28)]
+        for step in (26, 22):
+            while torch.cuda.mem_get_info()[0] - (left << 20) > 1 << step:
+                hold.append(torch.empty(1 << step, dtype=torch.uint8, device="cuda"))
+        for _ in range(2):
+            rc, err = product(cmb)
+            assert rc >= 0, (left, native.last_error())
+            assert err < TOL, left
+        del hold
         cmb.free()
 
 
