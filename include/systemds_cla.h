@@ -29,7 +29,10 @@
  * cla_stats_get. The right products (X %*% v, X %*% V), the specialised left vector product and
  * the chain built from them form every output cell's sum in a fixed order and are reproducible
  * bit for bit; the general left product, the self-product and the constant-column terms combine
- * partial sums with floating-point atomics and are reproducible to rounding only.
+ * partial sums with floating-point atomics and are reproducible to rounding only. The self-product of
+ * many columns has exact integer sums instead where a look at the block allows it: the same bits from
+ * every call, but for a call that is being captured before the block's first direct one (it cannot
+ * look, and its replay adds in double precision) and calls that find no memory for it.
  */
 #ifndef SYSTEMDS_CLA_H
 #define SYSTEMDS_CLA_H
@@ -210,7 +213,8 @@ int64_t cla_unary_agg(cla_handle h, int32_t op, double* out);
 /* ---- products, device buffers --------------------------------------------------------------
  * Same semantics; every pointer is a device address on the handle's device, `stream` is a
  * cudaStream_t (NULL = the legacy default stream). The call enqueues work and returns CLA_OK
- * without synchronising; no non-zero count is produced. Used for row-sharded multi-GPU runs,
+ * without synchronising, once the block has what it needs: a block's first call of a kind may build a
+ * plan or, for the self-product, look at the block, and waits for that. No non-zero count is produced. Used for row-sharded multi-GPU runs,
  * where the caller all-reduces the partial results of cla_lmm_dev / cla_tsmm_dev / cla_mmchain_dev. */
 int64_t cla_rmm_dev(cla_handle h, const double* dV, int32_t vRows, int32_t vCols, double* dOut, void* stream);
 int64_t cla_lmm_dev(cla_handle h, const double* dYt, int32_t yRows, double* dOut, void* stream);

@@ -557,6 +557,44 @@ def test_decompress_first_called_in_a_capture():
     cmb.free()
 
 
+@pytest.mark.parametrize("by_kind", [True, False])
+def test_self_product_first_called_in_a_capture(by_kind):
+    """A captured first call cannot look at the block: its replay does the sums in double precision, direct calls before and
+    after a replay in digits where the block suits them. A call captured later replays what direct calls give."""
+    import torch
+    from systemds_b200 import native
+    cmb = _six_kinds(20011, 257, by_kind)
+    X = torch.from_numpy(dense_of(cmb)).cuda()
+    want, bound = X.T @ X, 2 * 20011 * 2.0**-55 * (X.abs().T @ X.abs())
+    cmb.to_device()
+    lib, h = native.lib(), cmb.handle()
+    out, stream = torch.empty_like(want), torch.cuda.Stream()
+    first, later = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+
+    def call():
+        native.check(lib.cla_tsmm_dev(h, out.data_ptr(), stream.cuda_stream))
+
+    def result(f):
+        with torch.cuda.stream(stream):
+            out.zero_()
+            f()
+            stream.synchronize()
+            assert ((out - want).abs() <= bound).all()
+            return out.clone()
+
+    torch.cuda.synchronize()
+    with torch.cuda.graph(first, stream=stream, capture_error_mode="relaxed"):  # (the call grows its scratch)
+        call()
+    result(first.replay)
+    direct = result(call)
+    result(first.replay)
+    with torch.cuda.graph(later, stream=stream):
+        call()
+    assert torch.equal(result(later.replay), direct) and torch.equal(result(call), direct)
+    del first, later
+    cmb.free()
+
+
 @pytest.mark.parametrize("nCols", [128, 129, 300, 448, 449])
 @pytest.mark.parametrize("nRows", [77, 1000])
 def test_short_blocks_with_v_in_the_launch(nRows, nCols):
