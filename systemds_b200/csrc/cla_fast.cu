@@ -224,7 +224,7 @@ constexpr int VSTEP = 32;  // rows of a warp step: one 16-row block per half-war
 // dependent launch), and stores the result: nothing to clear beforehand. (Left to the last CTA of a chunk, without a second
 // launch: 18.2 instead of 14.3 us for the chain on 50,000 x 100, 17.6 instead of 14.2 for t(y) X on 250,000 x 40 -- one
 // CTA reads 148 partial rows too slowly.)
-// Measured (10M x 200, 256 values): 577 us, 3.6 TB/s; 634 with y loaded row by row, 685 for the one-row-step form before that, with
+// Measured (10M x 200, 256 values): 562 us, 3.7 TB/s, 577 with 16 warps; 634 with y loaded row by row, 685 for the one-row-step form before that, with
 // three instructions per address, a clear and a separately launched sum. 625,000 x 1000: 208 -> 187.
 // 100,000 x 500: 36.9 -> 30.5 us, 5000 x 500: 15.4 -> 10.4.
 // --------------------------------------------------------------------------------------------------

@@ -16,7 +16,7 @@
 //  * k_split_maps, k_split_cols (cla_generic.cu), k_split: dense maps, other columns by kind, decompressed rows -> planes [block of 128 columns][16 rows][digit][column][16 bytes], which is at once the layout of
 //    the operands in shared memory (K-major, no swizzle: a core matrix is 8 columns x 16 rows), so that a stage is copied as it lies.
 //  * k_syrk_i8: a CTA takes one pair of column blocks, half of the weights and a range of rows: bulk copies in a ring of
-//    four stages, one thread issues the products, four warps take the sums out of tensor memory at the end.
+//    four stages, a warp per sum issues its products, four warps take the sums out of tensor memory every 16,384 rows.
 //  * k_syrk_final: the integers to doubles, both triangles.
 //  * k_split_guard: the verdict over the guard's sums, which the same kernels form: planes of two digits a cell, "not zero" u and the
 //    leading seven bits of the magnitude a, and their four products.
