@@ -198,6 +198,11 @@ def _six_kinds(nRows, nCols, by_kind):
     return CompressedMatrixBlock(nRows, nCols, groups)
 
 
+def _entries_in_digits(got, want, X, oracles):
+    """Every entry for itself: 2^-50 of the sum of its terms' magnitudes is what a block may lose that is taken in digits."""
+    assert (np.abs(got - want) <= 2.0**-50 * (np.abs(X).T @ np.abs(X)) + oracles + 2.0**-52 * np.abs(want)).all()
+
+
 @pytest.mark.parametrize("nRows,nCols", [(11364, 176), (8193, 255), (20011, 257), (40001, 384), (4096, 500)])
 @pytest.mark.parametrize("by_kind", [True, False])
 def test_self_product_in_digits(oracle, nRows, nCols, by_kind):
@@ -216,6 +221,7 @@ def test_self_product_in_digits(oracle, nRows, nCols, by_kind):
     assert (np.abs(got - want) <= lost + oracles + 2.0**-52 * np.abs(want)).all()
     norms = np.sqrt(np.outer(np.diag(want), np.diag(want)))
     assert (np.abs(got - want) / norms).max() < 1e-15  # (the FP64 products: 4e-15 to 2e-14)
+    _entries_in_digits(got, want, X, oracles)
     assert np.array_equal(got, got.T)
     assert np.array_equal(got, np.array(CLALibTSMM.leftMultByTransposeSelf(cmb)))
     cmb.free()
@@ -227,6 +233,7 @@ def _self_product_in_digits(oracle, cmb):
     want = oracle.dense_tsmm_ld(X)
     norms = np.sqrt(np.outer(np.diag(want), np.diag(want)))
     assert (np.abs(got - want) / norms).max() < 1e-15
+    _entries_in_digits(got, want, X, X.shape[0] * 2.0**-64 * (np.abs(X).T @ np.abs(X)))
     assert np.array_equal(got, got.T)
     assert np.array_equal(got, np.array(CLALibTSMM.leftMultByTransposeSelf(cmb)))
 
@@ -344,6 +351,40 @@ def test_self_product_of_columns_of_two_scales(oracle, small, kinds, by_kind):
     for _ in range(2):
         got = np.array(CLALibTSMM.leftMultByTransposeSelf(cmb))
         assert (np.abs(got - want) <= nRows * 2.0**-55 * s).all(), (np.abs(got - want) / (s + 1e-300)).max()
+    cmb.free()
+
+
+@pytest.mark.parametrize("unused", [1e7, 1e18, 1e100])
+@pytest.mark.parametrize("kind", ["ddc", "sdc", "default", "rle"])
+def test_self_product_with_unused_tuples(oracle, kind, unused):
+    """A tuple that no row has lies far above the cells (bounds of the columns come from the dictionaries): a dense map and a column
+    of `kind` have one, in a block of dense maps for `ddc`."""
+    rng = np.random.default_rng(12)
+    n, groups = 12003, []
+    for c in range(200):
+        d = rng.uniform(0.5, 1.0, (6, 1)) * (1.0 if c % 2 else -1.0)
+        if c in (3, 140):
+            d[5] = unused
+        ids = rng.integers(0, 5, n)
+        rows = np.flatnonzero(rng.random(n) < 0.4)
+        if kind == "ddc" or c < 100:
+            groups.append(cg.ColGroupDDC([c], d, MapToFactory.create_from(ids, 6)))
+        elif kind == "rle":
+            starts = np.flatnonzero(np.diff(ids, prepend=-1))
+            groups.append(cg.ColGroupRLE.from_runs([c], d, starts, np.diff(starts, append=n), ids[starts], n))
+        elif kind == "sdc":
+            groups.append(cg.ColGroupSDCZeros([c], n, d, OffsetFactory.createOffset(rows), MapToFactory.create_from(ids[rows], 6)))
+        else:  # where every row is listed, the default tuple is the unused one
+            every = np.arange(n) if c == 140 else rows
+            groups.append(cg.ColGroupSDC([c], n, d[:5], d[5].copy(), OffsetFactory.createOffset(every), MapToFactory.create_from(ids[every], 5)))
+    cmb = CompressedMatrixBlock(n, 200, groups)
+    X = dense_of(cmb)
+    assert np.abs(X).max() <= 1.0
+    cmb.to_device()
+    want, s = oracle.dense_tsmm_ld(X), np.abs(X).T @ np.abs(X)
+    for _ in range(2):
+        got = np.array(CLALibTSMM.leftMultByTransposeSelf(cmb))
+        assert (np.abs(got - want) <= n * 2.0**-55 * s).all(), (np.abs(got - want) / (s + 1e-300)).max()
     cmb.free()
 
 
