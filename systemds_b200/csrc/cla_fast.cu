@@ -75,7 +75,9 @@ struct JointTerm {
   };
 };
 constexpr int JOINT_UNITS = 6;  // units per chunk, at most
-constexpr int JOINT_TAIL = 4;   // so many slots behind the last whole unit go by rows instead of taking a unit
+// So many slots behind the last whole unit go by rows instead of taking a unit. 1M rows of 16 values, us, by rows / as a unit: 98 columns (a tail of one) 37.5 / 38.9, 100 (two)
+// 38.3 / 38.9, 36 (two) 26.6 / 28.7, 102 (three) 38.9 / 38.9, 104 (four) 38.9 / 38.9, 108 (six) 39.2 / 38.9, 112 (eight) 40.5 / 38.9.
+constexpr int JOINT_TAIL = 4;
 struct FastPlan {
   bool ok = false;
   bool partial = false;      // only some groups are covered; the general kernels add the rest
@@ -1180,7 +1182,8 @@ __global__ void __launch_bounds__((JOINT ? RBJ_W : RB_W) * 32, 1) k_rmm_vec(cons
 // row sums are formed as in k_rmm_vec, scaled, put in shared memory, and multiplied into the column sums as in
 // k_lmm_vec with the id words still in registers (row loops not unrolled: the compiler would hoist a step's worth of
 // lookups and spill). The maps are read once instead of twice, the tables are staged once,
-// and u = X v never leaves the SM (it is stored only if the caller gave a buffer for it).
+// and u = X v never leaves the SM (it is stored only if the caller gave a buffer for it). With a step's row sums by eight products and a
+// shuffle per eight rows instead of ten products: 2M x 100 142.7 -> 141.4 us, 2M x 40 98.3 -> 93.9, 300,000 x 100 30.7 -> 30.3, 50,000 x 100 14.3 as before.
 // --------------------------------------------------------------------------------------------------
 constexpr int CH_W = 11;         // what fits next to seven units of 256 tuples
 constexpr int CH_T = CH_W * 32;
