@@ -92,7 +92,8 @@ static int64_t grow(Matrix* m, void** p, size_t* cur, size_t bytes) {
   }
   *p = nullptr;
   *cur = 0;
-  size_t want = bytes + bytes / 4 + 256;
+  // room for the next larger call; memory costs 8 us a MiB to get (t(X) X: most of a block's first call)
+  size_t want = bytes + std::min<size_t>(bytes / 4, 16 << 20) + 256;
   cudaError_t e = dev_malloc(m, p, want);
   if (e != cudaSuccess) return fail(CLA_ERR_NOMEM, std::string("cudaMalloc scratch: ") + cudaGetErrorString(e));
   *cur = want;

@@ -99,7 +99,7 @@ def test_self_product_where_device_memory_is_short():
         rc, err = product(cmb)
         assert rc >= 0 and err < TOL
         cmb.free()
-    # scratch of the FP64 products: n x 130 doubles and a quarter, 124 MiB; of the digits: planes of 256 columns x 7 bytes, 216
+    # scratch of the FP64 products: n x 130 doubles and 16 MiB, 115 MiB; of the digits: planes of 256 columns x 7 bytes, 188
     for left in (130, 150, 180, 260):
         torch.cuda.empty_cache()
         cmb = block.to_device()
