@@ -853,17 +853,14 @@ k_dec_cols(const DevGroup* __restrict__ groups, const int32_t* __restrict__ colS
 }
 
 // Warps of a CTA for n stretches of 32 columns. CTAs of five to eight warps overlap better than wider ones, whose warps all wait for
-// the slowest walk (250,001 x 500, 16 stretches: 273 us in two CTAs of eight, 292 in one; 200,003 x 384: 162 against 178 us),
-// as long as few of them are left without columns: warps that end at once hold their CTA's registers (100,000 x 350, 11 stretches in
-// two CTAs of six: 112 us, in one of eleven 104). A wide CTA counts as 6 % idle.
+// the slowest walk; of those the width that leaves the fewest warps without columns, which hold their CTA's registers. Decompress mixed, us, this
+// width and one CTA of n (or 16): 300,001 x 352 233 (6) and 252, 250,001 x 384 197 (6) and 223, 100,003 x 416 102 (7) and 108, x 480 99 (5) and 120, x 544 117 (6)
+// and 142, 40,001 x 400 47 (7) and 49, 250,001 x 500 273 (8) and 292; 100,003 x 288 74 (5) and 74, 30,001 x 352 34 and 34. t(X) X mixed,
+// 60,000 rows: x 288 155 and 156, x 352 169 and 178, x 400 277 and 281, x 480 271 and 295.
 static int dec_warps(int n) {
-  int best = n;
-  double cost = n > DC_WARPS ? 1.0 : (n > 8 ? 0.06 : 0.0);
-  for (int w = std::min(n, DC_WARPS); w >= 5; w--) {
-    const int all = (n + w - 1) / w * w;
-    const double c = (double)(all - n) / all + (w > 8 ? 0.06 : 0.0);
-    if (c < cost) best = w, cost = c;
-  }
+  int best = std::min(n, 8);
+  for (int w = best; w >= 5; w--)
+    if ((n + w - 1) / w * w < (n + best - 1) / best * best) best = w;  // (warps of a row of CTAs)
   return best;
 }
 
