@@ -75,12 +75,13 @@ __host__ __device__ constexpr bool sp_first(int t, int i, int j) {
 // found: 200,000 x 250 of lists, runs, small dictionaries and normal values 2^-51.3, six kinds of column on 4,096 to 40,001 rows 2^-51,
 // exponentially distributed values up to 2^e = 16 times their mean), some blocks whose lists have only a few rows in common are not.
 constexpr int SP_LOSS = -50;
-// Below these the FP64 products are as fast (us, FP64 / digits): 200,000 x 130 370 / 376, 200,000 x 150 320 / 353, 100,000 x 180 235 / 229; 2,500 x 250
+// Below these the FP64 products are as fast or nearly (us, FP64 / digits; mixed columns, whose kinds per 32 columns decide how they are decompressed): 200,000 x 130
+// 367 / 369, x 140 366 / 379, x 150 375 / 399, x 160 311 / 247, x 170 466 / 430, x 176 455 / 438, 100,000 x 180 234 / 230, 60,000 x 150 132 / 128; 2,500 x 250
 // 42 / 42, 5,000 x 250 44 / 44, 9,000 x 250 54 / 48, 12,000 x 180 47 / 47, 5,000 x 800 225 / 108.
 constexpr int SP_MIN_COLS = 176, SP_MIN_ROWS = 4096;
 constexpr int64_t SP_MIN_CELLS = 2000000;
 constexpr int SP_MAPS_COLS = 129;  // where k_split_maps takes the block (200,000 x 130 bytes 319 / 222, 1000 values 359 / 260; 16,000 x 130 47 / 38)
-constexpr size_t SP_CHUNK = 192ull << 20;  // bytes of a chunk of rows (200,000 x 250: 303 us in one chunk of 358 MB, 317 in two)
+constexpr size_t SP_CHUNK = 192ull << 20;  // bytes of a chunk of rows (200,000 x 250: 280 us in one chunk of 358 MB, 293 in two, 345 in four; 100 MB more cost a first call a millisecond)
 constexpr size_t SP_SMEM = (size_t)SP_RING + 1024;
 
 struct SplitPlan {
@@ -606,7 +607,7 @@ int64_t split_tsmm(Matrix* m, double* dOut, cudaStream_t s) {
   if (rc == CLA_OK && !m->split->ok) return 0;
   if (rc == CLA_OK) rc = split_run(m, S, m->split->expo, dOut, nullptr, s);
   if (rc != CLA_ERR_NOMEM) return rc < 0 ? rc : 1;
-  // Planes and sums can take more scratch than the FP64 products' chunk (100,000 x 130: 216 MiB against 124): no room, no digits from now on
+  // Planes and sums can take more scratch than the FP64 products' chunk (100,000 x 130: 188 MiB against 115): no room, no digits from now on
   m->split->ok = false;
   return 0;
 }
