@@ -126,12 +126,12 @@ int64_t col_minmax(Matrix* m, std::vector<double>& lo, std::vector<double>& hi, 
   if (!m->overlapping && !m->multiCover) {
     lo = m->colMin;
     hi = m->colMax;
-    for (auto& g : m->groups)
-      if (g.type == GT_UNC) {
+    for (size_t k = 0; k < m->hg.size(); k++)
+      if (const int gi = m->regToDev[k]; gi >= 0 && m->groups[gi].type == GT_UNC) {
+        const DevGroup& g = m->groups[gi];
+        const auto& cols = m->hg[k].cols;
         std::vector<double> glo(g.gCols, INFINITY), ghi(g.gCols, -INFINITY);
         if ((rc = dense_col_minmax(m, g.dense, m->nRows, g.gCols, glo, ghi, s)) < 0) return rc;
-        std::vector<int32_t> cols(g.gCols);
-        CLA_CUDA(cudaMemcpy(cols.data(), g.cols, sizeof(int32_t) * g.gCols, cudaMemcpyDeviceToHost));
         for (int j = 0; j < g.gCols; j++) {
           lo[cols[j]] = std::fmin(lo[cols[j]], glo[j]);
           hi[cols[j]] = std::fmax(hi[cols[j]], ghi[j]);
