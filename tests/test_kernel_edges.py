@@ -422,6 +422,18 @@ def test_decompress_columns(nRows, nCols):
     cmb.free()
 
 
+@pytest.mark.parametrize("stretches", [5, 8, 9, 11, 13, 17])
+def test_decompress_columns_in_rows_of_ctas(stretches):
+    """A kind per 32 columns, the last 32 cut short: one CTA along a row, several that come out even, and with warps left over."""
+    nRows, nCols = (4 << 20) // (stretches * 32 - 5) + 16, stretches * 32 - 5
+    cmb = datagen.random_cmb(stretches, nRows, [("ddc", "sdcz", "rle", "unc")[c // 32 % 4] for c in range(nCols)])
+    X = dense_of(cmb)
+    cmb.to_device()
+    for _ in range(3):  # by columns from the second call on
+        assert np.array_equal(np.array(CLALibDecompress.decompress(cmb)), X)
+    cmb.free()
+
+
 @pytest.mark.parametrize("nRows", [4096, 4127, 4161])
 @pytest.mark.parametrize("kinds", ["bytes", "chars", "mixed", "sparse", "cocoded"])
 def test_wide_right_operand(nRows, kinds):
